@@ -166,6 +166,7 @@ struct gs_ctx {
     /* per read */
     uint64_t *slot_cnt, *slot_off; size_t cap_slot_cnt, cap_slot_off;
     uint32_t *item_cnt, *item_off; size_t cap_item_cnt, cap_item_off;
+    uint32_t *item_read; size_t cap_item_read;
     uint32_t *rd_nf, *rd_nr; size_t cap_nf, cap_nr;
     uint64_t *rd_nseeds, *rd_npos; size_t cap_rns, cap_rnp;
     uint64_t *seed_off, *pos_off; size_t cap_so, cap_po;
@@ -292,6 +293,7 @@ extern "C" void gs_ctx_free(gs_ctx *c)
     if (c->st) cudaStreamSynchronize(c->st);
     cudaFree(c->d_seqs); cudaFree(c->d_offsets); cudaFree(c->d_lengths);
     cudaFree(c->slot_cnt); cudaFree(c->slot_off); cudaFree(c->item_cnt); cudaFree(c->item_off);
+    cudaFree(c->item_read);
     cudaFree(c->rd_nf); cudaFree(c->rd_nr); cudaFree(c->rd_nseeds); cudaFree(c->rd_npos);
     cudaFree(c->seed_off); cudaFree(c->pos_off);
     cudaFree(c->slots); cudaFree(c->hist); cudaFree(c->seeds); cudaFree(c->seed_pos);
@@ -530,6 +532,11 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.recmask = c->recmask;
     GS_CUDA(cudaMemsetAsync(c->recmask, 0, ((n_slots + 31) / 32 + 1) * sizeof(uint32_t), st));
     B.item_cap = n_items;
+    if (p->kernel == GS_KERNEL_BATCHED) {
+        RC(grow(c->item_read, c->cap_item_read, (size_t)n_items + 1, c->st));
+        B.item_read = c->item_read;
+        B.item_read_cap = c->cap_item_read;
+    }
     if (p->kernel == GS_KERNEL_PLAIN) {
         RC(grow(c->hist, c->cap_hist, c->h_small[2] + 1, c->st));
         B.hist = c->hist;
@@ -750,6 +757,8 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.recmask = c->recmask;
     GS_CUDA(cudaMemsetAsync(c->recmask, 0, ((c->cap_slots + 31) / 32 + 1) * sizeof(uint32_t), st));
     B.item_cap = c->g_items;
+    B.item_read = c->item_read;
+    B.item_read_cap = c->cap_item_read;
     /* the walker buffer as the sizing pass left it; walkers beyond it are
      * left to the leftover pass */
     if (c->last_walker_cap && c->walkers) {

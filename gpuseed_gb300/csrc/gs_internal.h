@@ -18,7 +18,8 @@
 #define GS_PCHUNK 30          /* read positions owned by one paired work item */
 #define GS_HANDOFF_LANES 2    /* default hand-over threshold of the batched search */
 #define GS_HANDOFF_STEPS 4
-#define GS_QUEUE_CHUNK 4      /* default work items per queue grab */
+#define GS_QUEUE_CHUNK 4      /* lockstep: default work items per queue grab */
+#define GS_QUEUE_CHUNK_MAX 16 /* batched start pass: most work items per queue grab */
 
 /* Device view of the index, passed by value to every kernel.
  * occ: one 32-byte block per 64 rows of the $-removed BWT string:
@@ -106,6 +107,8 @@ struct GsBatch {
     uint32_t *pmap;            /* position -> seed */
     uint64_t seed_cap, pos_cap;   /* output capacities (entries) */
     uint64_t slot_cap;             /* candidate slots allocated */
+    uint32_t *item_read;       /* batched start pass: the read of each work item */
+    uint64_t item_read_cap;    /* entries allocated */
     uint32_t item_cap;             /* work items the hand-over buffer is sized for */
     uint64_t cont_cap;             /* hand-over records allocated */
     uint32_t *queue;           /* [0]: work-queue head, [1]: status flags,

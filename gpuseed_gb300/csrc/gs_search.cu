@@ -62,8 +62,10 @@ int gs_build_kmer_table(const GsDevIndex &I, uint2 *table, cudaStream_t st)
  *      count(Xc) == count(X) > 0, if any.  Xc's interval is one step with X's
  *      first character from the kx-mer table entry of (X without its first
  *      character)·c;
- *   3. packing: entry.x = l, entry.y = size << 3 | code, code 0-3 the forced
- *      base, 4 none, 7 "size does not fit 29 bits: start from the 13-mer";
+ *   3. packing: entry.x = l, entry.y = the size, the forced code (0-3 the
+ *      base, 4 none, 7 "size does not fit 28 bits: start from the 13-mer")
+ *      and, where X has at most GS_EXT_ROWS rows, which of its one- and
+ *      two-base left extensions occur (gs_entry_* below);
  *   4. entry.z, entry.w = the packed entry of gs_kmer_rc(X), the kx-mer of
  *      X's reverse complement in the same bit order.
  * A candidate whose kx-mer is always followed by its neighbour's next base is
@@ -119,18 +121,68 @@ __global__ void gs_kmerx_code_kernel(GsDevIndex I, const uint4 *table, int kx, u
     }
 }
 
-__global__ void gs_kmerx_pack_kernel(uint4 *table, uint64_t n, const uint8_t *code)
+/* A packed half entry's second word (the first is l):
+ *   bits 0-2   forced code
+ *   bit 3      set: at most GS_EXT_ROWS rows, and
+ *     bits 4-11  the size
+ *     bits 12-15 base c: exactly one row of X is preceded by c
+ *     bits 16-31 bit 4*c + d: some row of X is preceded by c, and that by d
+ *              clear: bits 4-31 the size
+ * A candidate whose extension by the bases its read has next does not occur
+ * can reach no minimum length past it, and one whose extension is a single
+ * row that its neighbour's string shares is contained there: both end at
+ * their start, without a walk.  The walk pass was bound by the walks'
+ * dependent block loads, most of them of strings that a chance hit kept
+ * alive for a base or two: with the extensions, and with the item's bases
+ * loaded by the warp and its read found in a map instead of a search, a
+ * 2 M-read SMEM pass on 3.1 Gbp takes 16.6 ms instead of 24.2, a 40,000-read
+ * (2 kbp) MEM pass 7.2 instead of 10.4, a 1 M-read pass on 100 Mbp 7.9
+ * instead of 10.5.  255 rows is what the size's byte holds. */
+#define GS_EXT_ROWS 255u
+#define GS_ENTRY_EXT 8u
+
+__device__ __forceinline__ uint32_t gs_entry_size(uint32_t y)
+{
+    return (y & GS_ENTRY_EXT) ? (y >> 4) & 255u : y >> 4;
+}
+
+/* a thread per entry: rows l..u are read in order (their blocks, and those
+ * of their LF rows, are shared by neighbouring entries, whose strings and
+ * so whose rows are adjacent) */
+__global__ void gs_kmerx_pack_kernel(GsDevIndex I, uint4 *table, uint64_t n, const uint8_t *code)
 {
     for (uint64_t X = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; X < n;
          X += (uint64_t)gridDim.x * blockDim.x) {
         const uint4 e = table[X];
-        uint32_t size = e.x <= e.y ? e.y - e.x + 1u : 0u;
-        uint32_t c = code[X];
-        if (size >= (1u << 29)) {
-            size = 0;
-            c = 7;
+        const uint32_t size = e.x <= e.y ? e.y - e.x + 1u : 0u;
+        uint32_t y;
+        if (size >= (1u << 28)) {
+            y = 7u;
+        } else if (size > GS_EXT_ROWS) {
+            y = code[X] | (size << 4);
+        } else {
+            uint32_t seen = 0, multi = 0, two = 0, at = 0xffffffffu;
+            GsBlk B;
+            for (uint32_t i = 0; i < size; i++) {
+                const uint32_t row = e.x + i;
+                if (row == I.primary) continue;   /* the text starts with X */
+                const uint32_t ka = row - (row > I.primary ? 1u : 0u);
+                if ((ka >> 6) != at) {
+                    at = ka >> 6;
+                    B = gs_load_block(I.occ, at);
+                }
+                const uint32_t c = gs_block_base(B, ka);
+                multi |= seen & (1u << c);
+                seen |= 1u << c;
+                const uint32_t prev = gs_L2(I, c) + gs_occ_in_block(B, ka, c);
+                if (prev == I.primary) continue;   /* ... with cX */
+                const uint32_t kp = prev - (prev > I.primary ? 1u : 0u);
+                const GsBlk P = gs_load_block(I.occ, kp >> 6);
+                two |= 1u << (4u * c + gs_block_base(P, kp));
+            }
+            y = code[X] | GS_ENTRY_EXT | (size << 4) | ((seen & ~multi) << 12) | (two << 16);
         }
-        table[X] = make_uint4(e.x, (size << 3) | c, 0u, 0u);
+        table[X] = make_uint4(e.x, y, 0u, 0u);
     }
 }
 
@@ -156,7 +208,7 @@ int gs_build_kmerx_table(const GsDevIndex &I, uint4 *table, int kx, cudaStream_t
     gs_kmerx_code_kernel<<<152 * 64, 256, 0, st>>>(I, table, kx, n, code);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        gs_kmerx_pack_kernel<<<152 * 64, 256, 0, st>>>(table, n, code);
+        gs_kmerx_pack_kernel<<<152 * 64, 256, 0, st>>>(I, table, n, code);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
@@ -269,7 +321,7 @@ __device__ __forceinline__ bool gs_start(const GsDevIndex &I, const unsigned cha
             return true;
         }
         uint2 iv = gs_ld_entry(reinterpret_cast<const uint2 *>(&I.kmerx[pat]));
-        uint32_t code = iv.y & 7u, size = iv.y >> 3;
+        uint32_t code = iv.y & 7u, size = gs_entry_size(iv.y);
         if (code != 7u) {
             fcode = code;
             l = iv.x;
@@ -304,21 +356,6 @@ struct GsStart {
     bool ok, alive;
 };
 
-/* a start from one packed half of a start-table entry; false for code 7
- * (interval too wide to pack: the caller starts from the 13-mer) */
-__device__ __forceinline__ bool gs_entry_start(uint32_t x, uint32_t y, int anchor, int dir, int KT,
-                                               GsStart &S)
-{
-    const uint32_t code = y & 7u, size = y >> 3;
-    if (code == 7u) return false;
-    S.fcode = code;
-    S.l = x;
-    S.u = size ? x + size - 1u : x - 1u;
-    S.pos = anchor + dir * (KT - 1);
-    S.alive = size != 0;
-    return true;
-}
-
 /* gs_start of one candidate: the rare starts of a paired window (a
  * non-ACGT base in it, or an interval too wide to pack) */
 template <int NSTOP>
@@ -333,65 +370,80 @@ __device__ __forceinline__ GsStart gs_start_apart(const GsDevIndex &I, const uns
     return S;
 }
 
-/* Both candidates of read window R[s..s+KT-1] (KT = I.kx): the forward one
- * ending at s+KT-1 (vf) and the reverse one starting at s (vr), with the
- * same results as gs_start on each.  An ACGT-only window takes one paired
- * entry for both; a window with another base starts each candidate on its
- * own (the 13-mer rule and the wildcard steps depend on where the base
- * lies in each walk order). */
-template <int NSTOP>
-__device__ __forceinline__ void gs_start_pair(const GsDevIndex &I, const unsigned char *seq, int s,
-                                              int KT, int iL, bool vf, bool vr, GsStart &F,
-                                              GsStart &R, unsigned long long &w_kmer,
-                                              unsigned long long &w_blk)
+/* The bases around a lane's read window, from one 64-byte stretch of the
+ * read that the warp loads a word a lane: lane i gets the 2-bit codes of
+ * bases b0 + i .. b0 + i + 28 (the first at bits 0-1 of lo, the 17th at bits
+ * 0-1 of hi) and bit j of `odd` set when base b0 + i + j lies outside the
+ * read or is no plain base.  Plain letters are those whose complement code
+ * is 3 - code; the nibble tables give some other letters code 0 on both
+ * strands, which the callers look up one by one.  A word is loaded only if
+ * it holds a byte of the read. */
+__device__ __forceinline__ void gs_warp_bases(const unsigned char *seq, int iL, int b0, int lane,
+                                              uint32_t &lo, uint32_t &hi, uint32_t &odd)
 {
-    const int ef = s + KT - 1;
-    F.l = R.l = 1u;
-    F.u = R.u = 0u;
-    F.fcode = R.fcode = 4u;
-    F.ok = R.ok = F.alive = R.alive = false;
-    F.pos = ef - (GS_K0 - 1);
-    R.pos = s + (GS_K0 - 1);
-    if (!vf && !vr) return;
-    /* the reverse key: complement codes, R[s] at bits 0-1 */
-    uint32_t pr = 0;
-    bool bad = false;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-        if (j < KT) {
-            const uint32_t c = gs_comp_code(seq[s + j]);
-            bad |= c > 3u;
-            pr |= (c & 3u) << (j << 1);
+    const uintptr_t a0 = (uintptr_t)seq + (uintptr_t)(intptr_t)b0;
+    const int d = (int)(a0 & 3u);
+    const int p0 = b0 - d + 4 * lane;   /* read position of this lane's word */
+    uint32_t t = 0x000f0000u;
+    if (lane < 16 && p0 + 3 >= 0 && p0 < iL) {
+        const uint32_t b = __ldg((const uint32_t *)(a0 - (uintptr_t)d) + lane);
+        const uint32_t idx = b & 0x07070707u;
+        const uint32_t sel = (idx & 7u) | ((idx >> 4) & 0x70u) | ((idx >> 8) & 0x700u) |
+                             ((idx >> 12) & 0x7000u);
+        /* letter & 7: A 0, C 1, G 2, T 3, others 4 */
+        const uint32_t c = __byte_perm(0x01040004u, 0x02040403u, sel);
+        uint32_t v = c & 0x03030303u;
+        v = (v | (v >> 6)) & 0x000f000fu;
+        uint32_t iv = (c >> 2) & 0x01010101u;
+        iv = (iv | (iv >> 7)) & 0x00030003u;
+        iv = (iv | (iv >> 14)) & 0xfu;
+        if (p0 < 0) iv |= (1u << -p0) - 1u;
+        if (p0 + 4 > iL) iv |= 0xfu << (iL - p0);
+        t = ((v | (v >> 12)) & 0xffu) | ((iv & 0xfu) << 16);
+    }
+    /* words j..j+3 at lane j: 16 codes and 16 flags */
+    uint32_t n = __shfl_down_sync(0xffffffffu, t, 1);
+    t = (t & 0xffu) | ((n & 0xffu) << 8) | (t & 0xf0000u) | ((n & 0xf0000u) << 4);
+    n = __shfl_down_sync(0xffffffffu, t, 2);
+    const uint32_t c16 = (t & 0xffffu) | (n << 16);
+    uint32_t v = (t >> 16) | ((n >> 16) << 8);
+    v |= __shfl_down_sync(0xffffffffu, v, 4) << 16;
+    const int q = (lane + d) >> 2, sh = (lane + d) & 3;
+    const uint32_t x0 = __shfl_sync(0xffffffffu, c16, q);
+    const uint32_t x1 = __shfl_sync(0xffffffffu, c16, q + 4);
+    lo = __funnelshift_r(x0, x1, 2 * sh);
+    hi = x1 >> (2 * sh);
+    odd = __shfl_sync(0xffffffffu, v, q) >> sh;
+}
+
+/* What a start's entry says about the candidate's next two bases c, d of
+ * its walk (GS_START_*), for the candidate itself and, by a shuffle, for
+ * the one it may contain.  ok1/ok2: c, d are plain bases. */
+#define GS_START_ALIVE 1u
+#define GS_START_ONE 2u     /* its string extended by c is one row */
+#define GS_START_TWO 4u     /* extended by c and d it occurs ... */
+#define GS_START_KNOWN 8u   /* ... or, with this and not _TWO, does not */
+#define GS_CODE_UNKNOWN 5u  /* forced code of a start that no packed entry gave */
+#define GS_START_DEAD 16u   /* it ends before length k: no record */
+
+__device__ __forceinline__ uint32_t gs_start_flags(uint32_t y, uint32_t c, bool ok1, uint32_t d,
+                                                   bool ok2, int more)
+{
+    if (!(y & GS_ENTRY_EXT)) return GS_START_ALIVE;
+    if (!((y >> 4) & 255u)) return 0u;
+    uint32_t f = GS_START_ALIVE;
+    if (ok1) {
+        const uint32_t two = y >> (16u + 4u * c);
+        const bool one = (y >> (12u + c)) & 1u;
+        if (one) f |= GS_START_ONE;
+        if (!one && !(two & 15u)) f |= GS_START_DEAD;   /* more >= 1: k > the start's length */
+        if (ok2) {
+            f |= GS_START_KNOWN;
+            if ((two >> d) & 1u) f |= GS_START_TWO;
+            else if (more >= 2) f |= GS_START_DEAD;
         }
     }
-    if (!bad) {
-        /* the forward key (R[s+KT-1] at bits 0-1) is pr's reverse complement */
-        const uint32_t pf = gs_kmer_rc(pr, KT);
-        const uint4 e = gs_ld_pair(&I.kmerx[pf]);
-        /* code 7 (interval too wide to pack): gs_start's own 13-mer start */
-        bool wide = false;
-        if (vf) {
-            F.ok = true;
-            wide = !gs_entry_start(e.x, e.y, ef, -1, KT, F);
-        }
-        if (vr) {
-            R.ok = true;
-            wide |= !gs_entry_start(e.z, e.w, s, 1, KT, R);
-        }
-        if (!wide) {
-            w_kmer++;
-            return;
-        }
-    }
-    /* (the work counters count one lookup per candidate here) */
-    if (vf) {
-        F = gs_start_apart<NSTOP>(I, seq, ef, true, KT, iL);
-        w_kmer++;
-    }
-    if (vr) {
-        R = gs_start_apart<NSTOP>(I, seq, s, false, KT, iL);
-        w_kmer++;
-    }
+    return f;
 }
 
 /* ------------------------------------------------------------------ */
@@ -411,6 +463,32 @@ __global__ void gs_prepare_kernel(const uint32_t *lengths, uint32_t n_reads, int
         item_n[r] = (w + GS_PCHUNK - 1) / GS_PCHUNK;
     } else {
         item_n[r] = 2u * ((n + GS_CHUNK - 1) / GS_CHUNK);
+    }
+}
+
+/* the read of each work item, so that the start pass need not search
+ * item_off for it: a thread per read, or the warp for a read of many items */
+__global__ void __launch_bounds__(256) gs_item_map_kernel(const uint32_t *item_off, uint32_t n_reads,
+                                                          uint32_t *item_read, uint64_t cap)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t a = 0, e = 0;
+    if (r < n_reads) {
+        a = item_off[r];
+        e = item_off[r + 1];
+    }
+    const bool big = e - a > 16u;
+    if (!big)
+        for (uint32_t i = a; i < e; i++)
+            if (i < cap) item_read[i] = r;
+    uint32_t m = __ballot_sync(0xffffffffu, big);
+    while (m) {
+        const int src = __ffs(m) - 1;
+        m &= m - 1u;
+        const uint32_t a1 = __shfl_sync(0xffffffffu, a, src), e1 = __shfl_sync(0xffffffffu, e, src);
+        for (uint32_t i = a1 + (uint32_t)lane; i < e1; i += 32)
+            if (i < cap) item_read[i] = r - (uint32_t)lane + (uint32_t)src;
     }
 }
 
@@ -1016,10 +1094,10 @@ struct GsReserve {
 
 template <int NSTOP, int COUNT>
 __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch &B, uint32_t r,
-                                             uint32_t local, int lane, GsReserve &res,
-                                             unsigned long long &wk, unsigned long long &wb)
+                                             uint32_t local, uint32_t L, uint64_t off, int lane,
+                                             GsReserve &res, unsigned long long &wk,
+                                             unsigned long long &wb)
 {
-    const uint32_t L = B.lengths[r];
     const int k = B.k;
     const uint32_t n = L - (uint32_t)k + 1u;
     const uint32_t nch = (n + GS_CHUNK - 1) / GS_CHUNK;
@@ -1030,7 +1108,7 @@ __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch
     /* lane 31 only starts the next item's first candidate (which that item
      * owns: ceil(n / GS_CHUNK) items cover every candidate) */
     const bool owned = in_range && lane < GS_CHUNK;
-    const unsigned char *seq = (const unsigned char *)B.seqs + B.offsets[r];
+    const unsigned char *seq = (const unsigned char *)B.seqs + off;
     const int iL = (int)L;
     const int anchor = fwd ? (k - 1 + (int)ci) : ((int)n - 1 - (int)ci);
     const int dir = fwd ? -1 : 1;
@@ -1138,66 +1216,126 @@ __device__ __forceinline__ bool gs_push_walker(const GsBatch &B, const GsReserve
     return true;
 }
 
-/* J of an owned candidate from its neighbour's start, as in gs_start_item:
- * a forced code settles containment, otherwise the neighbour's interval is
- * J one base short (jpend) */
-__device__ __forceinline__ void gs_start_j(uint32_t cn, uint32_t fcode, bool nalive, uint32_t nl,
-                                           uint32_t nu, bool &killed, bool &jpend, uint32_t &jl,
-                                           uint32_t &ju)
+/* Whether a candidate that is to walk is contained in its neighbour at the
+ * start already (walk cleared), and whether it carries the neighbour's start
+ * interval as J, one base short.  cn: the neighbour's base; f, nf: the
+ * candidate's and the neighbour's GS_START_* flags. */
+__device__ __forceinline__ void gs_start_settle(uint32_t cn, uint32_t fcode, uint32_t f, uint32_t nf,
+                                                bool &walk, bool &j)
 {
-    if (cn > 3u) return;
+    if (cn > 3u) return;   /* the candidates beyond never started: no J */
     if (fcode < 4u) {
-        killed = (fcode == cn);
-    } else if (nalive) {
-        jl = nl;
-        ju = nu;
-        jpend = true;
+        walk = fcode != cn;   /* forced elsewhere: the neighbour's string does not occur */
+        return;
+    }
+    if (!(nf & GS_START_ALIVE)) return;
+    if (!(nf & GS_START_KNOWN)) {
+        j = true;
+    } else if (nf & GS_START_TWO) {
+        if (f & GS_START_ONE) walk = false;
+        else j = true;
+    } else if (fcode != 4u) {
+        j = true;   /* the sizes may be equal at the start already */
     }
 }
 
-/* A paired work item: the windows s = GS_PCHUNK*local - 1 + lane of read r
+/* A paired work item: the windows s = GS_PCHUNK*local - 1 + lane of a read
  * (lanes 1..GS_PCHUNK own theirs; lanes 0 and 31 start their windows only
  * for the neighbours' J), each window's forward candidate (ending at
  * s+KT-1, neighbour e+1 = lane+1) and reverse candidate (starting at s,
- * neighbour s-1 = lane-1) from one start-table entry.  Records, J and
- * walkers are those of gs_start_item for each candidate. */
-template <int NSTOP, int COUNT>
+ * neighbour s-1 = lane-1) from one start-table entry: its two keys are the
+ * window and its reverse complement.  A window that holds another letter
+ * than a plain base, or whose entry is too wide to pack, starts each
+ * candidate on its own.  No record is written here: a start is KT < k bases
+ * long.
+ *
+ * Which candidates walk.  Not those whose next one or two bases make a
+ * string that does not occur, where that keeps them below length k
+ * (GS_START_DEAD).  Not those contained in their neighbour: forced to its
+ * base, or a single row after one base where the neighbour's string, one
+ * base longer, still occurs (its own two-base extension: the same bases).
+ * Of the others, those whose neighbour's string no longer occurs after one
+ * base walk without J (at the start itself the sizes differ: no forced
+ * code). */
+template <int NSTOP>
 __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const GsBatch &B, uint32_t r,
-                                                   uint32_t local, int lane, GsReserve &res,
-                                                   unsigned long long &wk, unsigned long long &wb)
+                                                   uint32_t local, int iL, uint64_t off, int lane,
+                                                   GsReserve &res, unsigned long long &wk)
 {
-    const int iL = (int)B.lengths[r];
     const int k = B.k, KT = I.kx;
-    const uint32_t n = (uint32_t)(iL - k + 1);   /* candidates per strand (the item exists: L >= k) */
     const int s = (int)(local * GS_PCHUNK) - 1 + lane;
     const bool in_range = s >= 0 && s <= iL - KT;
     const bool owned = in_range && lane >= 1 && lane <= GS_PCHUNK;
     const bool vf = in_range && s >= k - KT;   /* forward candidate s+KT-1 >= k-1 */
     const bool vr = in_range && s <= iL - k;   /* reverse candidate s <= L-k */
-    const unsigned char *seq = (const unsigned char *)B.seqs + B.offsets[r];
+    const unsigned char *seq = (const unsigned char *)B.seqs + off;
     const int ef = s + KT - 1;
-    GsStart F, R;
-    gs_start_pair<NSTOP>(I, seq, s, KT, iL, vf, vr, F, R, wk, wb);
-    const uint32_t fnl = __shfl_down_sync(0xffffffffu, F.l, 1);
-    const uint32_t fnu = __shfl_down_sync(0xffffffffu, F.u, 1);
-    const int fna = __shfl_down_sync(0xffffffffu, F.alive ? 1 : 0, 1);
-    const uint32_t rnl = __shfl_up_sync(0xffffffffu, R.l, 1);
-    const uint32_t rnu = __shfl_up_sync(0xffffffffu, R.u, 1);
-    const int rna = __shfl_up_sync(0xffffffffu, R.alive ? 1 : 0, 1);
+    uint32_t lo, hi, odd;
+    gs_warp_bases(seq, iL, s - lane - 2, lane, lo, hi, odd);
+    /* bases s-2, s-1 (walk order of the forward candidate: s-1, s-2) and
+     * s+KT, s+KT+1 */
+    const uint32_t after = (uint32_t)((((uint64_t)hi << 32) | lo) >> (2 * (KT + 2)));
+    const uint32_t p1 = (lo >> 2) & 3u, p2 = lo & 3u, n1 = after & 3u, n2 = (after >> 2) & 3u;
+    const bool op1 = !(odd & 2u), op2 = !(odd & 1u);
+    const bool on1 = !((odd >> (KT + 2)) & 1u), on2 = !((odd >> (KT + 3)) & 1u);
 
-    bool fk = false, fj = false, rk = false, rj = false;
-    uint32_t fjl = 1, fju = 0, rjl = 1, rju = 0;
-    if (owned && vf && F.alive && ef + 1 < iL)
-        gs_start_j(gs_fwd_code(seq[ef + 1]), F.fcode, fna != 0, fnl, fnu, fk, fj, fjl, fju);
-    if (owned && vr && R.alive && s >= 1)
-        gs_start_j(gs_comp_code(seq[s - 1]), R.fcode, rna != 0, rnl, rnu, rk, rj, rjl, rju);
-
-    const bool wf = owned && vf && F.alive && !fk;
-    const bool wr = owned && vr && R.alive && !rk;
-    if (owned && vf && !wf) gs_write_record(B, r, n, true, ef, F.pos, F.l, F.u, F.ok, fk);
-    if (owned && vr && !wr) gs_write_record(B, r, n, false, s, R.pos, R.l, R.u, R.ok, rk);
+    uint32_t fl = 1u, fu = 0u, ff = 0u, fcode = 4u, rl = 1u, ru = 0u, rf = 0u, rcode = 4u;
+    if (vf || vr) {
+        bool apart = ((odd >> 2) & ((1u << KT) - 1u)) != 0u;
+        if (!apart) {
+            /* the reverse key: complement codes, R[s] at bits 0-1; the forward
+             * key (R[s+KT-1] at bits 0-1) is its reverse complement */
+            const uint32_t pr = ~__funnelshift_r(lo, hi, 4) & (0xffffffffu >> (32 - 2 * KT));
+            const uint4 e = gs_ld_pair(&I.kmerx[gs_kmer_rc(pr, KT)]);
+            const uint32_t fs = gs_entry_size(e.y), rs = gs_entry_size(e.w);
+            fcode = e.y & 7u;
+            rcode = e.w & 7u;
+            apart = (vf && fcode == 7u) || (vr && rcode == 7u);
+            if (vf) {
+                fl = e.x;
+                fu = e.x + fs - 1u;
+                ff = gs_start_flags(e.y, p1, op1, p2, op2, k - KT);
+            }
+            if (vr) {
+                rl = e.z;
+                ru = e.z + rs - 1u;
+                rf = gs_start_flags(e.w, 3u - n1, on1, 3u - n2, on2, k - KT);
+            }
+        }
+        wk += apart ? (vf ? 1u : 0u) + (vr ? 1u : 0u) : 1u;
+        if (apart) {
+            if (vf) {
+                const GsStart S = gs_start_apart<NSTOP>(I, seq, ef, true, KT, iL);
+                fl = S.l; fu = S.u; fcode = S.fcode < 4u ? S.fcode : GS_CODE_UNKNOWN;
+                ff = S.alive ? GS_START_ALIVE : 0u;
+            }
+            if (vr) {
+                const GsStart S = gs_start_apart<NSTOP>(I, seq, s, false, KT, iL);
+                rl = S.l; ru = S.u; rcode = S.fcode < 4u ? S.fcode : GS_CODE_UNKNOWN;
+                rf = S.alive ? GS_START_ALIVE : 0u;
+            }
+        }
+    }
+    const uint32_t nff = __shfl_down_sync(0xffffffffu, ff, 1);
+    const uint32_t nrf = __shfl_up_sync(0xffffffffu, rf, 1);
+    bool wf = owned && (ff & (GS_START_ALIVE | GS_START_DEAD)) == GS_START_ALIVE;
+    bool wr = owned && (rf & (GS_START_ALIVE | GS_START_DEAD)) == GS_START_ALIVE;
+    bool fj = false, rj = false;
+    if (wf && ef + 1 < iL) {
+        const uint32_t cn = on1 ? n1 : gs_fwd_code(seq[ef + 1]);
+        gs_start_settle(cn, fcode, ff, nff, wf, fj);
+    }
+    if (wr && s >= 1) {
+        const uint32_t cn = op1 ? 3u - p1 : gs_comp_code(seq[s - 1]);
+        gs_start_settle(cn, rcode, rf, nrf, wr, rj);
+    }
     const uint32_t mf = __ballot_sync(0xffffffffu, wf), mr = __ballot_sync(0xffffffffu, wr);
     if (!(mf | mr)) return;
+    const uint32_t fnl = __shfl_down_sync(0xffffffffu, fl, 1);
+    const uint32_t fnu = __shfl_down_sync(0xffffffffu, fu, 1);
+    const uint32_t rnl = __shfl_up_sync(0xffffffffu, rl, 1);
+    const uint32_t rnu = __shfl_up_sync(0xffffffffu, ru, 1);
+    const uint32_t n = (uint32_t)(iL - k + 1);   /* candidates per strand (the item exists: L >= k) */
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t cnt = (uint32_t)(__popc(mf) + __popc(mr));
     const uint32_t rem = res.end - res.next;
@@ -1211,12 +1349,12 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
             if ((uint64_t)g + gs_walker_chunk(B) >= B.walker_cap) res.full = 1u;
         }
     }
-    if (wf && !gs_push_walker(B, res, g, rem, (uint32_t)__popc(mf & lt), r, true, ef, F.l, F.u,
-                              fjl, fju, fj, iL))
-        gs_write_leftover(B, r, n, true, ef, F.l, F.u);
+    if (wf && !gs_push_walker(B, res, g, rem, (uint32_t)__popc(mf & lt), r, true, ef, fl, fu,
+                              fj ? fnl : 1u, fj ? fnu : 0u, fj, iL))
+        gs_write_leftover(B, r, n, true, ef, fl, fu);
     if (wr && !gs_push_walker(B, res, g, rem, (uint32_t)(__popc(mf) + __popc(mr & lt)), r, false,
-                              s, R.l, R.u, rjl, rju, rj, iL))
-        gs_write_leftover(B, r, n, false, s, R.l, R.u);
+                              s, rl, ru, rj ? rnl : 1u, rj ? rnu : 0u, rj, iL))
+        gs_write_leftover(B, r, n, false, s, rl, ru);
     if (rem < cnt) {
         res.next = (uint32_t)min((uint64_t)g + (cnt - rem), B.walker_cap);
         res.end = (uint32_t)min((uint64_t)g + gs_walker_chunk(B), B.walker_cap);
@@ -1235,22 +1373,36 @@ __global__ void __launch_bounds__(256, 5) gs_search_start(GsDevIndex I, GsBatch 
     unsigned long long wk = 0, wb = 0;
     GsReserve res = {0u, 0u, B.walker_cap == 0 ? 1u : 0u};
     const uint32_t n_items = B.item_off[B.n_reads];
+    if (n_items > B.item_read_cap) {
+        /* a captured pass replayed on larger input: report, do nothing */
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(B.queue + 1, GS_FLAG_OVERFLOW);
+        return;
+    }
     for (;;) {
         uint32_t first = 0;
         if (lane == 0) first = atomicAdd(B.queue, (uint32_t)queue_chunk);
         first = __shfl_sync(0xffffffffu, first, 0);
         if (first >= n_items) break;
-        uint32_t last = min(first + (uint32_t)queue_chunk, n_items);
-        uint32_t lo = 0, hi = B.n_reads;
-        while (lo + 1 < hi) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (B.item_off[mid] <= first) lo = mid; else hi = mid;
-        }
-        uint32_t r = lo;
-        for (uint32_t it = first; it < last; it++) {
-            while (B.item_off[r + 1] <= it) r++;
-            if (PAIRED) gs_start_pair_item<NSTOP, COUNT>(I, B, r, it - B.item_off[r], lane, res, wk, wb);
-            else gs_start_item<NSTOP, COUNT>(I, B, r, it - B.item_off[r], lane, res, wk, wb);
+        const uint32_t last = min(first + (uint32_t)queue_chunk, n_items);
+        /* up to 32 items at a time, each lane looking up one item's read */
+        for (uint32_t it = first; it < last; it += 32) {
+            const int m = (int)min(last - it, 32u);
+            uint32_t ir = 0, il = 0, iLen = 0;
+            uint64_t ioff = 0;
+            if (lane < m) {
+                ir = B.item_read[it + (uint32_t)lane];
+                il = it + (uint32_t)lane - B.item_off[ir];
+                iLen = B.lengths[ir];
+                ioff = B.offsets[ir];
+            }
+            for (int j = 0; j < m; j++) {
+                const uint32_t r = __shfl_sync(0xffffffffu, ir, j);
+                const uint32_t local = __shfl_sync(0xffffffffu, il, j);
+                const uint32_t L = __shfl_sync(0xffffffffu, iLen, j);
+                const uint64_t off = __shfl_sync(0xffffffffu, ioff, j);
+                if (PAIRED) gs_start_pair_item<NSTOP>(I, B, r, local, (int)L, off, lane, res, wk);
+                else gs_start_item<NSTOP, COUNT>(I, B, r, local, L, off, lane, res, wk, wb);
+            }
         }
     }
     /* unused entries of the last reservation: holes */
@@ -1553,7 +1705,6 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
     int dev = 0, sms = 0;
     GS_CUDA(cudaGetDevice(&dev));
     GS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (queue_chunk <= 0) queue_chunk = GS_QUEUE_CHUNK;
     const bool cnt = B.work != NULL, nstop = B.n_mode == GS_N_STOP;
     void (*start)(GsDevIndex, GsBatch, int) =
         B.paired ? (nstop ? (cnt ? gs_search_start<1, 1, true> : gs_search_start<1, 0, true>)
@@ -1569,11 +1720,22 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         ctas_per_sm = occ > 0 ? occ : 1;
     }
     uint32_t grid = (uint32_t)sms * (uint32_t)ctas_per_sm;
+    /* a captured pass knows its items only on the device: as many as the
+     * pass it was sized by */
+    const uint32_t items = n_items ? n_items : B.item_cap;
+    if (queue_chunk <= 0) {
+        /* an eighth of a warp's share of the items, 1 to GS_QUEUE_CHUNK_MAX */
+        const uint32_t share = items / (grid * 8u * 8u);
+        queue_chunk = share < 1u ? 1 : share > GS_QUEUE_CHUNK_MAX ? GS_QUEUE_CHUNK_MAX : (int)share;
+    }
     if (n_items) {
         uint32_t need = (n_items + (uint32_t)queue_chunk - 1) / (uint32_t)queue_chunk;
         if (need < grid * 8) grid = (need + 7) / 8;
     }
     if (grid == 0) grid = 1;
+    gs_item_map_kernel<<<(B.n_reads + 255) / 256, 256, 0, st>>>(B.item_off, B.n_reads, B.item_read,
+                                                                B.item_read_cap);
+    GS_CUDA(cudaGetLastError());
     GS_CUDA(cudaMemsetAsync(B.queue, 0, sizeof(uint32_t), st));
     GS_CUDA(cudaMemsetAsync(B.queue + 2, 0, 2 * sizeof(uint32_t), st));
     B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, GS_WALKER_CHUNK);
