@@ -1,26 +1,32 @@
 /*
  * gs_fm.cuh -- FM-index primitives on the device.
  *
- * The occurrence table in HBM: one 32-byte block per 64 rows of the
- * $-removed BWT string, {count of A, C, G, T before the block, H0, H1, L0,
- * L1}.  The counts are the reference's checkpoints (seed_gen.cu:52-58); the
- * block's 64 bases are stored bit-sliced instead of as 2-bit fields: H0/H1
- * hold their high bits and L0/L1 their low bits, base i of the block at bit
- * 31 - (i & 31) of word i >> 5 of each.  The loader converts the file's
- * packed words (16 bases per word, first base in the top bits) once
- * (gs_index.cu).  The arithmetic is the reference's (seed_gen.cu:195-216
- * occ, :329-368 occ pair, :455-484 LF); the counting is our own: the bases
- * equal to c among the first n of a block are the set bits of
- * (H ^ ~c1) & (L ^ ~c0) in the top n bits, two popcounts per query.
+ * The occurrence table in HBM: one 64-byte block per 64 rows of the BWT (its
+ * $ row included), a 16-byte slot per base c: {L2[c] + 1 + count of c before
+ * the block, the block's rows that hold c as a 64-bit mask (two words, row i
+ * at bit i & 31 of word i >> 5), 0}.  The $ row is set in no mask.  A step's
+ * bound with base c is then one 16-byte load, and the new bound is the
+ * slot's count plus the set bits of its mask below the bound's row: no
+ * counting of two-bit fields, no selection of the base's count, no
+ * correction for the $ row, no base offset to add.  The loader makes the
+ * blocks from the file's checkpoints and packed words once (gs_index.cu).
+ * Results are the reference's integers (seed_gen.cu:195-216 occ, :329-368
+ * occ pair, :455-484 LF).
+ *
+ * Before, a block of 32 bytes held 64 rows of the $-removed string as four
+ * counts and bit-sliced bases.  A query took two loads and about 30
+ * instructions, and the walk pass, which executes them without end, issued
+ * on two thirds of its slots.  The wider block costs HBM (3.1 GB at 3.1 Gbp
+ * instead of 1.55) and L2 reach, not loads: either form is one 64-byte fill
+ * a bound, and bounds 64 to 127 rows apart no longer share one.
+ * Measured (whole pass, the walk in brackets): 2 M reads on 3.1 Gbp 16.3 ->
+ * 15.5 ms (9.5 -> 8.7, its DRAM reads 16.0 -> 18.3 GB), 1 M reads on 100
+ * Mbp 7.7 -> 7.3 ms (4.1 -> 3.6), 40,000 long reads 7.1 -> 6.9 ms.
  */
 #ifndef GS_FM_CUH
 #define GS_FM_CUH
 
 #include "gs_internal.h"
-
-struct GsBlk {
-    uint32_t w[8];
-};
 
 /* one random read-only word with a 64-byte L2 fill (the default fills 128) */
 __device__ __forceinline__ uint32_t gs_ld64(const uint32_t *p)
@@ -30,141 +36,83 @@ __device__ __forceinline__ uint32_t gs_ld64(const uint32_t *p)
     return v;
 }
 
-__device__ __forceinline__ GsBlk gs_load_block(const uint32_t *occ, uint32_t blk)
-{
-    GsBlk b;
-    const uint32_t *p = occ + (size_t)blk * GS_BLOCK_WORDS;
-    asm("ld.global.nc.L2::64B.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(b.w[0]), "=r"(b.w[1]), "=r"(b.w[2]), "=r"(b.w[3]), "=r"(b.w[4]), "=r"(b.w[5]),
-          "=r"(b.w[6]), "=r"(b.w[7])
-        : "l"(p));
-    return b;
-}
-
 __device__ __forceinline__ uint32_t gs_sel4(uint32_t c, uint32_t a0, uint32_t a1, uint32_t a2,
                                             uint32_t a3)
 {
     return c == 0 ? a0 : c == 1 ? a1 : c == 2 ? a2 : a3;
 }
 
-__device__ __forceinline__ uint32_t gs_L2(const GsDevIndex &I, uint32_t c)
-{
-    return gs_sel4(c, I.L2[0], I.L2[1], I.L2[2], I.L2[3]);
-}
-
-/* bit-sliced match words of a block for base c: bit 31 - (i & 31) of word
- * i >> 5 is set when base i of the block is c */
-struct GsMatch {
+/* base c's slot of a row's block */
+struct GsSlot {
     uint32_t cnt, m0, m1;
 };
 
-__device__ __forceinline__ GsMatch gs_match(uint32_t cnt, uint32_t h0, uint32_t h1, uint32_t l0,
-                                            uint32_t l1, uint32_t c)
+/* rows & ~63 is the byte offset of a row's 64-byte block */
+__device__ __forceinline__ const char *gs_slot_at(const uint4 *occ, uint32_t row, uint32_t c)
 {
-    const uint32_t hx = ((c >> 1) & 1u) - 1u;   /* ~0 when c's high bit is 0 */
-    const uint32_t lx = (c & 1u) - 1u;
-    GsMatch m;
-    m.cnt = cnt;
-    m.m0 = (h0 ^ hx) & (l0 ^ lx);
-    m.m1 = (h1 ^ hx) & (l1 ^ lx);
-    return m;
+    return (const char *)occ + (size_t)(row & ~63u) + (c << 4);
 }
 
-/* count of c in string positions [0, k] given k's block matched for c: the
- * set bits among the top (k & 63) + 1 bits of m0:m1 */
-__device__ __forceinline__ uint32_t gs_occ_in_match(const GsMatch &m, uint32_t k)
+__device__ __forceinline__ GsSlot gs_load_slot(const uint4 *occ, uint32_t row, uint32_t c)
 {
-    const uint32_t j = k & 63u;
-    const uint32_t c0 = __popc(m.m0 >> (31u - ((j & 31u) | ((j >> 5) * 31u))));
-    const uint32_t c1 = j >= 32u ? __popc(m.m1 >> (63u - j)) : 0u;
-    return m.cnt + c0 + c1;
+    GsSlot s;
+    uint32_t pad;
+    asm("ld.global.nc.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];"
+        : "=r"(s.cnt), "=r"(s.m0), "=r"(s.m1), "=r"(pad)
+        : "l"(gs_slot_at(occ, row, c)));
+    return s;
 }
 
-/* count of c in string positions [0, k] given k's block */
-__device__ __forceinline__ uint32_t gs_occ_in_block(const GsBlk &b, uint32_t k, uint32_t c)
+/* the same when `yes`, as a predicated load instead of a branch; else the
+ * slot is left undefined */
+__device__ __forceinline__ GsSlot gs_load_slot_if(bool yes, const uint4 *occ, uint32_t row, uint32_t c)
 {
-    return gs_occ_in_match(gs_match(gs_sel4(c, b.w[0], b.w[1], b.w[2], b.w[3]), b.w[4], b.w[5],
-                                    b.w[6], b.w[7], c),
-                           k);
+    GsSlot s;
+    uint32_t pad;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+        "@q ld.global.nc.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+        : "=r"(s.cnt), "=r"(s.m0), "=r"(s.m1), "=r"(pad)
+        : "l"(gs_slot_at(occ, row, c)), "r"((int)yes));
+    return s;
 }
 
-/* base at string position k given k's block */
-__device__ __forceinline__ uint32_t gs_block_base(const GsBlk &b, uint32_t k)
+/* a with `s`, else b */
+__device__ __forceinline__ GsSlot gs_slot_sel(bool s, const GsSlot &a, const GsSlot &b)
 {
-    const uint32_t sh = 31u - (k & 31u);
-    const bool hi = (k & 32u) != 0;
-    const uint32_t h = ((hi ? b.w[5] : b.w[4]) >> sh) & 1u;
-    const uint32_t l = ((hi ? b.w[7] : b.w[6]) >> sh) & 1u;
-    return (h << 1) | l;
+    GsSlot r;
+    r.cnt = s ? a.cnt : b.cnt;
+    r.m0 = s ? a.m0 : b.m0;
+    r.m1 = s ? a.m1 : b.m1;
+    return r;
+}
+
+/* L2[c] + 1 + occurrences of c in rows [0, row): with the bits of the masks
+ * below row & 63 (PTX bmsk and shr clamp counts of 32 and more) */
+__device__ __forceinline__ uint32_t gs_slot_rank(const GsSlot &s, uint32_t row)
+{
+    const uint32_t j = row & 63u;
+    uint32_t w0, w1;
+    asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(w0) : "r"(j));
+    asm("shr.u32 %0, 0xffffffff, %1;" : "=r"(w1) : "r"(64u - j));
+    return s.cnt + __popc(s.m0 & w0) + __popc(s.m1 & w1);
 }
 
 /* One backward-search step with base c in [0,3]: [l,u] -> [l',u'].
- * Returns the number of 32-byte blocks read (0..2). */
+ * Returns the number of 32-byte blocks of 64 rows of the $-removed string
+ * that the canonical walk reads for it (0..2). */
 __device__ __forceinline__ int gs_step(const GsDevIndex &I, uint32_t &l, uint32_t &u, uint32_t c)
 {
     const bool lz = (l == 0);            /* occ(-1) = 0 */
     const bool uf = (u == I.seq_len);    /* occ(seq_len) = total */
     uint32_t la = l - 1u;
     la -= (la >= I.primary) ? 1u : 0u;
-    uint32_t ua = u - ((u >= I.primary) ? 1u : 0u);
-    uint32_t bl = la >> 6, bu = ua >> 6;
-    uint32_t ol = 0, ou;
-    int nb = 0;
-    GsBlk B;
-    if (!uf) {
-        B = gs_load_block(I.occ, bu);
-        ou = gs_occ_in_block(B, ua, c);
-        nb = 1;
-    } else {
-        ou = gs_sel4(c, I.L2[1], I.L2[2], I.L2[3], I.L2[4]) - gs_L2(I, c);
-    }
-    if (!lz) {
-        if (uf || bl != bu) {
-            B = gs_load_block(I.occ, bl);
-            nb++;
-        }
-        ol = gs_occ_in_block(B, la, c);
-    }
-    uint32_t base = gs_L2(I, c);
-    l = base + ol + 1u;
-    u = base + ou;
+    const uint32_t ua = u - ((u >= I.primary) ? 1u : 0u);
+    const int nb = (uf ? 0 : 1) + ((!lz && (uf || (la >> 6) != (ua >> 6))) ? 1 : 0);
+    const GsSlot A = gs_load_slot(I.occ, l, c);
+    const GsSlot E = gs_load_slot(I.occ, u + 1u, c);
+    l = gs_slot_rank(A, l);
+    u = gs_slot_rank(E, u + 1u) - 1u;
     return nb;
-}
-
-/* The part of a block one occurrence query with base c reads: the count
- * of c before the block and the four bit-slice words (a 4-byte and a
- * 16-byte load of the same 32-byte sector).  Their L2 fills are 64 bytes
- * (the block and its neighbour), not 128: config-3 search 101.25 -> 100.9
- * ms (256-byte fills: 101.5). */
-struct GsHalf {
-    uint32_t cnt, h0, h1, l0, l1;
-};
-
-__device__ __forceinline__ GsHalf gs_load_half(const uint32_t *occ, uint32_t blk, uint32_t c)
-{
-    GsHalf h;
-    const uint32_t *p = occ + (size_t)blk * GS_BLOCK_WORDS;
-    asm("ld.global.nc.L2::64B.u32 %0, [%1];" : "=r"(h.cnt) : "l"(p + c));
-    asm("ld.global.nc.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];"
-        : "=r"(h.h0), "=r"(h.h1), "=r"(h.l0), "=r"(h.l1)
-        : "l"(p + 4));
-    return h;
-}
-
-/* h = s ? a : h, word by word */
-__device__ __forceinline__ void gs_half_take(GsHalf &h, bool s, const GsHalf &a)
-{
-    h.cnt = s ? a.cnt : h.cnt;
-    h.h0 = s ? a.h0 : h.h0;
-    h.h1 = s ? a.h1 : h.h1;
-    h.l0 = s ? a.l0 : h.l0;
-    h.l1 = s ? a.l1 : h.l1;
-}
-
-/* count of c in string positions [0, k] given k's block */
-__device__ __forceinline__ uint32_t gs_occ_in_half(const GsHalf &b, uint32_t k, uint32_t c)
-{
-    return gs_occ_in_match(gs_match(b.cnt, b.h0, b.h1, b.l0, b.l1, c), k);
 }
 
 /* how many distinct values among those of a..d that are valid */
@@ -175,80 +123,90 @@ __device__ __forceinline__ int gs_distinct4(uint32_t a, bool va, uint32_t b, boo
            (int)(vd && !(va && d == a) && !(vb && d == b) && !(vc && d == c));
 }
 
-/* What one step of gs_step_pair touched, for the work counters: blocks
- * loaded for J alone, and the distinct 128-byte lines its bounds fall in
- * with this layout (256 rows a line) and with a 64-byte block of 192 rows
- * (384 rows a line). */
+/* What one step of gs_step_pair touched, for the work counters: slots
+ * loaded, those for J alone, and the distinct lines of 256 and 384 rows its
+ * bounds fall in. */
 struct GsStepTouch {
-    int jblocks, lines256, lines384;
+    int blocks, jblocks, lines256, lines384;
 };
 
-/* One backward step with base c of an interval I = [l,u] (only when doI)
- * and of a sub-interval J = [jl,ju] of it (jl > ju: none; left unchanged).  J's
- * bounds lie between I's, so their blocks are loaded only where they differ
- * from the blocks of I's bounds, and all loads are issued before any is
- * used.  Returns the number of 32-byte blocks loaded (0..4); jblocks gets
- * the number loaded for J alone. */
-__device__ __forceinline__ int gs_step_pair(const GsDevIndex &I, uint32_t &l, uint32_t &u,
-                                            uint32_t &jl, uint32_t &ju, uint32_t c, bool doI,
-                                            GsStepTouch &touch)
+/* One backward step with base c of an interval I = [l,e) (only when doI)
+ * and of an interval J = [jl,je) (jl >= je: none; left unchanged) that lies
+ * within it, or where doI is not set anywhere: e and je are one past the
+ * last row.  J's bounds lie between I's, so a slot is loaded only where its
+ * block differs from those of the bounds before it, by predicated loads that
+ * all issue before any is used. */
+template <int COUNT>
+__device__ __forceinline__ void gs_step_pair(const GsDevIndex &I, uint32_t &l, uint32_t &e,
+                                             uint32_t &jl, uint32_t &je, uint32_t c, bool doI,
+                                             GsStepTouch &touch)
 {
-    const uint32_t P = I.primary;
-    const bool lz = (l == 0), uf = (u == I.seq_len);
-    uint32_t la = l - 1u;
-    la -= (la >= P) ? 1u : 0u;
-    const uint32_t ua = u - ((u >= P) ? 1u : 0u);
-    const bool jn = jl <= ju;
-    const bool jlz = jn && jl == 0, juf = jn && ju == I.seq_len;
-    uint32_t jla = jl - 1u;
-    jla -= (jla >= P) ? 1u : 0u;
-    const uint32_t jua = ju - ((ju >= P) ? 1u : 0u);
-    const uint32_t bu = ua >> 6, bl = la >> 6, jbu = jua >> 6, jbl = jla >> 6;
-    /* distinct blocks: H0 = bu, H1 = bl, H2 = jbu, H3 = jbl */
-    const bool n0 = doI && !uf;
-    const bool n1 = doI && !lz && !(n0 && bl == bu);
-    const bool n2 = jn && !juf && !(n0 && jbu == bu) && !(n1 && jbu == bl);
-    const bool n3 = jn && !jlz && !(n0 && jbl == bu) && !(n1 && jbl == bl) && !(n2 && jbl == jbu);
-    GsHalf H0, H1, H2, H3;
-    if (n0) H0 = gs_load_half(I.occ, bu, c);
-    if (n1) H1 = gs_load_half(I.occ, bl, c);
-    if (n2) H2 = gs_load_half(I.occ, jbu, c);
-    if (n3) H3 = gs_load_half(I.occ, jbl, c);
-    const uint32_t base = gs_L2(I, c);
-    const uint32_t total = gs_sel4(c, I.L2[1], I.L2[2], I.L2[3], I.L2[4]) - base;
-    const uint32_t ou = uf ? total : gs_occ_in_half(H0, ua, c);
-    GsHalf X = H0;
-    gs_half_take(X, n1, H1);
-    const uint32_t ol = lz ? 0u : gs_occ_in_half(X, la, c);
-    if (jn) {
-        GsHalf Y = H1;
-        gs_half_take(Y, n0 && jbu == bu, H0);
-        gs_half_take(Y, n2, H2);
-        const uint32_t jou = juf ? total : gs_occ_in_half(Y, jua, c);
-        GsHalf Z = H2;
-        gs_half_take(Z, n1 && jbl == bl, H1);
-        gs_half_take(Z, n0 && jbl == bu, H0);
-        gs_half_take(Z, n3, H3);
-        const uint32_t jol = jlz ? 0u : gs_occ_in_half(Z, jla, c);
-        jl = base + jol + 1u;
-        ju = base + jou;
+    const bool jn = jl < je;
+    const uint32_t bl = l >> 6, be = e >> 6, bj = jl >> 6, bk = je >> 6;
+    const bool one = be == bl;                             /* I within a block: J too */
+    const bool jL = doI && bj == bl, jE = doI && bj == be;
+    const bool kL = doI && bk == bl, kE = doI && bk == be, kJ = bk == bj;
+    const bool n0 = doI, n1 = doI && !one, n2 = jn && !jL && !jE, n3 = jn && !kL && !kE && !kJ;
+    const GsSlot A = gs_load_slot_if(n0, I.occ, l, c);
+    GsSlot E = gs_load_slot_if(n1, I.occ, e, c);
+    GsSlot P = gs_load_slot_if(n2, I.occ, jl, c);
+    GsSlot Q = gs_load_slot_if(n3, I.occ, je, c);
+    E = gs_slot_sel(one, A, E);
+    P = gs_slot_sel(jL, A, gs_slot_sel(jE, E, P));
+    Q = gs_slot_sel(kL, A, gs_slot_sel(kE, E, gs_slot_sel(kJ, P, Q)));
+    if (COUNT) {
+        touch.blocks = (int)n0 + (int)n1 + (int)n2 + (int)n3;
+        touch.jblocks = (int)n2 + (int)n3;
+        touch.lines256 = gs_distinct4(e >> 8, doI, l >> 8, doI, je >> 8, jn, jl >> 8, jn);
+        touch.lines384 = gs_distinct4(e / 384u, doI, l / 384u, doI, je / 384u, jn, jl / 384u, jn);
     }
-    if (doI) {
-        l = base + ol + 1u;
-        u = base + ou;
-    }
-    const bool vu = doI && !uf, vl = doI && !lz, vju = jn && !juf, vjl = jn && !jlz;
-    touch.jblocks = (int)n2 + (int)n3;
-    touch.lines256 = gs_distinct4(ua >> 8, vu, la >> 8, vl, jua >> 8, vju, jla >> 8, vjl);
-    touch.lines384 = gs_distinct4(ua / 384u, vu, la / 384u, vl, jua / 384u, vju, jla / 384u, vjl);
-    return (int)n0 + (int)n1 + (int)n2 + (int)n3;
+    const uint32_t nl = gs_slot_rank(A, l), ne = gs_slot_rank(E, e);
+    const uint32_t njl = gs_slot_rank(P, jl), nje = gs_slot_rank(Q, je);
+    l = doI ? nl : l;
+    e = doI ? ne : e;
+    jl = jn ? njl : jl;
+    je = jn ? nje : je;
 }
 
-__device__ __forceinline__ int gs_step_pair(const GsDevIndex &I, uint32_t &l, uint32_t &u,
-                                            uint32_t &jl, uint32_t &ju, uint32_t c, bool doI)
+/* a whole block: every base's slot */
+struct GsBlk {
+    GsSlot s[4];
+};
+
+__device__ __forceinline__ GsBlk gs_load_block(const uint4 *occ, uint32_t row)
 {
-    GsStepTouch t;
-    return gs_step_pair(I, l, u, jl, ju, c, doI, t);
+    GsBlk b;
+    const char *p = (const char *)occ + (size_t)(row & ~63u);
+    uint32_t z0, z1;
+    asm("ld.global.nc.L2::64B.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(b.s[0].cnt), "=r"(b.s[0].m0), "=r"(b.s[0].m1), "=r"(z0), "=r"(b.s[1].cnt),
+          "=r"(b.s[1].m0), "=r"(b.s[1].m1), "=r"(z1)
+        : "l"(p));
+    asm("ld.global.nc.L2::64B.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(b.s[2].cnt), "=r"(b.s[2].m0), "=r"(b.s[2].m1), "=r"(z0), "=r"(b.s[3].cnt),
+          "=r"(b.s[3].m0), "=r"(b.s[3].m1), "=r"(z1)
+        : "l"(p + 32));
+    return b;
+}
+
+/* the base of a row that is not the $ row, given its block */
+__device__ __forceinline__ uint32_t gs_block_base(const GsBlk &b, uint32_t row)
+{
+    const uint32_t sh = row & 31u;
+    const bool hi = (row & 32u) != 0;
+    const uint32_t m1 = hi ? b.s[1].m1 : b.s[1].m0, m2 = hi ? b.s[2].m1 : b.s[2].m0,
+                   m3 = hi ? b.s[3].m1 : b.s[3].m0;
+    return (((m1 | m3) >> sh) & 1u) | ((((m2 | m3) >> sh) & 1u) << 1);
+}
+
+/* LF of a row whose base is c, given its block */
+__device__ __forceinline__ uint32_t gs_block_lf(const GsBlk &b, uint32_t row, uint32_t c)
+{
+    GsSlot s;
+    s.cnt = gs_sel4(c, b.s[0].cnt, b.s[1].cnt, b.s[2].cnt, b.s[3].cnt);
+    s.m0 = gs_sel4(c, b.s[0].m0, b.s[1].m0, b.s[2].m0, b.s[3].m0);
+    s.m1 = gs_sel4(c, b.s[0].m1, b.s[1].m1, b.s[2].m1, b.s[3].m1);
+    return gs_slot_rank(s, row);
 }
 
 /* LF of a BWT row (bwt_inv_psi_gpu, seed_gen.cu:455-484).  lf_mode
@@ -257,11 +215,9 @@ __device__ __forceinline__ int gs_step_pair(const GsDevIndex &I, uint32_t &l, ui
 __device__ __forceinline__ uint32_t gs_lf(const GsDevIndex &I, uint32_t k, int lf_mode)
 {
     if (k == I.primary) return 0;
-    uint32_t ka = k - ((k > I.primary) ? 1u : 0u);
-    if (lf_mode == GS_LF_GPUSEED && ka == I.primary) return 0;
-    GsBlk B = gs_load_block(I.occ, ka >> 6);
-    uint32_t c = gs_block_base(B, ka);
-    return gs_L2(I, c) + gs_occ_in_block(B, ka, c);
+    if (lf_mode == GS_LF_GPUSEED && k == I.primary + 1u) return 0;
+    const GsBlk B = gs_load_block(I.occ, k);
+    return gs_block_lf(B, k, gs_block_base(B, k));
 }
 
 #endif

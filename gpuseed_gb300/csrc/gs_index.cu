@@ -5,8 +5,8 @@
  * seed_gen.cu:2685-2736) with the same header checks, but reports failures as
  * GS_E* codes instead of exit(1) (:2692-2707, :2720-2724), and checks that
  * the .bwt holds every occurrence block seq_len needs (the reference does
- * not).  On the device the blocks are padded to whole 32-byte blocks so that
- * every lookup is a single aligned 256-bit load, the sampled SA gets its
+ * not).  On the device the blocks become 64-byte blocks with a slot per base
+ * (gs_fm.cuh), the sampled SA gets its
  * sa[0] = -1 sentinel (:2711) and the 13-mer table is built in HBM
  * (:2888-2895).
  */
@@ -18,7 +18,7 @@
 struct gs_index {
     int device;
     GsDevIndex dev;
-    uint32_t *d_occ;
+    uint4 *d_occ;
     uint32_t *d_sa;
     uint2 *d_kmer;
     uint4 *d_kmerx;
@@ -69,11 +69,10 @@ __global__ void gs_text_chain_kernel(GsDevIndex I, uint32_t *saf, uint8_t *t8, u
                 if (row != I.primary || s != 0) atomicAdd(&stat[1], 1ull);
                 break;
             }
-            const uint32_t ka = row - (row > I.primary ? 1u : 0u);
-            const GsBlk B = gs_load_block(I.occ, ka >> 6);
-            const uint32_t c = gs_block_base(B, ka);
+            const GsBlk B = gs_load_block(I.occ, row);
+            const uint32_t c = gs_block_base(B, row);
             t8[s - 1] = (uint8_t)c;
-            row = gs_L2(I, c) + gs_occ_in_block(B, ka, c);
+            row = gs_block_lf(B, row, c);
             s--;
             if (row % I.sa_intv == 0) {
                 /* the next chain's sample must continue this one */
@@ -162,36 +161,41 @@ int gs_build_text(GsDevIndex &I, uint32_t *saf, uint32_t *text, uint32_t *isa, c
     return GS_OK;
 }
 
-/* Longer start table by reference length: one table entry per distinct
- * kx-mer the text can hold (4^kx around seq_len) */
-/* the 16 high (hi) or low bits of a word of 16 two-bit bases, first base
- * (bits 30-31) at bit 15 */
-__device__ __forceinline__ uint32_t gs_slice16(uint32_t w, bool hi)
-{
-    uint32_t x = (hi ? w >> 1 : w) & 0x55555555u;
-    x = (x | (x >> 1)) & 0x33333333u;
-    x = (x | (x >> 2)) & 0x0f0f0f0fu;
-    x = (x | (x >> 4)) & 0x00ff00ffu;
-    return (x | (x >> 8)) & 0x0000ffffu;
-}
-
-/* The file's base words of each block (16 two-bit bases per word, first
- * base in the top bits, seed_gen.cu:52-58) become the bit-sliced words the
- * kernels read (gs_fm.cuh): H0, H1 = high bits of bases 0-31, 32-63, L0, L1
- * = low bits, base i at bit 31 - (i & 31).  The counts stay. */
-__global__ void gs_bitslice_kernel(uint32_t *occ, uint64_t nblk)
+/* The file's blocks (four checkpoint counts and 64 two-bit bases of the
+ * $-removed string, 16 per word, first base in the top bits,
+ * seed_gen.cu:52-58) become the blocks the kernels read (gs_fm.cuh), 64 rows
+ * of the BWT with its $ row.  Past the $ row, row r holds base r - 1 of the
+ * string, so a block starts with the last base of the file block before its
+ * own, and that base is taken back from its checkpoint.  Blocks that start
+ * at or past seq_len have no checkpoint of their own: the totals. */
+__global__ void gs_occ_kernel(const uint32_t *file, uint4 *occ, uint64_t nblk, uint32_t primary,
+                              uint4 L2, uint32_t seq_len)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t total[4] = {L2.x, L2.y - L2.x, L2.z - L2.y, L2.w - L2.z};
+    const uint32_t base[4] = {0u, L2.x, L2.y, L2.z};
     for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblk; b += stride) {
-        uint32_t *p = occ + b * GS_BLOCK_WORDS + 4;
-        const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3];
-        p[0] = (gs_slice16(w0, true) << 16) | gs_slice16(w1, true);
-        p[1] = (gs_slice16(w2, true) << 16) | gs_slice16(w3, true);
-        p[2] = (gs_slice16(w0, false) << 16) | gs_slice16(w1, false);
-        p[3] = (gs_slice16(w2, false) << 16) | gs_slice16(w3, false);
+        const uint64_t r0 = b * 64;
+        uint32_t cnt[4];
+        uint64_t m[4] = {0ull, 0ull, 0ull, 0ull};
+        for (int c = 0; c < 4; c++) cnt[c] = r0 < seq_len ? file[b * GS_BLOCK_WORDS + c] : total[c];
+        for (uint32_t i = 0; i < 64; i++) {
+            const uint64_t r = r0 + i;
+            if (r == primary || r > seq_len) continue;
+            const uint64_t s = r - (r > primary ? 1u : 0u);   /* place in the $-removed string */
+            const uint32_t w = file[(s >> 6) * GS_BLOCK_WORDS + 4 + ((s & 63u) >> 4)];
+            const uint32_t c = (w >> ((15u - (uint32_t)(s & 15u)) * 2u)) & 3u;
+            for (uint32_t q = 0; q < 4; q++) m[q] |= (uint64_t)(c == q) << i;
+            if (i == 0 && s < r0)
+                for (uint32_t q = 0; q < 4; q++) cnt[q] -= c == q;
+        }
+        for (int c = 0; c < 4; c++)
+            occ[b * 4 + c] = make_uint4(base[c] + 1u + cnt[c], (uint32_t)m[c], (uint32_t)(m[c] >> 32), 0u);
     }
 }
 
+/* Longer start table by reference length: one table entry per distinct
+ * kx-mer the text can hold (4^kx around seq_len) */
 static int auto_kmer_len(uint32_t seq_len)
 {
     if (seq_len > (1u << 30)) return 16;
@@ -244,8 +248,10 @@ static int upload(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *b
     gs_index *idx = (gs_index *)calloc(1, sizeof(gs_index));
     if (!idx) return GS_ENOMEM;
     idx->device = device;
-    uint64_t nblk = (uint64_t)seq_len / GS_OCC_INTERVAL + 2;
-    idx->occ_bytes = nblk * GS_BLOCK_WORDS * 4;
+    /* a step reads the block of one past its last row: up to row seq_len+1 */
+    const uint64_t nblk = ((uint64_t)seq_len + 1) / GS_OCC_INTERVAL + 1;
+    const uint64_t file_blk = (uint64_t)seq_len / GS_OCC_INTERVAL + 2;
+    idx->occ_bytes = nblk * 4 * sizeof(uint4);
     idx->sa_bytes = n_sa * 4;
     idx->kmer_bytes = (size_t)8 << (2 * GS_K0);
     cudaError_t e;
@@ -255,14 +261,22 @@ static int upload(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *b
         gs_index_free(idx);
         return gs_cuda_fail(e, "cudaMalloc(index)");
     }
-    uint64_t copy_words = bwt_words < nblk * GS_BLOCK_WORDS ? bwt_words : nblk * GS_BLOCK_WORDS;
-    if ((e = cudaMemset(idx->d_occ, 0, idx->occ_bytes)) != cudaSuccess ||
-        (e = cudaMemcpy(idx->d_occ, bwt, copy_words * 4, cudaMemcpyHostToDevice)) != cudaSuccess) {
+    const uint64_t file_words = file_blk * GS_BLOCK_WORDS;
+    const uint64_t copy_words = bwt_words < file_words ? bwt_words : file_words;
+    uint32_t *d_file = NULL;
+    if ((e = cudaMalloc(&d_file, file_words * 4)) != cudaSuccess ||
+        (e = cudaMemset(d_file, 0, file_words * 4)) != cudaSuccess ||
+        (e = cudaMemcpy(d_file, bwt, copy_words * 4, cudaMemcpyHostToDevice)) != cudaSuccess) {
+        cudaFree(d_file);
         gs_index_free(idx);
         return gs_cuda_fail(e, "index upload");
     }
-    gs_bitslice_kernel<<<152 * 8, 256>>>(idx->d_occ, nblk);
-    if ((e = cudaGetLastError()) != cudaSuccess) {
+    gs_occ_kernel<<<152 * 16, 256>>>(d_file, idx->d_occ, nblk, primary,
+                                     make_uint4(L2_1to4[0], L2_1to4[1], L2_1to4[2], L2_1to4[3]),
+                                     seq_len);
+    e = cudaGetLastError();
+    cudaFree(d_file);
+    if (e != cudaSuccess) {
         gs_index_free(idx);
         return gs_cuda_fail(e, "occurrence table layout");
     }

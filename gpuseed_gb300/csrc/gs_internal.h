@@ -11,7 +11,7 @@
 #include "../../include/gpuseed.h"
 
 #define GS_OCC_INTERVAL 64u   /* rows per occurrence block (seed_gen.cu:29) */
-#define GS_BLOCK_WORDS 8u     /* 4 counts + 4 bit-slice words of 64 bases = 32 bytes */
+#define GS_BLOCK_WORDS 8u     /* file block: 4 counts + 4 words of 16 bases = 32 bytes */
 #define GS_K0 13              /* k-mer table length (seed_gen.cu:2822) */
 #define GS_HIST 8             /* containment history depth of the batched search */
 #define GS_CHUNK 31           /* candidates owned by one warp work item */
@@ -22,10 +22,9 @@
 #define GS_QUEUE_CHUNK_MAX 16 /* batched start pass: most work items per queue grab */
 
 /* Device view of the index, passed by value to every kernel.
- * occ: one 32-byte block per 64 rows of the $-removed BWT string:
- *      {count of A, C, G, T before the block, H0, H1, L0, L1}: the high and
- *      low bits of the block's 64 bases, base i at bit 31 - (i & 31) of
- *      word i >> 5 (gs_fm.cuh).
+ * occ: one 64-byte block per 64 rows of the BWT: for each base a slot {L2[c]
+ *      + 1 + its count before the block, the mask of the block's rows that
+ *      hold it (2 words), 0} (gs_fm.cuh).
  * sa:  sampled suffix array, sa[0] = 0xffffffff (the $ row).
  * kmer: (l,u) of every 13-mer, base j at bits 2j, processed first.
  * Optional text structures, all built from occ and sa in HBM:
@@ -45,7 +44,7 @@
 #define GS_TEXT_MARK 0xf0000000u     /* jl of a text-mode walker */
 #define GS_REGIME_MARK 0xe0000000u   /* jl (+ steps) of a one-row walker without J */
 struct GsDevIndex {
-    const uint32_t *occ;
+    const uint4 *occ;
     const uint32_t *sa;
     const uint2 *kmer;
     const uint4 *kmerx;        /* optional table of all kx-mers, same bit order: x,y the

@@ -166,19 +166,17 @@ __global__ void gs_kmerx_pack_kernel(GsDevIndex I, uint4 *table, uint64_t n, con
             for (uint32_t i = 0; i < size; i++) {
                 const uint32_t row = e.x + i;
                 if (row == I.primary) continue;   /* the text starts with X */
-                const uint32_t ka = row - (row > I.primary ? 1u : 0u);
-                if ((ka >> 6) != at) {
-                    at = ka >> 6;
-                    B = gs_load_block(I.occ, at);
+                if ((row >> 6) != at) {
+                    at = row >> 6;
+                    B = gs_load_block(I.occ, row);
                 }
-                const uint32_t c = gs_block_base(B, ka);
+                const uint32_t c = gs_block_base(B, row);
                 multi |= seen & (1u << c);
                 seen |= 1u << c;
-                const uint32_t prev = gs_L2(I, c) + gs_occ_in_block(B, ka, c);
+                const uint32_t prev = gs_block_lf(B, row, c);
                 if (prev == I.primary) continue;   /* ... with cX */
-                const uint32_t kp = prev - (prev > I.primary ? 1u : 0u);
-                const GsBlk P = gs_load_block(I.occ, kp >> 6);
-                two |= 1u << (4u * c + gs_block_base(P, kp));
+                const GsBlk P = gs_load_block(I.occ, prev);
+                two |= 1u << (4u * c + gs_block_base(P, prev));
             }
             y = code[X] | GS_ENTRY_EXT | (size << 4) | ((seen & ~multi) << 12) | (two << 16);
         }
@@ -1008,11 +1006,13 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
         }
         /* settle over a wildcard: J unchanged */
     } else {
-        uint32_t nl = l, nu = u;
+        uint32_t nl = l, ne = u + 1u, je = ju + 1u;
         const bool had_j = jl <= ju;
         GsStepTouch touch;
-        int blocks = gs_step_pair(I, nl, nu, jl, ju, c, !settle, touch);
-        if (COUNT) wb += (unsigned long long)blocks;
+        gs_step_pair<COUNT>(I, nl, ne, jl, je, c, !settle, touch);
+        const uint32_t nu = ne - 1u;
+        ju = je - 1u;
+        if (COUNT) wb += (unsigned long long)touch.blocks;
         if (COUNT && wc) {
             wc->steps++;
             wc->lines256 += (unsigned long long)touch.lines256;
