@@ -559,6 +559,8 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
         const uint64_t per16 = p->walker_slots ? (uint64_t)p->walker_slots : c->walker_per16;
         const uint64_t units = (uint64_t)n_items * (B.paired ? 2u : 1u);
         uint64_t want = (units * per16 + 15u) / 16u + 32u;
+        /* a start-pass warp reserves 64 entries or more at a time */
+        if (!p->walker_slots) want += 64ull * (n_items < 8192u ? n_items : 8192u);
         if (want > (1ull << 31)) want = 1ull << 31;   /* 32-bit buffer counter */
         RC(grow(c->walkers, c->cap_walkers, (size_t)want, c->st));
         B.walkers = c->walkers;
@@ -651,7 +653,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     GS_CUDA(cudaEventRecord(c->ev1, st));
     RC(fetch_small(&c->h_small[5], c->queue + 1, 4, st));
     RC(fetch_small(&c->h_small[10], c->queue + 2, 4, st));
-    RC(fetch_small(&c->h_small[11], c->queue + 4, 4, st));
+    RC(fetch_small(&c->h_small[11], c->queue + 5, 4, st));
     if (B.work) RC(fetch_small(&c->h_small[6], c->d_work, 32, st));
     if (B.work) RC(fetch_small(&c->h_small[16], c->d_work + 4, 56, st));
     if (co) {

@@ -112,7 +112,8 @@ struct GsBatch {
     uint64_t cont_cap;             /* hand-over records allocated */
     uint32_t *queue;           /* [0]: work-queue head, [1]: status flags,
                                   [2]: hand-over count, [3]: tail-pass head,
-                                  [4]: text jobs queued (8 words, zeroed per pass) */
+                                  [4]: text-job entries reserved, [5]: text jobs in them
+                                  (8 words, zeroed per pass) */
     unsigned long long *work;  /* NULL or [kmer, occ blocks, lf steps, sa samples] */
     GsCont *cont;              /* NULL: no hand-over; else n_items * handoff_lanes entries */
     int32_t handoff_lanes;     /* hand over when at most this many owned lanes extend ... */
@@ -125,6 +126,7 @@ struct GsBatch {
     GsWalker *walkers;         /* batched search: survivors of the start pass */
     uint64_t walker_cap;       /* entries allocated (0: every walk is left to the leftover pass) */
     uint32_t walker_chunk;     /* entries a start-pass warp reserves at a time */
+    uint32_t text_chunk;       /* text jobs a walk-pass warp reserves at a time */
     struct GsTextJob *text_jobs;   /* walkers handed to the text pass */
     uint64_t text_cap;         /* entries allocated (0: text mode stays inline) */
 };

@@ -799,23 +799,32 @@ __global__ void __launch_bounds__(256, 5) gs_search_lockstep(GsDevIndex I, GsBat
 #define GS_WALKER_FWD 0x80000000u
 #define GS_WALKER_CHUNK 512u      /* most buffer entries a warp reserves at a time */
 
-/* entries a start-pass warp reserves at a time (gs_launch_batched sets it) */
+/* entries a start-pass warp reserves at a time (gs_launch_batched sets it):
+ * at least an item's walkers, 2 * GS_PCHUNK */
 __device__ __forceinline__ uint32_t gs_walker_chunk(const GsBatch &B)
 {
     return B.walker_chunk;
 }
 
 /* Sizes from the walker buffer's capacity and a grid of `warps` warps,
- * multiples of 32 from 32 to `most`: about 1/`parts` of a warp's share, so
+ * multiples of 32 from `least` to `most`: about 1/`parts` of a warp's share, so
  * that a small batch's buffer (start reservations) or walkers (walk-pass
  * windows) spread over every warp */
-static uint32_t gs_share_size(uint64_t cap, uint32_t warps, uint32_t parts, uint32_t most)
+static uint32_t gs_share_size(uint64_t cap, uint32_t warps, uint32_t parts, uint32_t least,
+                              uint32_t most)
 {
     uint64_t v = cap / ((uint64_t)warps * parts);
     v &= ~31ull;
-    if (v < 32u) v = 32u;
+    if (v < least) v = least;
     if (v > most) v = most;
     return (uint32_t)v;
+}
+/* entries of a list that a walk-pass warp reserves at a time: an eighth of
+ * its share of the capacity, 1 to 32 */
+static uint32_t gs_list_chunk(uint64_t cap, uint32_t warps)
+{
+    const uint64_t v = cap / ((uint64_t)warps * 8u);
+    return v < 1u ? 1u : v > 32u ? 32u : (uint32_t)v;
 }
 #define GS_WALK_WINDOW 512u       /* most buffer entries a walk-pass warp takes at a time */
 
@@ -1410,18 +1419,61 @@ __global__ void __launch_bounds__(256, 5) gs_search_start(GsDevIndex I, GsBatch 
     if (COUNT) gs_add_work(B, wk, wb);
 }
 
-template <int NSTOP, int COUNT>
-__global__ void __launch_bounds__(128, 8) gs_search_walk(GsDevIndex I, GsBatch B, uint32_t wsz)
+#define GS_WALK_WARPS 4
+
+/* A warp's part [next, end) of a list that all warps append to, in shared
+ * memory; full once the list gave no more room (no further atomics, so that
+ * the 32-bit counter cannot wrap) */
+struct GsListPart {
+    uint32_t next, end, full, used;
+};
+
+/* Places for the lanes of m in a list of `cap` entries with counter *count
+ * (at or past cap: no room): the rest of the warp's part, then a new part of
+ * `chunk` entries or more -- one atomic a part instead of one a push, on an
+ * address that every warp of the grid takes turns at. */
+__device__ __forceinline__ uint32_t gs_list_room(GsListPart &part, uint32_t *count, uint32_t chunk,
+                                                 uint32_t cap, uint32_t m, int lane)
 {
+    const uint32_t cnt = (uint32_t)__popc(m), rank = (uint32_t)__popc(m & ((1u << lane) - 1u));
+    const uint32_t at = part.next, rem = part.end - at, full = part.full;
+    __syncwarp();
+    uint32_t g = cap;
+    if (rem < cnt && !full) {
+        const uint32_t take = max(chunk, cnt - rem);
+        if (lane == 0) g = atomicAdd(count, take);
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (lane == 0) {
+            part.full = (uint64_t)g + take >= cap;
+            part.next = (uint32_t)min((uint64_t)g + (cnt - rem), (uint64_t)cap);
+            part.end = (uint32_t)min((uint64_t)g + take, (uint64_t)cap);
+        }
+    } else if (lane == 0) {
+        part.next = rem < cnt ? part.end : at + cnt;
+    }
+    __syncwarp();
+    const uint64_t j = rank < rem ? (uint64_t)at + rank : (uint64_t)g + (rank - rem);
+    return (uint32_t)min(j, (uint64_t)cap);
+}
+
+template <int NSTOP, int COUNT>
+__global__ void __launch_bounds__(GS_WALK_WARPS * 32, 8) gs_search_walk(GsDevIndex I, GsBatch B, uint32_t wsz)
+{
+    __shared__ GsListPart s_text[GS_WALK_WARPS];
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
+    GsListPart &text = s_text[threadIdx.x >> 5];
+    if (lane == 0) {
+        text.next = text.end = text.used = 0u;
+        text.full = B.text_cap == 0;
+    }
+    __syncwarp();
     unsigned long long wb = 0;
     /* walker indices fit 32 bits: the buffer holds at most 2^31 entries */
     uint32_t n_w = *(volatile uint32_t *)(B.queue + 2);
     if (n_w > B.walker_cap) n_w = (uint32_t)B.walker_cap;
     uint32_t win = 0, win_end = 0;   /* warp-uniform window of walker indices */
     bool have = false, exhausted = false, killed = false, jpend = false;
-    bool tfull = B.text_cap == 0;   /* warp-uniform: the text-job buffer is full */
     uint32_t r = 0, l = 0, u = 0, jl = 0, ju = 0, n = 0;
     int anchor = 0, pos = 0, iL = 0, dir = 0;
     bool fwd = false;
@@ -1483,22 +1535,17 @@ __global__ void __launch_bounds__(128, 8) gs_search_walk(GsDevIndex I, GsBatch B
         const bool tx = have && jl >= GS_TEXT_MARK;
         const uint32_t tm = __ballot_sync(0xffffffffu, tx);
         if (tm) {
-            uint32_t g = 0xffffffffu;
-            if (!tfull) {
-                const int lead = __ffs(tm) - 1;
-                if (lane == lead) g = atomicAdd(B.queue + 4, (uint32_t)__popc(tm));
-                g = __shfl_sync(0xffffffffu, g, lead);
-                if ((uint64_t)g + __popc(tm) > B.text_cap) tfull = true;
-            }
-            const uint64_t idx = (uint64_t)g + __popc(tm & lt);
+            const uint32_t cap = (uint32_t)B.text_cap;
+            const uint32_t j = gs_list_room(text, B.queue + 4, B.text_chunk, cap, tm, lane);
             if (tx) {
-                if (g != 0xffffffffu && idx < B.text_cap) {
+                if (j < cap) {
+                    atomicAdd(&text.used, 1u);
                     GsTextJob t;
                     t.r = r;
                     t.anchor = (uint32_t)anchor | (fwd ? GS_WALKER_FWD : 0u);
                     t.pos = (uint32_t)pos;
                     t.l = l;
-                    B.text_jobs[idx] = t;
+                    B.text_jobs[j] = t;
                     have = false;
                 } else {
                     jl = 1u;
@@ -1507,6 +1554,11 @@ __global__ void __launch_bounds__(128, 8) gs_search_walk(GsDevIndex I, GsBatch B
             }
         }
     }
+    /* what the warp reserved and did not fill */
+    __syncwarp();
+    for (uint32_t j = text.next + (uint32_t)lane; j < text.end; j += 32)
+        B.text_jobs[j].r = GS_WALKER_HOLE;
+    if (lane == 0 && text.used) atomicAdd(B.queue + 5, text.used);
     if (COUNT) {
         gs_add_work(B, 0, wb);
         unsigned long long v[7] = {wc.steps, wc.jsteps, wc.jblocks, wc.jshrank, wc.jwalkers,
@@ -1531,6 +1583,7 @@ __global__ void __launch_bounds__(256) gs_search_text(GsDevIndex I, GsBatch B)
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_jobs; j += stride) {
         const GsTextJob t = B.text_jobs[j];
         const uint32_t r = t.r;
+        if (r == GS_WALKER_HOLE) continue;
         const bool fwd = (t.anchor & GS_WALKER_FWD) != 0;
         const int anchor = (int)(t.anchor & ~GS_WALKER_FWD);
         const int dir = fwd ? -1 : 1;
@@ -1738,16 +1791,18 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
     GS_CUDA(cudaGetLastError());
     GS_CUDA(cudaMemsetAsync(B.queue, 0, sizeof(uint32_t), st));
     GS_CUDA(cudaMemsetAsync(B.queue + 2, 0, 2 * sizeof(uint32_t), st));
-    B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, GS_WALKER_CHUNK);
+    B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, 64u, GS_WALKER_CHUNK);
     start<<<grid, 256, 0, st>>>(I, B, queue_chunk);
     GS_CUDA(cudaGetLastError());
     if (B.walker_cap) {
         int wocc = 0;
-        GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wocc, walk, 128, 0));
+        GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wocc, walk, GS_WALK_WARPS * 32, 0));
         const uint32_t wgrid = (uint32_t)sms * (uint32_t)(wocc > 0 ? wocc : 4);
         /* the buffer's capacity stands for its walkers (the count is on the
          * device): about an eighth of a warp's share a window */
-        walk<<<wgrid, 128, 0, st>>>(I, B, gs_share_size(B.walker_cap, wgrid * 4u, 8u, GS_WALK_WINDOW));
+        B.text_chunk = gs_list_chunk(B.text_cap, wgrid * GS_WALK_WARPS);
+        walk<<<wgrid, GS_WALK_WARPS * 32, 0, st>>>(
+            I, B, gs_share_size(B.walker_cap, wgrid * GS_WALK_WARPS, 8u, 32u, GS_WALK_WINDOW));
         GS_CUDA(cudaGetLastError());
         if (B.text_cap) {
             void (*text)(GsDevIndex, GsBatch) =
