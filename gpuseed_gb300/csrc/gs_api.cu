@@ -189,7 +189,8 @@ struct gs_ctx {
     char *h_text[2];            /* pinned copy-out buffers */
     cudaEvent_t t_ev[2];
     uint64_t last_walkers, last_walker_cap;
-    uint32_t walker_per16;      /* automatic walker-buffer size, per 16 work items */
+    uint32_t walker_per16;      /* walker-buffer size per 16 work items, once a pass filled
+                                   the automatic one (0: not yet) */
     uint32_t *queue;
     uint64_t *d_max;
     unsigned long long *d_work;
@@ -555,8 +556,9 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
          * windows counts as two): as asked, or automatic -- 16 per item
          * with a start table (forced codes settle most candidates), all 31
          * without, and 1.5x more after a pass that filled its buffer */
-        if (!c->walker_per16) c->walker_per16 = I.kx > GS_K0 ? 256u : 512u;
-        const uint64_t per16 = p->walker_slots ? (uint64_t)p->walker_slots : c->walker_per16;
+        const uint32_t least = B.paired ? 256u : 512u;
+        uint64_t per16 = p->walker_slots ? (uint64_t)p->walker_slots : least;
+        if (!p->walker_slots && c->walker_per16 > per16) per16 = c->walker_per16;
         const uint64_t units = (uint64_t)n_items * (B.paired ? 2u : 1u);
         uint64_t want = (units * per16 + 15u) / 16u + 32u;
         /* a start-pass warp reserves 64 entries or more at a time */
@@ -687,7 +689,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     c->last_text_jobs = c->last_text_cap ? (c->h_small[11] & 0xffffffffu) : 0;
     if (!p->walker_slots && c->last_walker_cap && c->last_walkers >= c->last_walker_cap &&
         c->walker_per16 < 512u) {
-        c->walker_per16 += c->walker_per16 / 2;
+        c->walker_per16 = c->walker_per16 ? c->walker_per16 + c->walker_per16 / 2 : 384u;
         if (c->walker_per16 > 512u) c->walker_per16 = 512u;
     }
     if (B.work) memcpy(c->work, &c->h_small[6], sizeof(c->work));

@@ -303,8 +303,8 @@ static int upload(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *b
         gs_index_free(idx);
         return rc;
     }
-    /* the longer table is an accelerator: without room for it, run without */
-    for (int kx = auto_kmer_len(seq_len); kx > GS_K0; kx--)
+    /* the start table is an accelerator: without room for it, run without */
+    for (int kx = auto_kmer_len(seq_len); kx >= GS_K0; kx--)
         if (gs_index_set_kmer_len(idx, kx) == GS_OK) break;
     cudaGetLastError();
     *out = idx;
@@ -547,10 +547,14 @@ extern "C" int gs_index_set_kmer_len(gs_index *idx, int kx)
     }
     idx->dev.kmerx = NULL;
     idx->dev.kx = 0;
-    if (kx == GS_K0) return GS_OK;
     size_t bytes = (size_t)16 << (2 * kx);
     uint4 *t = NULL;
     cudaError_t e = cudaMalloc(&t, bytes);
+    if (e == cudaErrorMemoryAllocation && kx == GS_K0) {
+        /* the 13-mer table alone serves every kernel */
+        cudaGetLastError();
+        return GS_OK;
+    }
     if (e != cudaSuccess) return gs_cuda_fail(e, "cudaMalloc(k-mer start table)");
     int rc = gs_build_kmerx_table(idx->dev, t, kx, 0);
     if (rc == GS_OK && (e = cudaDeviceSynchronize()) != cudaSuccess) rc = gs_cuda_fail(e, "k-mer table");

@@ -47,12 +47,12 @@ struct GsDevIndex {
     const uint4 *occ;
     const uint32_t *sa;
     const uint2 *kmer;
-    const uint4 *kmerx;        /* optional table of all kx-mers, same bit order: x,y the
+    const uint4 *kmerx;        /* paired table of all kx-mers, same bit order (or NULL): x,y the
                                 * packed entry of X, z,w that of X's reverse complement */
     const uint32_t *saf;
     const uint32_t *text;
     const uint32_t *isa;
-    int32_t kx;                /* 14..16, or 0 when there is no longer table */
+    int32_t kx;                /* 13..16, or 0 when there is no paired table */
     uint32_t primary, seq_len, sa_intv, n_sa;
     uint32_t L2[5];
     uint32_t quirk_lo, quirk_n;

@@ -34,27 +34,51 @@
 /* ------------------------------------------------------------------ */
 /* 13-mer interval table (pre_calc_seed_intervals_gpu, seed_gen.cu:2648) */
 
-__global__ void gs_kmer_kernel(GsDevIndex I, uint2 *table, uint32_t n)
+/* The intervals of all strings of LV more bases than one whose interval is
+ * [l,u], each from the string one base shorter: an absent string keeps the
+ * empty interval at which it ended.  put(ext, l, u) gets each, the base
+ * processed first at bits 0-1 of ext. */
+template <int LV, class F>
+__device__ __forceinline__ void gs_kmer_expand(const GsDevIndex &I, uint32_t l, uint32_t u, int at,
+                                               uint32_t ext, const F &put)
 {
-    uint32_t patt = blockIdx.x * blockDim.x + threadIdx.x;
-    if (patt >= n) return;
+    if constexpr (LV == 0) {
+        put(ext, l, u);
+    } else {
+        for (uint32_t c = 0; c < 4; c++) {
+            uint32_t cl = l, cu = u;
+            if (l <= u) gs_step(I, cl, cu, c);
+            gs_kmer_expand<LV - 1>(I, cl, cu, at + 1, ext | (c << (2 * at)), put);
+        }
+    }
+}
+
+/* A thread per 10-mer: its interval, then its 64 13-mers, 94 steps instead
+ * of 13 for each (loading a 400 Mbp index, with its 15-mer table made the
+ * same way: 139 -> 102 ms) */
+__global__ void __launch_bounds__(256) gs_kmer_kernel(GsDevIndex I, uint2 *table)
+{
+    const int head = GS_K0 - 3;
+    const uint32_t patt = blockIdx.x * blockDim.x + threadIdx.x;
+    if (patt >= (1u << (2 * head))) return;
     uint32_t l = 0, u = I.seq_len;
-    for (int i = 0; i < GS_K0; i++) {
+    for (int i = 0; i < head; i++) {
         gs_step(I, l, u, (patt >> (i << 1)) & 3u);
         if (l > u) break;
     }
-    table[patt] = make_uint2(l, u);
+    gs_kmer_expand<3>(I, l, u, 0, 0u, [&](uint32_t ext, uint32_t cl, uint32_t cu) {
+        table[patt | (ext << (2 * head))] = make_uint2(cl, cu);
+    });
 }
 
 int gs_build_kmer_table(const GsDevIndex &I, uint2 *table, cudaStream_t st)
 {
-    uint32_t n = 1u << (2 * GS_K0);
-    gs_kmer_kernel<<<(n + 255) / 256, 256, 0, st>>>(I, table, n);
+    gs_kmer_kernel<<<(1u << (2 * (GS_K0 - 3))) / 256, 256, 0, st>>>(I, table);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }
 
-/* Longer start table, built in four passes over all kx-mers (base j at
+/* Start table, built in four passes over all kx-mers (base j at
  * bits 2j, processed first, i.e. the string's last character sits at bits
  * 0-1):
  *   1. (l,u) from the 13-mer prefix interval plus kx-13 steps;
@@ -82,42 +106,46 @@ __device__ __forceinline__ uint32_t gs_kmer_rc(uint32_t X, int kx)
     return (((b >> 1) & 0x55555555u) | ((b & 0x55555555u) << 1)) >> (32 - 2 * kx);
 }
 
-__global__ void gs_kmerx_kernel(GsDevIndex I, uint4 *table, int kx, uint64_t n)
+/* a thread per 13-mer: the intervals of its 4^(kx-13) kx-mers */
+template <int LV>
+__global__ void __launch_bounds__(256) gs_kmerx_kernel(GsDevIndex I, uint4 *table)
 {
-    for (uint64_t patt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; patt < n;
-         patt += (uint64_t)gridDim.x * blockDim.x) {
-        uint2 iv = __ldg(&I.kmer[patt & ((1u << (2 * GS_K0)) - 1u)]);
-        uint32_t l = iv.x, u = iv.y;
-        for (int i = GS_K0; i < kx && l <= u; i++) gs_step(I, l, u, (uint32_t)(patt >> (i << 1)) & 3u);
-        table[patt] = make_uint4(l, u, 0u, 0u);
+    const uint32_t patt = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint2 iv = __ldg(&I.kmer[patt]);
+    gs_kmer_expand<LV>(I, iv.x, iv.y, 0, 0u, [&](uint32_t ext, uint32_t l, uint32_t u) {
+        table[patt | ((uint64_t)ext << (2 * GS_K0))] = make_uint4(l, u, 0u, 0u);
+    });
+}
+
+/* The forced base of X = [l,u] (pass 2): c with count(Xc) == count(X) > 0, or
+ * 4.  raw(Y): the interval of a kx-mer. */
+template <class F>
+__device__ __forceinline__ uint32_t gs_forced_base(const GsDevIndex &I, uint64_t X, int kx, uint32_t l,
+                                                   uint32_t u, const F &raw)
+{
+    if (l > u) return 4u;
+    const uint64_t mask = (1ull << (2 * kx)) - 1u;
+    const uint32_t size = u - l + 1u, first = (uint32_t)(X >> (2 * (kx - 1))) & 3u;   /* X's first character */
+    for (uint32_t c = 0; c < 4; c++) {
+        uint2 y = raw(((X << 2) | c) & mask);
+        /* as many rows as X's at most come before the step */
+        if (y.x > y.y || y.y - y.x + 1u < size) continue;
+        gs_step(I, y.x, y.y, first);
+        if (y.x <= y.y && y.y - y.x + 1u == size) return c;
     }
+    return 4u;
 }
 
 __global__ void gs_kmerx_code_kernel(GsDevIndex I, const uint4 *table, int kx, uint64_t n,
                                      uint8_t *code)
 {
-    const uint64_t mask = n - 1;
     for (uint64_t X = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; X < n;
          X += (uint64_t)gridDim.x * blockDim.x) {
-        const uint4 e4 = table[X];
-        const uint2 e = make_uint2(e4.x, e4.y);
-        uint8_t out = 4;
-        if (e.x <= e.y) {
-            uint32_t size = e.y - e.x + 1u;
-            uint32_t first = (uint32_t)(X >> (2 * (kx - 1))) & 3u;   /* X's first character */
-            for (uint32_t c = 0; c < 4; c++) {
-                const uint4 y4 = table[((X << 2) | c) & mask];
-                const uint2 y = make_uint2(y4.x, y4.y);
-                if (y.x > y.y) continue;
-                uint32_t l = y.x, u = y.y;
-                gs_step(I, l, u, first);
-                if (l <= u && u - l + 1u == size) {
-                    out = (uint8_t)c;
-                    break;
-                }
-            }
-        }
-        code[X] = out;
+        const uint4 e = table[X];
+        code[X] = (uint8_t)gs_forced_base(I, X, kx, e.x, e.y, [&](uint64_t Y) {
+            const uint4 y = table[Y];
+            return make_uint2(y.x, y.y);
+        });
     }
 }
 
@@ -146,42 +174,57 @@ __device__ __forceinline__ uint32_t gs_entry_size(uint32_t y)
     return (y & GS_ENTRY_EXT) ? (y >> 4) & 255u : y >> 4;
 }
 
-/* a thread per entry: rows l..u are read in order (their blocks, and those
- * of their LF rows, are shared by neighbouring entries, whose strings and
- * so whose rows are adjacent) */
+/* The second word of X = [l,u].  Rows l..u are read in order (their blocks,
+ * and those of their LF rows, are shared by neighbouring entries, whose
+ * strings and so whose rows are adjacent). */
+__device__ __forceinline__ uint32_t gs_entry_word(const GsDevIndex &I, uint32_t l, uint32_t u,
+                                                  uint32_t code)
+{
+    const uint32_t size = l <= u ? u - l + 1u : 0u;
+    if (size >= (1u << 28)) return 7u;
+    if (size > GS_EXT_ROWS) return code | (size << 4);
+    uint32_t seen = 0, multi = 0, two = 0, at = 0xffffffffu;
+    GsBlk B;
+    for (uint32_t i = 0; i < size; i++) {
+        const uint32_t row = l + i;
+        if (row == I.primary) continue;   /* the text starts with X */
+        if ((row >> 6) != at) {
+            at = row >> 6;
+            B = gs_load_block(I.occ, row);
+        }
+        const uint32_t c = gs_block_base(B, row);
+        multi |= seen & (1u << c);
+        seen |= 1u << c;
+        const uint32_t prev = gs_block_lf(B, row, c);
+        if (prev == I.primary) continue;   /* ... with cX */
+        const GsBlk P = gs_load_block(I.occ, prev);
+        two |= 1u << (4u * c + gs_block_base(P, prev));
+    }
+    return code | GS_ENTRY_EXT | (size << 4) | ((seen & ~multi) << 12) | (two << 16);
+}
+
 __global__ void gs_kmerx_pack_kernel(GsDevIndex I, uint4 *table, uint64_t n, const uint8_t *code)
 {
     for (uint64_t X = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; X < n;
          X += (uint64_t)gridDim.x * blockDim.x) {
         const uint4 e = table[X];
-        const uint32_t size = e.x <= e.y ? e.y - e.x + 1u : 0u;
-        uint32_t y;
-        if (size >= (1u << 28)) {
-            y = 7u;
-        } else if (size > GS_EXT_ROWS) {
-            y = code[X] | (size << 4);
-        } else {
-            uint32_t seen = 0, multi = 0, two = 0, at = 0xffffffffu;
-            GsBlk B;
-            for (uint32_t i = 0; i < size; i++) {
-                const uint32_t row = e.x + i;
-                if (row == I.primary) continue;   /* the text starts with X */
-                if ((row >> 6) != at) {
-                    at = row >> 6;
-                    B = gs_load_block(I.occ, row);
-                }
-                const uint32_t c = gs_block_base(B, row);
-                multi |= seen & (1u << c);
-                seen |= 1u << c;
-                const uint32_t prev = gs_block_lf(B, row, c);
-                if (prev == I.primary) continue;   /* ... with cX */
-                const GsBlk P = gs_load_block(I.occ, prev);
-                two |= 1u << (4u * c + gs_block_base(P, prev));
-            }
-            y = code[X] | GS_ENTRY_EXT | (size << 4) | ((seen & ~multi) << 12) | (two << 16);
-        }
-        table[X] = make_uint4(e.x, y, 0u, 0u);
+        table[X] = make_uint4(e.x, gs_entry_word(I, e.x, e.y, code[X]), 0u, 0u);
     }
+}
+
+/* Passes 1 to 3 at once for kx = 13, whose raw intervals are the 13-mer
+ * table's.  (Pass 4 follows.)  Texts of up to 2^26 bases start from this
+ * table: nearly every 13-mer of theirs is forced or dead at once, where the
+ * plain table left every candidate to the walk (10,000 reads on 1 Mbp, a
+ * replayed pass: 430 -> 373 us), for 1 GiB and about 2 ms at load. */
+__global__ void __launch_bounds__(256) gs_kmer13_entries_kernel(GsDevIndex I, uint4 *table)
+{
+    const uint32_t X = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint2 e = __ldg(&I.kmer[X]);
+    const uint32_t code = gs_forced_base(I, X, GS_K0, e.x, e.y,
+                                         [&](uint64_t Y) { return __ldg(&I.kmer[Y]); });
+    uint2 *w = reinterpret_cast<uint2 *>(table);
+    w[2 * (uint64_t)X] = make_uint2(e.x, gs_entry_word(I, e.x, e.y, code));
 }
 
 /* pass 4: each entry's second half from the packed first half of its
@@ -198,8 +241,19 @@ __global__ void gs_kmerx_pair_kernel(uint4 *table, int kx, uint64_t n)
 
 int gs_build_kmerx_table(const GsDevIndex &I, uint4 *table, int kx, cudaStream_t st)
 {
-    uint64_t n = 1ull << (2 * kx);
-    gs_kmerx_kernel<<<152 * 64, 256, 0, st>>>(I, table, kx, n);
+    const uint64_t n = 1ull << (2 * kx);
+    const uint32_t n13 = 1u << (2 * GS_K0);
+    if (kx == GS_K0) {
+        gs_kmer13_entries_kernel<<<n13 / 256, 256, 0, st>>>(I, table);
+        GS_CUDA(cudaGetLastError());
+        gs_kmerx_pair_kernel<<<152 * 64, 256, 0, st>>>(table, kx, n);
+        GS_CUDA(cudaGetLastError());
+        return GS_OK;
+    }
+    void (*expand)(GsDevIndex, uint4 *) = kx == 14   ? gs_kmerx_kernel<1>
+                                          : kx == 15 ? gs_kmerx_kernel<2>
+                                                     : gs_kmerx_kernel<3>;
+    expand<<<n13 / 256, 256, 0, st>>>(I, table);
     GS_CUDA(cudaGetLastError());
     uint8_t *code = NULL;
     GS_CUDA(cudaMallocAsync(&code, n, st));
@@ -493,9 +547,9 @@ __global__ void __launch_bounds__(256) gs_item_map_kernel(const uint32_t *item_o
 int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t st)
 {
     uint32_t n = b.n_reads + 1;
-    /* the batched start pass pairs each window's two candidates when it
-     * starts from the longer table */
-    b.paired = kernel == GS_KERNEL_BATCHED && I.kx > GS_K0 && gs_start_len(I, b.k) == I.kx;
+    /* the batched start pass pairs each window's two candidates when they
+     * are longer than the paired table's strings */
+    b.paired = kernel == GS_KERNEL_BATCHED && I.kmerx && b.k > I.kx;
     /* counts are written in place and scanned into offsets */
     gs_prepare_kernel<<<(n + 255) / 256, 256, 0, st>>>(b.lengths, b.n_reads, b.k,
                                                         b.paired ? I.kx : 0, b.slot_off,
@@ -1311,7 +1365,7 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
                 rf = gs_start_flags(e.w, 3u - n1, on1, 3u - n2, on2, k - KT);
             }
         }
-        wk += apart ? (vf ? 1u : 0u) + (vr ? 1u : 0u) : 1u;
+        wk += (vf ? 1u : 0u) + (vr ? 1u : 0u);   /* entries: a paired one is two */
         if (apart) {
             if (vf) {
                 const GsStart S = gs_start_apart<NSTOP>(I, seq, ef, true, KT, iL);
