@@ -147,6 +147,11 @@ static int grow_host_keep(T *&p, size_t &cap, size_t n, size_t keep, cudaStream_
     return GS_OK;
 }
 
+/* h_small: [2] plain's longest read end, [6..9] work, [11] text bytes,
+ * [12..13] gs_seed's end and order, [16..22] walk counts, and */
+#define GS_H_TOTALS 24   /* 4: GsBatch.h_totals */
+#define GS_H_QUEUE 28    /* 4: the queue's 8 words at the end of the pass */
+
 struct gs_ctx {
     gs_index *idx;
     cudaStream_t st;
@@ -164,8 +169,10 @@ struct gs_ctx {
     uint64_t *d_offsets; size_t cap_offsets;
     uint32_t *d_lengths; size_t cap_lengths;
     /* per read */
-    uint64_t *slot_cnt, *slot_off; size_t cap_slot_cnt, cap_slot_off;
-    uint32_t *item_cnt, *item_off; size_t cap_item_cnt, cap_item_off;
+    uint64_t *slot_off; size_t cap_slot_off;
+    uint32_t *item_off; size_t cap_item_off;
+    GsParts parts;
+    uint64_t *d_totals;
     uint32_t *item_read; size_t cap_item_read;
     uint32_t *rd_nf, *rd_nr; size_t cap_nf, cap_nr;
     uint64_t *rd_nseeds, *rd_npos; size_t cap_rns, cap_rnp;
@@ -178,6 +185,7 @@ struct gs_ctx {
     uint64_t *seed_pos; size_t cap_seed_pos;
     uint32_t *pos; size_t cap_pos;
     uint32_t *pmap; size_t cap_pmap;
+    uint32_t *tile_seed; size_t cap_tile_seed;
     GsCont *cont; size_t cap_cont;
     GsWalker *walkers; size_t cap_walkers;
     GsTextJob *text_jobs; size_t cap_text_jobs;
@@ -197,7 +205,8 @@ struct gs_ctx {
     uint64_t work[4];
     uint64_t walk_counts[7];   /* count_work pass: gs_ctx_last_walk_counts */
     void *cub_tmp; size_t cap_cub;
-    uint64_t *h_small;          /* pinned scalars */
+    uint64_t *h_small;          /* pinned scalars (GS_H_*) */
+    uint32_t last_items;        /* work items of the last sized pass */
     /* host result */
     uint64_t *h_seed_off; size_t cap_h_so;
     uint64_t *h_pos_off; size_t cap_h_po;
@@ -248,6 +257,12 @@ extern "C" int gs_ctx_create(gs_index *idx, void *cuda_stream, gs_ctx **out)
     if (e == cudaSuccess) e = cudaMalloc(&c->d_max, 16);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_work, 128);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_small, 256);
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_totals, 4 * sizeof(uint64_t));
+    if (e == cudaSuccess) e = cudaMalloc(&c->parts.part, GS_PARTS_MOST * sizeof(GsPart) + 8);
+    if (e == cudaSuccess) {
+        c->parts.tickets = (uint32_t *)(c->parts.part + GS_PARTS_MOST);
+        e = cudaMemset(c->parts.tickets, 0, 8);
+    }
     if (e != cudaSuccess) {
         int rc = gs_cuda_fail(e, "gs_ctx_create");
         gs_ctx_free(c);
@@ -293,12 +308,13 @@ extern "C" void gs_ctx_free(gs_ctx *c)
     if (!c) return;
     if (c->st) cudaStreamSynchronize(c->st);
     cudaFree(c->d_seqs); cudaFree(c->d_offsets); cudaFree(c->d_lengths);
-    cudaFree(c->slot_cnt); cudaFree(c->slot_off); cudaFree(c->item_cnt); cudaFree(c->item_off);
+    cudaFree(c->slot_off); cudaFree(c->item_off);
+    cudaFree(c->parts.part); cudaFree(c->d_totals);
     cudaFree(c->item_read);
     cudaFree(c->rd_nf); cudaFree(c->rd_nr); cudaFree(c->rd_nseeds); cudaFree(c->rd_npos);
     cudaFree(c->seed_off); cudaFree(c->pos_off);
     cudaFree(c->slots); cudaFree(c->hist); cudaFree(c->seeds); cudaFree(c->seed_pos);
-    cudaFree(c->pos); cudaFree(c->pmap); cudaFree(c->queue); cudaFree(c->d_max);
+    cudaFree(c->pos); cudaFree(c->pmap); cudaFree(c->tile_seed); cudaFree(c->queue); cudaFree(c->d_max);
     cudaFree(c->cont);
     cudaFree(c->walkers);
     cudaFree(c->text_jobs);
@@ -408,16 +424,6 @@ static int fetch_small(uint64_t *dst, const void *src, size_t bytes, cudaStream_
     return GS_OK;
 }
 
-/* a chunk's per-read offsets made batch-wide */
-__global__ void gs_add_base_kernel(uint64_t *seed_off, uint64_t *pos_off, uint32_t n, uint64_t bs,
-                                   uint64_t bp)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        seed_off[i] += bs;
-        pos_off[i] += bp;
-    }
-}
-
 template <class In, class Out>
 static int exclusive_scan(gs_ctx *c, In in, Out out, size_t n)
 {
@@ -476,9 +482,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     c->have_host = c->have_dev = 0;
     c->n_reads = n_reads;
     size_t nr1 = (size_t)n_reads + 1;
-    RC(grow(c->slot_cnt, c->cap_slot_cnt, nr1, c->st));
     RC(grow(c->slot_off, c->cap_slot_off, nr1, c->st));
-    RC(grow(c->item_cnt, c->cap_item_cnt, nr1, c->st));
     RC(grow(c->item_off, c->cap_item_off, nr1, c->st));
     RC(grow(c->rd_nf, c->cap_nf, nr1, c->st));
     RC(grow(c->rd_nr, c->cap_nr, nr1, c->st));
@@ -507,15 +511,18 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     GS_CUDA(cudaEventRecord(c->ev0, st));
     if (B.work) GS_CUDA(cudaMemsetAsync(c->d_work, 0, 128, st));
     GS_CUDA(cudaMemsetAsync(c->queue, 0, 32, st));
-    B.slot_off = c->slot_cnt;
-    B.item_off = c->item_cnt;
-    RC(gs_launch_prepare(I, B, p->kernel, st));
-    RC(exclusive_scan(c, c->slot_cnt, c->slot_off, nr1));
-    RC(exclusive_scan(c, c->item_cnt, c->item_off, nr1));
+    B.parts = c->parts;
+    B.totals = c->d_totals;
+    B.h_totals = &c->h_small[GS_H_TOTALS];
     B.slot_off = c->slot_off;
     B.item_off = c->item_off;
-    RC(fetch_small(&c->h_small[0], c->slot_off + n_reads, 8, st));
-    RC(fetch_small(&c->h_small[1], c->item_off + n_reads, 4, st));
+    /* the item map before its size is known: what there is, and the rest
+     * once it is */
+    if (p->kernel == GS_KERNEL_BATCHED) {
+        B.item_read = c->item_read;
+        B.item_read_cap = c->item_read ? c->cap_item_read : 0;
+    }
+    RC(gs_launch_prepare(I, B, p->kernel, st));
     if (p->kernel == GS_KERNEL_PLAIN) {
         GS_CUDA(cudaMemsetAsync(c->d_max, 0, 8, st));
         if (n_reads)
@@ -524,8 +531,9 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
         RC(fetch_small(&c->h_small[2], c->d_max, 8, st));
     }
     GS_CUDA(cudaStreamSynchronize(st));
-    uint64_t n_slots = c->h_small[0];
-    uint32_t n_items = (uint32_t)(c->h_small[1] & 0xffffffffu);
+    const uint64_t n_slots = c->h_small[GS_H_TOTALS];
+    const uint32_t n_items = (uint32_t)(c->h_small[GS_H_TOTALS + 1] & 0xffffffffu);
+    c->last_items = n_items;
     RC(grow(c->slots, c->cap_slots, n_slots + 1, c->st));
     RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, c->st));
     B.slots = c->slots;
@@ -533,10 +541,11 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.recmask = c->recmask;
     GS_CUDA(cudaMemsetAsync(c->recmask, 0, ((n_slots + 31) / 32 + 1) * sizeof(uint32_t), st));
     B.item_cap = n_items;
-    if (p->kernel == GS_KERNEL_BATCHED) {
-        RC(grow(c->item_read, c->cap_item_read, (size_t)n_items + 1, c->st));
+    if (p->kernel == GS_KERNEL_BATCHED && n_items > B.item_read_cap) {
+        RC(grow(c->item_read, c->cap_item_read, (size_t)n_items, c->st));
         B.item_read = c->item_read;
         B.item_read_cap = c->cap_item_read;
+        RC(gs_launch_prepare(I, B, p->kernel, st));
     }
     if (p->kernel == GS_KERNEL_PLAIN) {
         RC(grow(c->hist, c->cap_hist, c->h_small[2] + 1, c->st));
@@ -592,15 +601,9 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.rd_nr = c->rd_nr;
     B.rd_nseeds = c->rd_nseeds;
     B.rd_npos = c->rd_npos;
-    GS_CUDA(cudaMemsetAsync(c->rd_nseeds + n_reads, 0, 8, st));
-    GS_CUDA(cudaMemsetAsync(c->rd_npos + n_reads, 0, 8, st));
     RC(gs_launch_finalize_count(I, B, st));
-    RC(exclusive_scan(c, c->rd_nseeds, c->seed_off, nr1));
-    RC(exclusive_scan(c, c->rd_npos, c->pos_off, nr1));
-    RC(fetch_small(&c->h_small[3], c->seed_off + n_reads, 8, st));
-    RC(fetch_small(&c->h_small[4], c->pos_off + n_reads, 8, st));
     GS_CUDA(cudaStreamSynchronize(st));
-    uint64_t n_seeds = c->h_small[3], n_pos = c->h_small[4];
+    const uint64_t n_seeds = c->h_small[GS_H_TOTALS + 2], n_pos = c->h_small[GS_H_TOTALS + 3];
     if (n_pos > 0xffffffffull * 4) {
         gs_set_error("batch emits %llu positions; split the batch", (unsigned long long)n_pos);
         return GS_EOVERFLOW;
@@ -609,12 +612,14 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     RC(grow(c->seed_pos, c->cap_seed_pos, n_seeds + 1, c->st));
     RC(grow(c->pos, c->cap_pos, n_pos + 1, c->st));
     RC(grow(c->pmap, c->cap_pmap, n_pos + 1, c->st));
+    RC(grow(c->tile_seed, c->cap_tile_seed, c->cap_pos / 32 + 1, c->st));
     B.seed_off = c->seed_off;
     B.pos_off = c->pos_off;
     B.seeds = c->seeds;
     B.seed_pos = c->seed_pos;
     B.pos = c->pos;
     B.pmap = c->pmap;
+    B.tile_seed = c->tile_seed;
     B.seed_cap = n_seeds + 1;
     B.pos_cap = n_pos + 1;
     if (fetch) {
@@ -624,6 +629,8 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
         RC(grow_host(c->h_pos, c->cap_h_pos, n_pos + 1));
     }
     if (co) {
+        B.base_s = co->base_s;
+        B.base_p = co->base_p;
         uint64_t ws = co->base_s + n_seeds + 1, wp = co->base_p + n_pos + 1;
         if (co->base_s == 0 && co->base_p == 0) {
             ws = (uint64_t)((double)ws * co->scale * 1.1);
@@ -646,16 +653,9 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
             GS_CUDA(cudaMemcpyAsync(c->h_seeds, c->seeds, n_seeds * sizeof(gs_seed_rec),
                                     cudaMemcpyDeviceToHost, c->st_copy));
     }
-    RC(gs_launch_locate(I, B, n_seeds, n_pos, st));
-    if (co && n_reads) {
-        gs_add_base_kernel<<<152 * 4, 256, 0, st>>>(c->seed_off, c->pos_off, n_reads, co->base_s,
-                                                    co->base_p);
-        GS_CUDA(cudaGetLastError());
-    }
+    RC(gs_launch_locate(I, B, n_pos, st));
     GS_CUDA(cudaEventRecord(c->ev1, st));
-    RC(fetch_small(&c->h_small[5], c->queue + 1, 4, st));
-    RC(fetch_small(&c->h_small[10], c->queue + 2, 4, st));
-    RC(fetch_small(&c->h_small[11], c->queue + 5, 4, st));
+    RC(fetch_small(&c->h_small[GS_H_QUEUE], c->queue, 32, st));
     if (B.work) RC(fetch_small(&c->h_small[6], c->d_work, 32, st));
     if (B.work) RC(fetch_small(&c->h_small[16], c->d_work + 4, 56, st));
     if (co) {
@@ -684,9 +684,10 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
         GS_CUDA(cudaMemcpyAsync(c->h_pos, c->pos, n_pos * 4, cudaMemcpyDeviceToHost, st));
     GS_CUDA(cudaStreamSynchronize(st));
     if (fetch) GS_CUDA(cudaStreamSynchronize(c->st_copy));
-    uint32_t flags = (uint32_t)(c->h_small[5] & 0xffffffffu);
-    c->last_walkers = c->last_walker_cap ? (c->h_small[10] & 0xffffffffu) : 0;
-    c->last_text_jobs = c->last_text_cap ? (c->h_small[11] & 0xffffffffu) : 0;
+    const uint32_t *queue = (const uint32_t *)&c->h_small[GS_H_QUEUE];
+    const uint32_t flags = queue[1];
+    c->last_walkers = c->last_walker_cap ? queue[2] : 0;
+    c->last_text_jobs = c->last_text_cap ? queue[5] : 0;
     if (!p->walker_slots && c->last_walker_cap && c->last_walkers >= c->last_walker_cap &&
         c->walker_per16 < 512u) {
         c->walker_per16 = c->walker_per16 ? c->walker_per16 + c->walker_per16 / 2 : 384u;
@@ -734,7 +735,6 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
 {
     const GsDevIndex &I = *gs_index_dev(c->idx);
     cudaStream_t st = c->st;
-    size_t nr1 = (size_t)n_reads + 1;
     GsBatch B;
     memset(&B, 0, sizeof(B));
     B.seqs = d_seqs;
@@ -749,20 +749,19 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.mem_next = p->mem_next;
     B.queue = c->queue;
     GS_CUDA(cudaMemsetAsync(c->queue, 0, 32, st));
-    B.slot_off = c->slot_cnt;
-    B.item_off = c->item_cnt;
-    RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
-    RC(exclusive_scan(c, c->slot_cnt, c->slot_off, nr1));
-    RC(exclusive_scan(c, c->item_cnt, c->item_off, nr1));
+    B.parts = c->parts;
+    B.totals = c->d_totals;
+    B.h_totals = &c->h_small[GS_H_TOTALS];
     B.slot_off = c->slot_off;
     B.item_off = c->item_off;
+    B.item_read = c->item_read;
+    B.item_read_cap = c->cap_item_read;
+    RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
     B.slots = c->slots;
     B.slot_cap = c->cap_slots;
     B.recmask = c->recmask;
     GS_CUDA(cudaMemsetAsync(c->recmask, 0, ((c->cap_slots + 31) / 32 + 1) * sizeof(uint32_t), st));
     B.item_cap = c->g_items;
-    B.item_read = c->item_read;
-    B.item_read_cap = c->cap_item_read;
     /* the walker buffer as the sizing pass left it; walkers beyond it are
      * left to the leftover pass */
     if (c->last_walker_cap && c->walkers) {
@@ -778,21 +777,19 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.rd_nr = c->rd_nr;
     B.rd_nseeds = c->rd_nseeds;
     B.rd_npos = c->rd_npos;
-    GS_CUDA(cudaMemsetAsync(c->rd_nseeds + n_reads, 0, 8, st));
-    GS_CUDA(cudaMemsetAsync(c->rd_npos + n_reads, 0, 8, st));
     RC(gs_launch_finalize_count(I, B, st));
-    RC(exclusive_scan(c, c->rd_nseeds, c->seed_off, nr1));
-    RC(exclusive_scan(c, c->rd_npos, c->pos_off, nr1));
     B.seed_off = c->seed_off;
     B.pos_off = c->pos_off;
     B.seeds = c->seeds;
     B.seed_pos = c->seed_pos;
     B.pos = c->pos;
     B.pmap = c->pmap;
+    B.tile_seed = c->tile_seed;
     B.seed_cap = c->cap_seeds < c->cap_seed_pos ? c->cap_seeds : c->cap_seed_pos;
     B.pos_cap = c->cap_pos < c->cap_pmap ? c->cap_pos : c->cap_pmap;
     RC(gs_launch_finalize_emit(I, B, st));
-    RC(gs_launch_locate(I, B, 0, 0, st));
+    RC(gs_launch_locate(I, B, UINT64_MAX, st));
+    RC(fetch_small(&c->h_small[GS_H_QUEUE], c->queue, 32, st));
     return GS_OK;
 }
 
@@ -813,12 +810,9 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
         GS_CUDA(cudaEventRecord(c->ev0, st));
         GS_CUDA(cudaGraphLaunch(c->gexec, st));
         GS_CUDA(cudaEventRecord(c->ev1, st));
-        GS_CUDA(cudaMemcpyAsync(&c->h_small[5], c->queue + 1, 4, cudaMemcpyDeviceToHost, st));
-        GS_CUDA(cudaMemcpyAsync(&c->h_small[3], c->seed_off + n_reads, 8, cudaMemcpyDeviceToHost, st));
-        GS_CUDA(cudaMemcpyAsync(&c->h_small[4], c->pos_off + n_reads, 8, cudaMemcpyDeviceToHost, st));
         GS_CUDA(cudaStreamSynchronize(st));
-        uint32_t flags = (uint32_t)(c->h_small[5] & 0xffffffffu);
-        uint64_t ns = c->h_small[3], np = c->h_small[4];
+        const uint32_t flags = ((const uint32_t *)&c->h_small[GS_H_QUEUE])[1];
+        const uint64_t ns = c->h_small[GS_H_TOTALS + 2], np = c->h_small[GS_H_TOTALS + 3];
         bool fits = !(flags & GS_FLAG_OVERFLOW) && ns <= c->cap_seeds && ns <= c->cap_seed_pos &&
                     np <= c->cap_pos && np <= c->cap_pmap;
         if (fits) {
@@ -844,7 +838,7 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
     RC(run_pipeline(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch));
     if (!c->slots || !c->seeds || !c->pos || !c->seed_pos || !c->pmap) return GS_OK;
     /* capture a pass with the capacities this one needed */
-    c->g_items = (uint32_t)(c->h_small[1] & 0xffffffffu);
+    c->g_items = c->last_items;
     cudaGraph_t g = NULL;
     GS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int rc = enqueue_pass(c, d_seqs, d_offsets, d_lengths, n_reads, p);

@@ -85,6 +85,25 @@ struct __align__(8) GsWalker {
     uint32_t l, u, jl, ju;
 };
 
+/* Per-read counts become offsets in two kernels that cut the reads the same
+ * way: the first sums each block's reads, its last block to finish turns the
+ * sums into offsets and totals; the second scans within the blocks.  A pair
+ * of counts is scanned at once (slots and work items; seeds and positions).
+ * Few reads take one block and the second kernel alone. */
+#define GS_PARTS_MOST 4864u   /* 32 blocks an SM: the last wave is a small part of all */
+struct GsPart {
+    unsigned long long a, b;
+};
+struct GsParts {
+    GsPart *part;      /* GS_PARTS_MOST entries, and tickets[2], zero between passes */
+    uint32_t *tickets;
+};
+static inline uint32_t gs_parts_of(uint32_t n_reads)
+{
+    const uint32_t p = (n_reads + 255u) / 256u;
+    return p < 1u ? 1u : p > GS_PARTS_MOST ? GS_PARTS_MOST : p;
+}
+
 /* Per-batch device arguments shared by the pipeline kernels. */
 struct GsBatch {
     const char *seqs;          /* ASCII bases */
@@ -92,6 +111,10 @@ struct GsBatch {
     const uint32_t *lengths;   /* per read */
     uint32_t n_reads;
     int32_t k, smem, n_mode, lf_mode;
+    GsParts parts;
+    uint64_t *totals;          /* slots, work items, seeds, positions of the pass, on the
+                                * device ... */
+    uint64_t *h_totals;        /* ... and in mapped host memory (or NULL) */
     uint64_t *slot_off;        /* per read (n+1): first candidate slot */
     uint32_t *item_off;        /* per read (n+1): first work item */
     GsRec *slots;              /* 2 * candidates; only slots holding a record are written */
@@ -104,6 +127,8 @@ struct GsBatch {
     uint64_t *seed_pos;        /* per output seed: index of its first position */
     uint32_t *pos;             /* output positions */
     uint32_t *pmap;            /* position -> seed */
+    uint32_t *tile_seed;       /* every 32nd position's seed (pos_cap / 32 + 1 entries) */
+    uint64_t base_s, base_p;      /* added to the offsets written (a chunk's place in its batch) */
     uint64_t seed_cap, pos_cap;   /* output capacities (entries) */
     uint64_t slot_cap;             /* candidate slots allocated */
     uint32_t *item_read;       /* batched start pass: the read of each work item */
@@ -217,9 +242,8 @@ int gs_launch_search(const GsDevIndex &idx, GsBatch &b, int kernel, int queue_ch
 int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t st);
 int gs_launch_finalize_count(const GsDevIndex &idx, GsBatch &b, cudaStream_t st);
 int gs_launch_finalize_emit(const GsDevIndex &idx, GsBatch &b, cudaStream_t st);
-/* n_seeds / n_pos: host-known totals, or 0 to size the grids by the
- * capacities and read the totals on the device (graph capture) */
-int gs_launch_locate(const GsDevIndex &idx, GsBatch &b, uint64_t n_seeds, uint64_t n_pos,
-                     cudaStream_t st);
+/* n_pos: the host-known total, or UINT64_MAX to size the grid by the
+ * capacity and read the total on the device (graph capture) */
+int gs_launch_locate(const GsDevIndex &idx, GsBatch &b, uint64_t n_pos, cudaStream_t st);
 
 #endif

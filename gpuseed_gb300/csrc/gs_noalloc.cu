@@ -32,8 +32,6 @@
  */
 #include "gs_internal.h"
 
-#include <cub/cub.cuh>
-
 #include <mutex>
 #include <string.h>
 
@@ -121,22 +119,22 @@ extern "C" int gs_seed_noalloc(gs_index *idx, const char *d_seqs, const uint64_t
     const size_t nr1 = (size_t)n_reads + 1;
 
     Carve cv = {scratch, 0, GS_NOALLOC_SCRATCH_BYTES};
-    uint64_t *slot_cnt = cv.take<uint64_t>(nr1), *slot_off = cv.take<uint64_t>(nr1);
-    uint32_t *item_cnt = cv.take<uint32_t>(nr1), *item_off = cv.take<uint32_t>(nr1);
+    uint64_t *slot_off = cv.take<uint64_t>(nr1);
+    uint32_t *item_off = cv.take<uint32_t>(nr1);
     uint32_t *rd_nf = cv.take<uint32_t>(nr1), *rd_nr = cv.take<uint32_t>(nr1);
     uint64_t *rd_nseeds = cv.take<uint64_t>(nr1), *rd_npos = cv.take<uint64_t>(nr1);
     uint32_t *queue = cv.take<uint32_t>(4);
-    size_t cub_bytes = 0, b2 = 0;
-    GS_CUDA(cub::DeviceScan::ExclusiveSum(NULL, cub_bytes, slot_cnt, slot_off, (int64_t)nr1, st));
-    GS_CUDA(cub::DeviceScan::ExclusiveSum(NULL, b2, item_cnt, item_off, (int64_t)nr1, st));
-    if (b2 > cub_bytes) cub_bytes = b2;
-    unsigned char *cub_tmp = cv.take<unsigned char>(cub_bytes + 256);
+    uint64_t *totals = cv.take<uint64_t>(4);
+    GsParts parts;
+    parts.part = cv.take<GsPart>(GS_PARTS_MOST);
+    parts.tickets = cv.take<uint32_t>(2);
     GsRec *slots = cv.take<GsRec>(GS_NOALLOC_MAX_SLOTS);
     uint32_t *recmask = cv.take<uint32_t>(GS_NOALLOC_MAX_SLOTS / 32 + 1);
     uint64_t *seed_pos = cv.take<uint64_t>(GS_NOALLOC_MAX_SEEDS);
     uint32_t *pmap = cv.take<uint32_t>(GS_NOALLOC_MAX_POS);
-    if (!slot_cnt || !slot_off || !item_cnt || !item_off || !rd_nf || !rd_nr || !rd_nseeds ||
-        !rd_npos || !queue || !cub_tmp || !slots || !recmask || !seed_pos || !pmap) {
+    uint32_t *tile_seed = cv.take<uint32_t>(GS_NOALLOC_MAX_POS / 32 + 1);
+    if (!slot_off || !item_off || !rd_nf || !rd_nr || !rd_nseeds || !rd_npos || !queue || !totals ||
+        !parts.part || !parts.tickets || !slots || !recmask || !seed_pos || !pmap || !tile_seed) {
         gs_set_error("gs_seed_noalloc: scratch layout exceeds %u bytes",
                      (unsigned)GS_NOALLOC_SCRATCH_BYTES);
         return GS_ENOMEM;
@@ -157,12 +155,14 @@ extern "C" int gs_seed_noalloc(gs_index *idx, const char *d_seqs, const uint64_t
     B.queue = queue;
     GS_CUDA(cudaMemsetAsync(queue, 0, 4 * sizeof(uint32_t), st));
 
+    GS_CUDA(cudaMemsetAsync(parts.tickets, 0, 2 * sizeof(uint32_t), st));
+
     /* slots and work items per read */
-    B.slot_off = slot_cnt;
-    B.item_off = item_cnt;
+    B.parts = parts;
+    B.totals = totals;
+    B.slot_off = slot_off;
+    B.item_off = item_off;
     NA_RC(gs_launch_prepare(I, B, GS_KERNEL_LOCKSTEP, st));
-    GS_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, slot_cnt, slot_off, (int64_t)nr1, st));
-    GS_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, item_cnt, item_off, (int64_t)nr1, st));
     uint64_t n_slots = 0;
     uint32_t n_items = 0;
     GS_CUDA(cudaMemcpyAsync(&n_slots, slot_off + n_reads, 8, cudaMemcpyDeviceToHost, st));
@@ -173,8 +173,6 @@ extern "C" int gs_seed_noalloc(gs_index *idx, const char *d_seqs, const uint64_t
                      "per call", (unsigned long long)n_slots, (unsigned)GS_NOALLOC_MAX_SLOTS);
         return GS_EINVAL;
     }
-    B.slot_off = slot_off;
-    B.item_off = item_off;
     B.slots = slots;
     B.slot_cap = GS_NOALLOC_MAX_SLOTS;
     B.recmask = recmask;
@@ -190,19 +188,22 @@ extern "C" int gs_seed_noalloc(gs_index *idx, const char *d_seqs, const uint64_t
     B.rd_nr = rd_nr;
     B.rd_nseeds = rd_nseeds;
     B.rd_npos = rd_npos;
-    GS_CUDA(cudaMemsetAsync(rd_nseeds + n_reads, 0, 8, st));
-    GS_CUDA(cudaMemsetAsync(rd_npos + n_reads, 0, 8, st));
     NA_RC(gs_launch_finalize_count(I, B, st));
-    GS_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, rd_nseeds, d_read_seed_off,
-                                          (int64_t)nr1, st));
-    GS_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, cub_bytes, rd_npos, d_read_pos_off, (int64_t)nr1,
-                                          st));
     uint64_t n_seeds = 0, n_pos = 0;
-    GS_CUDA(cudaMemcpyAsync(&n_seeds, d_read_seed_off + n_reads, 8, cudaMemcpyDeviceToHost, st));
-    GS_CUDA(cudaMemcpyAsync(&n_pos, d_read_pos_off + n_reads, 8, cudaMemcpyDeviceToHost, st));
+    GS_CUDA(cudaMemcpyAsync(&n_seeds, totals + 2, 8, cudaMemcpyDeviceToHost, st));
+    GS_CUDA(cudaMemcpyAsync(&n_pos, totals + 3, 8, cudaMemcpyDeviceToHost, st));
     GS_CUDA(cudaStreamSynchronize(st));
     *n_seeds_out = n_seeds;
     *n_pos_out = n_pos;
+    B.seed_off = d_read_seed_off;
+    B.pos_off = d_read_pos_off;
+    if (n_seeds > GS_NOALLOC_MAX_SEEDS || n_pos > GS_NOALLOC_MAX_POS || n_seeds > seed_cap ||
+        n_pos > pos_cap || (n_seeds && !d_seeds) || (n_pos && !d_pos)) {
+        /* no room for the seeds: the reads' offsets alone (seed_cap 0) */
+        B.mem_next = GS_MEM_NEXT_READ;
+        NA_RC(gs_launch_finalize_emit(I, B, st));
+        GS_CUDA(cudaStreamSynchronize(st));
+    }
     if (n_seeds > GS_NOALLOC_MAX_SEEDS || n_pos > GS_NOALLOC_MAX_POS) {
         gs_set_error("gs_seed_noalloc: %llu seeds / %llu positions, at most %u / %u per call",
                      (unsigned long long)n_seeds, (unsigned long long)n_pos,
@@ -215,16 +216,15 @@ extern "C" int gs_seed_noalloc(gs_index *idx, const char *d_seqs, const uint64_t
                      (unsigned long long)seed_cap, (unsigned long long)pos_cap);
         return GS_EOVERFLOW;
     }
-    B.seed_off = d_read_seed_off;
-    B.pos_off = d_read_pos_off;
     B.seeds = d_seeds;
     B.seed_pos = seed_pos;
     B.pos = d_pos;
     B.pmap = pmap;
+    B.tile_seed = tile_seed;
     B.seed_cap = n_seeds;
     B.pos_cap = n_pos;
     NA_RC(gs_launch_finalize_emit(I, B, st));
-    NA_RC(gs_launch_locate(I, B, n_seeds, n_pos, st));
+    NA_RC(gs_launch_locate(I, B, n_pos, st));
     uint32_t flags = 0;
     GS_CUDA(cudaMemcpyAsync(&flags, queue + 1, 4, cudaMemcpyDeviceToHost, st));
     GS_CUDA(cudaStreamSynchronize(st));

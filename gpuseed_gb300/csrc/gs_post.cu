@@ -9,13 +9,12 @@
  *   gs_finalize_count  lane per read (warp per long read): compacts the
  *                      read's candidate slots in place and counts the
  *                      seeds/positions the filters keep;
- *   (scan)             exclusive sums of those counts over reads;
- *   gs_finalize_emit   thread per read: merges the forward (ascending end)
+ *   gs_finalize_emit   thread per read: its offsets, and merges the forward (ascending end)
  *                      and reverse (ascending start) records by begin --
  *                      equal begins keep forward first, as the reference's
  *                      stable sort does -- and writes the output seeds;
- *   gs_expand          position -> seed map;
- *   gs_locate          thread per position: LF walk to a sampled row.
+ *   gs_locate          position -> seed map, and each position's row by an
+ *                      LF walk to a sampled row (or the full suffix array).
  *
  * Filter rules on the per-strand record lists (ascending end / start):
  *   SMEM forward: keep a record unless the next one has the same begin
@@ -27,6 +26,7 @@
  *        reverse: the same toward the previous record with the same end.
  */
 #include "gs_fm.cuh"
+#include "gs_scan.cuh"
 
 
 
@@ -277,9 +277,11 @@ __device__ __forceinline__ uint32_t gs_lane_compact(GsRec *slots, const uint32_t
  * lane; longer ones by the whole warp */
 #define GS_LANE_SLOTS 512u
 
-/* a read compacted and counted by the whole warp (long reads) */
+/* a read compacted and counted by the whole warp (long reads); lane 0 adds
+ * its seeds and positions to the sums */
 __device__ __noinline__ void gs_finalize_read_warp(const GsBatch &B, uint32_t r, uint64_t base,
-                                                   uint64_t next, int lane)
+                                                   uint64_t next, int lane, uint64_t &sum_s,
+                                                   uint64_t &sum_p)
 {
     uint32_t n = (uint32_t)((next - base) >> 1);
     GsRec *F = B.slots + base;
@@ -338,23 +340,26 @@ __device__ __noinline__ void gs_finalize_read_warp(const GsBatch &B, uint32_t r,
         B.rd_nr[r] = nr;
         B.rd_nseeds[r] = seeds;
         B.rd_npos[r] = npos;
+        sum_s += seeds;
+        sum_p += npos;
     }
 }
 
 /* 32 consecutive reads per warp: a lane compacts and counts its own read
  * when it spans at most GS_LANE_SLOTS slots (few instructions a read, the
  * warp's loads spread over 32 reads); the warp then takes its longer reads
- * one at a time. */
-__global__ void __launch_bounds__(256) gs_finalize_count(GsBatch B)
+ * one at a time.  The blocks' sums become the offsets of gs_finalize_emit. */
+__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r0 = warp * 32u; r0 < B.n_reads; r0 += nwarps * 32u) {
+    uint32_t first, last;
+    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    uint64_t sum_s = 0, sum_p = 0;
+    for (uint32_t r0 = first + (threadIdx.x & ~31u); r0 < last; r0 += GS_SCAN_THREADS) {
         const uint32_t r = r0 + (uint32_t)lane;
         uint64_t base = 0, next = 0;
         bool longr = false;
-        if (r < B.n_reads) {
+        if (r < last) {
             base = B.slot_off[r];
             next = B.slot_off[r + 1];
             if (next > B.slot_cap) {
@@ -379,6 +384,8 @@ __global__ void __launch_bounds__(256) gs_finalize_count(GsBatch B)
                 B.rd_nr[r] = nr;
                 B.rd_nseeds[r] = seeds;
                 B.rd_npos[r] = npos;
+                sum_s += seeds;
+                sum_p += npos;
             }
         }
         uint32_t lm = __ballot_sync(0xffffffffu, longr);
@@ -387,61 +394,95 @@ __global__ void __launch_bounds__(256) gs_finalize_count(GsBatch B)
             lm &= lm - 1u;
             const uint64_t b0 = __shfl_sync(0xffffffffu, base, src);
             const uint64_t b1 = __shfl_sync(0xffffffffu, next, src);
-            gs_finalize_read_warp(B, r0 + (uint32_t)src, b0, b1, lane);
+            gs_finalize_read_warp(B, r0 + (uint32_t)src, b0, b1, lane, sum_s, sum_p);
+        }
+    }
+    GsPart sum, total;
+    gs_block_scan(sum_s, sum_p, sum);
+    if (gs_parts_publish(B.parts, 1, sum, total) && threadIdx.x == 0) {
+        B.totals[2] = total.a;
+        B.totals[3] = total.b;
+        if (B.h_totals) {
+            B.h_totals[2] = total.a;
+            B.h_totals[3] = total.b;
         }
     }
 }
 
-__global__ void __launch_bounds__(128) gs_finalize_emit(GsBatch B, uint64_t *seed_pos)
+/* A thread per read: its seeds' and positions' offsets, and its seeds merged
+ * by begin. */
+__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, uint64_t *seed_pos)
 {
-    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= B.n_reads) return;
-    uint64_t base = B.slot_off[r];
-    uint32_t n = (uint32_t)((B.slot_off[r + 1] - base) >> 1);
-    const GsRec *F = B.slots + base;
-    const GsRec *Rv = F + n;
-    uint32_t nf = B.rd_nf[r], nr = B.rd_nr[r];
-    uint64_t s = B.seed_off[r];
-    uint64_t p = B.pos_off[r];
-    uint32_t a = 0, b = 0;
-    /* each record loaded once: the forward list's current and next, the
-     * reverse list's current and previous */
-    GsRec none;
-    none.x = none.y = 0;
-    none.l = 1u;
-    none.u = 0u;
-    GsRec fc = nf ? F[0] : none, fn = nf > 1 ? F[1] : none;
-    GsRec rc = nr ? Rv[0] : none, rp = none;
-    while (a < nf || b < nr) {
-        bool take_f;
-        if (a >= nf) take_f = false;
-        else if (b >= nr) take_f = true;
-        else take_f = ((uint32_t)fc.x & 0x7fffffffu) <= ((uint32_t)rc.x & 0x7fffffffu);
-        bool keep; uint32_t cnt, xl, xu;
-        GsRec R;
-        if (take_f) {
-            gs_fwd_rule_v(fc, fn, a + 1 < nf, B.smem, B.max_occ, keep, cnt, xl, xu);
-            R = fc;
-            a++;
-            fc = fn;
-            fn = a + 1 < nf ? F[a + 1] : none;
-        } else {
-            gs_rev_rule_v(rc, rp, b > 0, B.smem, B.max_occ, keep, cnt, xl, xu);
-            R = rc;
-            b++;
-            rp = rc;
-            rc = b < nr ? Rv[b] : none;
+    uint32_t first, last;
+    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    GsPart run = B.parts.part[blockIdx.x];
+    if (last == B.n_reads && threadIdx.x == 0) {
+        B.seed_off[B.n_reads] = B.totals[2] + B.base_s;
+        B.pos_off[B.n_reads] = B.totals[3] + B.base_p;
+    }
+    /* the offsets of all the block's reads first: the merges below then need
+     * no barrier, and a warp of short lists does not wait for one of long */
+    for (uint32_t r0 = first; r0 < last; r0 += GS_SCAN_THREADS) {
+        const uint32_t r = r0 + threadIdx.x;
+        const bool in = r < last;
+        GsPart t;
+        const GsPart x = gs_block_scan(in ? B.rd_nseeds[r] : 0ull, in ? B.rd_npos[r] : 0ull, t);
+        if (in) {
+            B.seed_off[r] = run.a + x.a + B.base_s;
+            B.pos_off[r] = run.b + x.b + B.base_p;
         }
-        if (keep && cnt) {
-            if (s < B.seed_cap) {
-                gs_seed_rec o;
-                o.x = R.x; o.y = R.y; o.l = R.l; o.u = R.u;
-                o.xl = xl; o.xu = xu; o.n_pos = cnt; o.pad = 0;
-                B.seeds[s] = o;
-                seed_pos[s] = p;
+        run.a += t.a;
+        run.b += t.b;
+    }
+    for (uint32_t r = first + threadIdx.x; r < last; r += GS_SCAN_THREADS) {
+        uint64_t s = B.seed_off[r] - B.base_s, p = B.pos_off[r] - B.base_p;   /* this thread's own */
+        const uint64_t base = B.slot_off[r];
+        const uint32_t n = (uint32_t)((B.slot_off[r + 1] - base) >> 1);
+        const GsRec *F = B.slots + base;
+        const GsRec *Rv = F + n;
+        const uint32_t nf = B.rd_nf[r], nr = B.rd_nr[r];
+        uint32_t a = 0, b = 0;
+        /* each record loaded once: the forward list's current and next, the
+         * reverse list's current and previous */
+        GsRec none;
+        none.x = none.y = 0;
+        none.l = 1u;
+        none.u = 0u;
+        GsRec fc = nf ? F[0] : none, fn = nf > 1 ? F[1] : none;
+        GsRec rc = nr ? Rv[0] : none, rp = none;
+        while (a < nf || b < nr) {
+            bool take_f;
+            if (a >= nf) take_f = false;
+            else if (b >= nr) take_f = true;
+            else take_f = ((uint32_t)fc.x & 0x7fffffffu) <= ((uint32_t)rc.x & 0x7fffffffu);
+            bool keep; uint32_t cnt, xl, xu;
+            GsRec R;
+            if (take_f) {
+                gs_fwd_rule_v(fc, fn, a + 1 < nf, B.smem, B.max_occ, keep, cnt, xl, xu);
+                R = fc;
+                a++;
+                fc = fn;
+                fn = a + 1 < nf ? F[a + 1] : none;
+            } else {
+                gs_rev_rule_v(rc, rp, b > 0, B.smem, B.max_occ, keep, cnt, xl, xu);
+                R = rc;
+                b++;
+                rp = rc;
+                rc = b < nr ? Rv[b] : none;
             }
-            s++;
-            p += cnt;
+            if (keep && cnt) {
+                if (s < B.seed_cap) {
+                    gs_seed_rec o;
+                    o.x = R.x; o.y = R.y; o.l = R.l; o.u = R.u;
+                    o.xl = xl; o.xu = xu; o.n_pos = cnt; o.pad = 0;
+                    B.seeds[s] = o;
+                    seed_pos[s] = p;
+                    for (uint64_t m = (p + 31u) >> 5; (m << 5) < p + cnt && (m << 5) < B.pos_cap; m++)
+                        B.tile_seed[m] = (uint32_t)s;
+                }
+                s++;
+                p += cnt;
+            }
         }
     }
 }
@@ -509,78 +550,87 @@ __global__ void __launch_bounds__(128) gs_mem_next_kernel(GsBatch B)
     }
 }
 
-__global__ void __launch_bounds__(256) gs_expand(const uint64_t *seed_pos, const gs_seed_rec *seeds,
-                                                 const uint64_t *n_seeds_dev, uint64_t seed_cap,
-                                                 uint32_t *pmap, uint64_t pos_cap)
-{
-    uint64_t n = *n_seeds_dev;
-    if (n > seed_cap) n = seed_cap;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += stride) {
-        uint64_t p = seed_pos[s];
-        uint32_t cnt = seeds[s].n_pos;
-        for (uint32_t i = 0; i < cnt && p + i < pos_cap; i++) pmap[p + i] = (uint32_t)s;
-    }
-}
+/* Positions: a warp takes a tile of them, 32 a round (they span at most 32
+ * seeds, as every seed has a position), from the seed of the tile's first
+ * position, which gs_finalize_emit noted.  It writes the position -> seed map
+ * for the text records and resolves each row.  A seed of many positions is
+ * spread over many warps.  Tiles of 32 to 256, so that few positions spread
+ * over many warps: a round of LF walks is up to sa_intv - 1 dependent pairs
+ * of loads. */
+#define GS_LOCATE_MOST 256u
 
-__global__ void __launch_bounds__(256) gs_locate(GsDevIndex I, const gs_seed_rec *seeds,
-                                                 const uint64_t *seed_pos, const uint32_t *pmap,
-                                                 const uint64_t *n_pos_dev, uint64_t pos_cap,
-                                                 uint32_t *out, int lf_mode, uint32_t *flags,
-                                                 unsigned long long *work)
+template <bool SAF>
+__global__ void __launch_bounds__(256, 8) gs_locate(GsDevIndex I, GsBatch B)
 {
-    uint64_t n_pos = *n_pos_dev;
-    if (n_pos > pos_cap) n_pos = pos_cap;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    /* base is the same for every lane of a warp, so warps stay whole */
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n_pos; base += stride) {
-        const uint64_t j = base + threadIdx.x;
-        uint32_t steps = 0;
-        const bool active = j < n_pos;
-        if (active) {
-            uint32_t s = pmap[j];
-            gs_seed_rec S = seeds[s];
-            /* the (j - first)-th row from l outside [xl, xu] */
-            uint32_t row = S.l + (uint32_t)(j - seed_pos[s]);
-            const uint32_t x0 = S.xl > S.l ? S.xl : S.l;
-            if (S.xl <= S.xu && S.xu >= x0 && row >= x0) row += S.xu - x0 + 1u;
-            /* locate_seeds_gpu (:668-684): LF until a sampled row; a
-             * consistent index reaches one within seq_len+1 steps.  With
-             * the full suffix array it is one read: the walk's result is
-             * SA[row], except that the LF quirk sends the rows whose walk
-             * passes row primary+1 to row 0, where sa[0] = -1 gives the
-             * steps taken minus one -- position - quirk_lo. */
-            const uint32_t cap = I.seq_len + 2u;
-            bool bad = false;
-            if (I.saf) {
-                uint32_t v = gs_ld64(&I.saf[row]);
-                if (lf_mode == GS_LF_GPUSEED && v - I.quirk_lo < I.quirk_n) v -= I.quirk_lo;
-                out[j] = v;
-            }
-            while (!I.saf && row % I.sa_intv) {
-                row = gs_lf(I, row, lf_mode);
-                if (++steps > cap) {
-                    bad = true;
-                    break;
+    /* a replayed pass with more output than it was sized for: the host sees
+     * the totals and sizes it again */
+    const uint64_t n_pos = B.totals[3], n_seeds = B.totals[2];
+    if (n_pos > B.pos_cap || n_seeds > B.seed_cap || n_seeds == 0) return;
+    const int lane = threadIdx.x & 31;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint32_t cap = I.seq_len + 2u;
+    const uint64_t share = ((n_pos + nwarps - 1) / nwarps + 31u) & ~31ull;
+    const uint64_t tile = share < GS_LOCATE_MOST ? share : GS_LOCATE_MOST;
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * tile < n_pos;
+         w += nwarps) {
+        const uint64_t p0 = w * tile;
+        const uint64_t p1 = p0 + tile < n_pos ? p0 + tile : n_pos;
+        uint64_t s0 = B.tile_seed[p0 >> 5];
+        for (uint64_t pb = p0; pb < p1; pb += 32) {
+            const uint64_t p = pb + (uint64_t)lane;
+            /* first positions of seeds s0+1 .. s0+32 */
+            const uint64_t at = s0 + 1u + (uint64_t)lane;
+            const uint64_t next = at < n_seeds ? B.seed_pos[at] : ~0ull;
+            int k = 0;   /* how many of them are at or before p */
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1)
+                if (__shfl_sync(0xffffffffu, next, k + step - 1) <= p) k += step;
+            if (__shfl_sync(0xffffffffu, next, k) <= p) k++;
+            const uint64_t s = s0 + (uint64_t)k;
+            uint32_t steps = 0;
+            const bool active = p < p1;
+            if (active) {
+                const gs_seed_rec S = B.seeds[s];
+                B.pmap[p] = (uint32_t)s;
+                /* the (p - first)-th row from l outside [xl, xu] */
+                uint32_t row = S.l + (uint32_t)(p - B.seed_pos[s]);
+                const uint32_t x0 = S.xl > S.l ? S.xl : S.l;
+                if (S.xl <= S.xu && S.xu >= x0 && row >= x0) row += S.xu - x0 + 1u;
+                /* locate_seeds_gpu (:668-684): LF until a sampled row; a
+                 * consistent index reaches one within seq_len+1 steps.  With
+                 * the full suffix array it is one read: the walk's result is
+                 * SA[row], except that the LF quirk sends the rows whose walk
+                 * passes row primary+1 to row 0, where sa[0] = -1 gives the
+                 * steps taken minus one -- position - quirk_lo. */
+                if (SAF) {
+                    uint32_t v = gs_ld64(&I.saf[row]);
+                    if (B.lf_mode == GS_LF_GPUSEED && v - I.quirk_lo < I.quirk_n) v -= I.quirk_lo;
+                    B.pos[p] = v;
+                } else {
+                    while (row % I.sa_intv && steps <= cap) {
+                        row = gs_lf(I, row, B.lf_mode);
+                        steps++;
+                    }
+                    if (steps > cap) {
+                        atomicOr(B.queue + 1, GS_FLAG_WALK);
+                        B.pos[p] = 0xffffffffu;
+                    } else {
+                        B.pos[p] = __ldg(&I.sa[row / I.sa_intv]) + steps;
+                    }
                 }
             }
-            if (bad) {
-                atomicOr(flags, GS_FLAG_WALK);
-                out[j] = 0xffffffffu;
-            } else if (!I.saf) {
-                out[j] = __ldg(&I.sa[row / I.sa_intv]) + steps;
+            if (B.work) {
+                unsigned long long st = steps, np = active ? 1ull : 0ull;
+                for (int off = 16; off; off >>= 1) {
+                    st += __shfl_xor_sync(0xffffffffu, st, off);
+                    np += __shfl_xor_sync(0xffffffffu, np, off);
+                }
+                if (lane == 0 && np) {
+                    atomicAdd(&B.work[2], st);
+                    atomicAdd(&B.work[3], np);
+                }
             }
-        }
-        if (work) {
-            unsigned long long st = steps, np = active ? 1ull : 0ull;
-            for (int off = 16; off; off >>= 1) {
-                st += __shfl_xor_sync(0xffffffffu, st, off);
-                np += __shfl_xor_sync(0xffffffffu, np, off);
-            }
-            if ((threadIdx.x & 31) == 0 && np) {
-                atomicAdd(&work[2], st);
-                atomicAdd(&work[3], np);
-            }
+            s0 = __shfl_sync(0xffffffffu, s, 31);
         }
     }
 }
@@ -588,10 +638,7 @@ __global__ void __launch_bounds__(256) gs_locate(GsDevIndex I, const gs_seed_rec
 int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
-    if (B.n_reads == 0) return GS_OK;
-    uint32_t grid = (B.n_reads + 255) / 256;
-    if (grid > 152u * 16u) grid = 152u * 16u;
-    gs_finalize_count<<<grid, 256, 0, st>>>(B);
+    gs_finalize_count<<<gs_parts_of(B.n_reads), GS_SCAN_THREADS, 0, st>>>(B);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }
@@ -599,36 +646,25 @@ int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 int gs_launch_finalize_emit(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
-    if (B.n_reads == 0) return GS_OK;
-    gs_finalize_emit<<<(B.n_reads + 127) / 128, 128, 0, st>>>(B, B.seed_pos);
+    gs_finalize_emit<<<gs_parts_of(B.n_reads), GS_SCAN_THREADS, 0, st>>>(B, B.seed_pos);
     GS_CUDA(cudaGetLastError());
-    if (!B.smem && B.mem_next == GS_MEM_NEXT_GPUSEED) {
+    if (B.n_reads && !B.smem && B.mem_next == GS_MEM_NEXT_GPUSEED) {
         gs_mem_next_kernel<<<(B.n_reads + 127) / 128, 128, 0, st>>>(B);
         GS_CUDA(cudaGetLastError());
     }
     return GS_OK;
 }
 
-int gs_launch_locate(const GsDevIndex &I, GsBatch &B, uint64_t n_seeds, uint64_t n_pos,
-                     cudaStream_t st)
+int gs_launch_locate(const GsDevIndex &I, GsBatch &B, uint64_t n_pos, cudaStream_t st)
 {
-    if (B.n_reads == 0 || B.seed_cap == 0 || B.pos_cap == 0) return GS_OK;
-    uint64_t ns = n_seeds ? n_seeds : B.seed_cap;
-    uint64_t np = n_pos ? n_pos : B.pos_cap;
-    if (n_seeds == 0 && n_pos == 0) {
-        /* totals known only on the device: persistent grids */
-        ns = ns < 152ull * 256 * 32 ? ns : 152ull * 256 * 32;
-        np = np < 152ull * 256 * 64 ? np : 152ull * 256 * 64;
-    } else if (n_pos == 0 || n_seeds == 0) {
-        return GS_OK;   /* nothing to locate */
-    }
-    gs_expand<<<(unsigned)((ns + 255) / 256), 256, 0, st>>>(B.seed_pos, B.seeds,
-                                                             B.seed_off + B.n_reads, B.seed_cap,
-                                                             B.pmap, B.pos_cap);
-    GS_CUDA(cudaGetLastError());
-    gs_locate<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(I, B.seeds, B.seed_pos, B.pmap,
-                                                             B.pos_off + B.n_reads, B.pos_cap,
-                                                             B.pos, B.lf_mode, B.queue + 1, B.work);
+    if (B.n_reads == 0 || B.seed_cap == 0 || B.pos_cap == 0 || n_pos == 0) return GS_OK;
+    uint64_t n = n_pos < B.pos_cap ? n_pos : B.pos_cap;
+    /* eight warps a block, a round of positions each, at most 16 blocks an SM
+     * (twice what is resident) */
+    uint64_t grid = (n + 255) / 256;
+    if (grid > 152ull * 16) grid = 152ull * 16;
+    if (I.saf) gs_locate<true><<<(unsigned)grid, 256, 0, st>>>(I, B);
+    else gs_locate<false><<<(unsigned)grid, 256, 0, st>>>(I, B);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }

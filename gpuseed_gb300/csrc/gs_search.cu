@@ -28,6 +28,7 @@
  *     after another, containment history in a per-read global array.
  */
 #include "gs_fm.cuh"
+#include "gs_scan.cuh"
 
 
 
@@ -501,59 +502,108 @@ __device__ __forceinline__ uint32_t gs_start_flags(uint32_t y, uint32_t c, bool 
 /* ------------------------------------------------------------------ */
 /* per-batch preparation: candidate slots and work items per read */
 
-__global__ void gs_prepare_kernel(const uint32_t *lengths, uint32_t n_reads, int k, int paired_kt,
-                                  uint64_t *slot_n, uint32_t *item_n)
+/* a read's slots (two a candidate) and work items */
+__device__ __forceinline__ void gs_read_counts(uint32_t L, int k, int paired_kt, uint32_t &slots,
+                                               uint32_t &items)
 {
-    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r > n_reads) return;
-    uint32_t n = 0;
-    if (r < n_reads && lengths[r] >= (uint32_t)k) n = lengths[r] - (uint32_t)k + 1u;
-    slot_n[r] = 2ull * n;
+    const uint32_t n = L >= (uint32_t)k ? L - (uint32_t)k + 1u : 0u;
+    slots = 2u * n;
     if (paired_kt) {
         /* windows s in [0, L-KT] (k >= KT, so L-KT+1 >= n) */
-        const uint32_t w = n ? lengths[r] - (uint32_t)paired_kt + 1u : 0u;
-        item_n[r] = (w + GS_PCHUNK - 1) / GS_PCHUNK;
+        const uint32_t w = n ? L - (uint32_t)paired_kt + 1u : 0u;
+        items = (w + GS_PCHUNK - 1) / GS_PCHUNK;
     } else {
-        item_n[r] = 2u * ((n + GS_CHUNK - 1) / GS_CHUNK);
+        items = 2u * ((n + GS_CHUNK - 1) / GS_CHUNK);
     }
 }
 
-/* the read of each work item, so that the start pass need not search
- * item_off for it: a thread per read, or the warp for a read of many items */
-__global__ void __launch_bounds__(256) gs_item_map_kernel(const uint32_t *item_off, uint32_t n_reads,
-                                                          uint32_t *item_read, uint64_t cap)
+__device__ __forceinline__ void gs_put_totals(const GsBatch &B, int at, const GsPart &t)
+{
+    if (threadIdx.x) return;
+    B.totals[at] = t.a;
+    B.totals[at + 1] = t.b;
+    if (B.h_totals) {
+        B.h_totals[at] = t.a;
+        B.h_totals[at + 1] = t.b;
+    }
+}
+
+__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_sum(GsBatch B, int paired_kt)
+{
+    uint32_t first, last;
+    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    unsigned long long a = 0, b = 0;
+    for (uint32_t r = first + threadIdx.x; r < last; r += GS_SCAN_THREADS) {
+        uint32_t slots, items;
+        gs_read_counts(B.lengths[r], B.k, paired_kt, slots, items);
+        a += slots;
+        b += items;
+    }
+    GsPart sum, total;
+    gs_block_scan(a, b, sum);
+    if (gs_parts_publish(B.parts, 0, sum, total)) gs_put_totals(B, 0, total);
+}
+
+/* Offsets of the reads' slots and work items, and the read of each work
+ * item, so that the start pass need not search item_off for it (a thread per
+ * read, or the warp for a read of many items). */
+__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_scan(GsBatch B, int paired_kt)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t a = 0, e = 0;
-    if (r < n_reads) {
-        a = item_off[r];
-        e = item_off[r + 1];
+    uint32_t first, last;
+    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    GsPart run = {0ull, 0ull};
+    if (gridDim.x > 1) run = B.parts.part[blockIdx.x];
+    for (uint32_t r0 = first; r0 < last; r0 += GS_SCAN_THREADS) {
+        const uint32_t r = r0 + threadIdx.x;
+        uint32_t slots = 0, items = 0;
+        if (r < last) gs_read_counts(B.lengths[r], B.k, paired_kt, slots, items);
+        GsPart t;
+        const GsPart x = gs_block_scan(slots, items, t);
+        const uint32_t a = (uint32_t)(run.b + x.b), e = a + items;
+        if (r < last) {
+            B.slot_off[r] = run.a + x.a;
+            B.item_off[r] = a;
+        }
+        if (B.item_read) {
+            const bool big = items > 16u;
+            if (!big)
+                for (uint32_t i = a; i < e; i++)
+                    if (i < B.item_read_cap) B.item_read[i] = r;
+            uint32_t m = __ballot_sync(0xffffffffu, big);
+            while (m) {
+                const int src = __ffs(m) - 1;
+                m &= m - 1u;
+                const uint32_t a1 = __shfl_sync(0xffffffffu, a, src), e1 = __shfl_sync(0xffffffffu, e, src);
+                for (uint32_t i = a1 + (uint32_t)lane; i < e1; i += 32)
+                    if (i < B.item_read_cap) B.item_read[i] = r - (uint32_t)lane + (uint32_t)src;
+            }
+        }
+        run.a += t.a;
+        run.b += t.b;
     }
-    const bool big = e - a > 16u;
-    if (!big)
-        for (uint32_t i = a; i < e; i++)
-            if (i < cap) item_read[i] = r;
-    uint32_t m = __ballot_sync(0xffffffffu, big);
-    while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1u;
-        const uint32_t a1 = __shfl_sync(0xffffffffu, a, src), e1 = __shfl_sync(0xffffffffu, e, src);
-        for (uint32_t i = a1 + (uint32_t)lane; i < e1; i += 32)
-            if (i < cap) item_read[i] = r - (uint32_t)lane + (uint32_t)src;
+    if (last == B.n_reads && (first < last || blockIdx.x == 0)) {
+        /* the block that holds the last read */
+        if (threadIdx.x == 0) {
+            B.slot_off[B.n_reads] = run.a;
+            B.item_off[B.n_reads] = (uint32_t)run.b;
+        }
+        if (gridDim.x == 1) gs_put_totals(B, 0, run);
     }
 }
 
 int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t st)
 {
-    uint32_t n = b.n_reads + 1;
     /* the batched start pass pairs each window's two candidates when they
      * are longer than the paired table's strings */
     b.paired = kernel == GS_KERNEL_BATCHED && I.kmerx && b.k > I.kx;
-    /* counts are written in place and scanned into offsets */
-    gs_prepare_kernel<<<(n + 255) / 256, 256, 0, st>>>(b.lengths, b.n_reads, b.k,
-                                                        b.paired ? I.kx : 0, b.slot_off,
-                                                        b.item_off);
+    const int kt = b.paired ? I.kx : 0;
+    const uint32_t parts = gs_parts_of(b.n_reads);
+    if (parts > 1) {
+        gs_prepare_sum<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
+        GS_CUDA(cudaGetLastError());
+    }
+    gs_prepare_scan<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }
@@ -1840,9 +1890,6 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         if (need < grid * 8) grid = (need + 7) / 8;
     }
     if (grid == 0) grid = 1;
-    gs_item_map_kernel<<<(B.n_reads + 255) / 256, 256, 0, st>>>(B.item_off, B.n_reads, B.item_read,
-                                                                B.item_read_cap);
-    GS_CUDA(cudaGetLastError());
     GS_CUDA(cudaMemsetAsync(B.queue, 0, sizeof(uint32_t), st));
     GS_CUDA(cudaMemsetAsync(B.queue + 2, 0, 2 * sizeof(uint32_t), st));
     B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, 64u, GS_WALKER_CHUNK);
