@@ -206,7 +206,10 @@ struct gs_ctx {
     uint64_t walk_counts[7];   /* count_work pass: gs_ctx_last_walk_counts */
     void *cub_tmp; size_t cap_cub;
     uint64_t *h_small;          /* pinned scalars (GS_H_*) */
-    uint32_t last_items;        /* work items of the last sized pass */
+    uint64_t last_slots;        /* slots, work items and reads of the last pass */
+    uint32_t last_items, last_reads;
+    char *h_stage; size_t cap_stage;   /* pinned: a small gs_seed batch's input, as one copy */
+    char *d_stage; size_t cap_d_stage;
     /* host result */
     uint64_t *h_seed_off; size_t cap_h_so;
     uint64_t *h_pos_off; size_t cap_h_po;
@@ -216,6 +219,7 @@ struct gs_ctx {
     uint64_t n_seeds, n_pos;
     int have_host, have_dev;
     float t_search, t_total;
+    int timing;                 /* events recorded, elapsed times not yet taken: GS_TIMING_* */
     /* captured pass */
     cudaGraphExec_t gexec;
     const char *g_seqs;
@@ -223,6 +227,7 @@ struct gs_ctx {
     const uint32_t *g_lens;
     uint32_t g_n;
     uint32_t g_gen;   /* index generation the graph was captured with */
+    uint64_t g_key;   /* and the workspace (workspace_key) */
     gs_params g_params;
     uint32_t g_items;
 };
@@ -326,6 +331,8 @@ extern "C" void gs_ctx_free(gs_ctx *c)
     cudaFree(c->d_work);
     cudaFree(c->cub_tmp);
     cudaFreeHost(c->h_small);
+    cudaFreeHost(c->h_stage);
+    cudaFree(c->d_stage);
     cudaFreeHost(c->h_seed_off); cudaFreeHost(c->h_pos_off);
     cudaFreeHost(c->h_seeds); cudaFreeHost(c->h_pos);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -382,9 +389,25 @@ extern "C" int gs_ctx_last_text_jobs(gs_ctx *c, uint64_t *n_jobs, uint64_t *capa
     return GS_OK;
 }
 
+#define GS_TIMING_PASS 1    /* ev0, ev_s0, ev_s1, ev1 */
+#define GS_TIMING_GRAPH 2   /* ev0, ev1: the whole pass stands for the search too */
+
+/* elapsed times of the last pass from its events, when they are asked for */
+static void take_timing(gs_ctx *c)
+{
+    if (c->timing) cudaEventElapsedTime(&c->t_total, c->ev0, c->ev1);
+    if (c->timing == GS_TIMING_PASS) cudaEventElapsedTime(&c->t_search, c->ev_s0, c->ev_s1);
+    if (c->timing == GS_TIMING_GRAPH) c->t_search = c->t_total;
+    c->timing = 0;
+}
+
 extern "C" int gs_ctx_last_timing(gs_ctx *c, float *search_ms, float *total_ms)
 {
     if (!c) return GS_EINVAL;
+    if (c->timing) {
+        GS_ON_DEVICE(gs_index_device(c->idx));
+        take_timing(c);
+    }
     if (search_ms) *search_ms = c->t_search;
     if (total_ms) *total_ms = c->t_total;
     return GS_OK;
@@ -469,29 +492,11 @@ static int check_params(const gs_params *p)
         if (_rc) return _rc;     \
     } while (0)
 
-/* One pass over n_reads device-resident reads.  fetch: copy the result to
- * the context's host arrays.  co (gs_seed's chunks): instead, copy this
- * chunk's result into the batch's host arrays on st_copy, batch-wide, and
- * return without waiting for that copy. */
-static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
-                        const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p,
-                        int fetch, GsChunkOut *co = NULL)
+/* the arguments of a pass that its sizes do not change; zero: the prepare
+ * kernels clear the queue and the first `mask_words` words of the record mask */
+static void batch_of(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
+                     const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p, GsBatch &B)
 {
-    const GsDevIndex &I = *gs_index_dev(c->idx);
-    cudaStream_t st = c->st;
-    c->have_host = c->have_dev = 0;
-    c->n_reads = n_reads;
-    size_t nr1 = (size_t)n_reads + 1;
-    RC(grow(c->slot_off, c->cap_slot_off, nr1, c->st));
-    RC(grow(c->item_off, c->cap_item_off, nr1, c->st));
-    RC(grow(c->rd_nf, c->cap_nf, nr1, c->st));
-    RC(grow(c->rd_nr, c->cap_nr, nr1, c->st));
-    RC(grow(c->rd_nseeds, c->cap_rns, nr1, c->st));
-    RC(grow(c->rd_npos, c->cap_rnp, nr1, c->st));
-    RC(grow(c->seed_off, c->cap_so, nr1, c->st));
-    RC(grow(c->pos_off, c->cap_po, nr1, c->st));
-
-    GsBatch B;
     memset(&B, 0, sizeof(B));
     B.seqs = d_seqs;
     B.offsets = d_offsets;
@@ -504,6 +509,250 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     B.max_occ = p->max_occ > 0 ? (uint32_t)p->max_occ : 0u;
     B.mem_next = p->mem_next;
     B.queue = c->queue;
+    B.parts = c->parts;
+    B.totals = c->d_totals;
+    B.h_totals = &c->h_small[GS_H_TOTALS];
+    B.slot_off = c->slot_off;
+    B.item_off = c->item_off;
+    B.rd_nf = c->rd_nf;
+    B.rd_nr = c->rd_nr;
+    B.rd_nseeds = c->rd_nseeds;
+    B.rd_npos = c->rd_npos;
+    B.seed_off = c->seed_off;
+    B.pos_off = c->pos_off;
+}
+
+static int grow_reads(gs_ctx *c, size_t nr1)
+{
+    RC(grow(c->slot_off, c->cap_slot_off, nr1, c->st));
+    RC(grow(c->item_off, c->cap_item_off, nr1, c->st));
+    RC(grow(c->rd_nf, c->cap_nf, nr1, c->st));
+    RC(grow(c->rd_nr, c->cap_nr, nr1, c->st));
+    RC(grow(c->rd_nseeds, c->cap_rns, nr1, c->st));
+    RC(grow(c->rd_npos, c->cap_rnp, nr1, c->st));
+    RC(grow(c->seed_off, c->cap_so, nr1, c->st));
+    RC(grow(c->pos_off, c->cap_po, nr1, c->st));
+    return GS_OK;
+}
+
+static int grow_outputs(gs_ctx *c, uint64_t n_seeds, uint64_t n_pos)
+{
+    RC(grow(c->seeds, c->cap_seeds, n_seeds + 1, c->st));
+    RC(grow(c->seed_pos, c->cap_seed_pos, n_seeds + 1, c->st));
+    RC(grow(c->pos, c->cap_pos, n_pos + 1, c->st));
+    RC(grow(c->pmap, c->cap_pmap, n_pos + 1, c->st));
+    RC(grow(c->tile_seed, c->cap_tile_seed, c->cap_pos / 32 + 1, c->st));
+    return GS_OK;
+}
+
+/* the output buffers as they are, with all their room */
+static void bind_outputs(gs_ctx *c, GsBatch &B)
+{
+    B.seeds = c->seeds;
+    B.seed_pos = c->seed_pos;
+    B.pos = c->pos;
+    B.pmap = c->pmap;
+    B.tile_seed = c->tile_seed;
+    B.seed_cap = c->cap_seeds < c->cap_seed_pos ? c->cap_seeds : c->cap_seed_pos;
+    B.pos_cap = c->cap_pos < c->cap_pmap ? c->cap_pos : c->cap_pmap;
+}
+
+static int grow_fetch(gs_ctx *c, size_t nr1, uint64_t n_seeds, uint64_t n_pos)
+{
+    RC(grow_host(c->h_seed_off, c->cap_h_so, nr1));
+    RC(grow_host(c->h_pos_off, c->cap_h_po, nr1));
+    RC(grow_host(c->h_seeds, c->cap_h_seeds, n_seeds + 1));
+    RC(grow_host(c->h_pos, c->cap_h_pos, n_pos + 1));
+    return GS_OK;
+}
+
+/* The batched search's walker and text-job buffers for n_items work items
+ * (B.paired set).  Entries per 16 work items of 31 candidates (a paired item
+ * of 30 windows counts as two): as asked, or automatic -- 16 per item with a
+ * start table (forced codes settle most candidates), all 31 without, and
+ * 1.5x more after a pass that filled its buffer. */
+static int size_walkers(gs_ctx *c, const GsDevIndex &I, const gs_params *p, uint32_t n_items, GsBatch &B)
+{
+    c->last_walker_cap = 0;
+    c->last_text_cap = 0;
+    if (p->walker_slots < 0) return GS_OK;
+    const uint32_t least = B.paired ? 256u : 512u;
+    uint64_t per16 = p->walker_slots ? (uint64_t)p->walker_slots : least;
+    if (!p->walker_slots && c->walker_per16 > per16) per16 = c->walker_per16;
+    const uint64_t units = (uint64_t)n_items * (B.paired ? 2u : 1u);
+    uint64_t want = (units * per16 + 15u) / 16u + 32u;
+    /* a start-pass warp reserves 64 entries or more at a time */
+    if (!p->walker_slots) want += 64ull * (n_items < 8192u ? n_items : 8192u);
+    if (want > (1ull << 31)) want = 1ull << 31;   /* 32-bit buffer counter */
+    RC(grow(c->walkers, c->cap_walkers, (size_t)want, c->st));
+    B.walkers = c->walkers;
+    B.walker_cap = want;
+    c->last_walker_cap = want;
+    /* walkers handed to the text pass: two per work item is far above what
+     * reads with a few differences per 100 bases need; without room a walker
+     * walks on in the walk pass */
+    if (I.text_min) {
+        uint64_t tw = units * 2u + 64u;
+        if (tw > (1ull << 31)) tw = 1ull << 31;
+        RC(grow(c->text_jobs, c->cap_text_jobs, (size_t)tw, c->st));
+        B.text_jobs = c->text_jobs;
+        B.text_cap = tw;
+        c->last_text_cap = tw;
+    }
+    return GS_OK;
+}
+
+/* what the end of a batched pass leaves in the queue words: the diagnostics,
+ * and a larger walker buffer next time where this one was full */
+static uint32_t read_queue(gs_ctx *c, const gs_params *p)
+{
+    const uint32_t *queue = (const uint32_t *)&c->h_small[GS_H_QUEUE];
+    c->last_walkers = c->last_walker_cap ? queue[2] : 0;
+    c->last_text_jobs = c->last_text_cap ? queue[5] : 0;
+    if (!p->walker_slots && c->last_walker_cap && c->last_walkers >= c->last_walker_cap &&
+        c->walker_per16 < 512u) {
+        c->walker_per16 = c->walker_per16 ? c->walker_per16 + c->walker_per16 / 2 : 384u;
+        if (c->walker_per16 > 512u) c->walker_per16 = 512u;
+    }
+    return queue[1];
+}
+
+static int walk_limit_error(void)
+{
+    gs_set_error("sampled-SA walk exceeded seq_len+2 steps: index inconsistent");
+    return GS_EWALK;
+}
+
+static int too_many_positions(uint64_t n_pos)
+{
+    gs_set_error("batch emits %llu positions; split the batch", (unsigned long long)n_pos);
+    return GS_EOVERFLOW;
+}
+
+/* The result of a small pass into the context's host arrays (mapped pinned
+ * memory), sizes read on the device: no copy has to wait for the host to
+ * learn them. */
+__global__ void __launch_bounds__(256) gs_copy_out_kernel(GsBatch B, uint64_t *seed_off, uint64_t *pos_off,
+                                                          uint4 *seeds, uint64_t seed_cap, uint32_t *pos,
+                                                          uint64_t pos_cap, uint32_t *queue)
+{
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    if (t < 8) queue[t] = B.queue[t];
+    if (!seed_off) return;
+    const uint64_t n_seeds = B.totals[2], n_pos = B.totals[3];
+    /* more than there is room for, here or there: the host makes room */
+    if (n_seeds > seed_cap || n_pos > pos_cap || n_seeds > B.seed_cap || n_pos > B.pos_cap) return;
+    for (uint64_t i = t; i <= B.n_reads; i += stride) {
+        seed_off[i] = B.seed_off[i];
+        pos_off[i] = B.pos_off[i];
+    }
+    const uint4 *src = reinterpret_cast<const uint4 *>(B.seeds);
+    for (uint64_t i = t; i < 2 * n_seeds; i += stride) seeds[i] = src[i];
+    for (uint64_t i = t; i < n_pos; i += stride) pos[i] = B.pos[i];
+}
+
+#define GS_RETRY 1   /* run_once: the batch needs more room than assumed */
+
+/* A whole batched pass with one synchronisation, for batches whose launches
+ * and waits would take as long as their kernels: everything is enqueued on
+ * sizes known beforehand.  exact: n_slots and n_items are the batch's
+ * (gs_seed counts them on the host); else they are what the context has
+ * room for or expects (see run_device), and a batch that needs more returns
+ * GS_RETRY.  Seeds and positions are written to what room there is, and once
+ * more when that was too little. */
+static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, const uint32_t *d_lengths,
+                    uint32_t n_reads, const gs_params *p, int fetch, uint64_t n_slots,
+                    uint32_t n_items, bool exact)
+{
+    const GsDevIndex &I = *gs_index_dev(c->idx);
+    cudaStream_t st = c->st;
+    const size_t nr1 = (size_t)n_reads + 1;
+    c->have_host = c->have_dev = 0;
+    c->n_reads = n_reads;
+    RC(grow_reads(c, nr1));
+    if (exact) {
+        RC(grow(c->slots, c->cap_slots, n_slots + 1, st));
+        RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, st));
+        RC(grow(c->item_read, c->cap_item_read, (size_t)n_items + 1, st));
+    }
+    /* a read has a handful of seeds, a seed a position or two */
+    const uint64_t want_s = 8ull * n_reads + n_slots / 32 + 256;
+    const uint64_t want_p = 16ull * n_reads + n_slots / 16 + 1024;
+    RC(grow_outputs(c, want_s, want_p));
+    if (fetch) RC(grow_fetch(c, nr1, want_s, want_p));
+    memset(c->work, 0, sizeof(c->work));
+    memset(c->walk_counts, 0, sizeof(c->walk_counts));
+    GsBatch B;
+    batch_of(c, d_seqs, d_offsets, d_lengths, n_reads, p, B);
+    B.item_read = c->item_read;
+    B.item_read_cap = c->cap_item_read;
+    B.slots = c->slots;
+    B.slot_cap = c->cap_slots;
+    B.recmask = c->recmask;
+    B.clear = 1;
+    B.clear_words = ((exact ? n_slots : c->cap_slots) + 31) / 32 + 1;
+    B.item_cap = n_items;
+    GS_CUDA(cudaEventRecord(c->ev0, st));
+    RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
+    RC(size_walkers(c, I, p, n_items, B));
+    GS_CUDA(cudaEventRecord(c->ev_s0, st));
+    RC(gs_launch_search(I, B, GS_KERNEL_BATCHED, p->queue_chunk, p->ctas_per_sm, n_items, st));
+    GS_CUDA(cudaEventRecord(c->ev_s1, st));
+    RC(gs_launch_finalize_count(I, B, st));
+    bind_outputs(c, B);
+    for (bool emit = true;;) {
+        if (emit) {
+            RC(gs_launch_finalize_emit(I, B, st));
+            RC(gs_launch_locate(I, B, UINT64_MAX, st));
+        }
+        const unsigned grid = n_reads < 152u * 16u ? (n_reads + 15u) / 16u : 152u;
+        gs_copy_out_kernel<<<grid, 256, 0, st>>>(
+            B, fetch ? c->h_seed_off : NULL, c->h_pos_off, (uint4 *)c->h_seeds, c->cap_h_seeds, c->h_pos,
+            c->cap_h_pos, (uint32_t *)&c->h_small[GS_H_QUEUE]);
+        GS_CUDA(cudaGetLastError());
+        GS_CUDA(cudaEventRecord(c->ev1, st));
+        GS_CUDA(cudaStreamSynchronize(st));
+        c->n_seeds = c->h_small[GS_H_TOTALS + 2];
+        c->n_pos = c->h_small[GS_H_TOTALS + 3];
+        const uint32_t flags = ((const uint32_t *)&c->h_small[GS_H_QUEUE])[1];
+        if (!exact && (flags & GS_FLAG_OVERFLOW)) return GS_RETRY;
+        if (c->n_pos > 0xffffffffull * 4) return too_many_positions(c->n_pos);
+        emit = c->n_seeds > B.seed_cap || c->n_pos > B.pos_cap;
+        const bool copy = fetch && (c->n_seeds > c->cap_h_seeds || c->n_pos > c->cap_h_pos);
+        if (!emit && !copy) break;
+        if (emit) {
+            RC(grow_outputs(c, c->n_seeds, c->n_pos));
+            bind_outputs(c, B);
+        }
+        if (copy) RC(grow_fetch(c, nr1, c->n_seeds, c->n_pos));
+    }
+    c->last_items = (uint32_t)c->h_small[GS_H_TOTALS + 1];
+    c->last_slots = c->h_small[GS_H_TOTALS];
+    c->last_reads = n_reads;
+    c->timing = GS_TIMING_PASS;
+    if (read_queue(c, p) & GS_FLAG_WALK) return walk_limit_error();
+    c->have_dev = 1;
+    c->have_host = fetch;
+    return GS_OK;
+}
+
+/* One pass over n_reads device-resident reads.  fetch: copy the result to
+ * the context's host arrays.  co (gs_seed's chunks): instead, copy this
+ * chunk's result into the batch's host arrays on st_copy, batch-wide, and
+ * return without waiting for that copy. */
+static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
+                        const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p,
+                        int fetch, GsChunkOut *co = NULL)
+{
+    const GsDevIndex &I = *gs_index_dev(c->idx);
+    cudaStream_t st = c->st;
+    c->have_host = c->have_dev = 0;
+    c->n_reads = n_reads;
+    const size_t nr1 = (size_t)n_reads + 1;
+    RC(grow_reads(c, nr1));
+    GsBatch B;
+    batch_of(c, d_seqs, d_offsets, d_lengths, n_reads, p, B);
     B.work = p->count_work ? c->d_work : NULL;
     memset(c->work, 0, sizeof(c->work));
     memset(c->walk_counts, 0, sizeof(c->walk_counts));
@@ -511,11 +760,6 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     GS_CUDA(cudaEventRecord(c->ev0, st));
     if (B.work) GS_CUDA(cudaMemsetAsync(c->d_work, 0, 128, st));
     GS_CUDA(cudaMemsetAsync(c->queue, 0, 32, st));
-    B.parts = c->parts;
-    B.totals = c->d_totals;
-    B.h_totals = &c->h_small[GS_H_TOTALS];
-    B.slot_off = c->slot_off;
-    B.item_off = c->item_off;
     /* the item map before its size is known: what there is, and the rest
      * once it is */
     if (p->kernel == GS_KERNEL_BATCHED) {
@@ -534,6 +778,8 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     const uint64_t n_slots = c->h_small[GS_H_TOTALS];
     const uint32_t n_items = (uint32_t)(c->h_small[GS_H_TOTALS + 1] & 0xffffffffu);
     c->last_items = n_items;
+    c->last_slots = n_slots;
+    c->last_reads = n_reads;
     RC(grow(c->slots, c->cap_slots, n_slots + 1, c->st));
     RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, c->st));
     B.slots = c->slots;
@@ -560,35 +806,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     }
     c->last_walker_cap = 0;
     c->last_text_cap = 0;
-    if (p->kernel == GS_KERNEL_BATCHED && p->walker_slots >= 0) {
-        /* entries per 16 work items of 31 candidates (a paired item of 30
-         * windows counts as two): as asked, or automatic -- 16 per item
-         * with a start table (forced codes settle most candidates), all 31
-         * without, and 1.5x more after a pass that filled its buffer */
-        const uint32_t least = B.paired ? 256u : 512u;
-        uint64_t per16 = p->walker_slots ? (uint64_t)p->walker_slots : least;
-        if (!p->walker_slots && c->walker_per16 > per16) per16 = c->walker_per16;
-        const uint64_t units = (uint64_t)n_items * (B.paired ? 2u : 1u);
-        uint64_t want = (units * per16 + 15u) / 16u + 32u;
-        /* a start-pass warp reserves 64 entries or more at a time */
-        if (!p->walker_slots) want += 64ull * (n_items < 8192u ? n_items : 8192u);
-        if (want > (1ull << 31)) want = 1ull << 31;   /* 32-bit buffer counter */
-        RC(grow(c->walkers, c->cap_walkers, (size_t)want, c->st));
-        B.walkers = c->walkers;
-        B.walker_cap = want;
-        c->last_walker_cap = want;
-        /* walkers handed to the text pass: two per work item is far above
-         * what reads with a few differences per 100 bases need; without
-         * room a walker walks on in the walk pass */
-        if (I.text_min) {
-            uint64_t tw = units * 2u + 64u;
-            if (tw > (1ull << 31)) tw = 1ull << 31;
-            RC(grow(c->text_jobs, c->cap_text_jobs, (size_t)tw, c->st));
-            B.text_jobs = c->text_jobs;
-            B.text_cap = tw;
-            c->last_text_cap = tw;
-        }
-    }
+    if (p->kernel == GS_KERNEL_BATCHED) RC(size_walkers(c, I, p, n_items, B));
 
     GS_CUDA(cudaEventRecord(c->ev_s0, st));
     RC(gs_launch_search(I, B, p->kernel, p->queue_chunk, p->ctas_per_sm, n_items, st));
@@ -597,37 +815,15 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
      * this chunk searched */
     if (co && co->wait_d2h) GS_CUDA(cudaStreamWaitEvent(st, c->ev_d2h, 0));
 
-    B.rd_nf = c->rd_nf;
-    B.rd_nr = c->rd_nr;
-    B.rd_nseeds = c->rd_nseeds;
-    B.rd_npos = c->rd_npos;
     RC(gs_launch_finalize_count(I, B, st));
     GS_CUDA(cudaStreamSynchronize(st));
     const uint64_t n_seeds = c->h_small[GS_H_TOTALS + 2], n_pos = c->h_small[GS_H_TOTALS + 3];
-    if (n_pos > 0xffffffffull * 4) {
-        gs_set_error("batch emits %llu positions; split the batch", (unsigned long long)n_pos);
-        return GS_EOVERFLOW;
-    }
-    RC(grow(c->seeds, c->cap_seeds, n_seeds + 1, c->st));
-    RC(grow(c->seed_pos, c->cap_seed_pos, n_seeds + 1, c->st));
-    RC(grow(c->pos, c->cap_pos, n_pos + 1, c->st));
-    RC(grow(c->pmap, c->cap_pmap, n_pos + 1, c->st));
-    RC(grow(c->tile_seed, c->cap_tile_seed, c->cap_pos / 32 + 1, c->st));
-    B.seed_off = c->seed_off;
-    B.pos_off = c->pos_off;
-    B.seeds = c->seeds;
-    B.seed_pos = c->seed_pos;
-    B.pos = c->pos;
-    B.pmap = c->pmap;
-    B.tile_seed = c->tile_seed;
+    if (n_pos > 0xffffffffull * 4) return too_many_positions(n_pos);
+    RC(grow_outputs(c, n_seeds, n_pos));
+    bind_outputs(c, B);
     B.seed_cap = n_seeds + 1;
     B.pos_cap = n_pos + 1;
-    if (fetch) {
-        RC(grow_host(c->h_seed_off, c->cap_h_so, nr1));
-        RC(grow_host(c->h_pos_off, c->cap_h_po, nr1));
-        RC(grow_host(c->h_seeds, c->cap_h_seeds, n_seeds + 1));
-        RC(grow_host(c->h_pos, c->cap_h_pos, n_pos + 1));
-    }
+    if (fetch) RC(grow_fetch(c, nr1, n_seeds, n_pos));
     if (co) {
         B.base_s = co->base_s;
         B.base_p = co->base_p;
@@ -684,23 +880,11 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
         GS_CUDA(cudaMemcpyAsync(c->h_pos, c->pos, n_pos * 4, cudaMemcpyDeviceToHost, st));
     GS_CUDA(cudaStreamSynchronize(st));
     if (fetch) GS_CUDA(cudaStreamSynchronize(c->st_copy));
-    const uint32_t *queue = (const uint32_t *)&c->h_small[GS_H_QUEUE];
-    const uint32_t flags = queue[1];
-    c->last_walkers = c->last_walker_cap ? queue[2] : 0;
-    c->last_text_jobs = c->last_text_cap ? queue[5] : 0;
-    if (!p->walker_slots && c->last_walker_cap && c->last_walkers >= c->last_walker_cap &&
-        c->walker_per16 < 512u) {
-        c->walker_per16 = c->walker_per16 ? c->walker_per16 + c->walker_per16 / 2 : 384u;
-        if (c->walker_per16 > 512u) c->walker_per16 = 512u;
-    }
+    const uint32_t flags = read_queue(c, p);
     if (B.work) memcpy(c->work, &c->h_small[6], sizeof(c->work));
     if (B.work) memcpy(c->walk_counts, &c->h_small[16], sizeof(c->walk_counts));
-    cudaEventElapsedTime(&c->t_search, c->ev_s0, c->ev_s1);
-    cudaEventElapsedTime(&c->t_total, c->ev0, c->ev1);
-    if (flags & GS_FLAG_WALK) {
-        gs_set_error("sampled-SA walk exceeded seq_len+2 steps: index inconsistent");
-        return GS_EWALK;
-    }
+    c->timing = GS_TIMING_PASS;
+    if (flags & GS_FLAG_WALK) return walk_limit_error();
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;
@@ -736,31 +920,15 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     const GsDevIndex &I = *gs_index_dev(c->idx);
     cudaStream_t st = c->st;
     GsBatch B;
-    memset(&B, 0, sizeof(B));
-    B.seqs = d_seqs;
-    B.offsets = d_offsets;
-    B.lengths = d_lengths;
-    B.n_reads = n_reads;
-    B.k = p->k;
-    B.smem = p->smem ? 1 : 0;
-    B.n_mode = p->n_mode;
-    B.lf_mode = p->lf_mode;
-    B.max_occ = p->max_occ > 0 ? (uint32_t)p->max_occ : 0u;
-    B.mem_next = p->mem_next;
-    B.queue = c->queue;
-    GS_CUDA(cudaMemsetAsync(c->queue, 0, 32, st));
-    B.parts = c->parts;
-    B.totals = c->d_totals;
-    B.h_totals = &c->h_small[GS_H_TOTALS];
-    B.slot_off = c->slot_off;
-    B.item_off = c->item_off;
+    batch_of(c, d_seqs, d_offsets, d_lengths, n_reads, p, B);
     B.item_read = c->item_read;
     B.item_read_cap = c->cap_item_read;
-    RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
     B.slots = c->slots;
     B.slot_cap = c->cap_slots;
     B.recmask = c->recmask;
-    GS_CUDA(cudaMemsetAsync(c->recmask, 0, ((c->cap_slots + 31) / 32 + 1) * sizeof(uint32_t), st));
+    B.clear = 1;
+    B.clear_words = (c->cap_slots + 31) / 32 + 1;
+    RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
     B.item_cap = c->g_items;
     /* the walker buffer as the sizing pass left it; walkers beyond it are
      * left to the leftover pass */
@@ -773,31 +941,31 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
         }
     }
     RC(gs_launch_search(I, B, GS_KERNEL_BATCHED, p->queue_chunk, p->ctas_per_sm, 0, st));
-    B.rd_nf = c->rd_nf;
-    B.rd_nr = c->rd_nr;
-    B.rd_nseeds = c->rd_nseeds;
-    B.rd_npos = c->rd_npos;
     RC(gs_launch_finalize_count(I, B, st));
-    B.seed_off = c->seed_off;
-    B.pos_off = c->pos_off;
-    B.seeds = c->seeds;
-    B.seed_pos = c->seed_pos;
-    B.pos = c->pos;
-    B.pmap = c->pmap;
-    B.tile_seed = c->tile_seed;
-    B.seed_cap = c->cap_seeds < c->cap_seed_pos ? c->cap_seeds : c->cap_seed_pos;
-    B.pos_cap = c->cap_pos < c->cap_pmap ? c->cap_pos : c->cap_pmap;
+    bind_outputs(c, B);
     RC(gs_launch_finalize_emit(I, B, st));
     RC(gs_launch_locate(I, B, UINT64_MAX, st));
     RC(fetch_small(&c->h_small[GS_H_QUEUE], c->queue, 32, st));
     return GS_OK;
 }
 
+/* A captured pass holds the workspace's addresses and sizes: another pass
+ * on the context may have replaced a buffer since. */
+static uint64_t workspace_key(const gs_ctx *c)
+{
+    const void *const p[] = {c->slot_off, c->item_off, c->item_read, c->rd_nf, c->rd_nr, c->rd_nseeds,
+                             c->rd_npos, c->seed_off, c->pos_off, c->slots, c->recmask, c->walkers,
+                             c->text_jobs, c->seeds, c->seed_pos, c->pos, c->pmap, c->tile_seed};
+    uint64_t h = 1469598103934665603ull;
+    for (const void *q : p) h = (h ^ (uint64_t)(uintptr_t)q) * 1099511628211ull;
+    return h;
+}
+
 static bool same_graph(const gs_ctx *c, const char *s, const uint64_t *o, const uint32_t *l,
                        uint32_t n, const gs_params *p)
 {
     return c->gexec && c->g_seqs == s && c->g_offs == o && c->g_lens == l && c->g_n == n &&
-           c->g_gen == gs_index_generation(c->idx) &&
+           c->g_gen == gs_index_generation(c->idx) && c->g_key == workspace_key(c) &&
            memcmp(&c->g_params, p, sizeof(gs_params)) == 0;
 }
 
@@ -816,16 +984,12 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
         bool fits = !(flags & GS_FLAG_OVERFLOW) && ns <= c->cap_seeds && ns <= c->cap_seed_pos &&
                     np <= c->cap_pos && np <= c->cap_pmap;
         if (fits) {
-            if (flags & GS_FLAG_WALK) {
-                gs_set_error("sampled-SA walk exceeded seq_len+2 steps: index inconsistent");
-                return GS_EWALK;
-            }
+            if (flags & GS_FLAG_WALK) return walk_limit_error();
             c->n_reads = n_reads;
             c->n_seeds = ns;
             c->n_pos = np;
             c->have_dev = 1;
-            cudaEventElapsedTime(&c->t_total, c->ev0, c->ev1);
-            c->t_search = c->t_total;
+            c->timing = GS_TIMING_GRAPH;
             if (fetch) RC(fetch_result(c));
             return GS_OK;
         }
@@ -859,8 +1023,36 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
     c->g_lens = d_lengths;
     c->g_n = n_reads;
     c->g_gen = gs_index_generation(c->idx);
+    c->g_key = workspace_key(c);
     c->g_params = *p;
     return GS_OK;
+}
+
+/* A pass over device-resident reads whose sizes the host does not know.  A
+ * context that has run before expects as many slots and work items a read
+ * as its last pass had, and a quarter more; where its buffers hold that, the
+ * batch runs without waiting for its sizes, and again with them if it needed
+ * more.  For up to GS_ONCE_READS reads: two waits of about 10 us each are
+ * what it saves (60,007 short reads 527 -> 457 us), and a batch that
+ * has to run again pays for little. */
+#define GS_ONCE_READS (1u << 17)
+#define GS_ONCE_SLOTS (1ull << 26)   /* the record mask is cleared over all the room there is */
+
+static int run_device(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
+                      const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p, int fetch)
+{
+    if (p->kernel == GS_KERNEL_BATCHED && !p->count_work && n_reads && n_reads <= GS_ONCE_READS &&
+        c->last_reads && c->slots && c->item_read && c->cap_slots <= GS_ONCE_SLOTS) {
+        const double per = 1.25 * (double)n_reads / (double)c->last_reads;
+        const uint64_t slots = (uint64_t)(per * (double)c->last_slots) + 1;
+        const uint64_t items = (uint64_t)(per * (double)c->last_items) + 1;
+        if (slots <= c->cap_slots && items <= c->cap_item_read && items <= 0xffffffffull) {
+            const int rc = run_once(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch, slots,
+                                    (uint32_t)items, false);
+            if (rc != GS_RETRY) return rc;
+        }
+    }
+    return run_pipeline(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch);
 }
 
 extern "C" int gs_seed_device(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
@@ -875,7 +1067,7 @@ extern "C" int gs_seed_device(gs_ctx *c, const char *d_seqs, const uint64_t *d_o
     GS_ON_DEVICE(gs_index_device(c->idx));
     if (p->graph && p->kernel == GS_KERNEL_BATCHED && !p->count_work && n_reads)
         return run_graph(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch_to_host);
-    return run_pipeline(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch_to_host);
+    return run_device(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch_to_host);
 }
 
 /* A large batch whose reads lie in order in `seqs` runs as chunks of reads:
@@ -942,9 +1134,11 @@ static int seed_chunked(gs_ctx *c, const char *seqs, const uint64_t *offsets, ui
         walkers += c->last_walkers;
         text_jobs += c->last_text_jobs;
         for (int w = 0; w < 4; w++) work[w] += c->work[w];
+        take_timing(c);
         t_search += c->t_search;
         t_total += c->t_total;
     }
+    c->timing = 0;
     /* no copy may outlive the call: the caller owns the host buffers */
     cudaStreamSynchronize(c->st_h2d);
     cudaStreamSynchronize(c->st_copy);
@@ -968,6 +1162,12 @@ static int seed_chunked(gs_ctx *c, const char *seqs, const uint64_t *offsets, ui
     return GS_OK;
 }
 
+/* gs_seed batches that the host sizes: at a few nanoseconds a read and a
+ * copy of the input into pinned memory, against the launches and the wait
+ * that size it on the device (about 40 us) */
+#define GS_HOST_READS 8192u
+#define GS_STAGE_BYTES ((uint64_t)4 << 20)
+
 extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
                        const uint32_t *lengths, uint32_t n_reads, const gs_params *p)
 {
@@ -977,6 +1177,33 @@ extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
     }
     RC(check_params(p));
     GS_ON_DEVICE(gs_index_device(c->idx));
+    if (n_reads && n_reads <= GS_HOST_READS && p->kernel == GS_KERNEL_BATCHED && !p->count_work) {
+        /* few enough reads to size the pass here: their slots, work items
+         * and the end of the last base */
+        const GsDevIndex &I = *gs_index_dev(c->idx);
+        const int kt = gs_paired_len(I, p->kernel, p->k);
+        uint64_t slots = 0, items = 0, end = 0;
+        for (uint32_t i = 0; i < n_reads; i++) {
+            uint32_t a, b;
+            gs_read_counts(lengths[i], p->k, kt, a, b);
+            slots += a;
+            items += b;
+            const uint64_t e = offsets[i] + lengths[i];
+            end = e > end ? e : end;
+        }
+        if (end <= GS_STAGE_BYTES && items <= 0xffffffffull) {
+            const size_t at_len = (size_t)n_reads * 8, at_seq = (at_len + (size_t)n_reads * 4 + 15) & ~(size_t)15;
+            RC(grow_host(c->h_stage, c->cap_stage, at_seq + end));
+            RC(grow(c->d_stage, c->cap_d_stage, at_seq + end + 16, c->st));
+            memcpy(c->h_stage, offsets, at_len);
+            memcpy(c->h_stage + at_len, lengths, (size_t)n_reads * 4);
+            memcpy(c->h_stage + at_seq, seqs, end);
+            GS_CUDA(cudaMemcpyAsync(c->d_stage, c->h_stage, at_seq + end, cudaMemcpyHostToDevice, c->st));
+            return run_once(c, c->d_stage + at_seq, (const uint64_t *)c->d_stage,
+                            (const uint32_t *)(c->d_stage + at_len), n_reads, p, 1, slots,
+                            (uint32_t)items, true);
+        }
+    }
     /* offsets and lengths first; the end of the last base comes from a
      * reduction on the device, then the bases themselves */
     RC(grow(c->d_offsets, c->cap_offsets, (size_t)n_reads + 1, c->st));
@@ -1001,7 +1228,7 @@ extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
     }
     RC(grow(c->d_seqs, c->cap_seqs, bytes + 1, c->st));
     if (bytes) GS_CUDA(cudaMemcpyAsync(c->d_seqs, seqs, bytes, cudaMemcpyHostToDevice, c->st));
-    return run_pipeline(c, c->d_seqs, c->d_offsets, c->d_lengths, n_reads, p, 1);
+    return run_device(c, c->d_seqs, c->d_offsets, c->d_lengths, n_reads, p, 1);
 }
 
 extern "C" int gs_result_host(gs_ctx *c, gs_result_view *out)
@@ -1262,6 +1489,7 @@ extern "C" int gs_autotune(gs_ctx *c, const char *d_seqs, const uint64_t *d_offs
         for (int rep = 0; rep < 2; rep++) {
             int rc = run_pipeline(c, d_seqs, d_offsets, d_lengths, n, &q, 0);
             if (rc) return rc;
+            take_timing(c);
             if (rep > 0 || n < 1000) best = c->t_search < best ? c->t_search : best;
         }
         ms = best;

@@ -56,7 +56,7 @@ __device__ __forceinline__ const char *gs_slot_at(const uint4 *occ, uint32_t row
 __device__ __forceinline__ GsSlot gs_load_slot(const uint4 *occ, uint32_t row, uint32_t c)
 {
     GsSlot s;
-    uint32_t pad;
+    [[maybe_unused]] uint32_t pad;
     asm("ld.global.nc.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];"
         : "=r"(s.cnt), "=r"(s.m0), "=r"(s.m1), "=r"(pad)
         : "l"(gs_slot_at(occ, row, c)));
@@ -68,7 +68,7 @@ __device__ __forceinline__ GsSlot gs_load_slot(const uint4 *occ, uint32_t row, u
 __device__ __forceinline__ GsSlot gs_load_slot_if(bool yes, const uint4 *occ, uint32_t row, uint32_t c)
 {
     GsSlot s;
-    uint32_t pad;
+    [[maybe_unused]] uint32_t pad;
     asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
         "@q ld.global.nc.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
         : "=r"(s.cnt), "=r"(s.m0), "=r"(s.m1), "=r"(pad)
@@ -177,7 +177,7 @@ __device__ __forceinline__ GsBlk gs_load_block(const uint4 *occ, uint32_t row)
 {
     GsBlk b;
     const char *p = (const char *)occ + (size_t)(row & ~63u);
-    uint32_t z0, z1;
+    [[maybe_unused]] uint32_t z0, z1;
     asm("ld.global.nc.L2::64B.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=r"(b.s[0].cnt), "=r"(b.s[0].m0), "=r"(b.s[0].m1), "=r"(z0), "=r"(b.s[1].cnt),
           "=r"(b.s[1].m0), "=r"(b.s[1].m1), "=r"(z1)

@@ -111,6 +111,8 @@ struct GsBatch {
     const uint32_t *lengths;   /* per read */
     uint32_t n_reads;
     int32_t k, smem, n_mode, lf_mode;
+    int32_t clear;             /* the prepare kernels zero the queue and ... */
+    uint64_t clear_words;      /* ... the first words of recmask */
     GsParts parts;
     uint64_t *totals;          /* slots, work items, seeds, positions of the pass, on the
                                 * device ... */
@@ -176,6 +178,28 @@ __host__ __device__ static inline uint32_t gs_comp_code(unsigned char ch)
 {
     /* pack_4bit_rev table (seed_gen.cu:2561): complement codes */
     return (0x14002035u >> ((ch & 7u) << 2)) & 15u;
+}
+
+/* the start table's length where the batched start pass pairs each window's
+ * two candidates on its entries -- they are longer than its strings -- else 0 */
+static inline int gs_paired_len(const GsDevIndex &I, int kernel, int k)
+{
+    return kernel == GS_KERNEL_BATCHED && I.kmerx && k > I.kx ? I.kx : 0;
+}
+
+/* a read's slots (two a candidate) and work items */
+__host__ __device__ static inline void gs_read_counts(uint32_t L, int k, int paired_kt, uint32_t &slots,
+                                                      uint32_t &items)
+{
+    const uint32_t n = L >= (uint32_t)k ? L - (uint32_t)k + 1u : 0u;
+    slots = 2u * n;
+    if (paired_kt) {
+        /* windows s in [0, L-KT] (k >= KT, so L-KT+1 >= n) */
+        const uint32_t w = n ? L - (uint32_t)paired_kt + 1u : 0u;
+        items = (w + GS_PCHUNK - 1) / GS_PCHUNK;
+    } else {
+        items = 2u * ((n + GS_CHUNK - 1) / GS_CHUNK);
+    }
 }
 
 /* Device result as the text formatter reads it (gs_text.cu). */

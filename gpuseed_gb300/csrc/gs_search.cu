@@ -502,21 +502,6 @@ __device__ __forceinline__ uint32_t gs_start_flags(uint32_t y, uint32_t c, bool 
 /* ------------------------------------------------------------------ */
 /* per-batch preparation: candidate slots and work items per read */
 
-/* a read's slots (two a candidate) and work items */
-__device__ __forceinline__ void gs_read_counts(uint32_t L, int k, int paired_kt, uint32_t &slots,
-                                               uint32_t &items)
-{
-    const uint32_t n = L >= (uint32_t)k ? L - (uint32_t)k + 1u : 0u;
-    slots = 2u * n;
-    if (paired_kt) {
-        /* windows s in [0, L-KT] (k >= KT, so L-KT+1 >= n) */
-        const uint32_t w = n ? L - (uint32_t)paired_kt + 1u : 0u;
-        items = (w + GS_PCHUNK - 1) / GS_PCHUNK;
-    } else {
-        items = 2u * ((n + GS_CHUNK - 1) / GS_CHUNK);
-    }
-}
-
 __device__ __forceinline__ void gs_put_totals(const GsBatch &B, int at, const GsPart &t)
 {
     if (threadIdx.x) return;
@@ -528,8 +513,19 @@ __device__ __forceinline__ void gs_put_totals(const GsBatch &B, int at, const Gs
     }
 }
 
+/* the pass's counters and record mask, where the host left that to the
+ * first kernel */
+__device__ __forceinline__ void gs_clear(const GsBatch &B)
+{
+    if (!B.clear) return;
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 8) B.queue[t] = 0u;
+    for (uint64_t i = t; i < B.clear_words; i += (uint64_t)gridDim.x * blockDim.x) B.recmask[i] = 0u;
+}
+
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_sum(GsBatch B, int paired_kt)
 {
+    gs_clear(B);
     uint32_t first, last;
     gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
     unsigned long long a = 0, b = 0;
@@ -550,6 +546,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_sum(GsBatch B, int
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_scan(GsBatch B, int paired_kt)
 {
     const int lane = threadIdx.x & 31;
+    if (gridDim.x == 1) gs_clear(B);
     uint32_t first, last;
     gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
     GsPart run = {0ull, 0ull};
@@ -594,10 +591,8 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_scan(GsBatch B, in
 
 int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t st)
 {
-    /* the batched start pass pairs each window's two candidates when they
-     * are longer than the paired table's strings */
-    b.paired = kernel == GS_KERNEL_BATCHED && I.kmerx && b.k > I.kx;
-    const int kt = b.paired ? I.kx : 0;
+    const int kt = gs_paired_len(I, kernel, b.k);
+    b.paired = kt != 0;
     const uint32_t parts = gs_parts_of(b.n_reads);
     if (parts > 1) {
         gs_prepare_sum<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
@@ -1479,8 +1474,10 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
 
 /* 5 CTAs of 256 per SM (48 registers, no spills): more lookups in flight
  * than 4 or 3 (config-3 search 101.1 / 101.8 / 104.5 ms) */
+#define GS_START_CTAS 5
+
 template <int NSTOP, int COUNT, bool PAIRED>
-__global__ void __launch_bounds__(256, 5) gs_search_start(GsDevIndex I, GsBatch B, int queue_chunk)
+__global__ void __launch_bounds__(256, GS_START_CTAS) gs_search_start(GsDevIndex I, GsBatch B, int queue_chunk)
 {
     const int lane = threadIdx.x & 31;
     unsigned long long wk = 0, wb = 0;
@@ -1524,6 +1521,7 @@ __global__ void __launch_bounds__(256, 5) gs_search_start(GsDevIndex I, GsBatch 
 }
 
 #define GS_WALK_WARPS 4
+#define GS_WALK_CTAS 8
 
 /* A warp's part [next, end) of a list that all warps append to, in shared
  * memory; full once the list gave no more room (no further atomics, so that
@@ -1561,7 +1559,7 @@ __device__ __forceinline__ uint32_t gs_list_room(GsListPart &part, uint32_t *cou
 }
 
 template <int NSTOP, int COUNT>
-__global__ void __launch_bounds__(GS_WALK_WARPS * 32, 8) gs_search_walk(GsDevIndex I, GsBatch B, uint32_t wsz)
+__global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_walk(GsDevIndex I, GsBatch B, uint32_t wsz)
 {
     __shared__ GsListPart s_text[GS_WALK_WARPS];
     const int lane = threadIdx.x & 31;
@@ -1871,11 +1869,7 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
     void (*walk)(GsDevIndex, GsBatch, uint32_t) =
         nstop ? (cnt ? gs_search_walk<1, 1> : gs_search_walk<1, 0>)
               : (cnt ? gs_search_walk<0, 1> : gs_search_walk<0, 0>);
-    if (ctas_per_sm <= 0) {
-        int occ = 0;
-        GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, start, 256, 0));
-        ctas_per_sm = occ > 0 ? occ : 1;
-    }
+    if (ctas_per_sm <= 0) ctas_per_sm = GS_START_CTAS;
     uint32_t grid = (uint32_t)sms * (uint32_t)ctas_per_sm;
     /* a captured pass knows its items only on the device: as many as the
      * pass it was sized by */
@@ -1890,15 +1884,14 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         if (need < grid * 8) grid = (need + 7) / 8;
     }
     if (grid == 0) grid = 1;
-    GS_CUDA(cudaMemsetAsync(B.queue, 0, sizeof(uint32_t), st));
-    GS_CUDA(cudaMemsetAsync(B.queue + 2, 0, 2 * sizeof(uint32_t), st));
     B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, 64u, GS_WALKER_CHUNK);
     start<<<grid, 256, 0, st>>>(I, B, queue_chunk);
     GS_CUDA(cudaGetLastError());
     if (B.walker_cap) {
-        int wocc = 0;
-        GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wocc, walk, GS_WALK_WARPS * 32, 0));
-        const uint32_t wgrid = (uint32_t)sms * (uint32_t)(wocc > 0 ? wocc : 4);
+        /* no more warps than the items can have walkers for, 32 each */
+        uint32_t wgrid = (uint32_t)sms * GS_WALK_CTAS;
+        const uint64_t most = (uint64_t)items * (2u * GS_PCHUNK) / (GS_WALK_WARPS * 32u) + 1u;
+        if (most < wgrid) wgrid = (uint32_t)most;
         /* the buffer's capacity stands for its walkers (the count is on the
          * device): about an eighth of a warp's share a window */
         B.text_chunk = gs_list_chunk(B.text_cap, wgrid * GS_WALK_WARPS);
@@ -1909,14 +1902,18 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
             void (*text)(GsDevIndex, GsBatch) =
                 nstop ? (cnt ? gs_search_text<1, 1> : gs_search_text<1, 0>)
                       : (cnt ? gs_search_text<0, 1> : gs_search_text<0, 0>);
-            text<<<(uint32_t)sms * 8u, 256, 0, st>>>(I, B);
+            uint32_t tgrid = (uint32_t)sms * 8u;
+            if (B.text_cap < (uint64_t)tgrid * 256u) tgrid = (uint32_t)(B.text_cap / 256u) + 1u;
+            text<<<tgrid, 256, 0, st>>>(I, B);
             GS_CUDA(cudaGetLastError());
         }
     }
     void (*leftover)(GsDevIndex, GsBatch) =
         nstop ? (cnt ? gs_search_leftover<1, 1> : gs_search_leftover<1, 0>)
               : (cnt ? gs_search_leftover<0, 1> : gs_search_leftover<0, 0>);
-    leftover<<<(uint32_t)sms * 8u, 256, 0, st>>>(I, B);
+    uint32_t lgrid = (uint32_t)sms * 8u;
+    if (B.n_reads < lgrid * 8u) lgrid = B.n_reads / 8u + 1u;
+    leftover<<<lgrid, 256, 0, st>>>(I, B);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }

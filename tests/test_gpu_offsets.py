@@ -15,6 +15,10 @@ from helpers import build_index, pack, sample_reads
 pytestmark = pytest.mark.gpu
 
 
+def text_of(codes):
+    return "".join("ACGT"[c] for c in codes)
+
+
 @pytest.fixture(scope="module")
 def copies(built, tmp_path_factory):
     import gpuseed_gb300 as gs
@@ -28,7 +32,7 @@ def copies(built, tmp_path_factory):
     codes = np.concatenate(parts)
     prefix = build_index(tmp_path_factory.mktemp("offsets"), codes)
     reads = sample_reads(codes, 4000, 12, lengths=(10, 19, 20, 40, 80, 150), err=0.01, n_rate=0.1)
-    return gs.Index(prefix), pyoracle.Index(prefix), reads
+    return gs.Index(prefix), pyoracle.Index(prefix), reads, codes
 
 
 @pytest.mark.parametrize("text", [0, 4], ids=["lf_walk", "full_sa"])
@@ -38,7 +42,7 @@ def test_offsets_and_positions(copies, n, text):
 
     import gpuseed_gb300 as gs
 
-    gidx, oidx, reads = copies
+    gidx, oidx, reads, _ = copies
     gidx.set_text(text)
     seqs, offs, lens = pack(reads[-n:])
     dev = [torch.from_numpy(np.frombuffer(seqs, np.uint8).copy()).cuda(),
@@ -57,3 +61,33 @@ def test_offsets_and_positions(copies, n, text):
                 assert got.read_records(r) == want.read_records(r), f"n={n} smem={smem} read {r}"
     ctx.close()
     gidx.set_text(0)
+
+
+def test_batches_of_any_size_through_one_context(copies):
+    """A context runs small batches in one go on the room and the sizes of
+    the passes before: reads with far more slots, seeds or positions than
+    those expected make it run again, with the same result."""
+    import torch
+
+    import gpuseed_gb300 as gs
+
+    gidx, oidx, reads, codes = copies
+    full = [r for r in reads if len(r) == 150]
+    # inside the repeated unit: one seed of 700 positions
+    unit = text_of(codes)[9005:9055].encode()
+    batches = [reads[:1], [b"ACGT"] * 40, reads[:700], full * 3, [unit] * 300, reads[5:9], reads * 3]
+    ctx = gs.Context(gidx)
+    for i, batch in enumerate(batches):
+        seqs, offs, lens = pack(batch)
+        want = oidx.seed(seqs, offs, lens, k=19, smem=True)
+        d = [torch.from_numpy(np.frombuffer(seqs, np.uint8).copy()).cuda(),
+             torch.from_numpy(offs.view(np.int64)).cuda(), torch.from_numpy(lens.view(np.int32)).cuda()]
+        torch.cuda.synchronize()
+        results = [ctx.seed(seqs, offs, lens, k=19, smem=True)]
+        for graph in (False, True, False, True):
+            results.append(ctx.seed_device(*(t.data_ptr() for t in d), lens.size, fetch=True, k=19,
+                                           smem=True, graph=graph))
+        for j, got in enumerate(results):
+            for r in range(lens.size):
+                assert got.read_records(r) == want.read_records(r), f"batch {i} call {j} read {r}"
+    ctx.close()
