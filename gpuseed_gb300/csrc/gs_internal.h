@@ -98,9 +98,9 @@ struct GsParts {
     GsPart *part;      /* GS_PARTS_MOST entries, and tickets[2], zero between passes */
     uint32_t *tickets;
 };
-static inline uint32_t gs_parts_of(uint32_t n_reads)
+static inline uint32_t gs_parts_of(uint32_t n_reads, uint32_t tile)
 {
-    const uint32_t p = (n_reads + 255u) / 256u;
+    const uint32_t p = (n_reads + tile - 1u) / tile;
     return p < 1u ? 1u : p > GS_PARTS_MOST ? GS_PARTS_MOST : p;
 }
 

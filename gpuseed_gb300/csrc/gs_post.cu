@@ -345,21 +345,24 @@ __device__ __noinline__ void gs_finalize_read_warp(const GsBatch &B, uint32_t r,
     }
 }
 
-/* 32 consecutive reads per warp: a lane compacts and counts its own read
- * when it spans at most GS_LANE_SLOTS slots (few instructions a read, the
- * warp's loads spread over 32 reads); the warp then takes its longer reads
- * one at a time.  The blocks' sums become the offsets of gs_finalize_emit. */
-__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B)
+/* Tiles of 256 reads, 32 consecutive ones per warp: a lane compacts and
+ * counts its own read when it spans at most GS_LANE_SLOTS slots (few
+ * instructions a read, the warp's loads spread over 32 reads); the warp then
+ * takes its longer reads one at a time.  Small batches have tiles of 8 reads
+ * and the warp takes its one read whatever its length (gs_finalize_tile).
+ * The blocks' sums become the offsets of gs_finalize_emit. */
+__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B, uint32_t tile)
 {
     const int lane = threadIdx.x & 31;
+    const uint32_t per_warp = tile / (GS_SCAN_THREADS / 32u);
     uint32_t first, last;
-    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    gs_part_reads(B.n_reads, tile, blockIdx.x, gridDim.x, first, last);
     uint64_t sum_s = 0, sum_p = 0;
-    for (uint32_t r0 = first + (threadIdx.x & ~31u); r0 < last; r0 += GS_SCAN_THREADS) {
+    for (uint32_t r0 = first + (threadIdx.x >> 5) * per_warp; r0 < last; r0 += tile) {
         const uint32_t r = r0 + (uint32_t)lane;
         uint64_t base = 0, next = 0;
         bool longr = false;
-        if (r < last) {
+        if (r < last && lane < (int)per_warp) {
             base = B.slot_off[r];
             next = B.slot_off[r + 1];
             if (next > B.slot_cap) {
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B)
                 B.rd_nseeds[r] = 0;
                 B.rd_npos[r] = 0;
                 atomicOr(B.queue + 1, GS_FLAG_OVERFLOW);
-            } else if (next - base > GS_LANE_SLOTS) {
+            } else if (next - base > GS_LANE_SLOTS || per_warp == 1u) {
                 longr = true;
             } else {
                 const uint32_t n = (uint32_t)((next - base) >> 1);
@@ -411,10 +414,11 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B)
 
 /* A thread per read: its seeds' and positions' offsets, and its seeds merged
  * by begin. */
-__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, uint64_t *seed_pos)
+__global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, uint64_t *seed_pos,
+                                                                    uint32_t tile)
 {
     uint32_t first, last;
-    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    gs_part_reads(B.n_reads, tile, blockIdx.x, gridDim.x, first, last);
     GsPart run = B.parts.part[blockIdx.x];
     if (last == B.n_reads && threadIdx.x == 0) {
         B.seed_off[B.n_reads] = B.totals[2] + B.base_s;
@@ -422,9 +426,9 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, u
     }
     /* the offsets of all the block's reads first: the merges below then need
      * no barrier, and a warp of short lists does not wait for one of long */
-    for (uint32_t r0 = first; r0 < last; r0 += GS_SCAN_THREADS) {
+    for (uint32_t r0 = first; r0 < last; r0 += tile) {
         const uint32_t r = r0 + threadIdx.x;
-        const bool in = r < last;
+        const bool in = r < last && threadIdx.x < tile;
         GsPart t;
         const GsPart x = gs_block_scan(in ? B.rd_nseeds[r] : 0ull, in ? B.rd_npos[r] : 0ull, t);
         if (in) {
@@ -434,7 +438,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, u
         run.a += t.a;
         run.b += t.b;
     }
-    for (uint32_t r = first + threadIdx.x; r < last; r += GS_SCAN_THREADS) {
+    for (uint32_t r = threadIdx.x < tile ? first + threadIdx.x : last; r < last; r += tile) {
         uint64_t s = B.seed_off[r] - B.base_s, p = B.pos_off[r] - B.base_p;   /* this thread's own */
         const uint64_t base = B.slot_off[r];
         const uint32_t n = (uint32_t)((B.slot_off[r + 1] - base) >> 1);
@@ -635,10 +639,20 @@ __global__ void __launch_bounds__(256, 8) gs_locate(GsDevIndex I, GsBatch B)
     }
 }
 
+/* Reads of a block of gs_finalize_count and _emit.  Up to 4096 reads take a
+ * warp each: a lane's way through its read's mask words and records is one
+ * chain of loads, 34 us for 300 reads of 100 to 250 bases, against 8 us
+ * by the warp; more reads than that fill the device a lane each. */
+static uint32_t gs_finalize_tile(uint32_t n_reads)
+{
+    return n_reads <= 4096u ? GS_SCAN_THREADS / 32u : GS_SCAN_THREADS;
+}
+
 int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
-    gs_finalize_count<<<gs_parts_of(B.n_reads), GS_SCAN_THREADS, 0, st>>>(B);
+    const uint32_t tile = gs_finalize_tile(B.n_reads);
+    gs_finalize_count<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, tile);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
 }
@@ -646,7 +660,8 @@ int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 int gs_launch_finalize_emit(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
-    gs_finalize_emit<<<gs_parts_of(B.n_reads), GS_SCAN_THREADS, 0, st>>>(B, B.seed_pos);
+    const uint32_t tile = gs_finalize_tile(B.n_reads);
+    gs_finalize_emit<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, B.seed_pos, tile);
     GS_CUDA(cudaGetLastError());
     if (B.n_reads && !B.smem && B.mem_next == GS_MEM_NEXT_GPUSEED) {
         gs_mem_next_kernel<<<(B.n_reads + 127) / 128, 128, 0, st>>>(B);

@@ -18,15 +18,15 @@
 
 #define GS_SCAN_THREADS 256u
 
-/* reads [first, last) of block b of `blocks`: multiples of the block's
- * threads, the same cut in both kernels */
-__device__ __forceinline__ void gs_part_reads(uint32_t n, uint32_t b, uint32_t blocks, uint32_t &first,
-                                              uint32_t &last)
+/* reads [first, last) of block b of `blocks`: whole tiles of reads (at most
+ * the block's threads), the same cut in both kernels */
+__device__ __forceinline__ void gs_part_reads(uint32_t n, uint32_t tile, uint32_t b, uint32_t blocks,
+                                              uint32_t &first, uint32_t &last)
 {
-    const uint32_t tiles = (n + GS_SCAN_THREADS - 1u) / GS_SCAN_THREADS;
+    const uint32_t tiles = (n + tile - 1u) / tile;
     const uint32_t per = (tiles + blocks - 1u) / blocks;
-    first = min(b * per * GS_SCAN_THREADS, n);
-    last = min(first + per * GS_SCAN_THREADS, n);
+    first = min(b * per * tile, n);
+    last = min(first + per * tile, n);
 }
 
 /* exclusive sums of (a, b) over the block's threads; (ta, tb): the totals */

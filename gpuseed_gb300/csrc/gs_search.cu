@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_sum(GsBatch B, int
 {
     gs_clear(B);
     uint32_t first, last;
-    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    gs_part_reads(B.n_reads, GS_SCAN_THREADS, blockIdx.x, gridDim.x, first, last);
     unsigned long long a = 0, b = 0;
     for (uint32_t r = first + threadIdx.x; r < last; r += GS_SCAN_THREADS) {
         uint32_t slots, items;
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_scan(GsBatch B, in
     const int lane = threadIdx.x & 31;
     if (gridDim.x == 1) gs_clear(B);
     uint32_t first, last;
-    gs_part_reads(B.n_reads, blockIdx.x, gridDim.x, first, last);
+    gs_part_reads(B.n_reads, GS_SCAN_THREADS, blockIdx.x, gridDim.x, first, last);
     GsPart run = {0ull, 0ull};
     if (gridDim.x > 1) run = B.parts.part[blockIdx.x];
     for (uint32_t r0 = first; r0 < last; r0 += GS_SCAN_THREADS) {
@@ -593,7 +593,7 @@ int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t 
 {
     const int kt = gs_paired_len(I, kernel, b.k);
     b.paired = kt != 0;
-    const uint32_t parts = gs_parts_of(b.n_reads);
+    const uint32_t parts = gs_parts_of(b.n_reads, GS_SCAN_THREADS);
     if (parts > 1) {
         gs_prepare_sum<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
         GS_CUDA(cudaGetLastError());
@@ -898,22 +898,15 @@ __global__ void __launch_bounds__(256, 5) gs_search_lockstep(GsDevIndex I, GsBat
 #define GS_WALKER_FWD 0x80000000u
 #define GS_WALKER_CHUNK 512u      /* most buffer entries a warp reserves at a time */
 
-/* entries a start-pass warp reserves at a time (gs_launch_batched sets it):
- * at least an item's walkers, 2 * GS_PCHUNK */
-__device__ __forceinline__ uint32_t gs_walker_chunk(const GsBatch &B)
-{
-    return B.walker_chunk;
-}
-
 /* Sizes from the walker buffer's capacity and a grid of `warps` warps,
- * multiples of 32 from `least` to `most`: about 1/`parts` of a warp's share, so
+ * multiples of 16 from `least` to `most`: about 1/`parts` of a warp's share, so
  * that a small batch's buffer (start reservations) or walkers (walk-pass
  * windows) spread over every warp */
 static uint32_t gs_share_size(uint64_t cap, uint32_t warps, uint32_t parts, uint32_t least,
                               uint32_t most)
 {
     uint64_t v = cap / ((uint64_t)warps * parts);
-    v &= ~31ull;
+    v &= ~15ull;
     if (v < least) v = least;
     if (v > most) v = most;
     return (uint32_t)v;
@@ -1200,6 +1193,36 @@ struct GsReserve {
     uint32_t next, end, full;
 };
 
+/* Room for an item's cnt walkers beyond the rem entries left: a new
+ * reservation of walker_chunk entries, or of all it needs.  Its first entry
+ * (walker_cap: none to be had) and size. */
+__device__ __forceinline__ uint32_t gs_reserve(const GsBatch &B, GsReserve &res, uint32_t cnt,
+                                               uint32_t rem, int lane, uint32_t &take)
+{
+    uint32_t g = 0;
+    take = 0;
+    if (rem >= cnt) return g;
+    take = max(B.walker_chunk, cnt - rem);
+    if (res.full) return (uint32_t)B.walker_cap;
+    if (lane == 0) g = atomicAdd(B.queue + 2, take);
+    g = __shfl_sync(0xffffffffu, g, 0);
+    if ((uint64_t)g + take >= B.walker_cap) res.full = 1u;
+    return g;
+}
+
+/* ... and the reservation after them */
+__device__ __forceinline__ void gs_reserved(const GsBatch &B, GsReserve &res, uint32_t cnt, uint32_t rem,
+                                            uint32_t g, uint32_t take)
+{
+    if (rem >= cnt) {
+        res.next += cnt;
+        return;
+    }
+    res.next = (uint32_t)min((uint64_t)g + (cnt - rem), B.walker_cap);
+    res.end = (uint32_t)min((uint64_t)g + take, B.walker_cap);
+    if (res.next > res.end) res.next = res.end;
+}
+
 template <int NSTOP, int COUNT>
 __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch &B, uint32_t r,
                                              uint32_t local, uint32_t L, uint64_t off, int lane,
@@ -1261,21 +1284,13 @@ __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch
     const uint32_t cnt = (uint32_t)__popc(wm);
     const uint32_t rank = (uint32_t)__popc(wm & ((1u << lane) - 1u));
     const uint32_t rem = res.end - res.next;
-    uint32_t g = 0;
-    if (rem < cnt) {
-        if (res.full) {
-            g = (uint32_t)B.walker_cap;
-        } else {
-            if (lane == 0) g = atomicAdd(B.queue + 2, gs_walker_chunk(B));
-            g = __shfl_sync(0xffffffffu, g, 0);
-            if ((uint64_t)g + gs_walker_chunk(B) >= B.walker_cap) res.full = 1u;
-        }
-    }
+    uint32_t take;
+    const uint32_t g = gs_reserve(B, res, cnt, rem, lane, take);
     if (walker) {
         uint64_t idx;
         if (rank < rem) idx = res.next + rank;
         else idx = (uint64_t)g + (rank - rem);
-        const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + gs_walker_chunk(B), B.walker_cap);
+        const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + take, B.walker_cap);
         /* the entry keeps 30 bits of anchor: reads of 2^30 bases or more
          * (none in practice) are left over too */
         if (idx < cap_end && iL < (1 << 30)) {
@@ -1291,27 +1306,22 @@ __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch
             gs_write_leftover(B, r, n, fwd, anchor, l, u);
         }
     }
-    if (rem < cnt) {
-        res.next = (uint32_t)min((uint64_t)g + (cnt - rem), B.walker_cap);
-        res.end = (uint32_t)min((uint64_t)g + gs_walker_chunk(B), B.walker_cap);
-        if (res.next > res.end) res.next = res.end;
-    } else {
-        res.next += cnt;
-    }
+    gs_reserved(B, res, cnt, rem, g, take);
 }
 
 /* one walker-buffer entry of a warp's reservation (rank among the warp's
  * walkers of this item); false when the buffer is full (or the read too
  * long for the entry's anchor bits): the walk is then left over */
 __device__ __forceinline__ bool gs_push_walker(const GsBatch &B, const GsReserve &res, uint32_t g,
-                                               uint32_t rem, uint32_t rank, uint32_t r, bool fwd,
+                                               uint32_t take, uint32_t rem, uint32_t rank,
+                                               uint32_t r, bool fwd,
                                                int anchor, uint32_t l, uint32_t u, uint32_t jl,
                                                uint32_t ju, bool jpend, int iL)
 {
     uint64_t idx;
     if (rank < rem) idx = res.next + rank;
     else idx = (uint64_t)g + (rank - rem);
-    const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + gs_walker_chunk(B), B.walker_cap);
+    const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + take, B.walker_cap);
     if (idx >= cap_end || iL >= (1 << 30)) return false;
     GsWalker w;
     w.r = r;
@@ -1447,29 +1457,15 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t cnt = (uint32_t)(__popc(mf) + __popc(mr));
     const uint32_t rem = res.end - res.next;
-    uint32_t g = 0;
-    if (rem < cnt) {
-        if (res.full) {
-            g = (uint32_t)B.walker_cap;
-        } else {
-            if (lane == 0) g = atomicAdd(B.queue + 2, gs_walker_chunk(B));
-            g = __shfl_sync(0xffffffffu, g, 0);
-            if ((uint64_t)g + gs_walker_chunk(B) >= B.walker_cap) res.full = 1u;
-        }
-    }
-    if (wf && !gs_push_walker(B, res, g, rem, (uint32_t)__popc(mf & lt), r, true, ef, fl, fu,
+    uint32_t take;
+    const uint32_t g = gs_reserve(B, res, cnt, rem, lane, take);
+    if (wf && !gs_push_walker(B, res, g, take, rem, (uint32_t)__popc(mf & lt), r, true, ef, fl, fu,
                               fj ? fnl : 1u, fj ? fnu : 0u, fj, iL))
         gs_write_leftover(B, r, n, true, ef, fl, fu);
-    if (wr && !gs_push_walker(B, res, g, rem, (uint32_t)(__popc(mf) + __popc(mr & lt)), r, false,
+    if (wr && !gs_push_walker(B, res, g, take, rem, (uint32_t)(__popc(mf) + __popc(mr & lt)), r, false,
                               s, rl, ru, rj ? rnl : 1u, rj ? rnu : 0u, rj, iL))
         gs_write_leftover(B, r, n, false, s, rl, ru);
-    if (rem < cnt) {
-        res.next = (uint32_t)min((uint64_t)g + (cnt - rem), B.walker_cap);
-        res.end = (uint32_t)min((uint64_t)g + gs_walker_chunk(B), B.walker_cap);
-        if (res.next > res.end) res.next = res.end;
-    } else {
-        res.next += cnt;
-    }
+    gs_reserved(B, res, cnt, rem, g, take);
 }
 
 /* 5 CTAs of 256 per SM (48 registers, no spills): more lookups in flight
@@ -1875,8 +1871,11 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
      * pass it was sized by */
     const uint32_t items = n_items ? n_items : B.item_cap;
     if (queue_chunk <= 0) {
-        /* an eighth of a warp's share of the items, 1 to GS_QUEUE_CHUNK_MAX */
-        const uint32_t share = items / (grid * 8u * 8u);
+        /* a warp's share of the items, 1 to GS_QUEUE_CHUNK_MAX: items take
+         * alike long, and each grab is a chain of three dependent accesses
+         * (60,007 short reads, 17 items a warp: start pass 123 -> 79 us
+         * against an eighth of a share) */
+        const uint32_t share = items / (grid * 8u);
         queue_chunk = share < 1u ? 1 : share > GS_QUEUE_CHUNK_MAX ? GS_QUEUE_CHUNK_MAX : (int)share;
     }
     if (n_items) {
@@ -1884,7 +1883,7 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         if (need < grid * 8) grid = (need + 7) / 8;
     }
     if (grid == 0) grid = 1;
-    B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, 64u, GS_WALKER_CHUNK);
+    B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, 16u, GS_WALKER_CHUNK);
     start<<<grid, 256, 0, st>>>(I, B, queue_chunk);
     GS_CUDA(cudaGetLastError());
     if (B.walker_cap) {
