@@ -6,19 +6,28 @@
  * it produces the .bwt/.sa pair in the layout the reference reads
  * (seed_gen.cu:2685-2736, :52-58) for a forward-strand text.
  *
- *   suffix array  prefix doubling (Manber-Myers) over dense 32-bit ranks:
- *                 initial keys pack the first 21 characters in base 5
- *                 ($ = 0 < A..T), every round sorts (rank[i], rank[i+h]) pairs
- *                 with a 64-bit LSD radix sort and re-ranks by a scan of
- *                 "key changed" flags, until all ranks are distinct;
- *   BWT           B[row] = T[SA[row]-1], the $ row dropped (primary);
- *   occurrences   per 64-row block: counts of A,C,G,T before the block
- *                 (scan of per-block counts) + 4 words of 16 bases, MSB
+ *   suffix array  prefix doubling over 32-bit ranks, a rank being the first
+ *                 place of its group: initial keys pack the first 21
+ *                 characters in base 5 ($ = 0 < A..T); each later round sorts
+ *                 (rank[i], rank[i+h]) with a 64-bit LSD radix sort for the
+ *                 suffixes whose rank is still shared, and only those;
+ *   BWT           B[row] = T[SA[row]-1], the $ row dropped (primary), packed
+ *                 into blocks of 64 rows: counts of A,C,G,T before the block
+ *                 (a scan of the blocks' counts) + 4 words of 16 bases, MSB
  *                 first;
  *   sampled SA    SA[i * sa_intv] for i >= 1.
  *
- * Memory: about 30 bytes per base on the device (keys and values double
- * buffered, ranks, flags); a 3.1 Gbp text needs ~95 GB of HBM.
+ * The blocks stay on the device for the index that is returned; they go to
+ * the host for the files alone.
+ *
+ * Bound by the first sort's seven passes and the start table's kernels, not
+ * by the host.  Ten million bases (an eighth of repeats), built, seeded with
+ * and freed: 6.7 ms, of which sorting is 1.9 (1.1 in the first round).  Six
+ * rounds over all suffixes, the host's pass over the codes and the blocks'
+ * round trip over the host took 16.5 ms, of which 4.4 were the sorts.
+ *
+ * Memory: about 33 bytes per base on the device (keys and values double
+ * buffered, ranks, suffix array, text); a 3.1 Gbp text needs ~103 GB of HBM.
  */
 #include "gs_internal.h"
 
@@ -27,12 +36,20 @@
 #include <stdlib.h>
 #include <string.h>
 
+/* what a round leaves for the host */
+struct GsSaState {
+    uint32_t left;       /* suffixes whose rank is shared */
+    uint32_t pad;
+    unsigned long long bad;   /* first code that is not 0..3, or ~0 */
+};
+
 static __global__ void init_keys21(const uint8_t *__restrict__ T, uint64_t n, uint64_t *keys,
-                                   uint32_t *vals)
+                                   uint32_t *vals, GsSaState *st)
 {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t k = 0;
+        if (i < n && T[i] > 3) atomicMin(&st->bad, (unsigned long long)i);
 #pragma unroll
         for (int j = 0; j < 21; j++) {
             uint64_t p = i + (uint64_t)j;
@@ -44,76 +61,141 @@ static __global__ void init_keys21(const uint8_t *__restrict__ T, uint64_t n, ui
     }
 }
 
-static __global__ void change_flags(const uint64_t *keys, uint64_t N, uint32_t *flags)
+/* Of the sorted keys, per place: where its group of this round's ranks (key
+ * >> shift) and its group of equal keys begin, once the marks (a place that
+ * begins one, else 0) are scanned by the larger of each half. */
+static __global__ void group_marks(const uint64_t *keys, uint64_t N, int shift, uint64_t *marks)
 {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < N;
-         j += (uint64_t)gridDim.x * blockDim.x)
-        flags[j] = (j == 0 || keys[j] != keys[j - 1]) ? 1u : 0u;
+         j += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = keys[j], before = j ? keys[j - 1] : k;
+        marks[j] = ((k >> shift) != (before >> shift) ? j << 32 : 0u) | (k != before ? j : 0u);
+    }
 }
 
-static __global__ void scatter_ranks(const uint32_t *sa, const uint32_t *g, uint64_t N, uint32_t *rank)
+struct GsMarkMax {
+    __host__ __device__ __forceinline__ uint64_t operator()(uint64_t a, uint64_t b) const
+    {
+        const uint64_t ah = a >> 32, bh = b >> 32, al = a & 0xffffffffu, bl = b & 0xffffffffu;
+        return ((ah > bh ? ah : bh) << 32) | (al > bl ? al : bl);
+    }
+};
+
+/* Places and ranks from the sorted keys, and the suffixes whose rank is
+ * still shared, in any order.  A group's places begin at its rank, key >>
+ * shift (the first round's one group at 0).  One count per warp and block
+ * goes to the list's end: the addition per warp alone took longer than the
+ * ranks' scattered writes. */
+static __global__ void __launch_bounds__(256)
+settle_ranks(const uint64_t *keys, const uint32_t *vals, const uint64_t *marks, uint64_t N, int shift,
+             uint32_t *sa, uint32_t *rank, uint32_t *next, GsSaState *st)
 {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < N;
-         j += (uint64_t)gridDim.x * blockDim.x)
-        rank[sa[j]] = g[j];
+    __shared__ uint32_t cnt[8];
+    __shared__ uint32_t base;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t j0 = (uint64_t)blockIdx.x * blockDim.x; j0 < N; j0 += stride) {
+        const uint64_t j = j0 + threadIdx.x;
+        bool shared = false;
+        uint32_t s = 0;
+        if (j < N) {
+            const uint64_t m = marks[j];
+            const uint64_t first = m & 0xffffffffu, at = (keys[j] >> shift) - (m >> 32);
+            s = vals[j];
+            sa[at + j] = s;
+            rank[s] = (uint32_t)(at + first);
+            shared = first != j || (j + 1 < N && (marks[j + 1] & 0xffffffffu) == first);
+        }
+        const uint32_t votes = __ballot_sync(0xffffffffu, shared);
+        if (lane == 0) cnt[warp] = __popc(votes);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t sum = 0;
+            for (int w = 0; w < 8; w++) {
+                const uint32_t c = cnt[w];
+                cnt[w] = sum;
+                sum += c;
+            }
+            base = sum ? atomicAdd(&st->left, sum) : 0u;
+        }
+        __syncthreads();
+        if (shared) next[base + cnt[warp] + __popc(votes & ((1u << lane) - 1u))] = s;
+        __syncthreads();
+    }
 }
 
-static __global__ void pair_keys(const uint32_t *rank, uint64_t n, uint64_t h, int b, uint64_t *keys,
-                                 uint32_t *vals)
+/* a suffix shorter than h has its $ among its first h characters, so its
+ * rank is not shared: those listed have a suffix h further on */
+static __global__ void pair_keys(const uint32_t *rank, const uint32_t *list, uint64_t left, uint64_t n,
+                                 uint64_t h, int b, uint64_t *keys)
 {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < left;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t hi = rank[i];
-        uint64_t lo = (i + h <= n) ? rank[i + h] : 0u;
-        keys[i] = (hi << b) | lo;
-        vals[i] = (uint32_t)i;
+        const uint64_t s = list[i];
+        keys[i] = ((uint64_t)rank[s] << b) | (s + h <= n ? rank[s + h] : 0u);
     }
 }
 
-/* B[row] with the $ row marked 4; primary = row of suffix 0 */
-static __global__ void bwt_rows(const uint8_t *T, const uint32_t *sa, uint64_t N, uint8_t *B,
-                                uint32_t *primary)
+/* the even bits of the result from the low 16 of x */
+__device__ __forceinline__ uint32_t even_bits(uint32_t x)
 {
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N;
-         r += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t p = sa[r];
-        if (p == 0) {
-            B[r] = 4;
-            *primary = (uint32_t)r;
-        } else {
-            B[r] = T[p - 1];
+    x = (x | (x << 8)) & 0x00ff00ffu;
+    x = (x | (x << 4)) & 0x0f0f0f0fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    return (x | (x << 1)) & 0x55555555u;
+}
+
+/* A warp per 64-row block of the $-removed string: its 4 packed words and its
+ * base counts; cnt[nblk] = 0.  Two rows a lane, a word from half a ballot of
+ * each bit of the bases (one thread per block, reading bytes that a pass
+ * before it had written, left sectors of 64 blocks to each load). */
+static __global__ void pack_blocks(const uint8_t *__restrict__ T, const uint32_t *__restrict__ sa,
+                                   uint64_t n, const uint32_t *rank, uint32_t *occ, uint4 *cnt,
+                                   uint64_t nblk)
+{
+    const uint32_t lane = threadIdx.x & 31u, primary = rank[0];   /* the row of the whole text */
+    const uint64_t stride = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; b <= nblk; b += stride) {
+        uint32_t in[2], lo[2], hi[2];
+        for (int q = 0; q < 2; q++) {
+            const uint64_t s = b * 64 + q * 32 + lane;
+            const bool ok = s < n;
+            const uint32_t c = ok ? T[sa[s + (s >= primary ? 1u : 0u)] - 1u] : 0u;
+            in[q] = __ballot_sync(0xffffffffu, ok);
+            lo[q] = __ballot_sync(0xffffffffu, c & 1u);
+            hi[q] = __ballot_sync(0xffffffffu, c & 2u);
+        }
+        if (lane == 0) {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            for (int q = 0; q < 2; q++) {
+                v.x += __popc(in[q] & ~hi[q] & ~lo[q]);
+                v.y += __popc(lo[q] & ~hi[q]);
+                v.z += __popc(hi[q] & ~lo[q]);
+                v.w += __popc(hi[q] & lo[q]);
+            }
+            cnt[b] = v;
+        }
+        if (lane < 4 && b < nblk) {
+            const uint32_t half = lane & 1u;   /* base i of a word at bits 2*(15-i) */
+            const uint32_t rl = __brev(lane < 2 ? lo[0] : lo[1]), rh = __brev(lane < 2 ? hi[0] : hi[1]);
+            occ[b * GS_BLOCK_WORDS + 4 + lane] =
+                even_bits((half ? rl : rl >> 16) & 0xffffu) | (even_bits((half ? rh : rh >> 16) & 0xffffu) << 1);
         }
     }
 }
 
-/* one thread per 64-row block of the $-removed string: 4 packed words and
- * the block's own base counts */
-static __global__ void pack_blocks(const uint8_t *B, uint64_t n, uint32_t primary, uint32_t *occ,
-                                   uint32_t *blkcnt, uint64_t nblk)
-{
-    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblk;
-         b += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t cnt[4] = {0, 0, 0, 0};
-        uint32_t w[4] = {0, 0, 0, 0};
-        for (int q = 0; q < 64; q++) {
-            uint64_t s = b * 64 + (uint64_t)q;
-            if (s >= n) break;
-            uint64_t r = s + (s >= primary ? 1u : 0u);
-            uint32_t c = B[r] & 3u;
-            cnt[c]++;
-            w[q >> 4] |= c << ((15 - (q & 15)) << 1);
-        }
-        for (int c = 0; c < 4; c++) blkcnt[(uint64_t)c * nblk + b] = cnt[c];
-        uint32_t *o = occ + b * GS_BLOCK_WORDS;
-        o[4] = w[0]; o[5] = w[1]; o[6] = w[2]; o[7] = w[3];
+struct GsCountSum {
+    __host__ __device__ __forceinline__ uint4 operator()(const uint4 &a, const uint4 &b) const
+    {
+        return make_uint4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
     }
-}
+};
 
-static __global__ void write_counts(const uint32_t *scan, uint64_t nblk, uint32_t *occ)
+static __global__ void write_counts(const uint4 *scan, uint64_t nblk, uint32_t *occ)
 {
     for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblk;
          b += (uint64_t)gridDim.x * blockDim.x)
-        for (int c = 0; c < 4; c++) occ[b * GS_BLOCK_WORDS + c] = scan[(uint64_t)c * nblk + b];
+        *reinterpret_cast<uint4 *>(occ + b * GS_BLOCK_WORDS) = scan[b];
 }
 
 static __global__ void gather_samples(const uint32_t *sa, uint64_t n_samples, uint32_t intv,
@@ -130,31 +212,28 @@ static unsigned grid_for(uint64_t n)
     return (unsigned)(g > 152ull * 64 ? 152ull * 64 : (g ? g : 1));
 }
 
+/* One device allocation, dealt out in pieces. */
 struct DevMem {
-    void *p[16];
-    int n;
-    DevMem() : n(0) {}
-    ~DevMem()
+    uint8_t *p;
+    size_t used;
+    DevMem() : p(NULL), used(0) {}
+    ~DevMem() { release(); }
+    void release()
     {
-        for (int i = 0; i < n; i++) cudaFree(p[i]);
+        cudaFree(p);
+        p = NULL;
     }
-    template <class T>
-    cudaError_t alloc(T *&ptr, size_t count)
+    cudaError_t alloc(size_t bytes)
     {
-        cudaError_t e = cudaMalloc(&ptr, count * sizeof(T) + 16);
-        if (e == cudaSuccess) p[n++] = ptr;
-        return e;
+        used = 0;
+        return cudaMalloc(&p, bytes);
     }
+    static size_t room(size_t bytes) { return (bytes + 271) & ~(size_t)255; }
     template <class T>
-    void release(T *&ptr)
+    void take(T *&ptr, size_t count)
     {
-        for (int i = 0; i < n; i++)
-            if (p[i] == (void *)ptr) {
-                cudaFree(ptr);
-                p[i] = p[--n];
-                ptr = NULL;
-                return;
-            }
+        ptr = (T *)(p + used);
+        used += room(count * sizeof(T));
     }
 };
 
@@ -164,157 +243,148 @@ struct DevMem {
         if (_e != cudaSuccess) return gs_cuda_fail(_e, #x);    \
     } while (0)
 
-/* Suffix array of T[0..n) + $ into d_sa (n+1 entries, device). */
-static int build_sa(const uint8_t *d_T, uint64_t n, uint32_t *d_sa_out)
+/* the built index on the device: blocks in the file's layout, of which the
+ * last may be part used, and samples */
+struct GsBuilt {
+    uint32_t primary, tot[4], L2[4];   /* L2: cumulative counts */
+    uint32_t *d_occ, *d_smp;
+    uint64_t nblk, n_samples;
+    DevMem mem;
+};
+
+static int build_device(const uint8_t *codes, uint64_t n, uint32_t sa_intv, GsBuilt &o)
 {
-    DevMem m;
     const uint64_t N = n + 1;
+    const uint64_t nblk = o.nblk = (n + 63) / 64;
+    o.n_samples = n / sa_intv;   /* rows intv, 2 intv, ... <= n */
+    cub::DoubleBuffer<uint64_t> keys;
+    cub::DoubleBuffer<uint32_t> vals;
     uint64_t *k0, *k1;
-    uint32_t *v0, *v1, *rank;
-    BCUDA(m.alloc(k0, N));
-    BCUDA(m.alloc(k1, N));
-    BCUDA(m.alloc(v0, N));
-    BCUDA(m.alloc(v1, N));
-    BCUDA(m.alloc(rank, N));
+    uint32_t *v0, *v1, *rank, *sa;
+    uint8_t *T, *tmp;
+    GsSaState *st;
+    size_t sort_bytes = 0, scan_bytes = 0, sum_bytes = 0;
+    BCUDA(cub::DeviceRadixSort::SortPairs(NULL, sort_bytes, keys, vals, N, 0, 64));
+    BCUDA(cub::DeviceScan::InclusiveScan(NULL, scan_bytes, (uint64_t *)NULL, (uint64_t *)NULL,
+                                         GsMarkMax(), N));
+    BCUDA(cub::DeviceScan::ExclusiveScan(NULL, sum_bytes, (uint4 *)NULL, (uint4 *)NULL, GsCountSum(),
+                                         make_uint4(0, 0, 0, 0), nblk + 1));
+    size_t tmp_bytes = sort_bytes > scan_bytes ? sort_bytes : scan_bytes;
+    if (sum_bytes > tmp_bytes) tmp_bytes = sum_bytes;
+    DevMem m;
+    BCUDA(m.alloc(2 * DevMem::room(N * 8) + 4 * DevMem::room(N * 4) + DevMem::room(n) +
+                  DevMem::room(tmp_bytes) + DevMem::room(sizeof(GsSaState))));
+    m.take(k0, N);
+    m.take(k1, N);
+    m.take(v0, N);
+    m.take(v1, N);
+    m.take(rank, N);
+    m.take(sa, N);
+    m.take(T, n);
+    m.take(tmp, tmp_bytes);
+    m.take(st, 1);
+    keys = cub::DoubleBuffer<uint64_t>(k0, k1);
+    vals = cub::DoubleBuffer<uint32_t>(v0, v1);
+
+    GsSaState h_st = {0, 0, ~0ull};
+    BCUDA(cudaMemcpyAsync(T, codes, n, cudaMemcpyHostToDevice, 0));
+    BCUDA(cudaMemcpyAsync(st, &h_st, sizeof(h_st), cudaMemcpyHostToDevice, 0));
     int b = 1;
-    while (b < 32 && (1ull << b) <= N + 1) b++;
-    cub::DoubleBuffer<uint64_t> keys(k0, k1);
-    cub::DoubleBuffer<uint32_t> vals(v0, v1);
-    init_keys21<<<grid_for(N), 256>>>(d_T, n, keys.Current(), vals.Current());
+    while (b < 32 && (1ull << b) < N) b++;
+    init_keys21<<<grid_for(N), 256>>>(T, n, keys.Current(), vals.Current(), st);
     BCUDA(cudaGetLastError());
-    size_t tmp_bytes = 0, scan_bytes = 0;
-    BCUDA(cub::DeviceRadixSort::SortPairs(NULL, tmp_bytes, keys, vals, N, 0, 64));
-    BCUDA(cub::DeviceScan::InclusiveSum(NULL, scan_bytes, v1, v1, N));
-    uint8_t *tmp = NULL;
-    size_t need = tmp_bytes > scan_bytes ? tmp_bytes : scan_bytes;
-    BCUDA(m.alloc(tmp, need));
-    int end_bit = 49;   /* 5^21 < 2^49 */
-    uint64_t h = 21;
-    for (int round = 0; round < 40; round++) {
-        BCUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, vals, N, 0, end_bit));
-        uint32_t *g = vals.Alternate();
-        change_flags<<<grid_for(N), 256>>>(keys.Current(), N, g);
-        BCUDA(cudaGetLastError());
-        BCUDA(cub::DeviceScan::InclusiveSum(tmp, scan_bytes, g, g, N));
-        uint32_t groups = 0;
-        BCUDA(cudaMemcpy(&groups, g + (N - 1), 4, cudaMemcpyDeviceToHost));
-        if ((uint64_t)groups == N) {
-            BCUDA(cudaMemcpy(d_sa_out, vals.Current(), N * 4, cudaMemcpyDeviceToDevice));
-            return GS_OK;
+    int end_bit = 49, shift = 63;   /* 5^21 < 2^49: one group */
+    uint64_t h = 21, left = N;
+    for (int round = 0; left; round++) {
+        if (round == 40) {
+            gs_set_error("suffix sorting did not converge");
+            return GS_EINVAL;
         }
-        scatter_ranks<<<grid_for(N), 256>>>(vals.Current(), g, N, rank);
+        /* a smaller sort may be of another kind, with its own needs */
+        size_t need = 0;
+        BCUDA(cub::DeviceRadixSort::SortPairs(NULL, need, keys, vals, left, 0, end_bit));
+        DevMem more;
+        if (need > tmp_bytes) BCUDA(more.alloc(need));
+        BCUDA(cub::DeviceRadixSort::SortPairs(need > tmp_bytes ? more.p : tmp, need, keys, vals, left, 0,
+                                              end_bit));
+        uint64_t *marks = keys.Alternate();
+        group_marks<<<grid_for(left), 256>>>(keys.Current(), left, shift, marks);
         BCUDA(cudaGetLastError());
-        pair_keys<<<grid_for(N), 256>>>(rank, n, h, b, keys.Current(), vals.Current());
+        need = scan_bytes;
+        BCUDA(cub::DeviceScan::InclusiveScan(tmp, need, marks, marks, GsMarkMax(), left));
+        BCUDA(cudaMemsetAsync(&st->left, 0, 4, 0));
+        settle_ranks<<<grid_for(left), 256>>>(keys.Current(), vals.Current(), marks, left, shift, sa, rank,
+                                              vals.Alternate(), st);
         BCUDA(cudaGetLastError());
+        BCUDA(cudaMemcpy(&h_st, st, sizeof(h_st), cudaMemcpyDeviceToHost));
+        if (h_st.bad != ~0ull) return GS_EINVAL;   /* the caller names the code */
+        left = h_st.left;
+        vals.selector ^= 1;
+        shift = b;
         end_bit = 2 * b;
+        if (left) pair_keys<<<grid_for(left), 256>>>(rank, vals.Current(), left, n, h, b, keys.Current());
+        BCUDA(cudaGetLastError());
         h *= 2;
     }
-    gs_set_error("suffix sorting did not converge");
-    return GS_EINVAL;
-}
 
-/* Builds the file-layout .bwt words and .sa samples on the host. */
-static int build_arrays(const uint8_t *codes, uint64_t n, uint32_t sa_intv, uint32_t *primary_out,
-                        uint32_t L2_out[4], uint32_t **bwt_out, uint64_t *bwt_words_out,
-                        uint32_t **samples_out, uint64_t *n_samples_out)
-{
-    DevMem m;
-    const uint64_t N = n + 1;
-    uint8_t *d_T, *d_B;
-    uint32_t *d_sa, *d_prim;
-    BCUDA(m.alloc(d_T, n));
-    BCUDA(cudaMemcpy(d_T, codes, n, cudaMemcpyHostToDevice));
-    BCUDA(m.alloc(d_sa, N));
-    {
-        int rc = build_sa(d_T, n, d_sa);   /* its sort buffers are freed on return */
-        if (rc) return rc;
-    }
-    DevMem m2;
-    BCUDA(m2.alloc(d_B, N));
-    BCUDA(m2.alloc(d_prim, 1));
-    bwt_rows<<<grid_for(N), 256>>>(d_T, d_sa, N, d_B, d_prim);
+    uint4 *cnt;
+    BCUDA(o.mem.alloc(DevMem::room((nblk + 1) * GS_BLOCK_WORDS * 4) + DevMem::room((o.n_samples + 1) * 4) +
+                      DevMem::room((nblk + 1) * 16)));
+    o.mem.take(o.d_occ, (nblk + 1) * GS_BLOCK_WORDS);
+    o.mem.take(o.d_smp, o.n_samples + 1);
+    o.mem.take(cnt, nblk + 1);
+    pack_blocks<<<grid_for((nblk + 1) * 32), 256>>>(T, sa, n, rank, o.d_occ, cnt, nblk);
     BCUDA(cudaGetLastError());
-    uint32_t primary = 0;
-    BCUDA(cudaMemcpy(&primary, d_prim, 4, cudaMemcpyDeviceToHost));
-    uint64_t nblk = (n + 63) / 64;
-    uint32_t *d_occ, *d_cnt;
-    BCUDA(m2.alloc(d_occ, (nblk + 1) * GS_BLOCK_WORDS));
-    BCUDA(m2.alloc(d_cnt, 4 * (nblk + 1)));
-    BCUDA(cudaMemset(d_cnt, 0, 4 * (nblk + 1) * 4));
-    pack_blocks<<<grid_for(nblk), 256>>>(d_B, n, primary, d_occ, d_cnt, nblk);
+    BCUDA(cub::DeviceScan::ExclusiveScan(tmp, sum_bytes, cnt, cnt, GsCountSum(), make_uint4(0, 0, 0, 0),
+                                         nblk + 1));
+    write_counts<<<grid_for(nblk), 256>>>(cnt, nblk, o.d_occ);
     BCUDA(cudaGetLastError());
-    /* exclusive scans of the 4 per-block count rows; the extra slot of each
-     * row is the total */
-    uint32_t *d_scan;
-    BCUDA(m2.alloc(d_scan, 4 * (nblk + 1)));
-    size_t sb = 0;
-    BCUDA(cub::DeviceScan::ExclusiveSum(NULL, sb, d_cnt, d_scan, nblk + 1));
-    uint8_t *d_tmp;
-    BCUDA(m2.alloc(d_tmp, sb + 16));
-    uint32_t *d_rows;
-    BCUDA(m2.alloc(d_rows, 4 * (nblk + 1)));
-    for (int c = 0; c < 4; c++) {
-        BCUDA(cudaMemcpy(d_rows + (uint64_t)c * (nblk + 1), d_cnt + (uint64_t)c * nblk, nblk * 4,
-                         cudaMemcpyDeviceToDevice));
-        BCUDA(cudaMemset(d_rows + (uint64_t)c * (nblk + 1) + nblk, 0, 4));
-        BCUDA(cub::DeviceScan::ExclusiveSum(d_tmp, sb, d_rows + (uint64_t)c * (nblk + 1),
-                                            d_scan + (uint64_t)c * (nblk + 1), nblk + 1));
-    }
-    /* re-stride the scans to the [c * nblk + b] layout write_counts reads */
-    for (int c = 0; c < 4; c++)
-        BCUDA(cudaMemcpy(d_cnt + (uint64_t)c * nblk, d_scan + (uint64_t)c * (nblk + 1), nblk * 4,
-                         cudaMemcpyDeviceToDevice));
-    write_counts<<<grid_for(nblk), 256>>>(d_cnt, nblk, d_occ);
-    BCUDA(cudaGetLastError());
-    uint32_t tot[4];
-    for (int c = 0; c < 4; c++)
-        BCUDA(cudaMemcpy(&tot[c], d_scan + (uint64_t)c * (nblk + 1) + nblk, 4, cudaMemcpyDeviceToHost));
-    uint64_t n_samples = n / sa_intv;   /* rows intv, 2 intv, ... <= n */
-    uint32_t *d_smp;
-    BCUDA(m2.alloc(d_smp, n_samples + 1));
-    if (n_samples) {
-        gather_samples<<<grid_for(n_samples), 256>>>(d_sa, n_samples, sa_intv, d_smp);
+    if (o.n_samples) {
+        gather_samples<<<grid_for(o.n_samples), 256>>>(sa, o.n_samples, sa_intv, o.d_smp);
         BCUDA(cudaGetLastError());
     }
-    /* host: bwa's layout (whole blocks, the last block's used words, final
-     * counts) */
+    BCUDA(cudaMemcpy(&o.primary, rank, 4, cudaMemcpyDeviceToHost));
+    BCUDA(cudaMemcpy(o.tot, cnt + nblk, 16, cudaMemcpyDeviceToHost));
+    for (uint32_t c = 0, sum = 0; c < 4; c++) o.L2[c] = sum += o.tot[c];
+    return GS_OK;
+}
+
+/* The file's .bwt words and .sa samples on the host: whole blocks, the last
+ * block's used words, final counts. */
+static int download(const GsBuilt &o, uint64_t n, uint32_t **bwt_out, uint64_t *bwt_words_out,
+                    uint32_t **samples_out)
+{
+    const uint64_t nblk = o.nblk;
     uint64_t words = 4 * (nblk + 1) + (n + 15) / 16;
     uint32_t *occ = (uint32_t *)malloc((nblk + 1) * GS_BLOCK_WORDS * 4);
     uint32_t *bwt = (uint32_t *)malloc(words * 4 + 16);
-    uint32_t *smp = (uint32_t *)malloc(n_samples * 4 + 16);
+    uint32_t *smp = (uint32_t *)malloc(o.n_samples * 4 + 16);
     if (!occ || !bwt || !smp) {
         free(occ); free(bwt); free(smp);
         return GS_ENOMEM;
     }
-    cudaError_t e = cudaMemcpy(occ, d_occ, nblk * GS_BLOCK_WORDS * 4, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && n_samples) e = cudaMemcpy(smp, d_smp, n_samples * 4, cudaMemcpyDeviceToHost);
+    cudaError_t e = cudaMemcpy(occ, o.d_occ, nblk * GS_BLOCK_WORDS * 4, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && o.n_samples)
+        e = cudaMemcpy(smp, o.d_smp, o.n_samples * 4, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         free(occ); free(bwt); free(smp);
         return gs_cuda_fail(e, "index download");
     }
     uint64_t k = 0;
     for (uint64_t bl = 0; bl < nblk; bl++) {
-        const uint32_t *o = occ + bl * GS_BLOCK_WORDS;
+        const uint32_t *ob = occ + bl * GS_BLOCK_WORDS;
         uint64_t rows = n - bl * 64 < 64 ? n - bl * 64 : 64;
         uint64_t nw = (rows + 15) / 16;
-        memcpy(bwt + k, o, 16);
-        memcpy(bwt + k + 4, o + 4, nw * 4);
+        memcpy(bwt + k, ob, 16);
+        memcpy(bwt + k + 4, ob + 4, nw * 4);
         k += 4 + nw;
     }
-    memcpy(bwt + k, tot, 16);
+    memcpy(bwt + k, o.tot, 16);
     k += 4;
     free(occ);
-    uint32_t L2[4];
-    L2[0] = tot[0];
-    L2[1] = L2[0] + tot[1];
-    L2[2] = L2[1] + tot[2];
-    L2[3] = L2[2] + tot[3];
-    *primary_out = primary;
-    memcpy(L2_out, L2, 16);
     *bwt_out = bwt;
     *bwt_words_out = k;
     *samples_out = smp;
-    *n_samples_out = n_samples;
     return GS_OK;
 }
 
@@ -350,9 +420,25 @@ static int write_files(const char *prefix, uint32_t primary, const uint32_t L2[4
     return ok ? GS_OK : GS_EIO;
 }
 
-int gs_index_from_host(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *bwt,
-                       uint64_t bwt_words, uint32_t sa_intv, const uint32_t *sa_samples,
-                       uint64_t n_samples, int device, gs_index **out);
+static int build(const uint8_t *codes, uint64_t n, uint32_t sa_intv, int device, const char *prefix,
+                 gs_index **out)
+{
+    GS_ON_DEVICE(device);
+    GsBuilt o;
+    int rc = build_device(codes, n, sa_intv, o);   /* its sort buffers are freed on return */
+    if (rc == GS_OK && prefix) {
+        uint32_t *bwt = NULL, *smp = NULL;
+        uint64_t words = 0;
+        rc = download(o, n, &bwt, &words, &smp);
+        if (rc == GS_OK)
+            rc = write_files(prefix, o.primary, o.L2, bwt, words, sa_intv, (uint32_t)n, smp, o.n_samples);
+        free(bwt);
+        free(smp);
+    }
+    if (rc == GS_OK && out)
+        rc = gs_index_from_device(o.primary, o.L2, o.d_occ, sa_intv, o.d_smp, o.n_samples, device, out);
+    return rc;
+}
 
 extern "C" int gs_index_build(const uint8_t *codes, uint64_t n, uint32_t sa_intv, int device,
                               const char *prefix, gs_index **out)
@@ -361,21 +447,13 @@ extern "C" int gs_index_build(const uint8_t *codes, uint64_t n, uint32_t sa_intv
         gs_set_error("gs_index_build: need 1 <= n < 2^32-1 codes, sa_intv > 0 and an output");
         return GS_EINVAL;
     }
-    for (uint64_t i = 0; i < n; i++)
+    const int rc = build(codes, n, sa_intv, device, prefix, out);
+    /* the device looks at the codes; a failure of any kind is put down to a
+     * bad one first */
+    for (uint64_t i = 0; rc != GS_OK && i < n; i++)
         if (codes[i] > 3) {
             gs_set_error("gs_index_build: code %u at %llu is not 0..3", codes[i], (unsigned long long)i);
             return GS_EINVAL;
         }
-    GS_ON_DEVICE(device);
-    uint32_t primary = 0, L2[4];
-    uint32_t *bwt = NULL, *smp = NULL;
-    uint64_t words = 0, n_samples = 0;
-    int rc = build_arrays(codes, n, sa_intv, &primary, L2, &bwt, &words, &smp, &n_samples);
-    if (rc == GS_OK && prefix)
-        rc = write_files(prefix, primary, L2, bwt, words, sa_intv, (uint32_t)n, smp, n_samples);
-    if (rc == GS_OK && out)
-        rc = gs_index_from_host(primary, L2, bwt, words, sa_intv, smp, n_samples, device, out);
-    free(bwt);
-    free(smp);
     return rc;
 }

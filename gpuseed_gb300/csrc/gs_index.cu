@@ -217,6 +217,65 @@ int gs_index_device(const gs_index *idx) { return idx->device; }
 float gs_index_l2_ratio(const gs_index *idx) { return idx->l2_hit_ratio; }
 size_t gs_index_occ_bytes(const gs_index *idx) { return idx->occ_bytes; }
 
+/* The index of a file's blocks and samples: the blocks on the device, each
+ * with room for GS_BLOCK_WORDS words; the samples where `kind` has them. */
+static int make_index(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *d_file, uint32_t sa_intv,
+                      const uint32_t *samples, uint64_t n_samples, cudaMemcpyKind kind, int device,
+                      gs_index **out)
+{
+    const uint32_t seq_len = L2_1to4[3];
+    gs_index *idx = (gs_index *)calloc(1, sizeof(gs_index));
+    if (!idx) return GS_ENOMEM;
+    idx->device = device;
+    /* a step reads the block of one past its last row: up to row seq_len+1 */
+    const uint64_t nblk = ((uint64_t)seq_len + 1) / GS_OCC_INTERVAL + 1;
+    idx->occ_bytes = nblk * 4 * sizeof(uint4);
+    idx->sa_bytes = (n_samples + 1) * 4;
+    idx->kmer_bytes = (size_t)8 << (2 * GS_K0);
+    cudaError_t e;
+    if ((e = cudaMalloc(&idx->d_occ, idx->occ_bytes)) != cudaSuccess ||
+        (e = cudaMalloc(&idx->d_sa, idx->sa_bytes)) != cudaSuccess ||
+        (e = cudaMalloc(&idx->d_kmer, idx->kmer_bytes)) != cudaSuccess) {
+        gs_index_free(idx);
+        return gs_cuda_fail(e, "cudaMalloc(index)");
+    }
+    gs_occ_kernel<<<152 * 16, 256>>>(d_file, idx->d_occ, nblk, primary,
+                                     make_uint4(L2_1to4[0], L2_1to4[1], L2_1to4[2], L2_1to4[3]),
+                                     seq_len);
+    if ((e = cudaGetLastError()) != cudaSuccess) {
+        gs_index_free(idx);
+        return gs_cuda_fail(e, "occurrence table layout");
+    }
+    uint32_t minus1 = 0xffffffffu;
+    if ((e = cudaMemcpy(idx->d_sa, &minus1, 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (n_samples && (e = cudaMemcpy(idx->d_sa + 1, samples, n_samples * 4, kind)) != cudaSuccess)) {
+        gs_index_free(idx);
+        return gs_cuda_fail(e, "sa upload");
+    }
+    GsDevIndex &D = idx->dev;
+    D.occ = idx->d_occ;
+    D.sa = idx->d_sa;
+    D.kmer = idx->d_kmer;
+    D.primary = primary;
+    D.seq_len = seq_len;
+    D.sa_intv = sa_intv;
+    D.n_sa = (uint32_t)(n_samples + 1);
+    D.L2[0] = 0;
+    for (int c = 0; c < 4; c++) D.L2[c + 1] = L2_1to4[c];
+    int rc = gs_build_kmer_table(D, idx->d_kmer, 0);
+    if (rc == GS_OK && (e = cudaDeviceSynchronize()) != cudaSuccess) rc = gs_cuda_fail(e, "kmer table");
+    if (rc) {
+        gs_index_free(idx);
+        return rc;
+    }
+    /* the start table is an accelerator: without room for it, run without */
+    for (int kx = auto_kmer_len(seq_len); kx >= GS_K0; kx--)
+        if (gs_index_set_kmer_len(idx, kx) == GS_OK) break;
+    cudaGetLastError();
+    *out = idx;
+    return GS_OK;
+}
+
 static int upload(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *bwt,
                   uint64_t bwt_words, uint32_t sa_intv, const uint32_t *samples,
                   uint64_t n_samples, int device, gs_index **out)
@@ -245,70 +304,29 @@ static int upload(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *b
         return GS_EFORMAT;
     }
     GS_ON_DEVICE(device);
-    gs_index *idx = (gs_index *)calloc(1, sizeof(gs_index));
-    if (!idx) return GS_ENOMEM;
-    idx->device = device;
-    /* a step reads the block of one past its last row: up to row seq_len+1 */
-    const uint64_t nblk = ((uint64_t)seq_len + 1) / GS_OCC_INTERVAL + 1;
-    const uint64_t file_blk = (uint64_t)seq_len / GS_OCC_INTERVAL + 2;
-    idx->occ_bytes = nblk * 4 * sizeof(uint4);
-    idx->sa_bytes = n_sa * 4;
-    idx->kmer_bytes = (size_t)8 << (2 * GS_K0);
-    cudaError_t e;
-    if ((e = cudaMalloc(&idx->d_occ, idx->occ_bytes)) != cudaSuccess ||
-        (e = cudaMalloc(&idx->d_sa, idx->sa_bytes)) != cudaSuccess ||
-        (e = cudaMalloc(&idx->d_kmer, idx->kmer_bytes)) != cudaSuccess) {
-        gs_index_free(idx);
-        return gs_cuda_fail(e, "cudaMalloc(index)");
-    }
-    const uint64_t file_words = file_blk * GS_BLOCK_WORDS;
+    const uint64_t file_words = ((uint64_t)seq_len / GS_OCC_INTERVAL + 2) * GS_BLOCK_WORDS;
     const uint64_t copy_words = bwt_words < file_words ? bwt_words : file_words;
     uint32_t *d_file = NULL;
+    cudaError_t e;
     if ((e = cudaMalloc(&d_file, file_words * 4)) != cudaSuccess ||
         (e = cudaMemset(d_file, 0, file_words * 4)) != cudaSuccess ||
         (e = cudaMemcpy(d_file, bwt, copy_words * 4, cudaMemcpyHostToDevice)) != cudaSuccess) {
         cudaFree(d_file);
-        gs_index_free(idx);
         return gs_cuda_fail(e, "index upload");
     }
-    gs_occ_kernel<<<152 * 16, 256>>>(d_file, idx->d_occ, nblk, primary,
-                                     make_uint4(L2_1to4[0], L2_1to4[1], L2_1to4[2], L2_1to4[3]),
-                                     seq_len);
-    e = cudaGetLastError();
+    int rc = make_index(primary, L2_1to4, d_file, sa_intv, samples, n_samples, cudaMemcpyHostToDevice, device,
+                        out);
     cudaFree(d_file);
-    if (e != cudaSuccess) {
-        gs_index_free(idx);
-        return gs_cuda_fail(e, "occurrence table layout");
-    }
-    uint32_t minus1 = 0xffffffffu;
-    if ((e = cudaMemcpy(idx->d_sa, &minus1, 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (n_samples && (e = cudaMemcpy(idx->d_sa + 1, samples, n_samples * 4,
-                                      cudaMemcpyHostToDevice)) != cudaSuccess)) {
-        gs_index_free(idx);
-        return gs_cuda_fail(e, "sa upload");
-    }
-    GsDevIndex &D = idx->dev;
-    D.occ = idx->d_occ;
-    D.sa = idx->d_sa;
-    D.kmer = idx->d_kmer;
-    D.primary = primary;
-    D.seq_len = seq_len;
-    D.sa_intv = sa_intv;
-    D.n_sa = (uint32_t)n_sa;
-    D.L2[0] = 0;
-    for (int c = 0; c < 4; c++) D.L2[c + 1] = L2_1to4[c];
-    int rc = gs_build_kmer_table(D, idx->d_kmer, 0);
-    if (rc == GS_OK && (e = cudaDeviceSynchronize()) != cudaSuccess) rc = gs_cuda_fail(e, "kmer table");
-    if (rc) {
-        gs_index_free(idx);
-        return rc;
-    }
-    /* the start table is an accelerator: without room for it, run without */
-    for (int kx = auto_kmer_len(seq_len); kx >= GS_K0; kx--)
-        if (gs_index_set_kmer_len(idx, kx) == GS_OK) break;
-    cudaGetLastError();
-    *out = idx;
-    return GS_OK;
+    return rc;
+}
+
+int gs_index_from_device(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *d_blocks,
+                         uint32_t sa_intv, const uint32_t *d_samples, uint64_t n_samples, int device,
+                         gs_index **out)
+{
+    *out = NULL;
+    return make_index(primary, L2_1to4, d_blocks, sa_intv, d_samples, n_samples, cudaMemcpyDeviceToDevice,
+                      device, out);
 }
 
 extern "C" int gs_index_from_host(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *bwt,

@@ -251,6 +251,12 @@ struct GsDeviceGuard {
     GsDeviceGuard gs_device_guard_;  \
     GS_CUDA(gs_device_guard_.enter(dev))
 
+/* the index of built blocks (the file's layout, GS_BLOCK_WORDS words each) and
+ * samples; they may be freed on return */
+int gs_index_from_device(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *d_blocks,
+                         uint32_t sa_intv, const uint32_t *d_samples, uint64_t n_samples, int device,
+                         gs_index **out);
+
 /* kernel launchers (defined next to their kernels) */
 int gs_build_kmer_table(const GsDevIndex &idx, uint2 *table, cudaStream_t st);
 int gs_launch_text_lengths(const GsTextArgs &a, cudaStream_t st);
