@@ -932,19 +932,28 @@ __global__ void __launch_bounds__(256, 5) gs_search_lockstep(GsDevIndex I, GsBat
 #define GS_WALKER_JPEND 0x40000000u   /* anchor flag: J is one base short of I's far end */
 #define GS_WALKER_FWD 0x80000000u
 #define GS_WALKER_CHUNK 512u      /* most buffer entries a warp reserves at a time */
+#define GS_WALK_WINDOW 512u       /* ... and a walk-pass warp takes */
 
-/* Sizes from the walker buffer's capacity and a grid of `warps` warps,
- * multiples of 16 from `least` to `most`: about 1/`parts` of a warp's share, so
- * that a small batch's buffer (start reservations) or walkers (walk-pass
- * windows) spread over every warp */
-static uint32_t gs_share_size(uint64_t cap, uint32_t warps, uint32_t parts, uint32_t least,
-                              uint32_t most)
+/* Buffer entries a start-pass warp reserves at a time, a multiple of 16: a
+ * 32nd of its share of the capacity, 32 to 512.  The capacity is all
+ * candidates, of which a tenth or so become walkers, so what stays unused of
+ * the last reservations counts against them (each warp a 16th: 2.9 M entries
+ * for 1.6 M walkers); less than an item's walkers is a reservation an item
+ * (16 entries at 60,007 short reads: start pass 85 -> 104 us). */
+static uint32_t gs_walker_chunk(uint64_t cap, uint32_t warps)
 {
-    uint64_t v = cap / ((uint64_t)warps * parts);
-    v &= ~15ull;
-    if (v < least) v = least;
-    if (v > most) v = most;
-    return (uint32_t)v;
+    const uint64_t v = cap / ((uint64_t)warps * 32u) & ~15ull;
+    return v < 32u ? 32u : v > GS_WALKER_CHUNK ? GS_WALKER_CHUNK : (uint32_t)v;
+}
+
+/* Buffer entries a walk-pass warp takes at a time: an eighth of its share of
+ * the entries in use, 32 to 512, so that the walks spread over every warp
+ * (sized by the buffer's capacity, 100,000 reads of 150 were 3,100 windows
+ * of 512 for 4,900 warps: walk pass 538 -> 456 us on 100 Mbp; 150,001
+ * reads, 740 -> 622). */
+__device__ __forceinline__ uint32_t gs_walk_window(uint32_t n_w, uint32_t warps)
+{
+    return min(max((n_w / (warps * 8u)) & ~31u, 32u), GS_WALK_WINDOW);
 }
 /* entries of a list that a walk-pass warp reserves at a time: an eighth of
  * its share of the capacity, 1 to 32 */
@@ -953,7 +962,6 @@ static uint32_t gs_list_chunk(uint64_t cap, uint32_t warps)
     const uint64_t v = cap / ((uint64_t)warps * 8u);
     return v < 1u ? 1u : v > 32u ? 32u : (uint32_t)v;
 }
-#define GS_WALK_WINDOW 512u       /* most buffer entries a walk-pass warp takes at a time */
 
 /* Text mode.  A walker whose interval is one row [l,l] and whose J is
  * empty can no longer be contained: its walk only extends one occurrence,
@@ -1596,7 +1604,7 @@ __device__ __forceinline__ uint32_t gs_list_room(GsListPart &part, uint32_t *cou
 }
 
 template <int NSTOP, int COUNT>
-__global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_walk(GsDevIndex I, GsBatch B, uint32_t wsz)
+__global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_walk(GsDevIndex I, GsBatch B)
 {
     __shared__ GsListPart s_text[GS_WALK_WARPS];
     const int lane = threadIdx.x & 31;
@@ -1611,6 +1619,7 @@ __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_wa
     /* walker indices fit 32 bits: the buffer holds at most 2^31 entries */
     uint32_t n_w = *(volatile uint32_t *)(B.queue + 2);
     if (n_w > B.walker_cap) n_w = (uint32_t)B.walker_cap;
+    const uint32_t wsz = gs_walk_window(n_w, gridDim.x * GS_WALK_WARPS);
     uint32_t win = 0, win_end = 0;   /* warp-uniform window of walker indices */
     bool have = false, exhausted = false, killed = false, jpend = false;
     uint32_t r = 0, l = 0, u = 0, jl = 0, ju = 0, n = 0;
@@ -1906,7 +1915,7 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
                           : (cnt ? gs_search_start<0, 1, true> : gs_search_start<0, 0, true>))
                  : (nstop ? (cnt ? gs_search_start<1, 1, false> : gs_search_start<1, 0, false>)
                           : (cnt ? gs_search_start<0, 1, false> : gs_search_start<0, 0, false>));
-    void (*walk)(GsDevIndex, GsBatch, uint32_t) =
+    void (*walk)(GsDevIndex, GsBatch) =
         nstop ? (cnt ? gs_search_walk<1, 1> : gs_search_walk<1, 0>)
               : (cnt ? gs_search_walk<0, 1> : gs_search_walk<0, 0>);
     if (ctas_per_sm <= 0) ctas_per_sm = GS_START_CTAS;
@@ -1927,7 +1936,7 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         if (need < grid * 8) grid = (need + 7) / 8;
     }
     if (grid == 0) grid = 1;
-    B.walker_chunk = gs_share_size(B.walker_cap, grid * 8u, 16u, 16u, GS_WALKER_CHUNK);
+    B.walker_chunk = gs_walker_chunk(B.walker_cap, grid * 8u);
     start<<<grid, 256, 0, st>>>(I, B, queue_chunk);
     GS_CUDA(cudaGetLastError());
     if (B.walker_cap) {
@@ -1938,8 +1947,7 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         /* the buffer's capacity stands for its walkers (the count is on the
          * device): about an eighth of a warp's share a window */
         B.text_chunk = gs_list_chunk(B.text_cap, wgrid * GS_WALK_WARPS);
-        walk<<<wgrid, GS_WALK_WARPS * 32, 0, st>>>(
-            I, B, gs_share_size(B.walker_cap, wgrid * GS_WALK_WARPS, 8u, 32u, GS_WALK_WINDOW));
+        walk<<<wgrid, GS_WALK_WARPS * 32, 0, st>>>(I, B);
         GS_CUDA(cudaGetLastError());
         if (B.text_cap) {
             void (*text)(GsDevIndex, GsBatch) =
