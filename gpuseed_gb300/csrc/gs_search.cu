@@ -83,14 +83,13 @@ int gs_build_kmer_table(const GsDevIndex &I, uint2 *table, cudaStream_t st)
  * bits 2j, processed first, i.e. the string's last character sits at bits
  * 0-1):
  *   1. (l,u) from the 13-mer prefix interval plus kx-13 steps;
- *   2. the forced right extension of each kx-mer X: the base c with
- *      count(Xc) == count(X) > 0, if any.  Xc's interval is one step with X's
+ *   2. what follows each kx-mer X: the forced right extension, i.e. the base
+ *      c with count(Xc) == count(X) > 0, if any; for an X of one to three
+ *      rows, the base after each row's X.  Xc's interval is one step with X's
  *      first character from the kx-mer table entry of (X without its first
  *      character)·c;
- *   3. packing: entry.x = l, entry.y = the size, the forced code (0-3 the
- *      base, 4 none, 7 "size does not fit 28 bits: start from the 13-mer")
- *      and, where X has at most GS_EXT_ROWS rows, which of its one- and
- *      two-base left extensions occur (gs_entry_* below);
+ *   3. packing: entry.x = l, entry.y = the size, the forced base and what the
+ *      rows' left contexts are (gs_entry_* below);
  *   4. entry.z, entry.w = the packed entry of gs_kmer_rc(X), the kx-mer of
  *      X's reverse complement in the same bit order.
  * A candidate whose kx-mer is always followed by its neighbour's next base is
@@ -118,45 +117,99 @@ __global__ void __launch_bounds__(256) gs_kmerx_kernel(GsDevIndex I, uint4 *tabl
     });
 }
 
-/* The forced base of X = [l,u] (pass 2): c with count(Xc) == count(X) > 0, or
- * 4.  raw(Y): the interval of a kx-mer. */
+/* What follows X = [l,u] (pass 2): c with count(Xc) == count(X) > 0, or 4;
+ * for one to three rows whose X all have a base after them, GS_RIGHTS | the
+ * rows' bases in row order (rows are sorted by what follows X), 2 bits each.
+ * raw(Y): the interval of a kx-mer. */
+#define GS_RIGHTS 0x40u
+#define GS_ROWS_MOST 3u
+
 template <class F>
-__device__ __forceinline__ uint32_t gs_forced_base(const GsDevIndex &I, uint64_t X, int kx, uint32_t l,
-                                                   uint32_t u, const F &raw)
+__device__ __forceinline__ uint32_t gs_right_code(const GsDevIndex &I, uint64_t X, int kx, uint32_t l,
+                                                  uint32_t u, const F &raw)
 {
     if (l > u) return 4u;
     const uint64_t mask = (1ull << (2 * kx)) - 1u;
     const uint32_t size = u - l + 1u, first = (uint32_t)(X >> (2 * (kx - 1))) & 3u;   /* X's first character */
+    const bool few = size <= GS_ROWS_MOST;
+    uint32_t forced = 4u, rows = 0u, rights = 0u;
     for (uint32_t c = 0; c < 4; c++) {
         uint2 y = raw(((X << 2) | c) & mask);
         /* as many rows as X's at most come before the step */
-        if (y.x > y.y || y.y - y.x + 1u < size) continue;
+        if (y.x > y.y || (!few && y.y - y.x + 1u < size)) continue;
         gs_step(I, y.x, y.y, first);
-        if (y.x <= y.y && y.y - y.x + 1u == size) return c;
+        const uint32_t n = y.x <= y.y ? y.y - y.x + 1u : 0u;
+        if (n == size) forced = c;
+        if (!few) {
+            if (n == size) break;
+            continue;
+        }
+        for (uint32_t i = 0; i < n; i++) rights |= c << (2u * (rows + i));
+        rows += n;
     }
-    return 4u;
+    return few && rows == size ? GS_RIGHTS | rights : forced;
 }
 
-__global__ void gs_kmerx_code_kernel(GsDevIndex I, const uint4 *table, int kx, uint64_t n,
-                                     uint8_t *code)
+/* The X of a block's GS_DENSE that occur, dense: most kx-mers of a table of
+ * about as many entries as the text has bases occur nowhere, and the chains
+ * of loads of the others, which bound these kernels, would hold warps of a few
+ * busy lanes.  entry(X): the interval; none(X, iv) and some(X, iv): what is
+ * done for either.  The 13-mer entries of ten million bases, 1.6 ms with a
+ * thread per entry, take 0.77 in blocks of 32 registers a thread, 8 an SM, and
+ * 0.87 in 5 an SM; one round of blocks after another overlaps one's chains
+ * with the next's entries, where blocks, or warps, that stay and keep what is
+ * left over for their next entries take 1.2 and 1.0 ms. */
+#define GS_DENSE 2048u
+
+template <class E, class N, class S>
+__device__ __forceinline__ void gs_dense(const E &entry, const N &none, const S &some)
 {
-    for (uint64_t X = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; X < n;
-         X += (uint64_t)gridDim.x * blockDim.x) {
-        const uint4 e = table[X];
-        code[X] = (uint8_t)gs_forced_base(I, X, kx, e.x, e.y, [&](uint64_t Y) {
-            const uint4 y = table[Y];
-            return make_uint2(y.x, y.y);
-        });
+    __shared__ uint16_t list[GS_DENSE];
+    __shared__ uint32_t count;
+    const uint64_t X0 = (uint64_t)blockIdx.x * GS_DENSE;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < GS_DENSE; i += 256u) {
+        const uint2 iv = entry(X0 + i);
+        const bool occurs = iv.x <= iv.y;
+        if (!occurs) none(X0 + i, iv);
+        const uint32_t m = __ballot_sync(0xffffffffu, occurs);
+        uint32_t at = 0;
+        if (lane == 0 && m) at = atomicAdd(&count, (uint32_t)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (occurs) list[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < count; i += 256u) {
+        const uint64_t X = X0 + list[i];
+        some(X, entry(X));
     }
 }
 
-/* A packed half entry's second word (the first is l):
- *   bits 0-2   forced code
- *   bit 3      set: at most GS_EXT_ROWS rows, and
- *     bits 4-11  the size
- *     bits 12-15 base c: exactly one row of X is preceded by c
- *     bits 16-31 bit 4*c + d: some row of X is preceded by c, and that by d
- *              clear: bits 4-31 the size
+__global__ void __launch_bounds__(256, 8) gs_kmerx_code_kernel(GsDevIndex I, const uint4 *table, int kx,
+                                                            uint8_t *code)
+{
+    const auto entry = [&](uint64_t X) {
+        const uint4 e = table[X];
+        return make_uint2(e.x, e.y);
+    };
+    gs_dense(
+        entry, [&](uint64_t X, uint2) { code[X] = 4u; },
+        [&](uint64_t X, uint2 iv) { code[X] = (uint8_t)gs_right_code(I, X, kx, iv.x, iv.y, entry); });
+}
+
+/* A packed half entry's second word (the first is l).  Bits 0-2:
+ *   5, 6, 7  one, two, three rows, each with the bases before its X (nearest
+ *            in the high bits) and the base after: six before, 14 bits a
+ *            row from bit 3 (one and two rows), or three, 8 bits (three);
+ *   0-3, 4   the forced base, or none, and
+ *     bit 3 set: at most GS_EXT_ROWS rows, and
+ *       bits 4-11  the size
+ *       bits 12-15 base c: exactly one row of X is preceded by c
+ *       bits 16-31 bit 4*c + d: some row of X is preceded by c, and that by d
+ *     bit 3 clear: bits 4-31 the size (4 and size 0: it does not fit).
+ * (Rows whose context reaches an end of the text take the second form.)
  * A candidate whose extension by the bases its read has next does not occur
  * can reach no minimum length past it, and one whose extension is a single
  * row that its neighbour's string shares is contained there: both end at
@@ -166,23 +219,82 @@ __global__ void gs_kmerx_code_kernel(GsDevIndex I, const uint4 *table, int kx, u
  * loaded by the warp and its read found in a map instead of a search, a
  * 2 M-read SMEM pass on 3.1 Gbp takes 16.6 ms instead of 24.2, a 40,000-read
  * (2 kbp) MEM pass 7.2 instead of 10.4, a 1 M-read pass on 100 Mbp 7.9
- * instead of 10.5.  255 rows is what the size's byte holds. */
+ * instead of 10.5.  With the few rows' contexts a start plays its walk out
+ * over up to six bases, its neighbour's with it, and a quarter (3.1 Gbp) to
+ * half (100 Mbp) of the walkers that were left end there: walk passes of the
+ * same three 8.45 -> 7.28, 3.33 -> 2.89 and 3.45 -> 2.70 ms.
+ * 255 rows is what the size's byte holds. */
 #define GS_EXT_ROWS 255u
 #define GS_ENTRY_EXT 8u
+#define GS_ENTRY_WIDE 4u
+
+__device__ __forceinline__ uint32_t gs_entry_rows(uint32_t y) { return (y & 7u) > 4u ? (y & 7u) - 4u : 0u; }
 
 __device__ __forceinline__ uint32_t gs_entry_size(uint32_t y)
 {
-    return (y & GS_ENTRY_EXT) ? (y >> 4) & 255u : y >> 4;
+    const uint32_t rows = gs_entry_rows(y);
+    return rows ? rows : (y & GS_ENTRY_EXT) ? (y >> 4) & 255u : y >> 4;
 }
 
-/* The second word of X = [l,u].  Rows l..u are read in order (their blocks,
- * and those of their LF rows, are shared by neighbouring entries, whose
- * strings and so whose rows are adjacent). */
+/* row i's context in an entry of n rows: the bases before it in 12 bits (the
+ * last six 0 where there are three), and the base after */
+__device__ __forceinline__ void gs_entry_row(uint32_t y, uint32_t n, uint32_t i, uint32_t &left,
+                                             uint32_t &right)
+{
+    const bool six = n < 3u;
+    const uint32_t f = y >> (3u + i * (six ? 14u : 8u));
+    left = six ? f & 0xfffu : (f & 0x3fu) << 6;
+    right = (six ? f >> 12 : f >> 6) & 3u;
+}
+
+/* the forced base, or 4 */
+__device__ __forceinline__ uint32_t gs_entry_forced(uint32_t y)
+{
+    const uint32_t n = gs_entry_rows(y);
+    if (!n) return y & 7u;
+    uint32_t left, first, right;
+    gs_entry_row(y, n, 0u, left, first);
+    uint32_t forced = first;
+    for (uint32_t i = 1; i < n; i++) {
+        gs_entry_row(y, n, i, left, right);
+        if (right != first) forced = 4u;
+    }
+    return forced;
+}
+
+/* The second word of X = [l,u] from what follows it (gs_right_code).  Rows
+ * l..u are read in order (their blocks, and those of their LF rows, are
+ * shared by neighbouring entries, whose strings and so whose rows are
+ * adjacent). */
 __device__ __forceinline__ uint32_t gs_entry_word(const GsDevIndex &I, uint32_t l, uint32_t u,
                                                   uint32_t code)
 {
     const uint32_t size = l <= u ? u - l + 1u : 0u;
-    if (size >= (1u << 28)) return 7u;
+    if (size >= (1u << 28)) return GS_ENTRY_WIDE;
+    if (code & GS_RIGHTS) {
+        const bool six = size < 3u;
+        uint32_t y = 4u + size;
+        bool end = false;
+        for (uint32_t i = 0; i < size && !end; i++) {
+            uint32_t row = l + i, left = 0;
+            for (int at = six ? 10 : 4; at >= 0 && !end; at -= 2) {
+                end = row == I.primary;   /* the text begins here */
+                if (end) break;
+                const GsBlk B = gs_load_block(I.occ, row);
+                const uint32_t c = gs_block_base(B, row);
+                left |= c << at;
+                if (at) row = gs_block_lf(B, row, c);
+            }
+            const uint32_t right = (code >> (2u * i)) & 3u;
+            y |= (left | right << (six ? 12 : 6)) << (3u + i * (six ? 14u : 8u));
+        }
+        if (!end) return y;
+        /* all rows followed by one base: forced */
+        uint32_t forced = code & 3u;
+        for (uint32_t i = 1; i < size; i++)
+            if (((code >> (2u * i)) & 3u) != (code & 3u)) forced = 4u;
+        code = forced;
+    }
     if (size > GS_EXT_ROWS) return code | (size << 4);
     uint32_t seen = 0, multi = 0, two = 0, at = 0xffffffffu;
     GsBlk B;
@@ -204,28 +316,35 @@ __device__ __forceinline__ uint32_t gs_entry_word(const GsDevIndex &I, uint32_t 
     return code | GS_ENTRY_EXT | (size << 4) | ((seen & ~multi) << 12) | (two << 16);
 }
 
-__global__ void gs_kmerx_pack_kernel(GsDevIndex I, uint4 *table, uint64_t n, const uint8_t *code)
+#define GS_ENTRY_NONE (4u | GS_ENTRY_EXT)   /* no rows */
+
+__global__ void __launch_bounds__(256, 8) gs_kmerx_pack_kernel(GsDevIndex I, uint4 *table, const uint8_t *code)
 {
-    for (uint64_t X = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; X < n;
-         X += (uint64_t)gridDim.x * blockDim.x) {
-        const uint4 e = table[X];
-        table[X] = make_uint4(e.x, gs_entry_word(I, e.x, e.y, code[X]), 0u, 0u);
-    }
+    gs_dense(
+        [&](uint64_t X) {
+            const uint4 e = table[X];
+            return make_uint2(e.x, e.y);
+        },
+        [&](uint64_t X, uint2 iv) { table[X] = make_uint4(iv.x, GS_ENTRY_NONE, 0u, 0u); },
+        [&](uint64_t X, uint2 iv) {
+            table[X] = make_uint4(iv.x, gs_entry_word(I, iv.x, iv.y, code[X]), 0u, 0u);
+        });
 }
 
 /* Passes 1 to 3 at once for kx = 13, whose raw intervals are the 13-mer
  * table's.  (Pass 4 follows.)  Texts of up to 2^26 bases start from this
  * table: nearly every 13-mer of theirs is forced or dead at once, where the
  * plain table left every candidate to the walk (10,000 reads on 1 Mbp, a
- * replayed pass: 430 -> 373 us), for 1 GiB and about 2 ms at load. */
-__global__ void __launch_bounds__(256) gs_kmer13_entries_kernel(GsDevIndex I, uint4 *table)
+ * replayed pass: 430 -> 373 us), for 1 GiB and about 1.5 ms at load. */
+__global__ void __launch_bounds__(256, 8) gs_kmer13_entries_kernel(GsDevIndex I, uint4 *table)
 {
-    const uint32_t X = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint2 e = __ldg(&I.kmer[X]);
-    const uint32_t code = gs_forced_base(I, X, GS_K0, e.x, e.y,
-                                         [&](uint64_t Y) { return __ldg(&I.kmer[Y]); });
-    uint2 *w = reinterpret_cast<uint2 *>(table);
-    w[2 * (uint64_t)X] = make_uint2(e.x, gs_entry_word(I, e.x, e.y, code));
+    const auto entry = [&](uint64_t X) { return __ldg(&I.kmer[X]); };
+    gs_dense(
+        entry, [&](uint64_t X, uint2 iv) { table[X] = make_uint4(iv.x, GS_ENTRY_NONE, 0u, 0u); },
+        [&](uint64_t X, uint2 iv) {
+            const uint32_t code = gs_right_code(I, X, GS_K0, iv.x, iv.y, entry);
+            table[X] = make_uint4(iv.x, gs_entry_word(I, iv.x, iv.y, code), 0u, 0u);
+        });
 }
 
 /* Pass 4: each entry's second half from the packed first half of its reverse
@@ -284,7 +403,7 @@ int gs_build_kmerx_table(const GsDevIndex &I, uint4 *table, int kx, cudaStream_t
     const uint64_t n = 1ull << (2 * kx);
     const uint32_t n13 = 1u << (2 * GS_K0);
     if (kx == GS_K0) {
-        gs_kmer13_entries_kernel<<<n13 / 256, 256, 0, st>>>(I, table);
+        gs_kmer13_entries_kernel<<<n13 / GS_DENSE, 256, 0, st>>>(I, table);
         GS_CUDA(cudaGetLastError());
         GS_CUDA(gs_kmerx_pair(table, kx, st));
         return GS_OK;
@@ -296,10 +415,10 @@ int gs_build_kmerx_table(const GsDevIndex &I, uint4 *table, int kx, cudaStream_t
     GS_CUDA(cudaGetLastError());
     uint8_t *code = NULL;
     GS_CUDA(cudaMallocAsync(&code, n, st));
-    gs_kmerx_code_kernel<<<152 * 64, 256, 0, st>>>(I, table, kx, n, code);
+    gs_kmerx_code_kernel<<<(unsigned)(n / GS_DENSE), 256, 0, st>>>(I, table, kx, code);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        gs_kmerx_pack_kernel<<<152 * 64, 256, 0, st>>>(I, table, n, code);
+        gs_kmerx_pack_kernel<<<(unsigned)(n / GS_DENSE), 256, 0, st>>>(I, table, code);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = gs_kmerx_pair(table, kx, st);
@@ -409,8 +528,8 @@ __device__ __forceinline__ bool gs_start(const GsDevIndex &I, const unsigned cha
             return true;
         }
         uint2 iv = gs_ld_entry(reinterpret_cast<const uint2 *>(&I.kmerx[pat]));
-        uint32_t code = iv.y & 7u, size = gs_entry_size(iv.y);
-        if (code != 7u) {
+        if (iv.y != GS_ENTRY_WIDE) {
+            const uint32_t code = gs_entry_forced(iv.y), size = gs_entry_size(iv.y);
             fcode = code;
             l = iv.x;
             u = size ? iv.x + size - 1u : iv.x - 1u;
@@ -504,28 +623,64 @@ __device__ __forceinline__ void gs_warp_bases(const unsigned char *seq, int iL, 
     odd = __shfl_sync(0xffffffffu, v, q) >> sh;
 }
 
-/* What a start's entry says about the candidate's next two bases c, d of
- * its walk (GS_START_*), for the candidate itself and, by a shuffle, for
- * the one it may contain.  ok1/ok2: c, d are plain bases. */
+/* What a start's entry says about the candidate's next bases, for the
+ * candidate itself and, by a shuffle, for the one it may contain. */
 #define GS_START_ALIVE 1u
-#define GS_START_ONE 2u     /* its string extended by c is one row */
-#define GS_START_TWO 4u     /* extended by c and d it occurs ... */
+#define GS_START_ONE 2u     /* its string extended by the next base is one row */
+#define GS_START_TWO 4u     /* extended by the next two it occurs ... */
 #define GS_START_KNOWN 8u   /* ... or, with this and not _TWO, does not */
 #define GS_CODE_UNKNOWN 5u  /* forced code of a start that no packed entry gave */
 #define GS_START_DEAD 16u   /* it ends before length k: no record */
+#define GS_START_ROWS 32u   /* its few rows' contexts settle J: */
+#define GS_START_IN 64u     /*   contained in its neighbour */
+#define GS_START_J 128u     /*   walks with its neighbour's interval */
 
-__device__ __forceinline__ uint32_t gs_start_flags(uint32_t y, uint32_t c, bool ok1, uint32_t d,
-                                                   bool ok2, int more)
+/* walk: the next six bases of the walk, the nearest at bits 10-11, nv of them
+ * plain; cn: the neighbour's base (4 or more: none); more: bases that the
+ * start lacks to length k, at least 1.
+ *
+ * With the rows' contexts the walk is played out: each row stays for as many
+ * bases as match, and is one of J's rows if the neighbour's base follows.
+ * a, b: how far J's rows and the others get, of the `cap` bases known.  The
+ * candidate is contained where the last of the others has gone and a J row
+ * is left (a > b); it has no use for J where that cannot be (a < b, or both
+ * end at the same base); otherwise both last as far as is known. */
+__device__ __forceinline__ uint32_t gs_start_flags(uint32_t y, uint32_t walk, int nv, uint32_t cn,
+                                                   int more)
 {
-    if (!(y & GS_ENTRY_EXT)) return GS_START_ALIVE;
-    if (!((y >> 4) & 255u)) return 0u;
+    const uint32_t n = gs_entry_rows(y);
     uint32_t f = GS_START_ALIVE;
-    if (ok1) {
+    if (n) {
+        const int cap = min(nv, n < 3u ? 6 : 3);
+        int a = -1, b = -1;
+#pragma unroll
+        for (uint32_t i = 0; i < GS_ROWS_MOST; i++) {
+            if (i < n) {
+                uint32_t left, right;
+                gs_entry_row(y, n, i, left, right);
+                const int m = min(__clz((left ^ walk) << 20) >> 1, cap);
+                if (right == cn) a = max(a, m);
+                else b = max(b, m);
+            }
+        }
+        const int m = max(a, b);
+        f |= GS_START_ROWS;
+        if (m < cap && m < more) f |= GS_START_DEAD;
+        if (cap >= 2) f |= GS_START_KNOWN;
+        if (m >= 2) f |= GS_START_TWO;
+        if (a > b) f |= GS_START_IN;
+        else if (a == b && a == cap) f |= GS_START_J;
+        return f;
+    }
+    if (!(y & GS_ENTRY_EXT)) return f;
+    if (!((y >> 4) & 255u)) return 0u;
+    if (nv >= 1) {
+        const uint32_t c = (walk >> 10) & 3u, d = (walk >> 8) & 3u;
         const uint32_t two = y >> (16u + 4u * c);
         const bool one = (y >> (12u + c)) & 1u;
         if (one) f |= GS_START_ONE;
-        if (!one && !(two & 15u)) f |= GS_START_DEAD;   /* more >= 1: k > the start's length */
-        if (ok2) {
+        if (!one && !(two & 15u)) f |= GS_START_DEAD;
+        if (nv >= 2) {
             f |= GS_START_KNOWN;
             if ((two >> d) & 1u) f |= GS_START_TWO;
             else if (more >= 2) f |= GS_START_DEAD;
@@ -1390,6 +1545,11 @@ __device__ __forceinline__ bool gs_push_walker(const GsBatch &B, const GsReserve
 __device__ __forceinline__ void gs_start_settle(uint32_t cn, uint32_t fcode, uint32_t f, uint32_t nf,
                                                 bool &walk, bool &j)
 {
+    if (f & GS_START_ROWS) {
+        walk = !(f & GS_START_IN);
+        j = (f & GS_START_J) != 0u;
+        return;
+    }
     if (cn > 3u) return;   /* the candidates beyond never started: no J */
     if (fcode < 4u) {
         walk = fcode != cn;   /* forced elsewhere: the neighbour's string does not occur */
@@ -1418,8 +1578,8 @@ __device__ __forceinline__ void gs_start_settle(uint32_t cn, uint32_t fcode, uin
  *
  * Which candidates walk.  Not those whose next one or two bases make a
  * string that does not occur, where that keeps them below length k
- * (GS_START_DEAD).  Not those contained in their neighbour: forced to its
- * base, or a single row after one base where the neighbour's string, one
+ * (GS_START_DEAD).  Not those contained in their neighbour: by their few
+ * rows' contexts (gs_start_flags), forced to its base, or a single row after one base where the neighbour's string, one
  * base longer, still occurs (its own two-base extension: the same bases).
  * Of the others, those whose neighbour's string no longer occurs after one
  * base walk without J (at the start itself the sizes differ: no forced
@@ -1438,35 +1598,40 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
     const unsigned char *seq = (const unsigned char *)B.seqs + off;
     const int ef = s + KT - 1;
     uint32_t lo, hi, odd;
-    gs_warp_bases(seq, iL, s - lane - 2, lane, lo, hi, odd);
-    /* bases s-2, s-1 (walk order of the forward candidate: s-1, s-2) and
-     * s+KT, s+KT+1 */
-    const uint32_t after = (uint32_t)((((uint64_t)hi << 32) | lo) >> (2 * (KT + 2)));
-    const uint32_t p1 = (lo >> 2) & 3u, p2 = lo & 3u, n1 = after & 3u, n2 = (after >> 2) & 3u;
-    const bool op1 = !(odd & 2u), op2 = !(odd & 1u);
-    const bool on1 = !((odd >> (KT + 2)) & 1u), on2 = !((odd >> (KT + 3)) & 1u);
+    gs_warp_bases(seq, iL, s - lane - 6, lane, lo, hi, odd);
+    /* the walks' next six bases, the nearest at bits 10-11: s-1, s-2, ...
+     * forward, the complements of s+KT, s+KT+1, ... reverse; how many are
+     * plain; and the neighbours' bases, s+KT and s-1 */
+    const uint32_t before = lo & 0xfffu;
+    const uint32_t after = (uint32_t)((((uint64_t)hi << 32) | lo) >> (2 * (KT + 6))) & 0xfffu;
+    const uint32_t rev = __brev(~after << 20);   /* the 12 bits reversed */
+    const uint32_t rwalk = ((rev >> 1) & 0x555u) | ((rev & 0x555u) << 1);
+    const uint32_t ob = odd << 26, oa = (odd >> (KT + 6)) & 0x3fu;
+    const int fnv = ob ? __clz(ob) : 6, rnv = oa ? __ffs(oa) - 1 : 6;
+    uint32_t fcn = 4u, rcn = 4u;
+    if (ef + 1 < iL && in_range) fcn = rnv > 0 ? after & 3u : gs_fwd_code(seq[ef + 1]);
+    if (s >= 1 && in_range) rcn = fnv > 0 ? 3u - (before >> 10) : gs_comp_code(seq[s - 1]);
 
     uint32_t fl = 1u, fu = 0u, ff = 0u, fcode = 4u, rl = 1u, ru = 0u, rf = 0u, rcode = 4u;
     if (vf || vr) {
-        bool apart = ((odd >> 2) & ((1u << KT) - 1u)) != 0u;
+        bool apart = ((odd >> 6) & ((1u << KT) - 1u)) != 0u;
         if (!apart) {
             /* the reverse key: complement codes, R[s] at bits 0-1; the forward
              * key (R[s+KT-1] at bits 0-1) is its reverse complement */
-            const uint32_t pr = ~__funnelshift_r(lo, hi, 4) & (0xffffffffu >> (32 - 2 * KT));
+            const uint32_t pr = ~__funnelshift_r(lo, hi, 12) & (0xffffffffu >> (32 - 2 * KT));
             const uint4 e = gs_ld_pair(&I.kmerx[gs_kmer_rc(pr, KT)]);
-            const uint32_t fs = gs_entry_size(e.y), rs = gs_entry_size(e.w);
             fcode = e.y & 7u;
             rcode = e.w & 7u;
-            apart = (vf && fcode == 7u) || (vr && rcode == 7u);
+            apart = (vf && e.y == GS_ENTRY_WIDE) || (vr && e.w == GS_ENTRY_WIDE);
             if (vf) {
                 fl = e.x;
-                fu = e.x + fs - 1u;
-                ff = gs_start_flags(e.y, p1, op1, p2, op2, k - KT);
+                fu = e.x + gs_entry_size(e.y) - 1u;
+                ff = gs_start_flags(e.y, before, fnv, fcn, k - KT);
             }
             if (vr) {
                 rl = e.z;
-                ru = e.z + rs - 1u;
-                rf = gs_start_flags(e.w, 3u - n1, on1, 3u - n2, on2, k - KT);
+                ru = e.z + gs_entry_size(e.w) - 1u;
+                rf = gs_start_flags(e.w, rwalk, rnv, rcn, k - KT);
             }
         }
         wk += (vf ? 1u : 0u) + (vr ? 1u : 0u);   /* entries: a paired one is two */
@@ -1488,14 +1653,8 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
     bool wf = owned && (ff & (GS_START_ALIVE | GS_START_DEAD)) == GS_START_ALIVE;
     bool wr = owned && (rf & (GS_START_ALIVE | GS_START_DEAD)) == GS_START_ALIVE;
     bool fj = false, rj = false;
-    if (wf && ef + 1 < iL) {
-        const uint32_t cn = on1 ? n1 : gs_fwd_code(seq[ef + 1]);
-        gs_start_settle(cn, fcode, ff, nff, wf, fj);
-    }
-    if (wr && s >= 1) {
-        const uint32_t cn = op1 ? 3u - p1 : gs_comp_code(seq[s - 1]);
-        gs_start_settle(cn, rcode, rf, nrf, wr, rj);
-    }
+    if (wf) gs_start_settle(fcn, fcode, ff, nff, wf, fj);
+    if (wr) gs_start_settle(rcn, rcode, rf, nrf, wr, rj);
     const uint32_t mf = __ballot_sync(0xffffffffu, wf), mr = __ballot_sync(0xffffffffu, wr);
     if (!(mf | mr)) return;
     const uint32_t fnl = __shfl_down_sync(0xffffffffu, fl, 1);
@@ -1944,8 +2103,6 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         uint32_t wgrid = (uint32_t)sms * GS_WALK_CTAS;
         const uint64_t most = (uint64_t)items * (2u * GS_PCHUNK) / (GS_WALK_WARPS * 32u) + 1u;
         if (most < wgrid) wgrid = (uint32_t)most;
-        /* the buffer's capacity stands for its walkers (the count is on the
-         * device): about an eighth of a warp's share a window */
         B.text_chunk = gs_list_chunk(B.text_cap, wgrid * GS_WALK_WARPS);
         walk<<<wgrid, GS_WALK_WARPS * 32, 0, st>>>(I, B);
         GS_CUDA(cudaGetLastError());
