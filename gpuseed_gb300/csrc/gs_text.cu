@@ -58,30 +58,52 @@ __device__ __forceinline__ uint32_t gs_header_len(const GsTextArgs &a, uint32_t 
            gs_ndig(a.first_read_no + r) + (uint32_t)(sizeof(k_h2) - 1);
 }
 
-/* per read: the seed -> read map, header and end tokens */
-template <int WRITE>
+/* per read: the seed -> read map and the lengths of its header and end */
 __global__ void gs_text_reads(GsTextArgs a)
 {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.n_reads) return;
     const uint64_t s0 = a.seed_off[r], s1 = a.seed_off[r + 1];
-    const uint64_t th = 2ull * r + s0 + a.pos_off[r];
-    const uint64_t te = 2ull * r + 1ull + s1 + a.pos_off[r + 1];
-    if (!WRITE) {
-        for (uint64_t s = s0; s < s1; s++) a.sread[s] = r;
-        a.off[th] = gs_header_len(a, r);
-        a.off[te] = 1;
-        return;
-    }
-    char *p = a.text + a.off[th];
-    p = gs_put_str(p, k_h0, sizeof(k_h0) - 1);
-    p = a.smem ? gs_put_str(p, "SMEM", 4) : gs_put_str(p, "MEM", 3);
-    p = gs_put_str(p, k_h1, sizeof(k_h1) - 1);
-    const uint32_t no = a.first_read_no + r;
-    p = gs_put_u32(p, no, gs_ndig(no));
-    gs_put_str(p, k_h2, sizeof(k_h2) - 1);
-    a.text[a.off[te]] = '\n';
+    for (uint64_t s = s0; s < s1; s++) a.sread[s] = r;
+    a.off[2ull * r + s0 + a.pos_off[r]] = gs_header_len(a, r);
+    a.off[2ull * r + 1ull + s1 + a.pos_off[r + 1]] = 1;
 }
+
+/* Headers and ends, a warp per read.  A header is 160 bytes, of which only
+ * the number differs between reads: the block keeps the rest in shared
+ * memory, and a warp's lanes write consecutive bytes.  Bound by the stores
+ * (100,000 reads, 16 MB: GS_TEXT_FIGURES with a thread per read, whose
+ * single bytes lay 160 and more apart). */
+#define GS_HEADER_MOST 192u
+
+__global__ void __launch_bounds__(256) gs_text_headers(GsTextArgs a)
+{
+    __shared__ char text[GS_HEADER_MOST];
+    const uint32_t n0 = (uint32_t)sizeof(k_h0) - 1u, n1 = a.smem ? 4u : 3u;
+    const uint32_t n2 = (uint32_t)sizeof(k_h1) - 1u, n3 = (uint32_t)sizeof(k_h2) - 1u;
+    const uint32_t front = n0 + n1 + n2;   /* ... the number, and n3 more */
+    for (uint32_t i = threadIdx.x; i < front + n3; i += 256u)
+        text[i] = i < n0             ? k_h0[i]
+                  : i < n0 + n1      ? (a.smem ? "SMEM" : "MEM")[i - n0]
+                  : i < front        ? k_h1[i - n0 - n1]
+                                     : k_h2[i - front];
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t r = blockIdx.x * 8ull + (threadIdx.x >> 5); r < a.n_reads; r += gridDim.x * 8ull) {
+        char *p = a.text + a.off[2ull * r + a.seed_off[r] + a.pos_off[r]];
+        const uint32_t no = a.first_read_no + (uint32_t)r, nd = gs_ndig(no);
+        for (uint32_t i = lane; i < front; i += 32u) p[i] = text[i];
+        if (lane < nd) {
+            uint32_t v = no;
+            for (uint32_t i = nd - 1u; i > lane; i--) v /= 10u;
+            p[front + lane] = (char)('0' + v % 10u);
+        }
+        for (uint32_t i = lane; i < n3; i += 32u) p[front + nd + i] = text[front + i];
+        if (lane == 31u)
+            a.text[a.off[2ull * r + 1ull + a.seed_off[r + 1] + a.pos_off[r + 1]]] = '\n';
+    }
+}
+static_assert(sizeof(k_h0) + sizeof(k_h1) + sizeof(k_h2) + 4 <= GS_HEADER_MOST, "header room");
 
 /* per seed with positions: "\nRead[b, e] -> " */
 template <int WRITE>
@@ -130,9 +152,13 @@ __global__ void gs_text_positions(GsTextArgs a)
 static int gs_text_pass(const GsTextArgs &a, bool write, cudaStream_t st)
 {
     if (a.n_reads) {
-        uint32_t g = (a.n_reads + 255) / 256;
-        if (write) gs_text_reads<1><<<g, 256, 0, st>>>(a);
-        else gs_text_reads<0><<<g, 256, 0, st>>>(a);
+        if (write) {
+            /* four rounds of a full device's blocks at most */
+            const uint32_t g = (a.n_reads + 7) / 8;
+            gs_text_headers<<<g < 152u * 32u ? g : 152u * 32u, 256, 0, st>>>(a);
+        } else {
+            gs_text_reads<<<(a.n_reads + 255) / 256, 256, 0, st>>>(a);
+        }
         GS_CUDA(cudaGetLastError());
     }
     if (a.n_seeds) {
