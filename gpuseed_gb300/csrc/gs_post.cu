@@ -412,11 +412,148 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B, 
     }
 }
 
-/* A thread per read: its seeds' and positions' offsets, and its seeds merged
- * by begin. */
+/* an output seed and, at the tiles of 32 positions that begin in it, its number */
+__device__ __forceinline__ void gs_put_seed(const GsBatch &B, uint64_t *seed_pos, uint64_t s, uint64_t p,
+                                            const gs_seed_rec &o)
+{
+    if (s >= B.seed_cap) return;
+    B.seeds[s] = o;
+    seed_pos[s] = p;
+    for (uint64_t m = (p + 31u) >> 5; (m << 5) < p + o.n_pos && (m << 5) < B.pos_cap; m++)
+        B.tile_seed[m] = (uint32_t)s;
+}
+
+/* A read's seeds from place s and position p, merged by begin by one thread,
+ * from records a and b on. */
+__device__ __forceinline__ void gs_emit_lane(const GsBatch &B, uint64_t *seed_pos, const GsRec *F, uint32_t nf,
+                                             const GsRec *Rv, uint32_t nr, uint32_t a, uint32_t b,
+                                             uint64_t s, uint64_t p)
+{
+    /* each record loaded once: the forward list's current and next, the
+     * reverse list's current and previous */
+    GsRec none;
+    none.x = none.y = 0;
+    none.l = 1u;
+    none.u = 0u;
+    GsRec fc = a < nf ? F[a] : none, fn = a + 1 < nf ? F[a + 1] : none;
+    GsRec rc = b < nr ? Rv[b] : none, rp = b ? Rv[b - 1] : none;
+    while (a < nf || b < nr) {
+        bool take_f;
+        if (a >= nf) take_f = false;
+        else if (b >= nr) take_f = true;
+        else take_f = ((uint32_t)fc.x & 0x7fffffffu) <= ((uint32_t)rc.x & 0x7fffffffu);
+        bool keep; uint32_t cnt, xl, xu;
+        GsRec R;
+        if (take_f) {
+            gs_fwd_rule_v(fc, fn, a + 1 < nf, B.smem, B.max_occ, keep, cnt, xl, xu);
+            R = fc;
+            a++;
+            fc = fn;
+            fn = a + 1 < nf ? F[a + 1] : none;
+        } else {
+            gs_rev_rule_v(rc, rp, b > 0, B.smem, B.max_occ, keep, cnt, xl, xu);
+            R = rc;
+            b++;
+            rp = rc;
+            rc = b < nr ? Rv[b] : none;
+        }
+        if (keep && cnt) {
+            gs_seed_rec o;
+            o.x = R.x; o.y = R.y; o.l = R.l; o.u = R.u;
+            o.xl = xl; o.xu = xu; o.n_pos = cnt; o.pad = 0;
+            gs_put_seed(B, seed_pos, s, p, o);
+            s++;
+            p += cnt;
+        }
+    }
+}
+
+/* how many of the warp's values, ascending by lane, are below v (or_equal: at
+ * most v) */
+__device__ __forceinline__ uint32_t gs_warp_below(uint32_t value, uint32_t v, bool or_equal)
+{
+    uint32_t k = 0;
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t x = __shfl_sync(0xffffffffu, value, k + step - 1);
+        if (or_equal ? x <= v : x < v) k += step;
+    }
+    const uint32_t x = __shfl_sync(0xffffffffu, value, k);
+    return k + ((or_equal ? x <= v : x < v) ? 1u : 0u);
+}
+
+/* ... by the warp, 32 merged records a round: a record of the next 32 of its
+ * list has its rank in the round by its lane and the other list's records
+ * before it.  Both lists ascend by begin wherever a match has no longer one
+ * ending before it; a round whose lists do not goes on with one thread. */
+__device__ __forceinline__ void gs_emit_warp(const GsBatch &B, uint64_t *seed_pos, const GsRec *F, uint32_t nf,
+                                             const GsRec *Rv, uint32_t nr, uint64_t s, uint64_t p, int lane,
+                                             gs_seed_rec *round)
+{
+    uint32_t a = 0, b = 0;
+    GsRec none;
+    none.x = none.y = 0;
+    none.l = 1u;
+    none.u = 0u;
+    while (a < nf || b < nr) {
+        const uint32_t i = a + (uint32_t)lane, j = b + (uint32_t)lane;
+        const bool hf = i < nf, hr = j < nr;
+        const GsRec f = hf ? F[i] : none, fn = i + 1u < nf ? F[i + 1u] : none;
+        const GsRec r = hr ? Rv[j] : none, rp = hr && j ? Rv[j - 1u] : none;
+        const uint32_t fx = hf ? (uint32_t)f.x & 0x7fffffffu : 0xffffffffu;
+        const uint32_t rx = hr ? (uint32_t)r.x & 0x7fffffffu : 0xffffffffu;
+        const bool down = __shfl_up_sync(0xffffffffu, fx, 1) > fx || __shfl_up_sync(0xffffffffu, rx, 1) > rx;
+        if (__any_sync(0xffffffffu, down)) {
+            if (lane == 0) gs_emit_lane(B, seed_pos, F, nf, Rv, nr, a, b, s, p);
+            return;
+        }
+        const uint32_t fk = (uint32_t)lane + gs_warp_below(rx, fx, false);
+        const uint32_t rk = (uint32_t)lane + gs_warp_below(fx, rx, true);
+        const bool tf = hf && fk < 32u, tr = hr && rk < 32u;
+        bool keep; uint32_t cnt;
+        gs_seed_rec o;
+        o.pad = 0;
+        if (tf) {
+            gs_fwd_rule_v(f, fn, i + 1u < nf, B.smem, B.max_occ, keep, cnt, o.xl, o.xu);
+            o.x = f.x; o.y = f.y; o.l = f.l; o.u = f.u;
+            o.n_pos = keep ? cnt : 0u;
+            round[fk] = o;
+        }
+        if (tr) {
+            gs_rev_rule_v(r, rp, j > 0, B.smem, B.max_occ, keep, cnt, o.xl, o.xu);
+            o.x = r.x; o.y = r.y; o.l = r.l; o.u = r.u;
+            o.n_pos = keep ? cnt : 0u;
+            round[rk] = o;
+        }
+        __syncwarp();
+        const uint32_t na = (uint32_t)__popc(__ballot_sync(0xffffffffu, tf));
+        const uint32_t nb = (uint32_t)__popc(__ballot_sync(0xffffffffu, tr));
+        const bool in = (uint32_t)lane < na + nb;
+        if (in) o = round[lane];
+        const uint32_t n = in ? o.n_pos : 0u;
+        unsigned long long sum = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long x = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += x;
+        }
+        const uint32_t kept = __ballot_sync(0xffffffffu, n != 0u);
+        if (n) gs_put_seed(B, seed_pos, s + (uint32_t)__popc(kept & ((1u << lane) - 1u)), p + sum - n, o);
+        s += (uint32_t)__popc(kept);
+        p += __shfl_sync(0xffffffffu, sum, 31);
+        a += na;
+        b += nb;
+        __syncwarp();
+    }
+}
+
+/* A thread per read, or a warp where the tile has one a warp: its seeds' and
+ * positions' offsets, and its seeds merged by begin. */
+template <bool WARP>
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, uint64_t *seed_pos,
                                                                     uint32_t tile)
 {
+    __shared__ gs_seed_rec rounds[WARP ? GS_SCAN_THREADS : 1u];
     uint32_t first, last;
     gs_part_reads(B.n_reads, tile, blockIdx.x, gridDim.x, first, last);
     GsPart run = B.parts.part[blockIdx.x];
@@ -438,56 +575,16 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, u
         run.a += t.a;
         run.b += t.b;
     }
-    for (uint32_t r = threadIdx.x < tile ? first + threadIdx.x : last; r < last; r += tile) {
-        uint64_t s = B.seed_off[r] - B.base_s, p = B.pos_off[r] - B.base_p;   /* this thread's own */
+    if (WARP) __syncthreads();   /* another thread's offsets */
+    const uint32_t at = WARP ? threadIdx.x >> 5 : threadIdx.x;
+    for (uint32_t r = at < tile ? first + at : last; r < last; r += tile) {
+        const uint64_t s = B.seed_off[r] - B.base_s, p = B.pos_off[r] - B.base_p;
         const uint64_t base = B.slot_off[r];
         const uint32_t n = (uint32_t)((B.slot_off[r + 1] - base) >> 1);
         const GsRec *F = B.slots + base;
-        const GsRec *Rv = F + n;
         const uint32_t nf = B.rd_nf[r], nr = B.rd_nr[r];
-        uint32_t a = 0, b = 0;
-        /* each record loaded once: the forward list's current and next, the
-         * reverse list's current and previous */
-        GsRec none;
-        none.x = none.y = 0;
-        none.l = 1u;
-        none.u = 0u;
-        GsRec fc = nf ? F[0] : none, fn = nf > 1 ? F[1] : none;
-        GsRec rc = nr ? Rv[0] : none, rp = none;
-        while (a < nf || b < nr) {
-            bool take_f;
-            if (a >= nf) take_f = false;
-            else if (b >= nr) take_f = true;
-            else take_f = ((uint32_t)fc.x & 0x7fffffffu) <= ((uint32_t)rc.x & 0x7fffffffu);
-            bool keep; uint32_t cnt, xl, xu;
-            GsRec R;
-            if (take_f) {
-                gs_fwd_rule_v(fc, fn, a + 1 < nf, B.smem, B.max_occ, keep, cnt, xl, xu);
-                R = fc;
-                a++;
-                fc = fn;
-                fn = a + 1 < nf ? F[a + 1] : none;
-            } else {
-                gs_rev_rule_v(rc, rp, b > 0, B.smem, B.max_occ, keep, cnt, xl, xu);
-                R = rc;
-                b++;
-                rp = rc;
-                rc = b < nr ? Rv[b] : none;
-            }
-            if (keep && cnt) {
-                if (s < B.seed_cap) {
-                    gs_seed_rec o;
-                    o.x = R.x; o.y = R.y; o.l = R.l; o.u = R.u;
-                    o.xl = xl; o.xu = xu; o.n_pos = cnt; o.pad = 0;
-                    B.seeds[s] = o;
-                    seed_pos[s] = p;
-                    for (uint64_t m = (p + 31u) >> 5; (m << 5) < p + cnt && (m << 5) < B.pos_cap; m++)
-                        B.tile_seed[m] = (uint32_t)s;
-                }
-                s++;
-                p += cnt;
-            }
-        }
+        if (WARP) gs_emit_warp(B, seed_pos, F, nf, F + n, nr, s, p, threadIdx.x & 31, rounds + (threadIdx.x & ~31u));
+        else gs_emit_lane(B, seed_pos, F, nf, F + n, nr, 0, 0, s, p);
     }
 }
 
@@ -639,19 +736,30 @@ __global__ void __launch_bounds__(256, 8) gs_locate(GsDevIndex I, GsBatch B)
     }
 }
 
-/* Reads of a block of gs_finalize_count and _emit.  Up to 4096 reads take a
- * warp each: a lane's way through its read's mask words and records is one
- * chain of loads, 34 us for 300 reads of 100 to 250 bases, against 8 us
- * by the warp; more reads than that fill the device a lane each. */
-static uint32_t gs_finalize_tile(uint32_t n_reads)
+/* Reads of a block of gs_finalize_count and _emit: a warp's each, or a lane's.
+ * A lane's way through its read's mask words and records is one chain of
+ * loads: 34 us for the count of 300 reads of 100 to 250 bases and 17 for
+ * their merges, against 9 and 6 by the warp.  10,000 reads of 100 keep enough
+ * lanes busy (13 and 7 us, 19 and 13 by the warp), so the line lies between.
+ * Long reads are a warp's work in any number, by their average, 16 items of a
+ * strand's candidates (about GS_LANE_SLOTS): 40,000 reads of 2 kbp, blocks of
+ * 256 on an SM each, 409 -> 186 us and 355 -> 110. */
+#define GS_WARP_READS 4096u
+
+static bool gs_finalize_by_warp(const GsBatch &B)
 {
-    return n_reads <= 4096u ? GS_SCAN_THREADS / 32u : GS_SCAN_THREADS;
+    return B.n_reads <= GS_WARP_READS || (uint64_t)B.item_cap * (B.paired ? 2u : 1u) > 16ull * B.n_reads;
+}
+
+static uint32_t gs_finalize_tile(const GsBatch &B)
+{
+    return gs_finalize_by_warp(B) ? GS_SCAN_THREADS / 32u : GS_SCAN_THREADS;
 }
 
 int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
-    const uint32_t tile = gs_finalize_tile(B.n_reads);
+    const uint32_t tile = gs_finalize_tile(B);
     gs_finalize_count<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, tile);
     GS_CUDA(cudaGetLastError());
     return GS_OK;
@@ -660,8 +768,10 @@ int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 int gs_launch_finalize_emit(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
-    const uint32_t tile = gs_finalize_tile(B.n_reads);
-    gs_finalize_emit<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, B.seed_pos, tile);
+    const uint32_t tile = gs_finalize_tile(B);
+    void (*emit)(GsBatch, uint64_t *, uint32_t) =
+        gs_finalize_by_warp(B) ? gs_finalize_emit<true> : gs_finalize_emit<false>;
+    emit<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, B.seed_pos, tile);
     GS_CUDA(cudaGetLastError());
     if (B.n_reads && !B.smem && B.mem_next == GS_MEM_NEXT_GPUSEED) {
         gs_mem_next_kernel<<<(B.n_reads + 127) / 128, 128, 0, st>>>(B);
