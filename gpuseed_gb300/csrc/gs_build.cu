@@ -7,7 +7,7 @@
  * (seed_gen.cu:2685-2736, :52-58) for a forward-strand text.
  *
  *   suffix array  prefix doubling over 32-bit ranks, a rank being the first
- *                 place of its group: initial keys pack the first 21
+ *                 place of its group: initial keys pack the first 17 (20)
  *                 characters in base 5 ($ = 0 < A..T); each later round sorts
  *                 (rank[i], rank[i+h]) with a 64-bit LSD radix sort for the
  *                 suffixes whose rank is still shared, and only those;
@@ -20,9 +20,9 @@
  * The blocks stay on the device for the index that is returned; they go to
  * the host for the files alone.
  *
- * Bound by the first sort's seven passes and the start table's kernels, not
+ * Bound by the first sort's five passes and the start table's kernels, not
  * by the host.  Ten million bases (an eighth of repeats), built, seeded with
- * and freed: 6.7 ms, of which sorting is 1.9 (1.1 in the first round).  Six
+ * and freed: 6.6 ms, of which sorting is 1.7 (0.9 in the first round).  Six
  * rounds over all suffixes, the host's pass over the codes and the blocks'
  * round trip over the host took 16.5 ms, of which 4.4 were the sorts.
  *
@@ -43,15 +43,17 @@ struct GsSaState {
     unsigned long long bad;   /* first code that is not 0..3, or ~0 */
 };
 
-static __global__ void init_keys21(const uint8_t *__restrict__ T, uint64_t n, uint64_t *keys,
-                                   uint32_t *vals, GsSaState *st)
+/* keys of the first H characters, by 5 (0: past the end) */
+template <int H>
+static __global__ void init_keys(const uint8_t *__restrict__ T, uint64_t n, uint64_t *keys, uint32_t *vals,
+                                 GsSaState *st)
 {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t k = 0;
         if (i < n && T[i] > 3) atomicMin(&st->bad, (unsigned long long)i);
 #pragma unroll
-        for (int j = 0; j < 21; j++) {
+        for (int j = 0; j < H; j++) {
             uint64_t p = i + (uint64_t)j;
             uint64_t c = p < n ? (uint64_t)T[p] + 1u : 0u;
             k = k * 5u + c;
@@ -291,10 +293,15 @@ static int build_device(const uint8_t *codes, uint64_t n, uint32_t sa_intv, GsBu
     BCUDA(cudaMemcpyAsync(st, &h_st, sizeof(h_st), cudaMemcpyHostToDevice, 0));
     int b = 1;
     while (b < 32 && (1ull << b) < N) b++;
-    init_keys21<<<grid_for(N), 256>>>(T, n, keys.Current(), vals.Current(), st);
+    /* as many characters as five or six passes of 8 bits sort (5^17 < 2^40,
+     * 5^20 < 2^47): 17 tell apart all but the repeats of texts well below 4^17
+     * (21 took a seventh pass: the first sort of ten million bases .82 ms) */
+    const bool few = n < (1ull << 29);
+    if (few) init_keys<17><<<grid_for(N), 256>>>(T, n, keys.Current(), vals.Current(), st);
+    else init_keys<20><<<grid_for(N), 256>>>(T, n, keys.Current(), vals.Current(), st);
     BCUDA(cudaGetLastError());
-    int end_bit = 49, shift = 63;   /* 5^21 < 2^49: one group */
-    uint64_t h = 21, left = N;
+    int end_bit = few ? 40 : 47, shift = 63;   /* one group */
+    uint64_t h = few ? 17 : 20, left = N;
     for (int round = 0; left; round++) {
         if (round == 40) {
             gs_set_error("suffix sorting did not converge");
