@@ -64,15 +64,16 @@ __device__ __forceinline__ GsSlot gs_load_slot(const uint4 *occ, uint32_t row, u
 }
 
 /* the same when `yes`, as a predicated load instead of a branch; else the
- * slot is left undefined */
-__device__ __forceinline__ GsSlot gs_load_slot_if(bool yes, const uint4 *occ, uint32_t row, uint32_t c)
+ * slot is left undefined.  Of a table whose blocks have 4 << sh slots. */
+__device__ __forceinline__ GsSlot gs_load_slot_if(bool yes, const uint4 *occ, uint32_t row, uint32_t c,
+                                                  uint32_t sh)
 {
     GsSlot s;
     [[maybe_unused]] uint32_t pad;
     asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
         "@q ld.global.nc.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
         : "=r"(s.cnt), "=r"(s.m0), "=r"(s.m1), "=r"(pad)
-        : "l"(gs_slot_at(occ, row, c)), "r"((int)yes));
+        : "l"((const char *)occ + ((size_t)(row & ~63u) << sh) + (c << 4)), "r"((int)yes));
     return s;
 }
 
@@ -130,27 +131,34 @@ struct GsStepTouch {
     int blocks, jblocks, lines256, lines384;
 };
 
-/* One backward step with base c of an interval I = [l,e) (only when doI)
- * and of an interval J = [jl,je) (jl >= je: none; left unchanged) that lies
- * within it, or where doI is not set anywhere: e and je are one past the
- * last row.  J's bounds lie between I's, so a slot is loaded only where its
- * block differs from those of the bounds before it, by predicated loads that
- * all issue before any is used. */
+/* A table of blocks of 4 << sh slots, and a slot: one base of occ (sh 0), or
+ * a base and the next of occ2 (sh 2) */
+struct GsStepBy {
+    const uint4 *occ;
+    uint32_t sh, c;
+};
+
+/* One backward step of an interval I = [l,e) (only when doI) and of an
+ * interval J = [jl,je) (jl >= je: none; left unchanged): e and je are one
+ * past the last row.  With `within`, J lies within I and both step by the same
+ * slot: J's bounds lie between I's, so a slot is loaded only where its block
+ * differs from those of the bounds before it.  Predicated loads, all of which
+ * issue before any is used. */
 template <int COUNT>
-__device__ __forceinline__ void gs_step_pair(const GsDevIndex &I, uint32_t &l, uint32_t &e,
-                                             uint32_t &jl, uint32_t &je, uint32_t c, bool doI,
+__device__ __forceinline__ void gs_step_pair(const GsStepBy &by_i, const GsStepBy &by_j, bool within,
+                                             uint32_t &l, uint32_t &e, uint32_t &jl, uint32_t &je, bool doI,
                                              GsStepTouch &touch)
 {
     const bool jn = jl < je;
     const uint32_t bl = l >> 6, be = e >> 6, bj = jl >> 6, bk = je >> 6;
     const bool one = be == bl;                             /* I within a block: J too */
-    const bool jL = doI && bj == bl, jE = doI && bj == be;
-    const bool kL = doI && bk == bl, kE = doI && bk == be, kJ = bk == bj;
+    const bool jL = within && bj == bl, jE = within && bj == be;
+    const bool kL = within && bk == bl, kE = within && bk == be, kJ = bk == bj;
     const bool n0 = doI, n1 = doI && !one, n2 = jn && !jL && !jE, n3 = jn && !kL && !kE && !kJ;
-    const GsSlot A = gs_load_slot_if(n0, I.occ, l, c);
-    GsSlot E = gs_load_slot_if(n1, I.occ, e, c);
-    GsSlot P = gs_load_slot_if(n2, I.occ, jl, c);
-    GsSlot Q = gs_load_slot_if(n3, I.occ, je, c);
+    const GsSlot A = gs_load_slot_if(n0, by_i.occ, l, by_i.c, by_i.sh);
+    GsSlot E = gs_load_slot_if(n1, by_i.occ, e, by_i.c, by_i.sh);
+    GsSlot P = gs_load_slot_if(n2, by_j.occ, jl, by_j.c, by_j.sh);
+    GsSlot Q = gs_load_slot_if(n3, by_j.occ, je, by_j.c, by_j.sh);
     E = gs_slot_sel(one, A, E);
     P = gs_slot_sel(jL, A, gs_slot_sel(jE, E, P));
     Q = gs_slot_sel(kL, A, gs_slot_sel(kE, E, gs_slot_sel(kJ, P, Q)));

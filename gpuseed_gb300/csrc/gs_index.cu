@@ -18,12 +18,12 @@
 struct gs_index {
     int device;
     GsDevIndex dev;
-    uint4 *d_occ;
+    uint4 *d_occ, *d_occ2;
     uint32_t *d_sa;
     uint2 *d_kmer;
     uint4 *d_kmerx;
     uint32_t *d_saf, *d_text, *d_isa;
-    size_t occ_bytes, sa_bytes, kmer_bytes, kmerx_bytes, text_bytes;
+    size_t occ_bytes, occ2_bytes, sa_bytes, kmer_bytes, kmerx_bytes, text_bytes;
     float l2_hit_ratio;
     uint32_t gen;   /* bumped whenever device pointers change */
 };
@@ -194,6 +194,45 @@ __global__ void gs_occ_kernel(const uint32_t *file, uint4 *occ, uint64_t nblk, u
     }
 }
 
+/* The same for steps of two bases: per 64 rows a slot for each base c of a row
+ * and base d of the row that c steps to, at 4c + d, 256 bytes a block (the
+ * four d of a c one 64-byte fill).  Its count is where the block's first row
+ * comes to by c and then d, its mask the block's rows that hold c and whose
+ * next hold d; $ rows are in none, at either step.  Four bytes a base of
+ * the text, at every size: 100 Mbp, whose occurrence table alone the L2 holds,
+ * gains as well.  A warp a block: the rows of one base step to rows in a
+ * row, so the 64 steps read few blocks (10 Mbp 62 us). */
+__global__ void gs_occ2_kernel(GsDevIndex I, uint4 *occ2, uint64_t nblk)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t stride = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nblk; b += stride) {
+        const uint32_t c = (lane >> 2) & 3u, d = lane & 3u;
+        uint32_t m[2];
+        for (uint32_t h = 0; h < 2; h++) {
+            const uint64_t r = b * 64u + h * 32u + lane;
+            bool in = r <= I.seq_len && r != I.primary;
+            uint32_t rc = 0, rd = 0;
+            if (in) {
+                const GsBlk B = gs_load_block(I.occ, (uint32_t)r);
+                rc = gs_block_base(B, (uint32_t)r);
+                const uint32_t prev = gs_block_lf(B, (uint32_t)r, rc);
+                in = prev != I.primary;
+                if (in) rd = gs_block_base(gs_load_block(I.occ, prev), prev);
+            }
+            const uint32_t v = __ballot_sync(0xffffffffu, in);
+            const uint32_t c0 = __ballot_sync(0xffffffffu, rc & 1u), c1 = __ballot_sync(0xffffffffu, rc & 2u);
+            const uint32_t d0 = __ballot_sync(0xffffffffu, rd & 1u), d1 = __ballot_sync(0xffffffffu, rd & 2u);
+            m[h] = v & (c & 1u ? c0 : ~c0) & (c & 2u ? c1 : ~c1) & (d & 1u ? d0 : ~d0) & (d & 2u ? d1 : ~d1);
+        }
+        if (lane < 16u) {
+            const uint32_t at = gs_load_slot(I.occ, (uint32_t)(b * 64u), c).cnt;
+            const uint32_t cnt = gs_slot_rank(gs_load_slot(I.occ, at, d), at);
+            occ2[b * 16u + lane] = make_uint4(cnt, m[0], m[1], 0u);
+        }
+    }
+}
+
 /* Longer start table by reference length: one table entry per distinct
  * kx-mer the text can hold (4^kx around seq_len) */
 static int auto_kmer_len(uint32_t seq_len)
@@ -272,6 +311,19 @@ static int make_index(uint32_t primary, const uint32_t L2_1to4[4], const uint32_
     for (int kx = auto_kmer_len(seq_len); kx >= GS_K0; kx--)
         if (gs_index_set_kmer_len(idx, kx) == GS_OK) break;
     cudaGetLastError();
+    /* and so are the steps of two bases */
+    if (cudaMalloc(&idx->d_occ2, nblk * 16 * sizeof(uint4)) == cudaSuccess) {
+        gs_occ2_kernel<<<152 * 32, 256>>>(D, idx->d_occ2, nblk);
+        if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
+            gs_index_free(idx);
+            return gs_cuda_fail(e, "occurrence table layout");
+        }
+        idx->occ2_bytes = nblk * 16 * sizeof(uint4);
+        D.occ2 = idx->d_occ2;
+    } else {
+        cudaGetLastError();
+        idx->d_occ2 = NULL;
+    }
     *out = idx;
     return GS_OK;
 }
@@ -422,6 +474,7 @@ extern "C" void gs_index_free(gs_index *idx)
 {
     if (!idx) return;
     cudaFree(idx->d_occ);
+    cudaFree(idx->d_occ2);
     cudaFree(idx->d_sa);
     cudaFree(idx->d_kmer);
     cudaFree(idx->d_kmerx);
@@ -441,7 +494,7 @@ extern "C" int gs_index_get_info(const gs_index *idx, gs_index_info *out)
     for (int c = 0; c < 5; c++) out->L2[c] = idx->dev.L2[c];
     out->device = idx->device;
     out->device_bytes =
-        idx->occ_bytes + idx->sa_bytes + idx->kmer_bytes + idx->kmerx_bytes + idx->text_bytes;
+        idx->occ_bytes + idx->occ2_bytes + idx->sa_bytes + idx->kmer_bytes + idx->kmerx_bytes + idx->text_bytes;
     out->kmer_len = idx->dev.kx ? idx->dev.kx : GS_K0;
     out->text_min = idx->d_saf ? (idx->dev.text_min ? idx->dev.text_min : -1) : 0;
     return GS_OK;

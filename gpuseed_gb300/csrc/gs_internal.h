@@ -45,6 +45,7 @@
 #define GS_REGIME_MARK 0xe0000000u   /* jl (+ steps) of a one-row walker without J */
 struct GsDevIndex {
     const uint4 *occ;
+    const uint4 *occ2;         /* steps of two bases (gs_occ2_kernel), or NULL */
     const uint32_t *sa;
     const uint2 *kmer;
     const uint4 *kmerx;        /* paired table of all kx-mers, same bit order (or NULL): x,y the

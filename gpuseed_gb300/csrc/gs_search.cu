@@ -1272,18 +1272,43 @@ struct GsWalkCounts {
     unsigned long long steps, jsteps, jblocks, jshrank, jwalkers, lines256, lines384;
 };
 
+/* Steps of two bases (the walk pass).  A walk is a chain of dependent steps,
+ * each of which waits for slots at random places of the occurrence table.
+ * occ2 has a slot for each base and the base after, so one step by a slot of
+ * the same form goes two bases.
+ *   - At odd read positions only: the neighbour's walk, a base ahead or
+ *     behind in the same warp, then comes by the same strings, and so the same
+ *     slots, as this one's J.  Without that nearly every slot was a fill
+ *     of its own: 2 M reads on 3.1 Gbp 13.9 GB of DRAM reads, 17.4 without.
+ *   - J's step to I's far end goes on with I's first step, J by two bases and
+ *     I by the second of them, at the parity that makes it the neighbour's own
+ *     first step of two (11.7 GB).
+ *   - Contained at the first base is contained at the second, unless I ends
+ *     between: an empty I is not taken, and the next step is with the first
+ *     base alone (or J's alone) and the walk's last.
+ * Walk pass before and after: 2 M reads 7.26 -> 5.18 ms, 40,000 long reads
+ * 2.77 -> 2.19, 1 M reads on 100 Mbp 2.72 -> 2.32, 300 reads 89 -> 63 us.
+ *
+ * The walk pass's bases ahead: those of the next step and of the one after
+ * (0, no base, past the read), here before they are needed; alone: the two
+ * together end the walk. */
+struct GsAhead {
+    unsigned char first, second;
+    bool alone;
+};
+
 template <int NSTOP, int COUNT, bool TEXT, bool PRE = false>
 __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned char *seq, int iL,
                                              bool fwd, int dir, uint32_t &l, uint32_t &u,
                                              uint32_t &jl, uint32_t &ju, int &pos, bool &jpend,
                                              bool &killed, unsigned long long &wb,
                                              GsWalkCounts *wc = nullptr,
-                                             unsigned char *pre = nullptr)
+                                             GsAhead *pre = nullptr)
 {
     /* TEXT: text-mode states run here; otherwise the caller hands a walker
      * that enters text mode to the text pass */
     const bool text = TEXT && jl >= GS_TEXT_MARK;
-    bool settle = false;
+    bool settle = false, two = false, fused = false;
     int np = pos;
     uint32_t c;
     if (text) {
@@ -1296,14 +1321,30 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
         jpend = false;
         np = settle ? pos : pos + dir;
         if (np < 0 || np >= iL) return false;
-        const unsigned char ch = PRE ? *pre : seq[np];
+        const unsigned char ch = PRE ? pre->first : seq[np];
         c = fwd ? gs_fwd_code(ch) : gs_comp_code(ch);
-        /* PRE: this step's base is here already, the next step's comes while
+        /* PRE: this step's bases are here already, the next step's come while
          * this one waits for its slots (1 M reads on 100 Mbp 7.27 -> 7.08 ms,
          * 2 M on 3.1 Gbp 15.34 -> 15.28, 300 reads' walk -5 us) */
-        if (PRE && np + dir >= 0 && np + dir < iL) *pre = seq[np + dir];
+        if (PRE) {
+            const uint32_t d = fwd ? gs_fwd_code(pre->second) : gs_comp_code(pre->second);
+            const bool both = I.occ2 && !pre->alone && c <= 3u && d <= 3u;
+            two = both && !settle && (np & 1);
+            fused = both && settle && (np & 1);
+            const bool ahead = two || fused;
+            const int n1 = np + dir + dir, n2 = n1 + dir;
+            const unsigned char x = n1 >= 0 && n1 < iL ? seq[n1] : 0;
+            const unsigned char y = ahead && n2 >= 0 && n2 < iL ? seq[n2] : 0;
+            pre->first = ahead ? x : pre->second;
+            pre->second = ahead ? y : x;
+            if (ahead) {
+                np += dir;
+                c = c << 2 | d;
+            }
+        }
     }
-    if (c > 3u) {
+    const bool doI = !settle || fused;
+    if (!two && !fused && c > 3u) {
         if (!settle) {
             if (NSTOP) return false;
             pos = np;   /* wildcard: both intervals unchanged, so no new equality */
@@ -1314,9 +1355,11 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
         uint32_t nl = l, ne = u + 1u, je = ju + 1u;
         const bool had_j = jl <= ju;
         GsStepTouch touch;
-        gs_step_pair<COUNT>(I, nl, ne, jl, je, c, !settle, touch);
+        uint32_t njl = jl;
+        const GsStepBy by_i = {two ? I.occ2 : I.occ, two ? 2u : 0u, fused ? c & 3u : c};
+        const GsStepBy by_j = {two || fused ? I.occ2 : I.occ, two || fused ? 2u : 0u, c};
+        gs_step_pair<COUNT>(by_i, by_j, !settle, nl, ne, njl, je, doI, touch);
         const uint32_t nu = ne - 1u;
-        ju = je - 1u;
         if (COUNT) wb += (unsigned long long)touch.blocks;
         if (COUNT && wc) {
             wc->steps++;
@@ -1325,9 +1368,18 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
             if (had_j) {
                 wc->jsteps++;
                 wc->jblocks += (unsigned long long)touch.jblocks;
-                if (!settle && nl <= nu && nu - nl < u - l) wc->jshrank++;
+                if (doI && nl <= nu && nu - nl < u - l) wc->jshrank++;
             }
         }
+        if (PRE && (two || fused) && nl > nu) {
+            /* it ends at one of the two: by the first alone */
+            pre->alone = true;
+            pre->first = seq[np - dir];
+            jpend = fused;
+            return true;
+        }
+        jl = njl;
+        ju = je - 1u;
         if (text) {
             l = nl;
             u = nu;
@@ -1339,7 +1391,7 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
             ju = 0u;
             return true;
         }
-        if (!settle) {
+        if (doI) {
             if (nl > nu) return false;   /* natural end at pos */
             l = nl;
             u = nu;
@@ -1350,6 +1402,7 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
         killed = true;
         return false;
     }
+    if (PRE && pre->alone) return false;   /* the second base ends it */
     /* one row and no J: count the steps taken so (J's words are free);
      * after text_min of them the occurrence is no chance hit, and with 16
      * bases or more left the walker enters text mode */
@@ -1357,7 +1410,7 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
         if (jl < GS_REGIME_MARK) {
             jl = GS_REGIME_MARK;
             ju = 0u;
-        } else if (++jl - GS_REGIME_MARK >= (uint32_t)I.text_min &&
+        } else if ((jl += two ? 2u : 1u) - GS_REGIME_MARK >= (uint32_t)I.text_min &&
                    (fwd ? pos : iL - 1 - pos) >= 16) {
             jl = GS_TEXT_MARK;
         }
@@ -1785,7 +1838,7 @@ __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_wa
     int anchor = 0, pos = 0, iL = 0, dir = 0;
     bool fwd = false;
     const unsigned char *seq = NULL;
-    unsigned char pre = 0;   /* the next step's base */
+    GsAhead pre = {0, 0, false};
     GsWalkCounts wc = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
     for (;;) {
         uint32_t need = __ballot_sync(0xffffffffu, !have);
@@ -1823,8 +1876,10 @@ __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_wa
                     have = true;
                     killed = false;
                     jpend = (w.anchor & GS_WALKER_JPEND) != 0;
-                    const int np = jpend ? pos : pos + dir;
-                    if (np >= 0 && np < iL) pre = seq[np];
+                    const int np = jpend ? pos : pos + dir, nn = np + dir;
+                    pre.first = np >= 0 && np < iL ? seq[np] : 0;
+                    pre.second = nn >= 0 && nn < iL ? seq[nn] : 0;
+                    pre.alone = false;
                     if (COUNT && (jpend || jl <= ju)) wc.jwalkers++;
                 }
             }
