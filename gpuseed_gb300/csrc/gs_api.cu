@@ -436,14 +436,14 @@ __global__ void gs_max_end_kernel(const uint64_t *off, const uint32_t *len, uint
  * large copy-out on another stream. */
 __global__ void gs_fetch_small_kernel(uint32_t *dst, const uint32_t *src, uint32_t n_words)
 {
+    gs_after_previous();
     if (threadIdx.x < n_words) dst[threadIdx.x] = src[threadIdx.x];
 }
 
 static int fetch_small(uint64_t *dst, const void *src, size_t bytes, cudaStream_t st)
 {
-    gs_fetch_small_kernel<<<1, 32, 0, st>>>((uint32_t *)dst, (const uint32_t *)src,
-                                            (uint32_t)(bytes / 4));
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(gs_launch_after(gs_fetch_small_kernel, 1, 32, st, (uint32_t *)dst, (const uint32_t *)src,
+                            (uint32_t)(bytes / 4)));
     return GS_OK;
 }
 
@@ -636,6 +636,7 @@ __global__ void __launch_bounds__(256) gs_copy_out_kernel(GsBatch B, uint64_t *s
                                                           uint4 *seeds, uint64_t seed_cap, uint32_t *pos,
                                                           uint64_t pos_cap, uint32_t *queue)
 {
+    gs_after_previous();
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     if (t < 8) queue[t] = B.queue[t];
@@ -707,10 +708,9 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
             RC(gs_launch_locate(I, B, UINT64_MAX, st));
         }
         const unsigned grid = n_reads < 152u * 16u ? (n_reads + 15u) / 16u : 152u;
-        gs_copy_out_kernel<<<grid, 256, 0, st>>>(
-            B, fetch ? c->h_seed_off : NULL, c->h_pos_off, (uint4 *)c->h_seeds, c->cap_h_seeds, c->h_pos,
-            c->cap_h_pos, (uint32_t *)&c->h_small[GS_H_QUEUE]);
-        GS_CUDA(cudaGetLastError());
+        GS_CUDA(gs_launch_after(gs_copy_out_kernel, grid, 256, st, B, fetch ? c->h_seed_off : NULL,
+                                c->h_pos_off, (uint4 *)c->h_seeds, c->cap_h_seeds, c->h_pos, c->cap_h_pos,
+                                (uint32_t *)&c->h_small[GS_H_QUEUE]));
         GS_CUDA(cudaEventRecord(c->ev1, st));
         GS_CUDA(cudaStreamSynchronize(st));
         c->n_seeds = c->h_small[GS_H_TOTALS + 2];

@@ -353,6 +353,7 @@ __device__ __noinline__ void gs_finalize_read_warp(const GsBatch &B, uint32_t r,
  * The blocks' sums become the offsets of gs_finalize_emit. */
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_count(GsBatch B, uint32_t tile)
 {
+    gs_after_previous();
     const int lane = threadIdx.x & 31;
     const uint32_t per_warp = tile / (GS_SCAN_THREADS / 32u);
     uint32_t first, last;
@@ -553,6 +554,7 @@ template <bool WARP>
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, uint64_t *seed_pos,
                                                                     uint32_t tile)
 {
+    gs_after_previous();
     __shared__ gs_seed_rec rounds[WARP ? GS_SCAN_THREADS : 1u];
     uint32_t first, last;
     gs_part_reads(B.n_reads, tile, blockIdx.x, gridDim.x, first, last);
@@ -605,6 +607,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_finalize_emit(GsBatch B, u
  * rows from l outside that interval.  Thread per read, after the emit. */
 __global__ void __launch_bounds__(128) gs_mem_next_kernel(GsBatch B)
 {
+    gs_after_previous();
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= B.n_reads) return;
     const uint64_t s0 = B.seed_off[r], s1 = B.seed_off[r + 1];
@@ -663,6 +666,7 @@ __global__ void __launch_bounds__(128) gs_mem_next_kernel(GsBatch B)
 template <bool SAF>
 __global__ void __launch_bounds__(256, 8) gs_locate(GsDevIndex I, GsBatch B)
 {
+    gs_after_previous();
     /* a replayed pass with more output than it was sized for: the host sees
      * the totals and sizes it again */
     const uint64_t n_pos = B.totals[3], n_seeds = B.totals[2];
@@ -760,8 +764,7 @@ int gs_launch_finalize_count(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
 {
     (void)I;
     const uint32_t tile = gs_finalize_tile(B);
-    gs_finalize_count<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, tile);
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(gs_launch_after(gs_finalize_count, gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, st, B, tile));
     return GS_OK;
 }
 
@@ -771,8 +774,7 @@ int gs_launch_finalize_emit(const GsDevIndex &I, GsBatch &B, cudaStream_t st)
     const uint32_t tile = gs_finalize_tile(B);
     void (*emit)(GsBatch, uint64_t *, uint32_t) =
         gs_finalize_by_warp(B) ? gs_finalize_emit<true> : gs_finalize_emit<false>;
-    emit<<<gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, 0, st>>>(B, B.seed_pos, tile);
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(gs_launch_after(emit, gs_parts_of(B.n_reads, tile), GS_SCAN_THREADS, st, B, B.seed_pos, tile));
     if (B.n_reads && !B.smem && B.mem_next == GS_MEM_NEXT_GPUSEED) {
         gs_mem_next_kernel<<<(B.n_reads + 127) / 128, 128, 0, st>>>(B);
         GS_CUDA(cudaGetLastError());
@@ -788,8 +790,6 @@ int gs_launch_locate(const GsDevIndex &I, GsBatch &B, uint64_t n_pos, cudaStream
      * (twice what is resident) */
     uint64_t grid = (n + 255) / 256;
     if (grid > 152ull * 16) grid = 152ull * 16;
-    if (I.saf) gs_locate<true><<<(unsigned)grid, 256, 0, st>>>(I, B);
-    else gs_locate<false><<<(unsigned)grid, 256, 0, st>>>(I, B);
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(gs_launch_after(I.saf ? gs_locate<true> : gs_locate<false>, (unsigned)grid, 256, st, I, B));
     return GS_OK;
 }

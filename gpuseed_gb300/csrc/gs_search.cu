@@ -715,6 +715,7 @@ __device__ __forceinline__ void gs_clear(const GsBatch &B)
 
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_sum(GsBatch B, int paired_kt)
 {
+    gs_after_previous();
     gs_clear(B);
     uint32_t first, last;
     gs_part_reads(B.n_reads, GS_SCAN_THREADS, blockIdx.x, gridDim.x, first, last);
@@ -735,6 +736,7 @@ __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_sum(GsBatch B, int
  * read, or the warp for a read of many items). */
 __global__ void __launch_bounds__(GS_SCAN_THREADS) gs_prepare_scan(GsBatch B, int paired_kt)
 {
+    gs_after_previous();
     const int lane = threadIdx.x & 31;
     if (gridDim.x == 1) gs_clear(B);
     uint32_t first, last;
@@ -788,8 +790,13 @@ int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t 
         gs_prepare_sum<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
         GS_CUDA(cudaGetLastError());
     }
-    gs_prepare_scan<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
-    GS_CUDA(cudaGetLastError());
+    if (parts > 1) {
+        GS_CUDA(gs_launch_after(gs_prepare_scan, parts, GS_SCAN_THREADS, st, b, kt));
+    } else {
+        /* the pass's first kernel: after all that the stream holds */
+        gs_prepare_scan<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
+        GS_CUDA(cudaGetLastError());
+    }
     return GS_OK;
 }
 
@@ -1736,6 +1743,7 @@ __device__ __forceinline__ void gs_start_pair_item(const GsDevIndex &I, const Gs
 template <int NSTOP, int COUNT, bool PAIRED>
 __global__ void __launch_bounds__(256, GS_START_CTAS) gs_search_start(GsDevIndex I, GsBatch B, int queue_chunk)
 {
+    gs_after_previous();
     const int lane = threadIdx.x & 31;
     unsigned long long wk = 0, wb = 0;
     GsReserve res = {0u, 0u, B.walker_cap == 0 ? 1u : 0u};
@@ -1818,6 +1826,7 @@ __device__ __forceinline__ uint32_t gs_list_room(GsListPart &part, uint32_t *cou
 template <int NSTOP, int COUNT>
 __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_walk(GsDevIndex I, GsBatch B)
 {
+    gs_after_previous();
     __shared__ GsListPart s_text[GS_WALK_WARPS];
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -1941,6 +1950,7 @@ __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_wa
 template <int NSTOP, int COUNT>
 __global__ void __launch_bounds__(256) gs_search_text(GsDevIndex I, GsBatch B)
 {
+    gs_after_previous();
     uint64_t n_jobs = B.queue[4];
     if (n_jobs > B.text_cap) n_jobs = B.text_cap;
     unsigned long long wb = 0;
@@ -1977,6 +1987,7 @@ __global__ void __launch_bounds__(256) gs_search_text(GsDevIndex I, GsBatch B)
 template <int NSTOP, int COUNT>
 __global__ void __launch_bounds__(256) gs_search_leftover(GsDevIndex I, GsBatch B)
 {
+    gs_after_previous();
     if (!(*(volatile uint32_t *)(B.queue + 1) & GS_FLAG_LEFTOVER)) return;
     const int lane = threadIdx.x & 31;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2151,24 +2162,21 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
     }
     if (grid == 0) grid = 1;
     B.walker_chunk = gs_walker_chunk(B.walker_cap, grid * 8u);
-    start<<<grid, 256, 0, st>>>(I, B, queue_chunk);
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(gs_launch_after(start, grid, 256, st, I, B, queue_chunk));
     if (B.walker_cap) {
         /* no more warps than the items can have walkers for, 32 each */
         uint32_t wgrid = (uint32_t)sms * GS_WALK_CTAS;
         const uint64_t most = (uint64_t)items * (2u * GS_PCHUNK) / (GS_WALK_WARPS * 32u) + 1u;
         if (most < wgrid) wgrid = (uint32_t)most;
         B.text_chunk = gs_list_chunk(B.text_cap, wgrid * GS_WALK_WARPS);
-        walk<<<wgrid, GS_WALK_WARPS * 32, 0, st>>>(I, B);
-        GS_CUDA(cudaGetLastError());
+        GS_CUDA(gs_launch_after(walk, wgrid, GS_WALK_WARPS * 32, st, I, B));
         if (B.text_cap) {
             void (*text)(GsDevIndex, GsBatch) =
                 nstop ? (cnt ? gs_search_text<1, 1> : gs_search_text<1, 0>)
                       : (cnt ? gs_search_text<0, 1> : gs_search_text<0, 0>);
             uint32_t tgrid = (uint32_t)sms * 8u;
             if (B.text_cap < (uint64_t)tgrid * 256u) tgrid = (uint32_t)(B.text_cap / 256u) + 1u;
-            text<<<tgrid, 256, 0, st>>>(I, B);
-            GS_CUDA(cudaGetLastError());
+            GS_CUDA(gs_launch_after(text, tgrid, 256, st, I, B));
         }
     }
     void (*leftover)(GsDevIndex, GsBatch) =
@@ -2176,8 +2184,7 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
               : (cnt ? gs_search_leftover<0, 1> : gs_search_leftover<0, 0>);
     uint32_t lgrid = (uint32_t)sms * 8u;
     if (B.n_reads < lgrid * 8u) lgrid = B.n_reads / 8u + 1u;
-    leftover<<<lgrid, 256, 0, st>>>(I, B);
-    GS_CUDA(cudaGetLastError());
+    GS_CUDA(gs_launch_after(leftover, lgrid, 256, st, I, B));
     return GS_OK;
 }
 
