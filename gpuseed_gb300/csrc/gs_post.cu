@@ -655,17 +655,50 @@ __global__ void __launch_bounds__(128) gs_mem_next_kernel(GsBatch B)
 }
 
 /* Positions: a warp takes a tile of them, 32 a round (they span at most 32
- * seeds, as every seed has a position), from the seed of the tile's first
+ * seeds, as every seed has a position), from the seed of the round's first
  * position, which gs_finalize_emit noted.  It writes the position -> seed map
  * for the text records and resolves each row.  A seed of many positions is
  * spread over many warps.  Tiles of 32 to 256, so that few positions spread
- * over many warps: a round of LF walks is up to sa_intv - 1 dependent pairs
- * of loads. */
+ * over many warps.
+ *
+ * With the full suffix array a row is one read.  Else it is a chain of LF
+ * steps, up to sa_intv - 1 of them, whose latency bounds the kernel: a tile's
+ * rows go through shared memory, and a lane whose row is resolved takes the
+ * next, so that a warp does not wait for the longest chain of each 32 (1 M
+ * reads on 100 Mbp, 2.3 M positions 246 -> 208 us; 150,001 reads 166 -> 131).
+ * A tile of one round has nothing to hand out: each lane runs its own chain
+ * (10,000 reads on 5 Mbp 38 us, 47 through shared memory). */
 #define GS_LOCATE_MOST 256u
+
+/* the row of position p (in the round from pb), and its seed */
+__device__ __forceinline__ uint32_t gs_position_row(const GsBatch &B, uint64_t pb, uint64_t p, bool in,
+                                                    uint64_t n_seeds, int lane)
+{
+    const uint64_t s0 = __ldg(&B.tile_seed[pb >> 5]);
+    /* first positions of seeds s0+1 .. s0+32 */
+    const uint64_t at = s0 + 1u + (uint64_t)lane;
+    const uint64_t next = at < n_seeds ? __ldg(&B.seed_pos[at]) : ~0ull;
+    int k = 0;   /* how many of them are at or before p */
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1)
+        if (__shfl_sync(0xffffffffu, next, k + step - 1) <= p) k += step;
+    if (__shfl_sync(0xffffffffu, next, k) <= p) k++;
+    const uint64_t s = s0 + (uint64_t)k;
+    if (!in) return 0u;
+    const uint4 *rec = reinterpret_cast<const uint4 *>(B.seeds + s);
+    const uint4 S = __ldg(rec), T = __ldg(rec + 1);   /* x y l u, xl xu n_pos pad */
+    B.pmap[p] = (uint32_t)s;
+    /* the (p - first)-th row from l outside [xl, xu] */
+    uint32_t row = S.z + (uint32_t)(p - __ldg(&B.seed_pos[s]));
+    const uint32_t x0 = T.x > S.z ? T.x : S.z;
+    if (T.x <= T.y && T.y >= x0 && row >= x0) row += T.y - x0 + 1u;
+    return row;
+}
 
 template <bool SAF>
 __global__ void __launch_bounds__(256, 8) gs_locate(GsDevIndex I, GsBatch B)
 {
+    __shared__ uint32_t rows[SAF ? 1 : 8][GS_LOCATE_MOST];
     gs_after_previous();
     /* a replayed pass with more output than it was sized for: the host sees
      * the totals and sizes it again */
@@ -679,63 +712,87 @@ __global__ void __launch_bounds__(256, 8) gs_locate(GsDevIndex I, GsBatch B)
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * tile < n_pos;
          w += nwarps) {
         const uint64_t p0 = w * tile;
-        const uint64_t p1 = p0 + tile < n_pos ? p0 + tile : n_pos;
-        uint64_t s0 = B.tile_seed[p0 >> 5];
-        for (uint64_t pb = p0; pb < p1; pb += 32) {
-            const uint64_t p = pb + (uint64_t)lane;
-            /* first positions of seeds s0+1 .. s0+32 */
-            const uint64_t at = s0 + 1u + (uint64_t)lane;
-            const uint64_t next = at < n_seeds ? B.seed_pos[at] : ~0ull;
-            int k = 0;   /* how many of them are at or before p */
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1)
-                if (__shfl_sync(0xffffffffu, next, k + step - 1) <= p) k += step;
-            if (__shfl_sync(0xffffffffu, next, k) <= p) k++;
-            const uint64_t s = s0 + (uint64_t)k;
-            uint32_t steps = 0;
-            const bool active = p < p1;
-            if (active) {
-                const gs_seed_rec S = B.seeds[s];
-                B.pmap[p] = (uint32_t)s;
-                /* the (p - first)-th row from l outside [xl, xu] */
-                uint32_t row = S.l + (uint32_t)(p - B.seed_pos[s]);
-                const uint32_t x0 = S.xl > S.l ? S.xl : S.l;
-                if (S.xl <= S.xu && S.xu >= x0 && row >= x0) row += S.xu - x0 + 1u;
-                /* locate_seeds_gpu (:668-684): LF until a sampled row; a
-                 * consistent index reaches one within seq_len+1 steps.  With
-                 * the full suffix array it is one read: the walk's result is
-                 * SA[row], except that the LF quirk sends the rows whose walk
-                 * passes row primary+1 to row 0, where sa[0] = -1 gives the
-                 * steps taken minus one -- position - quirk_lo. */
-                if (SAF) {
-                    uint32_t v = gs_ld64(&I.saf[row]);
-                    if (B.lf_mode == GS_LF_GPUSEED && v - I.quirk_lo < I.quirk_n) v -= I.quirk_lo;
-                    B.pos[p] = v;
-                } else {
-                    while (row % I.sa_intv && steps <= cap) {
+        const uint32_t n = (uint32_t)(p0 + tile < n_pos ? tile : n_pos - p0);
+        if (SAF) {
+            /* the chain's result is SA[row], except that the LF quirk sends
+             * the rows whose chain passes row primary+1 to row 0, where
+             * sa[0] = -1 gives the steps taken minus one: position -
+             * quirk_lo. */
+            for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+                const uint64_t p = p0 + i0 + (uint32_t)lane;
+                const bool in = i0 + (uint32_t)lane < n;
+                const uint32_t row = gs_position_row(B, p0 + i0, p, in, n_seeds, lane);
+                if (!in) continue;
+                uint32_t v = gs_ld64(&I.saf[row]);
+                if (B.lf_mode == GS_LF_GPUSEED && v - I.quirk_lo < I.quirk_n) v -= I.quirk_lo;
+                B.pos[p] = v;
+            }
+            if (B.work && lane == 0) atomicAdd(&B.work[3], (unsigned long long)n);
+            continue;
+        }
+        /* locate_seeds_gpu (:668-684): LF until a sampled row; a consistent
+         * index reaches one within seq_len+1 steps */
+        unsigned long long all = 0;
+        const auto resolve = [&](uint64_t p, uint32_t row, uint32_t steps) {
+            uint32_t v = 0xffffffffu;
+            if (steps > cap) atomicOr(B.queue + 1, GS_FLAG_WALK);
+            else v = __ldg(&I.sa[row / I.sa_intv]) + steps;
+            B.pos[p] = v;
+            all += steps;
+        };
+        if (n <= 32u) {
+            const uint64_t p = p0 + (uint32_t)lane;
+            uint32_t row = gs_position_row(B, p0, p, (uint32_t)lane < n, n_seeds, lane), steps = 0;
+            if ((uint32_t)lane < n) {
+                while (row % I.sa_intv && steps <= cap) {
+                    row = gs_lf(I, row, B.lf_mode);
+                    steps++;
+                }
+                resolve(p, row, steps);
+            }
+        } else {
+            uint32_t *list = rows[threadIdx.x >> 5];
+            for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+                const uint32_t i = i0 + (uint32_t)lane;
+                const uint32_t row = gs_position_row(B, p0 + i0, p0 + i, i < n, n_seeds, lane);
+                if (i < n) list[i] = row;
+            }
+            __syncwarp();
+            uint32_t i = 0, row = 0, steps = 0, taken = 0;
+            bool have = false;
+            for (;;) {
+                const uint32_t need = __ballot_sync(0xffffffffu, !have);
+                if (need && taken < n) {
+                    if (!have) {
+                        i = taken + (uint32_t)__popc(need & ((1u << lane) - 1u));
+                        have = i < n;
+                        if (have) {
+                            row = list[i];
+                            steps = 0;
+                        }
+                    }
+                    taken += (uint32_t)__popc(need);
+                } else if (need == 0xffffffffu) {
+                    break;
+                }
+                if (have) {
+                    if (row % I.sa_intv == 0 || steps > cap) {
+                        resolve(p0 + i, row, steps);
+                        have = false;
+                    } else {
                         row = gs_lf(I, row, B.lf_mode);
                         steps++;
                     }
-                    if (steps > cap) {
-                        atomicOr(B.queue + 1, GS_FLAG_WALK);
-                        B.pos[p] = 0xffffffffu;
-                    } else {
-                        B.pos[p] = __ldg(&I.sa[row / I.sa_intv]) + steps;
-                    }
                 }
             }
-            if (B.work) {
-                unsigned long long st = steps, np = active ? 1ull : 0ull;
-                for (int off = 16; off; off >>= 1) {
-                    st += __shfl_xor_sync(0xffffffffu, st, off);
-                    np += __shfl_xor_sync(0xffffffffu, np, off);
-                }
-                if (lane == 0 && np) {
-                    atomicAdd(&B.work[2], st);
-                    atomicAdd(&B.work[3], np);
-                }
+            __syncwarp();
+        }
+        if (B.work) {
+            for (int off = 16; off; off >>= 1) all += __shfl_xor_sync(0xffffffffu, all, off);
+            if (lane == 0) {
+                atomicAdd(&B.work[2], all);
+                atomicAdd(&B.work[3], (unsigned long long)n);
             }
-            s0 = __shfl_sync(0xffffffffu, s, 31);
         }
     }
 }
@@ -786,10 +843,11 @@ int gs_launch_locate(const GsDevIndex &I, GsBatch &B, uint64_t n_pos, cudaStream
 {
     if (B.n_reads == 0 || B.seed_cap == 0 || B.pos_cap == 0 || n_pos == 0) return GS_OK;
     uint64_t n = n_pos < B.pos_cap ? n_pos : B.pos_cap;
-    /* eight warps a block, a round of positions each, at most 16 blocks an SM
-     * (twice what is resident) */
+    /* eight warps a block, a round of positions each, at most what is
+     * resident, 8 blocks an SM (twice that where a position is one read) */
+    const uint64_t most = 152ull * (I.saf ? 16u : 8u);
     uint64_t grid = (n + 255) / 256;
-    if (grid > 152ull * 16) grid = 152ull * 16;
+    if (grid > most) grid = most;
     GS_CUDA(gs_launch_after(I.saf ? gs_locate<true> : gs_locate<false>, (unsigned)grid, 256, st, I, B));
     return GS_OK;
 }
