@@ -6,8 +6,8 @@
  * cannot afford the device-wide synchronisation cudaMalloc/cudaFree imply
  * while other streams are busy.  gs_seed_device() grows a per-context
  * workspace with cudaMalloc; gs_seed_noalloc() instead keeps every scratch
- * buffer of the pass (candidate slots, per-read counters, work queue, scan
- * temporaries, the position-to-seed map) in one file-scope device array of
+ * buffer of the pass (candidate slots, per-read counters, work queue, block
+ * sums, the position-to-seed map) in one file-scope device array of
  * GS_NOALLOC_SCRATCH_BYTES, which every GPU that loads the library holds
  * until the process exits.  The caller passes the reads and the output
  * buffers; results are written only there.

@@ -156,10 +156,12 @@ int gs_index_kmer_table(const gs_index *idx, uint64_t first, uint64_t count, uin
 int gs_index_build(const uint8_t *codes, uint64_t n, uint32_t sa_intv, int device,
                    const char *prefix, gs_index **out);
 /* Length of the k-mer start table (13..16).  Loading picks 16 above 2^30
- * bases, 15 above 2^28, 14 above 2^26, else 13 (16 * 4^len bytes of HBM:
- * each len-mer's entry and its reverse complement's, so that one lookup
- * starts both strands' candidates of a read window; a lower length is taken
- * when the memory is not there).  A candidate starts from the interval of
+ * bases, 15 above 2^28, 14 above 2^26, else 13 (16 * 4^len bytes of HBM, 1 GiB
+ * at 13 and 64 GiB at 16: each len-mer's entry and its reverse complement's,
+ * so that one lookup starts both strands' candidates of a read window, with
+ * what precedes and follows the string's rows, so that most candidates end
+ * there; a lower length, or none but the plain 13-mer table, is taken when
+ * the memory is not there).  A candidate starts from the interval of
  * its first len bases instead of 13 + len-13 steps: the SA interval of a
  * string does not depend on how it is found, so results do not change;
  * seeding uses it only when k > len.  Call while no pass runs on a context
@@ -234,24 +236,25 @@ void *gs_ctx_stream(gs_ctx *ctx);
  * from CUDA events recorded on the context stream. */
 int gs_ctx_last_timing(gs_ctx *ctx, float *search_ms, float *total_ms);
 /* Work of the last pass run with count_work = 1: start-table lookups,
- * 32-byte occurrence blocks of the search, LF steps and SA samples of the
+ * occurrence blocks of the search, LF steps and SA samples of the
  * locate stage.  With the plain kernel the search counts are the canonical
- * containment-stopped walk (the algorithmic work); with the other kernels
- * they are the lookups those kernels execute. */
+ * containment-stopped walk (the algorithmic work, blocks of 32 bytes for 64
+ * rows); with the other kernels they are the lookups those kernels execute:
+ * start-table entries (a paired lookup is two) and 16-byte slots of the
+ * occurrence tables, by one base or two. */
 int gs_ctx_last_work(gs_ctx *ctx, uint64_t out[4]);
 
 /* Batched search, last pass run with count_work = 1 (one pass, not
- * chunks): the walk pass's steps, its steps with a neighbour interval J, the
- * 32-byte blocks it loaded for J alone (J's bounds outside the blocks of
- * I's), the steps with J that shrank I, the walkers that started with J,
- * and the distinct 128-byte lines its steps' bounds fall in -- with this
- * occurrence table (256 rows a line) and as if blocks held 192 rows in 64
- * bytes (384 rows a line).  No counterpart in the reference: these bound
+ * chunks): the walk pass's steps (of one base or two), its steps with a
+ * neighbour interval J, the slots it loaded for J alone (J's bounds outside
+ * the 64-row blocks of I's), the steps with J that shrank I, the walkers that
+ * started with J, and the distinct groups of 256 rows, and of 384, that its
+ * steps' bounds fall in.  No counterpart in the reference: these bound
  * what another containment test or block size could save. */
 int gs_ctx_last_walk_counts(gs_ctx *ctx, uint64_t out[7]);
 /* Batched search (GS_KERNEL_BATCHED): candidates of the last call that the
- * start pass handed to the walk pass, and the walker buffer's capacity
- * (handed beyond it: walked in the start pass instead). */
+ * start pass reserved walker entries for, and the walker buffer's capacity
+ * (beyond it: walked in the leftover pass instead). */
 int gs_ctx_last_walkers(gs_ctx *ctx, uint64_t *n_walkers, uint64_t *capacity);
 /* Walkers the last batched pass handed to its text pass, and the room it had
  * for them (0, 0 without text mode). */
