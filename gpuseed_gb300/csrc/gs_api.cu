@@ -206,7 +206,7 @@ struct gs_ctx {
     uint64_t walk_counts[7];   /* count_work pass: gs_ctx_last_walk_counts */
     void *cub_tmp; size_t cap_cub;
     uint64_t *h_small;          /* pinned scalars (GS_H_*) */
-    uint64_t last_slots;        /* slots, work items and reads of the last pass */
+    uint64_t last_slots;        /* slots, work items and reads of the last pass that succeeded */
     uint32_t last_items, last_reads;
     char *h_stage; size_t cap_stage;   /* pinned: a small gs_seed batch's input, as one copy */
     char *d_stage; size_t cap_d_stage;
@@ -674,9 +674,11 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     RC(grow_reads(c, nr1));
     if (exact) {
         RC(grow(c->slots, c->cap_slots, n_slots + 1, st));
-        RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, st));
         RC(grow(c->item_read, c->cap_item_read, (size_t)n_items + 1, st));
     }
+    /* a bit for every slot there is, also where a pass before had no memory
+     * for the bits of the slots it got */
+    RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, st));
     /* a read has a handful of seeds, a seed a position or two */
     const uint64_t want_s = 8ull * n_reads + n_slots / 32 + 256;
     const uint64_t want_p = 16ull * n_reads + n_slots / 16 + 1024;
@@ -727,11 +729,11 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
         }
         if (copy) RC(grow_fetch(c, nr1, c->n_seeds, c->n_pos));
     }
+    c->timing = GS_TIMING_PASS;
+    if (read_queue(c, p) & GS_FLAG_WALK) return walk_limit_error();
     c->last_items = (uint32_t)c->h_small[GS_H_TOTALS + 1];
     c->last_slots = c->h_small[GS_H_TOTALS];
     c->last_reads = n_reads;
-    c->timing = GS_TIMING_PASS;
-    if (read_queue(c, p) & GS_FLAG_WALK) return walk_limit_error();
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;
@@ -777,9 +779,6 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     GS_CUDA(cudaStreamSynchronize(st));
     const uint64_t n_slots = c->h_small[GS_H_TOTALS];
     const uint32_t n_items = (uint32_t)(c->h_small[GS_H_TOTALS + 1] & 0xffffffffu);
-    c->last_items = n_items;
-    c->last_slots = n_slots;
-    c->last_reads = n_reads;
     RC(grow(c->slots, c->cap_slots, n_slots + 1, c->st));
     RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, c->st));
     B.slots = c->slots;
@@ -885,6 +884,9 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     if (B.work) memcpy(c->walk_counts, &c->h_small[16], sizeof(c->walk_counts));
     c->timing = GS_TIMING_PASS;
     if (flags & GS_FLAG_WALK) return walk_limit_error();
+    c->last_items = n_items;
+    c->last_slots = n_slots;
+    c->last_reads = n_reads;
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;

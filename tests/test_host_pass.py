@@ -1,0 +1,81 @@
+"""The seeding context's host code on a fake CUDA runtime: what a pass is
+sized by, and what a failed one leaves behind."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from hostlib import build_host
+
+ENOMEM = -4
+
+
+class Pass(C.Structure):
+    _fields_ = [(n, C.c_uint64) for n in ("passes", "n_items", "item_cap", "item_read_cap", "slot_cap",
+                                          "walker_cap", "clear_words", "mask_words", "items", "slots",
+                                          "seeds_a_read", "pos_a_read")]
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    L = build_host("pass", tmp_path_factory.mktemp("host"))
+    L.fake_pass.restype = C.POINTER(Pass)
+    L.fake_index.restype = C.c_void_p
+    L.gs_last_error.restype = C.c_char_p
+    return L
+
+
+class Seeder:
+    """A context, and passes over reads of given lengths"""
+
+    def __init__(self, L):
+        self.L, self.h = L, C.c_void_p()
+        assert L.gs_ctx_create(C.c_void_p(L.fake_index()), None, C.byref(self.h)) == 0
+        p = L.fake_pass().contents
+        p.seeds_a_read, p.pos_a_read = 2, 3
+
+    def run(self, lengths, device=True, fetch=0, **kw):
+        import gpuseed_gb300 as gs
+        p = gs.Context.params(**dict({"k": 19, "smem": True}, **kw))
+        lens = np.asarray(lengths, np.uint32)
+        self.offs = np.zeros(lens.size, np.uint64)
+        self.offs[1:] = np.cumsum(lens[:-1], dtype=np.uint64)
+        self.lens, self.seqs = lens, np.zeros(int(lens.sum(dtype=np.uint64)) + 1, np.uint8)
+        a = [C.c_void_p(v.ctypes.data) for v in (self.seqs, self.offs, self.lens)]
+        if device:
+            rc = self.L.gs_seed_device(self.h, *a, lens.size, C.byref(p), fetch)
+        else:
+            rc = self.L.gs_seed(self.h, *a, lens.size, C.byref(p))
+        assert self.L.fake_errors() == 0
+        return rc
+
+    @property
+    def last(self):
+        return self.L.fake_pass().contents
+
+    def close(self):
+        self.L.gs_ctx_free(self.h)
+
+
+@pytest.fixture
+def seeder(host):
+    s = Seeder(host)
+    yield s
+    host.fake_fail(0)
+    s.close()
+
+
+def test_record_mask_of_a_pass_that_had_no_memory(seeder):
+    """Each allocation of a pass larger than the one before fails in turn; the
+    batch then runs in parts, on the same context.  No pass clears or marks
+    more of the record mask than there is (the slots may have been had, and
+    the mask not)."""
+    assert seeder.run([100] * 2000) == 0
+    for at in range(1, 40):
+        seeder.L.fake_fail(at)
+        rc = seeder.run([100 + at] * (2000 + 600 * at))
+        seeder.L.fake_fail(0)
+        assert rc in (0, ENOMEM)
+        for _ in range(2):
+            assert seeder.run([100] * 1500) == 0
+            assert (seeder.last.slot_cap + 31) // 32 <= seeder.last.mask_words
