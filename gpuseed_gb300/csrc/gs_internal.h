@@ -60,6 +60,14 @@ struct GsDevIndex {
     int32_t text_min;
 };
 
+/* whether a walker's jl is text mode's state: an index without text mode has
+ * rows up to 2^32 - 2, the marks among them (with it, gs_index_set_text keeps
+ * the rows below) */
+__host__ __device__ static inline bool gs_text_mode(int32_t text_min, uint32_t jl)
+{
+    return text_min != 0 && jl >= GS_TEXT_MARK;
+}
+
 /* Candidate slot written by the search kernels; y == 0 marks "no record". */
 struct GsRec {
     int32_t x, y;

@@ -1314,7 +1314,7 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
 {
     /* TEXT: text-mode states run here; otherwise the caller hands a walker
      * that enters text mode to the text pass */
-    const bool text = TEXT && jl >= GS_TEXT_MARK;
+    const bool text = TEXT && gs_text_mode(I.text_min, jl);
     bool settle = false, two = false, fused = false;
     int np = pos;
     uint32_t c;
@@ -1906,7 +1906,7 @@ __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_wa
         }
         /* walkers that entered text mode go to the text pass, so that no
          * lane of this pass runs the compare; without room they walk on */
-        const bool tx = have && jl >= GS_TEXT_MARK;
+        const bool tx = have && gs_text_mode(I.text_min, jl);
         const uint32_t tm = __ballot_sync(0xffffffffu, tx);
         if (tm) {
             const uint32_t cap = (uint32_t)B.text_cap;

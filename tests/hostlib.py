@@ -14,8 +14,4 @@ def build_host(name, out_dir):
     subprocess.run([gbuild._nvcc(), *gbuild.ARCH, "-O1", "-std=c++17", "-cudart", "none", "-shared",
                     "-Xcompiler", "-fPIC,-Wall,-Wno-unused-function", "-Xlinker", "-Bsymbolic", "-I",
                     gbuild.INCLUDE, os.path.join(HERE, "host", name + ".cu"), "-o", so], check=True)
-    L = C.CDLL(so)
-    for f in ("fake_held", "fake_pinned_bytes"):
-        getattr(L, f).restype = C.c_size_t
-    L.fake_have.argtypes = [C.c_size_t]
-    return L
+    return C.CDLL(so)

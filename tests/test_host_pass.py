@@ -21,7 +21,7 @@ def host(tmp_path_factory):
     L = build_host("pass", tmp_path_factory.mktemp("host"))
     L.fake_pass.restype = C.POINTER(Pass)
     L.fake_index.restype = C.c_void_p
-    L.gs_last_error.restype = C.c_char_p
+    L.fake_pinned_bytes.restype = C.c_size_t
     return L
 
 
