@@ -93,6 +93,32 @@ struct __align__(8) GsWalker {
     uint32_t anchor;    /* bits 0-29: anchor; bit 30: J pending; bit 31: forward strand */
     uint32_t l, u, jl, ju;
 };
+#define GS_WALKER_HOLE 0xffffffffu    /* r of an entry that holds no walker */
+#define GS_WALKER_JPEND 0x40000000u   /* anchor flag: J is one base short of I's far end */
+#define GS_WALKER_FWD 0x80000000u
+
+/* A walker into entry idx of the buffer, of which the warp has those below
+ * `end`.  False without an entry, and for a read of 2^30 bases or more, whose
+ * anchors do not fit one: its entry becomes a hole. */
+__host__ __device__ static inline bool gs_put_walker(GsWalker *walkers, uint64_t idx, uint64_t end, uint32_t r,
+                                                     bool fwd, int anchor, uint32_t l, uint32_t u, uint32_t jl,
+                                                     uint32_t ju, bool jpend, int iL)
+{
+    if (idx >= end) return false;
+    if (iL >= (1 << 30)) {
+        walkers[idx].r = GS_WALKER_HOLE;
+        return false;
+    }
+    GsWalker w;
+    w.r = r;
+    w.anchor = (uint32_t)anchor | (fwd ? GS_WALKER_FWD : 0u) | (jpend ? GS_WALKER_JPEND : 0u);
+    w.l = l;
+    w.u = u;
+    w.jl = jl;
+    w.ju = ju;
+    walkers[idx] = w;
+    return true;
+}
 
 /* Per-read counts become offsets in two kernels that cut the reads the same
  * way: the first sums each block's reads, its last block to finish turns the

@@ -1090,9 +1090,6 @@ __global__ void __launch_bounds__(256, 5) gs_search_lockstep(GsDevIndex I, GsBat
  *     walker ends, from a per-warp window of the buffer; walkers that reach
  *     one row without J go to gs_search_text. */
 
-#define GS_WALKER_HOLE 0xffffffffu
-#define GS_WALKER_JPEND 0x40000000u   /* anchor flag: J is one base short of I's far end */
-#define GS_WALKER_FWD 0x80000000u
 #define GS_WALKER_CHUNK 512u      /* most buffer entries a warp reserves at a time */
 #define GS_WALK_WINDOW 512u       /* ... and a walk-pass warp takes */
 
@@ -1487,6 +1484,22 @@ __device__ __forceinline__ void gs_reserved(const GsBatch &B, GsReserve &res, ui
     if (res.next > res.end) res.next = res.end;
 }
 
+/* one walker-buffer entry of a warp's reservation (rank among the warp's
+ * walkers of this item); false when the buffer is full (or the read too
+ * long for the entry's anchor bits): the walk is then left over */
+__device__ __forceinline__ bool gs_push_walker(const GsBatch &B, const GsReserve &res, uint32_t g,
+                                               uint32_t take, uint32_t rem, uint32_t rank,
+                                               uint32_t r, bool fwd,
+                                               int anchor, uint32_t l, uint32_t u, uint32_t jl,
+                                               uint32_t ju, bool jpend, int iL)
+{
+    uint64_t idx;
+    if (rank < rem) idx = res.next + rank;
+    else idx = (uint64_t)g + (rank - rem);
+    const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + take, B.walker_cap);
+    return gs_put_walker(B.walkers, idx, cap_end, r, fwd, anchor, l, u, jl, ju, jpend, iL);
+}
+
 template <int NSTOP, int COUNT>
 __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch &B, uint32_t r,
                                              uint32_t local, uint32_t L, uint64_t off, int lane,
@@ -1550,52 +1563,9 @@ __device__ __forceinline__ void gs_start_item(const GsDevIndex &I, const GsBatch
     const uint32_t rem = res.end - res.next;
     uint32_t take;
     const uint32_t g = gs_reserve(B, res, cnt, rem, lane, take);
-    if (walker) {
-        uint64_t idx;
-        if (rank < rem) idx = res.next + rank;
-        else idx = (uint64_t)g + (rank - rem);
-        const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + take, B.walker_cap);
-        /* the entry keeps 30 bits of anchor: reads of 2^30 bases or more
-         * (none in practice) are left over too */
-        if (idx < cap_end && iL < (1 << 30)) {
-            GsWalker w;
-            w.r = r;
-            w.anchor = (uint32_t)anchor | (fwd ? GS_WALKER_FWD : 0u) | (jpend ? GS_WALKER_JPEND : 0u);
-            w.l = l;
-            w.u = u;
-            w.jl = jl;
-            w.ju = ju;
-            B.walkers[idx] = w;
-        } else {
-            gs_write_leftover(B, r, n, fwd, anchor, l, u);
-        }
-    }
+    if (walker && !gs_push_walker(B, res, g, take, rem, rank, r, fwd, anchor, l, u, jl, ju, jpend, iL))
+        gs_write_leftover(B, r, n, fwd, anchor, l, u);
     gs_reserved(B, res, cnt, rem, g, take);
-}
-
-/* one walker-buffer entry of a warp's reservation (rank among the warp's
- * walkers of this item); false when the buffer is full (or the read too
- * long for the entry's anchor bits): the walk is then left over */
-__device__ __forceinline__ bool gs_push_walker(const GsBatch &B, const GsReserve &res, uint32_t g,
-                                               uint32_t take, uint32_t rem, uint32_t rank,
-                                               uint32_t r, bool fwd,
-                                               int anchor, uint32_t l, uint32_t u, uint32_t jl,
-                                               uint32_t ju, bool jpend, int iL)
-{
-    uint64_t idx;
-    if (rank < rem) idx = res.next + rank;
-    else idx = (uint64_t)g + (rank - rem);
-    const uint64_t cap_end = rank < rem ? res.end : min((uint64_t)g + take, B.walker_cap);
-    if (idx >= cap_end || iL >= (1 << 30)) return false;
-    GsWalker w;
-    w.r = r;
-    w.anchor = (uint32_t)anchor | (fwd ? GS_WALKER_FWD : 0u) | (jpend ? GS_WALKER_JPEND : 0u);
-    w.l = l;
-    w.u = u;
-    w.jl = jl;
-    w.ju = ju;
-    B.walkers[idx] = w;
-    return true;
 }
 
 /* Whether a candidate that is to walk is contained in its neighbour at the

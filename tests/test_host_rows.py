@@ -10,6 +10,7 @@ from hostlib import build_host
 def rows(tmp_path_factory):
     L = build_host("rows", tmp_path_factory.mktemp("host"))
     L.rows_text_mode.argtypes = [C.c_int32, C.c_uint32]
+    L.rows_put_walker.argtypes = [C.c_uint64, C.c_int32, C.POINTER(C.c_uint32 * 6)]
     return L
 
 
@@ -20,3 +21,17 @@ def test_a_row_is_no_text_state(rows, jl):
     marks, has walkers in it."""
     assert not rows.rows_text_mode(0, jl)
     assert rows.rows_text_mode(4, jl) == (jl >= 0xf0000000)
+
+
+@pytest.mark.parametrize("length", [150, 2**30 - 1, 2**30, 2**31 - 1])
+@pytest.mark.parametrize("entry", [0, 2, 3])
+def test_a_reserved_entry_is_a_walker_or_a_hole(rows, entry, length):
+    """The walk pass reads every entry a warp reserved: none may keep what an
+    earlier pass left there, also where the read's anchors do not fit."""
+    w = (C.c_uint32 * 6)()
+    there = rows.rows_put_walker(entry, length, C.byref(w))
+    assert there == (entry < 3 and length < 2**30)
+    if there:
+        assert list(w) == [7, 0x80000000 | 0x40000000 | 5, 1, 2, 3, 4]
+    else:
+        assert w[0] == (0xffffffff if entry < 3 else 0x55555555)
