@@ -291,7 +291,9 @@ struct GsDeviceGuard {
  * ends, and waits at its start (gs_after_previous) until that has ended and
  * its writes are seen.  Every kernel launched so, and every kernel such a
  * launch can follow, begins with the wait, whatever it then does: the one
- * after it waits for it alone.  A pass's first kernel is launched plainly,
+ * after it waits for it alone.  What a pass's kernels write is read by plain
+ * loads: a read-only one (__ldg) may see it as it was when its kernel started,
+ * which can be before it was written.  A pass's first kernel is launched plainly,
  * after all that the stream holds.  The gaps between a small pass's nine
  * kernels were a tenth of it: one read 93 -> 83 us, 300 reads 178 -> 166; a
  * replayed graph has none to lose (10,000 reads 287 us either way). */

@@ -674,10 +674,12 @@ __global__ void __launch_bounds__(128) gs_mem_next_kernel(GsBatch B)
 __device__ __forceinline__ uint32_t gs_position_row(const GsBatch &B, uint64_t pb, uint64_t p, bool in,
                                                     uint64_t n_seeds, int lane)
 {
-    const uint64_t s0 = __ldg(&B.tile_seed[pb >> 5]);
+    /* plain loads: the kernel before this one, which may not have ended when
+     * this one starts, writes all of these */
+    const uint64_t s0 = B.tile_seed[pb >> 5];
     /* first positions of seeds s0+1 .. s0+32 */
     const uint64_t at = s0 + 1u + (uint64_t)lane;
-    const uint64_t next = at < n_seeds ? __ldg(&B.seed_pos[at]) : ~0ull;
+    const uint64_t next = at < n_seeds ? B.seed_pos[at] : ~0ull;
     int k = 0;   /* how many of them are at or before p */
 #pragma unroll
     for (int step = 16; step >= 1; step >>= 1)
@@ -686,10 +688,10 @@ __device__ __forceinline__ uint32_t gs_position_row(const GsBatch &B, uint64_t p
     const uint64_t s = s0 + (uint64_t)k;
     if (!in) return 0u;
     const uint4 *rec = reinterpret_cast<const uint4 *>(B.seeds + s);
-    const uint4 S = __ldg(rec), T = __ldg(rec + 1);   /* x y l u, xl xu n_pos pad */
-    B.pmap[p] = (uint32_t)s;
+    const uint4 S = rec[0], T = rec[1];   /* x y l u, xl xu n_pos pad */
     /* the (p - first)-th row from l outside [xl, xu] */
-    uint32_t row = S.z + (uint32_t)(p - __ldg(&B.seed_pos[s]));
+    uint32_t row = S.z + (uint32_t)(p - B.seed_pos[s]);
+    B.pmap[p] = (uint32_t)s;
     const uint32_t x0 = T.x > S.z ? T.x : S.z;
     if (T.x <= T.y && T.y >= x0 && row >= x0) row += T.y - x0 + 1u;
     return row;
