@@ -952,14 +952,24 @@ static int enqueue_pass(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
 }
 
 /* A captured pass holds the workspace's addresses and sizes: another pass
- * on the context may have replaced a buffer since. */
+ * on the context may have replaced a buffer since, and a larger one may lie
+ * where the captured one lay. */
 static uint64_t workspace_key(const gs_ctx *c)
 {
-    const void *const p[] = {c->slot_off, c->item_off, c->item_read, c->rd_nf, c->rd_nr, c->rd_nseeds,
-                             c->rd_npos, c->seed_off, c->pos_off, c->slots, c->recmask, c->walkers,
-                             c->text_jobs, c->seeds, c->seed_pos, c->pos, c->pmap, c->tile_seed};
+    const struct {
+        const void *p;
+        size_t cap;
+    } held[] = {{c->slot_off, c->cap_slot_off}, {c->item_off, c->cap_item_off}, {c->item_read, c->cap_item_read},
+                {c->rd_nf, c->cap_nf}, {c->rd_nr, c->cap_nr}, {c->rd_nseeds, c->cap_rns}, {c->rd_npos, c->cap_rnp},
+                {c->seed_off, c->cap_so}, {c->pos_off, c->cap_po}, {c->slots, c->cap_slots},
+                {c->recmask, c->cap_recmask}, {c->walkers, c->cap_walkers}, {c->text_jobs, c->cap_text_jobs},
+                {c->seeds, c->cap_seeds}, {c->seed_pos, c->cap_seed_pos}, {c->pos, c->cap_pos},
+                {c->pmap, c->cap_pmap}, {c->tile_seed, c->cap_tile_seed}};
     uint64_t h = 1469598103934665603ull;
-    for (const void *q : p) h = (h ^ (uint64_t)(uintptr_t)q) * 1099511628211ull;
+    for (const auto &b : held) {
+        h = (h ^ (uint64_t)(uintptr_t)b.p) * 1099511628211ull;
+        h = (h ^ (uint64_t)b.cap) * 1099511628211ull;
+    }
     return h;
 }
 

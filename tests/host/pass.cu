@@ -106,6 +106,19 @@ static void fake_kernel(const std::string &name, void **args)
 }
 
 extern "C" {
+/* whether a pass captured now would be replayed once buffer `which`, where it
+ * lies, has room for 100 entries more; -1: there is no such buffer */
+int fake_replayed_when_larger(gs_ctx *c, int which)
+{
+    size_t *const cap[] = {&c->cap_slots, &c->cap_item_read, &c->cap_recmask, &c->cap_walkers, &c->cap_seeds,
+                           &c->cap_seed_pos, &c->cap_pos, &c->cap_pmap, &c->cap_tile_seed};
+    if (which >= (int)(sizeof(cap) / sizeof(cap[0]))) return -1;
+    *cap[which] += 100;
+    const int same = same_graph(c, c->g_seqs, c->g_offs, c->g_lens, c->g_n, &c->g_params);
+    *cap[which] -= 100;
+    return same;
+}
+
 FakePass *fake_pass(void) { return &pass; }
 gs_index *fake_index(void)
 {

@@ -79,3 +79,15 @@ def test_record_mask_of_a_pass_that_had_no_memory(seeder):
         for _ in range(2):
             assert seeder.run([100] * 1500) == 0
             assert (seeder.last.slot_cap + 31) // 32 <= seeder.last.mask_words
+
+
+def test_captured_pass_of_smaller_buffers(seeder):
+    """A captured pass stops at the sizes it was captured with: it is not
+    replayed where a buffer is larger since, although it lies where it lay."""
+    assert seeder.run([100] * 2000, graph=1) == 0
+    answers = []
+    for which in range(20):
+        answers.append(seeder.L.fake_replayed_when_larger(seeder.h, which))
+        if answers[-1] < 0:
+            break
+    assert answers == [0] * 9 + [-1]
