@@ -206,8 +206,8 @@ struct gs_ctx {
     uint64_t walk_counts[7];   /* count_work pass: gs_ctx_last_walk_counts */
     void *cub_tmp; size_t cap_cub;
     uint64_t *h_small;          /* pinned scalars (GS_H_*) */
-    uint64_t last_slots;        /* slots, work items and reads of the last pass that succeeded */
-    uint32_t last_items, last_reads;
+    uint32_t last_items;        /* work items of the last pass that succeeded */
+    double slots_a_read, items_a_read;   /* what passes have had (note_sizes) */
     char *h_stage; size_t cap_stage;   /* pinned: a small gs_seed batch's input, as one copy */
     char *d_stage; size_t cap_d_stage;
     /* host result */
@@ -602,6 +602,19 @@ static int size_walkers(gs_ctx *c, const GsDevIndex &I, const gs_params *p, uint
     return GS_OK;
 }
 
+/* A batch's slots and work items a read are expected to be the last one's, or
+ * those of batches before it that had more, an eighth less for each since: two
+ * kinds of batches taking turns are both expected. */
+static void note_sizes(gs_ctx *c, uint32_t n_reads, uint64_t slots, uint32_t items)
+{
+    c->last_items = items;
+    if (!n_reads) return;
+    const double s = (double)slots / n_reads, i = (double)items / n_reads;
+    const double s0 = c->slots_a_read * 0.875, i0 = c->items_a_read * 0.875;
+    c->slots_a_read = s > s0 ? s : s0;
+    c->items_a_read = i > i0 ? i : i0;
+}
+
 /* what the end of a batched pass leaves in the queue words: the diagnostics,
  * and a larger walker buffer next time where this one was full */
 static uint32_t read_queue(gs_ctx *c, const gs_params *p)
@@ -658,10 +671,11 @@ __global__ void __launch_bounds__(256) gs_copy_out_kernel(GsBatch B, uint64_t *s
 /* A whole batched pass with one synchronisation, for batches whose launches
  * and waits would take as long as their kernels: everything is enqueued on
  * sizes known beforehand.  exact: n_slots and n_items are the batch's
- * (gs_seed counts them on the host); else they are what the context has
- * room for or expects (see run_device), and a batch that needs more returns
- * GS_RETRY.  Seeds and positions are written to what room there is, and once
- * more when that was too little. */
+ * (gs_seed counts them on the host); else they are what the context expects
+ * (run_device).  Grids, walkers and the record mask are sized by them, so a
+ * batch that needs more is not searched: its kernels return at once, and it
+ * returns GS_RETRY.  Seeds and positions are written to what room there is,
+ * and once more when that was too little. */
 static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, const uint32_t *d_lengths,
                     uint32_t n_reads, const gs_params *p, int fetch, uint64_t n_slots,
                     uint32_t n_items, bool exact)
@@ -672,10 +686,8 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     c->have_host = c->have_dev = 0;
     c->n_reads = n_reads;
     RC(grow_reads(c, nr1));
-    if (exact) {
-        RC(grow(c->slots, c->cap_slots, n_slots + 1, st));
-        RC(grow(c->item_read, c->cap_item_read, (size_t)n_items + 1, st));
-    }
+    RC(grow(c->slots, c->cap_slots, n_slots + 1, st));
+    RC(grow(c->item_read, c->cap_item_read, (size_t)n_items + 1, st));
     /* a bit for every slot there is, also where a pass before had no memory
      * for the bits of the slots it got */
     RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, st));
@@ -689,12 +701,12 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     GsBatch B;
     batch_of(c, d_seqs, d_offsets, d_lengths, n_reads, p, B);
     B.item_read = c->item_read;
-    B.item_read_cap = c->cap_item_read;
+    B.item_read_cap = n_items;
     B.slots = c->slots;
-    B.slot_cap = c->cap_slots;
+    B.slot_cap = n_slots;
     B.recmask = c->recmask;
     B.clear = 1;
-    B.clear_words = ((exact ? n_slots : c->cap_slots) + 31) / 32 + 1;
+    B.clear_words = (n_slots + 31) / 32 + 1;
     B.item_cap = n_items;
     GS_CUDA(cudaEventRecord(c->ev0, st));
     RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
@@ -731,9 +743,7 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     }
     c->timing = GS_TIMING_PASS;
     if (read_queue(c, p) & GS_FLAG_WALK) return walk_limit_error();
-    c->last_items = (uint32_t)c->h_small[GS_H_TOTALS + 1];
-    c->last_slots = c->h_small[GS_H_TOTALS];
-    c->last_reads = n_reads;
+    note_sizes(c, n_reads, c->h_small[GS_H_TOTALS], (uint32_t)c->h_small[GS_H_TOTALS + 1]);
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;
@@ -884,9 +894,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     if (B.work) memcpy(c->walk_counts, &c->h_small[16], sizeof(c->walk_counts));
     c->timing = GS_TIMING_PASS;
     if (flags & GS_FLAG_WALK) return walk_limit_error();
-    c->last_items = n_items;
-    c->last_slots = n_slots;
-    c->last_reads = n_reads;
+    note_sizes(c, n_reads, n_slots, n_items);
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;
@@ -1041,24 +1049,28 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
 }
 
 /* A pass over device-resident reads whose sizes the host does not know.  A
- * context that has run before expects as many slots and work items a read
- * as its last pass had, and a quarter more; where its buffers hold that, the
- * batch runs without waiting for its sizes, and again with them if it needed
- * more.  For up to GS_ONCE_READS reads: two waits of about 10 us each are
- * what it saves (60,007 short reads 527 -> 457 us), and a batch that
- * has to run again pays for little. */
+ * context that has run before expects as many slots and work items a read as
+ * note_sizes kept, and a quarter more; where its buffers hold that, the batch
+ * runs without waiting for its sizes, and again with them if it needed more.
+ * Few reads may differ much and many lie near their average, so that a batch
+ * is also expected to be a small one of any kind.  For up to GS_ONCE_READS
+ * reads: two waits of about 10 us each are what it saves (60,007 short reads
+ * 527 -> 457 us), and a batch that has to run again pays for little. */
 #define GS_ONCE_READS (1u << 17)
-#define GS_ONCE_SLOTS (1ull << 26)   /* the record mask is cleared over all the room there is */
+#define GS_ONCE_SLOTS (1ull << 26)   /* the record mask is cleared for all of them */
 
 static int run_device(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
                       const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p, int fetch)
 {
     if (p->kernel == GS_KERNEL_BATCHED && !p->count_work && n_reads && n_reads <= GS_ONCE_READS &&
-        c->last_reads && c->slots && c->item_read && c->cap_slots <= GS_ONCE_SLOTS) {
-        const double per = 1.25 * (double)n_reads / (double)c->last_reads;
-        const uint64_t slots = (uint64_t)(per * (double)c->last_slots) + 1;
-        const uint64_t items = (uint64_t)(per * (double)c->last_items) + 1;
-        if (slots <= c->cap_slots && items <= c->cap_item_read && items <= 0xffffffffull) {
+        c->slots_a_read > 0.) {
+        const uint64_t least_s = 64ull * n_reads + 16384u, least_i = (uint64_t)n_reads + 256u;
+        uint64_t slots = (uint64_t)(1.25 * c->slots_a_read * (double)n_reads) + 1;
+        uint64_t items = (uint64_t)(1.25 * c->items_a_read * (double)n_reads) + 1;
+        if ((slots < c->cap_slots || slots <= least_s) && (items < c->cap_item_read || items <= least_i) &&
+            slots <= GS_ONCE_SLOTS) {
+            slots = slots > least_s ? slots : least_s;
+            items = items > least_i ? items : least_i;
             const int rc = run_once(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch, slots,
                                     (uint32_t)items, false);
             if (rc != GS_RETRY) return rc;

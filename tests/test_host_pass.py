@@ -91,3 +91,29 @@ def test_captured_pass_of_smaller_buffers(seeder):
         if answers[-1] < 0:
             break
     assert answers == [0] * 9 + [-1]
+
+
+def test_a_pass_is_sized_for_its_batch(seeder):
+    """Batches of any size after one another: the pass whose result is taken
+    was sized for the batch's work items, slots and walkers, whatever the
+    batches before it had, and a full walker buffer that was sized for fewer
+    items is no reason for a larger one."""
+    rng = np.random.default_rng(1)
+    batches = [[100] * 3000, [12] * 500, [100] * 3000, [150] * 40, [9000], [150] * 100, [30] * 3000, [250] * 3000]
+    batches += [[int(np.exp(rng.uniform(2.3, 7)))] * int(np.exp(rng.uniform(0, 8))) for _ in range(60)]
+    for batch in batches:
+        assert seeder.run(batch) == 0
+        p = seeder.last
+        assert p.items <= p.item_cap and p.slots <= p.slot_cap, batch[:1]
+        assert p.items * 16 < p.walker_cap, batch[:1]
+
+
+def test_alike_batches_run_once(seeder):
+    """Batches of one kind, or of two that take turns, are searched once each
+    from the second on."""
+    for kinds in ([100], [100, 150], [100, 10]):
+        for i in range(8):
+            before = seeder.last.passes
+            assert seeder.run([kinds[i % len(kinds)]] * 3000) == 0
+            assert i < 2 or seeder.last.passes == before + 1, f"{kinds} {i}"
+            assert i < 2 or seeder.last.clear_words, "in one go"
