@@ -133,10 +133,22 @@ struct GsParts {
     GsPart *part;      /* GS_PARTS_MOST entries, and tickets[2], zero between passes */
     uint32_t *tickets;
 };
-static inline uint32_t gs_parts_of(uint32_t n_reads, uint32_t tile)
+__host__ __device__ static inline uint32_t gs_parts_of(uint32_t n_reads, uint32_t tile)
 {
     const uint32_t p = (n_reads + tile - 1u) / tile;
     return p < 1u ? 1u : p > GS_PARTS_MOST ? GS_PARTS_MOST : p;
+}
+
+/* Whether the first kernel clears the record mask (GS_CLEAR_WORDS a thread at
+ * most) or a memset before it does.  A captured pass's mask is the context's,
+ * which other batches may have made large: 200 reads after 2 M in the same
+ * context, one block clearing 40 MB, took 2.16 ms a replay and take 0.20.  One
+ * block's 16,000 words cost what a memset does (the pass 110 us either way),
+ * 130,000 are 123 against 112. */
+#define GS_CLEAR_WORDS 64u
+__host__ __device__ static inline bool gs_clear_in_kernel(uint32_t n_reads, uint32_t tile, uint64_t words)
+{
+    return words <= (uint64_t)GS_CLEAR_WORDS * tile * gs_parts_of(n_reads, tile);
 }
 
 /* Per-batch device arguments shared by the pipeline kernels. */
@@ -146,7 +158,7 @@ struct GsBatch {
     const uint32_t *lengths;   /* per read */
     uint32_t n_reads;
     int32_t k, smem, n_mode, lf_mode;
-    int32_t clear;             /* the prepare kernels zero the queue and ... */
+    int32_t clear;             /* gs_launch_prepare zeroes the queue and ... */
     uint64_t clear_words;      /* ... the first words of recmask */
     GsParts parts;
     uint64_t *totals;          /* slots, work items, seeds, positions of the pass, on the

@@ -786,6 +786,10 @@ int gs_launch_prepare(const GsDevIndex &I, GsBatch &b, int kernel, cudaStream_t 
     const int kt = gs_paired_len(I, kernel, b.k);
     b.paired = kt != 0;
     const uint32_t parts = gs_parts_of(b.n_reads, GS_SCAN_THREADS);
+    if (b.clear && !gs_clear_in_kernel(b.n_reads, GS_SCAN_THREADS, b.clear_words)) {
+        GS_CUDA(cudaMemsetAsync(b.recmask, 0, b.clear_words * sizeof(uint32_t), st));
+        b.clear_words = 0;
+    }
     if (parts > 1) {
         gs_prepare_sum<<<parts, GS_SCAN_THREADS, 0, st>>>(b, kt);
         GS_CUDA(cudaGetLastError());

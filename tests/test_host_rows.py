@@ -10,6 +10,7 @@ from hostlib import build_host
 def rows(tmp_path_factory):
     L = build_host("rows", tmp_path_factory.mktemp("host"))
     L.rows_text_mode.argtypes = [C.c_int32, C.c_uint32]
+    L.rows_clear_in_kernel.argtypes = [C.c_uint32, C.c_uint32, C.c_uint64]
     L.rows_put_walker.argtypes = [C.c_uint64, C.c_int32, C.POINTER(C.c_uint32 * 6)]
     return L
 
@@ -35,3 +36,13 @@ def test_a_reserved_entry_is_a_walker_or_a_hole(rows, entry, length):
         assert list(w) == [7, 0x80000000 | 0x40000000 | 5, 1, 2, 3, 4]
     else:
         assert w[0] == (0xffffffff if entry < 3 else 0x55555555)
+
+
+@pytest.mark.parametrize("reads", [1, 200, 256, 257, 10_000, 131_072])
+def test_who_clears_the_record_mask(rows, reads):
+    """The first kernel of a small batch does not clear the mask that a large
+    one left: a thread has at most 64 words of it."""
+    threads = 256 * min(-(-reads // 256), 4864)
+    assert rows.rows_clear_in_kernel(reads, 256, 64 * threads)
+    assert not rows.rows_clear_in_kernel(reads, 256, 64 * threads + 1)
+    assert not rows.rows_clear_in_kernel(reads, 256, 10**9 // 32 * 64)
