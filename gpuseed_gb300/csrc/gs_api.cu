@@ -156,7 +156,10 @@ struct gs_ctx {
     gs_index *idx;
     cudaStream_t st;
     bool own_stream;
-    cudaEvent_t ev0, ev_s0, ev_s1, ev1;
+    /* a pass's begin and end and its search's: the last one's to end, and at
+     * [timed ^ 1] those that the next records */
+    struct { cudaEvent_t ev0, s0, s1, ev1; } times[2];
+    int timed;
     cudaStream_t st_copy;       /* copies seeds out while positions are located */
     cudaEvent_t ev_emit;
     /* gs_seed in chunks: reads go up on st_h2d, each chunk's results come
@@ -247,10 +250,9 @@ extern "C" int gs_ctx_create(gs_index *idx, void *cuda_stream, gs_ctx **out)
         e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
         c->own_stream = true;
     }
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev_s0);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev_s1);
-    if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
+    for (auto &t : c->times)
+        for (cudaEvent_t *ev : {&t.ev0, &t.s0, &t.s1, &t.ev1})
+            if (e == cudaSuccess) e = cudaEventCreate(ev);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_emit, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st_h2d, cudaStreamNonBlocking);
@@ -335,10 +337,9 @@ extern "C" void gs_ctx_free(gs_ctx *c)
     cudaFree(c->d_stage);
     cudaFreeHost(c->h_seed_off); cudaFreeHost(c->h_pos_off);
     cudaFreeHost(c->h_seeds); cudaFreeHost(c->h_pos);
-    if (c->ev0) cudaEventDestroy(c->ev0);
-    if (c->ev_s0) cudaEventDestroy(c->ev_s0);
-    if (c->ev_s1) cudaEventDestroy(c->ev_s1);
-    if (c->ev1) cudaEventDestroy(c->ev1);
+    for (auto &t : c->times)
+        for (cudaEvent_t ev : {t.ev0, t.s0, t.s1, t.ev1})
+            if (ev) cudaEventDestroy(ev);
     if (c->ev_emit) cudaEventDestroy(c->ev_emit);
     if (c->st_copy) {
         cudaStreamSynchronize(c->st_copy);
@@ -389,14 +390,23 @@ extern "C" int gs_ctx_last_text_jobs(gs_ctx *c, uint64_t *n_jobs, uint64_t *capa
     return GS_OK;
 }
 
-#define GS_TIMING_PASS 1    /* ev0, ev_s0, ev_s1, ev1 */
+#define GS_TIMING_PASS 1    /* ev0, s0, s1, ev1 */
 #define GS_TIMING_GRAPH 2   /* ev0, ev1: the whole pass stands for the search too */
+
+/* the pass that recorded times[timed ^ 1] is the last; one that fails before
+ * leaves the times as they were */
+static void timed(gs_ctx *c, int what)
+{
+    c->timed ^= 1;
+    c->timing = what;
+}
 
 /* elapsed times of the last pass from its events, when they are asked for */
 static void take_timing(gs_ctx *c)
 {
-    if (c->timing) cudaEventElapsedTime(&c->t_total, c->ev0, c->ev1);
-    if (c->timing == GS_TIMING_PASS) cudaEventElapsedTime(&c->t_search, c->ev_s0, c->ev_s1);
+    const auto &t = c->times[c->timed];
+    if (c->timing) cudaEventElapsedTime(&c->t_total, t.ev0, t.ev1);
+    if (c->timing == GS_TIMING_PASS) cudaEventElapsedTime(&c->t_search, t.s0, t.s1);
     if (c->timing == GS_TIMING_GRAPH) c->t_search = c->t_total;
     c->timing = 0;
 }
@@ -708,12 +718,12 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     B.clear = 1;
     B.clear_words = (n_slots + 31) / 32 + 1;
     B.item_cap = n_items;
-    GS_CUDA(cudaEventRecord(c->ev0, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].ev0, st));
     RC(gs_launch_prepare(I, B, GS_KERNEL_BATCHED, st));
     RC(size_walkers(c, I, p, n_items, B));
-    GS_CUDA(cudaEventRecord(c->ev_s0, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].s0, st));
     RC(gs_launch_search(I, B, GS_KERNEL_BATCHED, p->queue_chunk, p->ctas_per_sm, n_items, st));
-    GS_CUDA(cudaEventRecord(c->ev_s1, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].s1, st));
     RC(gs_launch_finalize_count(I, B, st));
     bind_outputs(c, B);
     for (bool emit = true;;) {
@@ -725,7 +735,7 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
         GS_CUDA(gs_launch_after(gs_copy_out_kernel, grid, 256, st, B, fetch ? c->h_seed_off : NULL,
                                 c->h_pos_off, (uint4 *)c->h_seeds, c->cap_h_seeds, c->h_pos, c->cap_h_pos,
                                 (uint32_t *)&c->h_small[GS_H_QUEUE]));
-        GS_CUDA(cudaEventRecord(c->ev1, st));
+        GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].ev1, st));
         GS_CUDA(cudaStreamSynchronize(st));
         c->n_seeds = c->h_small[GS_H_TOTALS + 2];
         c->n_pos = c->h_small[GS_H_TOTALS + 3];
@@ -741,7 +751,7 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
         }
         if (copy) RC(grow_fetch(c, nr1, c->n_seeds, c->n_pos));
     }
-    c->timing = GS_TIMING_PASS;
+    timed(c, GS_TIMING_PASS);
     if (read_queue(c, p) & GS_FLAG_WALK) return walk_limit_error();
     note_sizes(c, n_reads, c->h_small[GS_H_TOTALS], (uint32_t)c->h_small[GS_H_TOTALS + 1]);
     c->have_dev = 1;
@@ -769,7 +779,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     memset(c->work, 0, sizeof(c->work));
     memset(c->walk_counts, 0, sizeof(c->walk_counts));
 
-    GS_CUDA(cudaEventRecord(c->ev0, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].ev0, st));
     if (B.work) GS_CUDA(cudaMemsetAsync(c->d_work, 0, 128, st));
     GS_CUDA(cudaMemsetAsync(c->queue, 0, 32, st));
     /* the item map before its size is known: what there is, and the rest
@@ -817,9 +827,9 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     c->last_text_cap = 0;
     if (p->kernel == GS_KERNEL_BATCHED) RC(size_walkers(c, I, p, n_items, B));
 
-    GS_CUDA(cudaEventRecord(c->ev_s0, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].s0, st));
     RC(gs_launch_search(I, B, p->kernel, p->queue_chunk, p->ctas_per_sm, n_items, st));
-    GS_CUDA(cudaEventRecord(c->ev_s1, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].s1, st));
     /* the previous chunk's results are copied out of the buffers below while
      * this chunk searched */
     if (co && co->wait_d2h) GS_CUDA(cudaStreamWaitEvent(st, c->ev_d2h, 0));
@@ -859,7 +869,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
                                     cudaMemcpyDeviceToHost, c->st_copy));
     }
     RC(gs_launch_locate(I, B, n_pos, st));
-    GS_CUDA(cudaEventRecord(c->ev1, st));
+    GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].ev1, st));
     RC(fetch_small(&c->h_small[GS_H_QUEUE], c->queue, 32, st));
     if (B.work) RC(fetch_small(&c->h_small[6], c->d_work, 32, st));
     if (B.work) RC(fetch_small(&c->h_small[16], c->d_work + 4, 56, st));
@@ -892,7 +902,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     const uint32_t flags = read_queue(c, p);
     if (B.work) memcpy(c->work, &c->h_small[6], sizeof(c->work));
     if (B.work) memcpy(c->walk_counts, &c->h_small[16], sizeof(c->walk_counts));
-    c->timing = GS_TIMING_PASS;
+    timed(c, GS_TIMING_PASS);
     if (flags & GS_FLAG_WALK) return walk_limit_error();
     note_sizes(c, n_reads, n_slots, n_items);
     c->have_dev = 1;
@@ -995,9 +1005,9 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
     cudaStream_t st = c->st;
     if (same_graph(c, d_seqs, d_offsets, d_lengths, n_reads, p)) {
         c->have_host = c->have_dev = 0;
-        GS_CUDA(cudaEventRecord(c->ev0, st));
+        GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].ev0, st));
         GS_CUDA(cudaGraphLaunch(c->gexec, st));
-        GS_CUDA(cudaEventRecord(c->ev1, st));
+        GS_CUDA(cudaEventRecord(c->times[c->timed ^ 1].ev1, st));
         GS_CUDA(cudaStreamSynchronize(st));
         const uint32_t flags = ((const uint32_t *)&c->h_small[GS_H_QUEUE])[1];
         const uint64_t ns = c->h_small[GS_H_TOTALS + 2], np = c->h_small[GS_H_TOTALS + 3];
@@ -1009,7 +1019,7 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
             c->n_seeds = ns;
             c->n_pos = np;
             c->have_dev = 1;
-            c->timing = GS_TIMING_GRAPH;
+            timed(c, GS_TIMING_GRAPH);
             if (fetch) RC(fetch_result(c));
             return GS_OK;
         }
@@ -1162,7 +1172,6 @@ static int seed_chunked(gs_ctx *c, const char *seqs, const uint64_t *offsets, ui
         t_search += c->t_search;
         t_total += c->t_total;
     }
-    c->timing = 0;
     /* no copy may outlive the call: the caller owns the host buffers */
     cudaStreamSynchronize(c->st_h2d);
     cudaStreamSynchronize(c->st_copy);

@@ -117,3 +117,29 @@ def test_alike_batches_run_once(seeder):
             assert seeder.run([kinds[i % len(kinds)]] * 3000) == 0
             assert i < 2 or seeder.last.passes == before + 1, f"{kinds} {i}"
             assert i < 2 or seeder.last.clear_words, "in one go"
+
+
+def _timing(s):
+    t = C.c_float(), C.c_float()
+    assert s.L.gs_ctx_last_timing(s.h, C.byref(t[0]), C.byref(t[1])) == 0
+    return t[0].value, t[1].value
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("ask", [False, True], ids=["later", "before"])
+def test_timing_after_a_failed_pass(host, ask, graph):
+    """The times are of the last pass that ended, also when they are asked for
+    after one that failed on the way (each allocation in turn)."""
+    for at in range(1, 30):
+        s = Seeder(host)
+        assert s.run([100] * 2000, graph=graph) == 0
+        assert s.run([100] * 2000, graph=graph) == 0
+        want = _timing(s) if ask else None
+        host.fake_fail(at)
+        rc = s.run([120] * 4000, graph=graph)
+        host.fake_fail(0)
+        search, total = _timing(s)
+        assert 0 < search <= total
+        if rc and ask:
+            assert (search, total) == want
+        s.close()
