@@ -28,9 +28,6 @@ struct gs_index {
     uint32_t gen;   /* bumped whenever device pointers change */
 };
 
-extern "C" int gs_index_set_kmer_len(gs_index *idx, int kx);
-extern "C" int gs_index_set_text(gs_index *idx, int min_steps);
-
 #define GS_SAF_UNSET 0xfffffffeu
 #define GS_CHAIN_MAX (1u << 20)   /* LF steps one chain may take */
 
@@ -256,6 +253,67 @@ int gs_index_device(const gs_index *idx) { return idx->device; }
 float gs_index_l2_ratio(const gs_index *idx) { return idx->l2_hit_ratio; }
 size_t gs_index_occ_bytes(const gs_index *idx) { return idx->occ_bytes; }
 
+/* a step reads the block of one past its last row: up to row seq_len+1 */
+static uint64_t occ_blocks(uint32_t seq_len) { return ((uint64_t)seq_len + 1) / GS_OCC_INTERVAL + 1; }
+
+static void drop_start(gs_index *idx)
+{
+    cudaFree(idx->d_kmerx);
+    idx->d_kmerx = NULL;
+    idx->kmerx_bytes = 0;
+    idx->dev.kmerx = NULL;
+    idx->dev.kx = 0;
+}
+
+/* the start table of kx bases, in place of the one there is */
+static int make_start(gs_index *idx, int kx)
+{
+    drop_start(idx);
+    const size_t bytes = (size_t)16 << (2 * kx);
+    uint4 *t = NULL;
+    cudaError_t e = cudaMalloc(&t, bytes);
+    if (e != cudaSuccess) return gs_cuda_fail(e, "cudaMalloc(k-mer start table)");
+    int rc = gs_build_kmerx_table(idx->dev, t, kx, 0);
+    if (rc == GS_OK && (e = cudaDeviceSynchronize()) != cudaSuccess) rc = gs_cuda_fail(e, "k-mer table");
+    if (rc) {
+        cudaFree(t);
+        return rc;
+    }
+    idx->d_kmerx = t;
+    idx->kmerx_bytes = bytes;
+    idx->dev.kmerx = t;
+    idx->dev.kx = kx;
+    return GS_OK;
+}
+
+static void drop_two_base(gs_index *idx)
+{
+    cudaFree(idx->d_occ2);
+    idx->d_occ2 = NULL;
+    idx->occ2_bytes = 0;
+    idx->dev.occ2 = NULL;
+}
+
+/* the table for steps of two bases, where there is memory for it */
+static int make_two_base(gs_index *idx)
+{
+    const uint64_t nblk = occ_blocks(idx->dev.seq_len);
+    cudaError_t e;
+    if (cudaMalloc(&idx->d_occ2, nblk * 16 * sizeof(uint4)) != cudaSuccess) {
+        cudaGetLastError();
+        idx->d_occ2 = NULL;
+        return GS_OK;
+    }
+    gs_occ2_kernel<<<152 * 32, 256>>>(idx->dev, idx->d_occ2, nblk);
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
+        drop_two_base(idx);
+        return gs_cuda_fail(e, "occurrence table layout");
+    }
+    idx->occ2_bytes = nblk * 16 * sizeof(uint4);
+    idx->dev.occ2 = idx->d_occ2;
+    return GS_OK;
+}
+
 /* The index of a file's blocks and samples: the blocks on the device, each
  * with room for GS_BLOCK_WORDS words; the samples where `kind` has them. */
 static int make_index(uint32_t primary, const uint32_t L2_1to4[4], const uint32_t *d_file, uint32_t sa_intv,
@@ -266,8 +324,7 @@ static int make_index(uint32_t primary, const uint32_t L2_1to4[4], const uint32_
     gs_index *idx = (gs_index *)calloc(1, sizeof(gs_index));
     if (!idx) return GS_ENOMEM;
     idx->device = device;
-    /* a step reads the block of one past its last row: up to row seq_len+1 */
-    const uint64_t nblk = ((uint64_t)seq_len + 1) / GS_OCC_INTERVAL + 1;
+    const uint64_t nblk = occ_blocks(seq_len);
     idx->occ_bytes = nblk * 4 * sizeof(uint4);
     idx->sa_bytes = (n_samples + 1) * 4;
     idx->kmer_bytes = (size_t)8 << (2 * GS_K0);
@@ -309,20 +366,12 @@ static int make_index(uint32_t primary, const uint32_t L2_1to4[4], const uint32_
     }
     /* the start table is an accelerator: without room for it, run without */
     for (int kx = auto_kmer_len(seq_len); kx >= GS_K0; kx--)
-        if (gs_index_set_kmer_len(idx, kx) == GS_OK) break;
+        if (make_start(idx, kx) == GS_OK) break;
     cudaGetLastError();
     /* and so are the steps of two bases */
-    if (cudaMalloc(&idx->d_occ2, nblk * 16 * sizeof(uint4)) == cudaSuccess) {
-        gs_occ2_kernel<<<152 * 32, 256>>>(D, idx->d_occ2, nblk);
-        if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
-            gs_index_free(idx);
-            return gs_cuda_fail(e, "occurrence table layout");
-        }
-        idx->occ2_bytes = nblk * 16 * sizeof(uint4);
-        D.occ2 = idx->d_occ2;
-    } else {
-        cudaGetLastError();
-        idx->d_occ2 = NULL;
+    if ((rc = make_two_base(idx))) {
+        gs_index_free(idx);
+        return rc;
     }
     *out = idx;
     return GS_OK;
@@ -611,31 +660,12 @@ extern "C" int gs_index_set_kmer_len(gs_index *idx, int kx)
     GS_ON_DEVICE(idx->device);
     GS_CUDA(cudaDeviceSynchronize());
     idx->gen++;
-    if (idx->d_kmerx) {
-        cudaFree(idx->d_kmerx);
-        idx->d_kmerx = NULL;
-        idx->kmerx_bytes = 0;
-    }
-    idx->dev.kmerx = NULL;
-    idx->dev.kx = 0;
-    size_t bytes = (size_t)16 << (2 * kx);
-    uint4 *t = NULL;
-    cudaError_t e = cudaMalloc(&t, bytes);
-    if (e == cudaErrorMemoryAllocation && kx == GS_K0) {
-        /* the 13-mer table alone serves every kernel */
-        cudaGetLastError();
+    if (kx == GS_K0) {
+        /* the 13-mer table and the occurrence table alone serve every kernel */
+        drop_start(idx);
+        drop_two_base(idx);
         return GS_OK;
     }
-    if (e != cudaSuccess) return gs_cuda_fail(e, "cudaMalloc(k-mer start table)");
-    int rc = gs_build_kmerx_table(idx->dev, t, kx, 0);
-    if (rc == GS_OK && (e = cudaDeviceSynchronize()) != cudaSuccess) rc = gs_cuda_fail(e, "k-mer table");
-    if (rc) {
-        cudaFree(t);
-        return rc;
-    }
-    idx->d_kmerx = t;
-    idx->kmerx_bytes = bytes;
-    idx->dev.kmerx = t;
-    idx->dev.kx = kx;
-    return GS_OK;
+    const int rc = make_start(idx, kx);
+    return rc || idx->d_occ2 ? rc : make_two_base(idx);
 }

@@ -161,11 +161,15 @@ int gs_index_build(const uint8_t *codes, uint64_t n, uint32_t sa_intv, int devic
  * so that one lookup starts both strands' candidates of a read window, with
  * what precedes and follows the string's rows, so that most candidates end
  * there; a lower length, or none but the plain 13-mer table, is taken when
- * the memory is not there).  A candidate starts from the interval of
- * its first len bases instead of 13 + len-13 steps: the SA interval of a
- * string does not depend on how it is found, so results do not change;
- * seeding uses it only when k > len.  Call while no pass runs on a context
- * of this index. */
+ * the memory is not there).  It also makes a table for steps of two bases, 4
+ * bytes a base, where there is memory left.  A candidate starts from the
+ * interval of its first len bases instead of 13 + len-13 steps: the SA
+ * interval of a string does not depend on how it is found, so results do not
+ * change; seeding uses it only when k > len.  14 to 16: makes that table, and
+ * the two-base table where there is none.  13: frees both; seeding then starts
+ * from the plain 13-mer table and steps by one base, slower, in the least
+ * memory (for a process that holds many small genomes).  Call while no pass
+ * runs on a context of this index. */
 int gs_index_set_kmer_len(gs_index *idx, int kmer_len);
 /* Text structures in HBM, built from the .bwt and .sa by one pass of LF
  * chains: 4 * seq_len bytes of full suffix array, seq_len / 4 of packed
