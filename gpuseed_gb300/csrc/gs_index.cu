@@ -586,6 +586,38 @@ static void drop_text(gs_index *idx)
     D.text_min = 0;
 }
 
+static int make_text(gs_index *idx)
+{
+    GsDevIndex &D = idx->dev;
+    if (D.seq_len >= GS_REGIME_MARK) {
+        gs_set_error("text structures need seq_len below %u", GS_REGIME_MARK);
+        return GS_EINVAL;
+    }
+    const size_t saf_b = ((size_t)D.seq_len + 1) * 4;
+    const size_t text_b = (((size_t)D.seq_len + 15) / 16 + 2) * 4;
+    const size_t isa_b = ((size_t)D.seq_len / GS_ISA_STEP + 1) * 4;
+    cudaError_t e;
+    if ((e = cudaMalloc(&idx->d_saf, saf_b)) != cudaSuccess ||
+        (e = cudaMalloc(&idx->d_text, text_b)) != cudaSuccess ||
+        (e = cudaMalloc(&idx->d_isa, isa_b)) != cudaSuccess) {
+        drop_text(idx);
+        return gs_cuda_fail(e, "cudaMalloc(text structures)");
+    }
+    GsDevIndex B = D;
+    int rc = gs_build_text(B, idx->d_saf, idx->d_text, idx->d_isa, 0);
+    if (rc) {
+        drop_text(idx);
+        return rc;
+    }
+    idx->text_bytes = saf_b + text_b + isa_b;
+    D.saf = idx->d_saf;
+    D.text = idx->d_text;
+    D.isa = idx->d_isa;
+    D.quirk_lo = B.quirk_lo;
+    D.quirk_n = B.quirk_n;
+    return GS_OK;
+}
+
 extern "C" int gs_index_set_text(gs_index *idx, int min_steps)
 {
     if (!idx) return GS_EINVAL;
@@ -596,36 +628,17 @@ extern "C" int gs_index_set_text(gs_index *idx, int min_steps)
         drop_text(idx);
         return GS_OK;
     }
-    GsDevIndex &D = idx->dev;
     if (!idx->d_saf) {
-        if (D.seq_len >= GS_REGIME_MARK) {
-            gs_set_error("text structures need seq_len below %u", GS_REGIME_MARK);
-            return GS_EINVAL;
+        int rc = make_text(idx);
+        /* asked for, where the two-base table was not */
+        if (rc == GS_ENOMEM && idx->d_occ2) {
+            drop_two_base(idx);
+            rc = make_text(idx);
+            if (rc) make_two_base(idx);   /* it did not help */
         }
-        const size_t saf_b = ((size_t)D.seq_len + 1) * 4;
-        const size_t text_b = (((size_t)D.seq_len + 15) / 16 + 2) * 4;
-        const size_t isa_b = ((size_t)D.seq_len / GS_ISA_STEP + 1) * 4;
-        cudaError_t e;
-        if ((e = cudaMalloc(&idx->d_saf, saf_b)) != cudaSuccess ||
-            (e = cudaMalloc(&idx->d_text, text_b)) != cudaSuccess ||
-            (e = cudaMalloc(&idx->d_isa, isa_b)) != cudaSuccess) {
-            drop_text(idx);
-            return gs_cuda_fail(e, "cudaMalloc(text structures)");
-        }
-        GsDevIndex B = D;
-        int rc = gs_build_text(B, idx->d_saf, idx->d_text, idx->d_isa, 0);
-        if (rc) {
-            drop_text(idx);
-            return rc;
-        }
-        idx->text_bytes = saf_b + text_b + isa_b;
-        D.saf = idx->d_saf;
-        D.text = idx->d_text;
-        D.isa = idx->d_isa;
-        D.quirk_lo = B.quirk_lo;
-        D.quirk_n = B.quirk_n;
+        if (rc) return rc;
     }
-    D.text_min = min_steps > 0 ? min_steps : 0;
+    idx->dev.text_min = min_steps > 0 ? min_steps : 0;
     return GS_OK;
 }
 
@@ -666,6 +679,11 @@ extern "C" int gs_index_set_kmer_len(gs_index *idx, int kx)
         drop_two_base(idx);
         return GS_OK;
     }
-    const int rc = make_start(idx, kx);
-    return rc || idx->d_occ2 ? rc : make_two_base(idx);
+    int rc = make_start(idx, kx);
+    if (rc == GS_ENOMEM && idx->d_occ2) {
+        drop_two_base(idx);
+        rc = make_start(idx, kx);
+    }
+    const int rc2 = idx->d_occ2 ? GS_OK : make_two_base(idx);
+    return rc ? rc : rc2;
 }

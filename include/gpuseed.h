@@ -185,6 +185,8 @@ int gs_index_set_kmer_len(gs_index *idx, int kmer_len);
  * of its own; it takes the row where the match ends from the inverse-SA
  * samples.  Seeds and positions do not change.  min_steps > 0: build if
  * needed and use both; < 0: build if needed, locate only; 0: free them.
+ * Where there is no memory for them, the table for steps of two bases, which
+ * loading made unasked, is freed for them (gs_index_set_kmer_len likewise).
  * Call while no pass runs on a context of this index. */
 int gs_index_set_text(gs_index *idx, int min_steps);
 /* Copies entries [first, first+count) of a text structure to host memory:

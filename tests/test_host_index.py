@@ -55,3 +55,42 @@ def test_least_memory(host, index):
     info = _info(host, index)
     assert info.kmer_len == 14
     assert info.device_bytes - full == pytest.approx(3 * START, abs=MIB)
+
+
+@pytest.mark.parametrize("room", [48, 52, 60, 64, 200])
+def test_asked_for_comes_before_unasked(host, index, room):
+    """The text structures (4 + 1/4 + 2 bytes a base, and one while they are
+    made: 58 MiB) and a start table fit where they fit before loading made a
+    two-base table (32 MiB) of its own accord."""
+    full = _info(host, index).device_bytes
+    assert host.gs_index_set_kmer_len(index, 14) == 0
+    held = _info(host, index).device_bytes
+    assert held > full
+    host.fake_have(held - TWO_BASE + room * MIB)
+    fits = room >= 59
+    assert host.gs_index_set_text(index, 4) == (0 if fits else -4)
+    info = _info(host, index)
+    assert info.text_min == (4 if fits else 0)
+    if not fits:
+        assert info.device_bytes == held
+    kept = room >= 59 + 32     # the two-base table: where both fit, or the text did not even without it
+    if fits:
+        assert info.device_bytes == pytest.approx(held + 6.25 * BASES - (0 if kept else TWO_BASE), abs=MIB)
+    # a longer start table in the place of this one
+    host.fake_have(info.device_bytes + 12 * START - (TWO_BASE if kept else 0))
+    assert host.gs_index_set_kmer_len(index, 15) == 0
+    assert _info(host, index).kmer_len == 15
+
+
+def test_each_allocation_of_the_text_fails(host, index):
+    """One allocation fails: the structures are made without the two-base
+    table; when the next fails too, the call says so and frees all it took."""
+    for at in range(1, 6):
+        assert host.gs_index_set_kmer_len(index, 14) == 0
+        held = _info(host, index).device_bytes
+        host.fake_fail(at)
+        assert host.gs_index_set_text(index, 4) == 0
+        host.fake_fail(0)
+        info = _info(host, index)
+        assert info.device_bytes == pytest.approx(held + 6.25 * BASES - TWO_BASE, abs=MIB)
+        assert host.gs_index_set_text(index, 0) == 0
