@@ -210,7 +210,8 @@ struct gs_ctx {
     void *cub_tmp; size_t cap_cub;
     uint64_t *h_small;          /* pinned scalars (GS_H_*) */
     uint32_t last_items;        /* work items of the last pass that succeeded */
-    double slots_a_read, items_a_read;   /* what passes have had (note_sizes) */
+    struct { double slots, items, seeds, pos; } a_read;   /* what passes have had (note_sizes), */
+    bool ran;                                             /* ... once one has */
     char *h_stage; size_t cap_stage;   /* pinned: a small gs_seed batch's input, as one copy */
     char *d_stage; size_t cap_d_stage;
     /* host result */
@@ -612,17 +613,23 @@ static int size_walkers(gs_ctx *c, const GsDevIndex &I, const gs_params *p, uint
     return GS_OK;
 }
 
-/* A batch's slots and work items a read are expected to be the last one's, or
- * those of batches before it that had more, an eighth less for each since: two
- * kinds of batches taking turns are both expected. */
+/* What a batch has a read -- slots, work items, seeds, positions -- is expected
+ * to be what the last one had, or those of batches before it that had more, an
+ * eighth less for each since: two kinds of batches taking turns are both
+ * expected. */
 static void note_sizes(gs_ctx *c, uint32_t n_reads, uint64_t slots, uint32_t items)
 {
     c->last_items = items;
     if (!n_reads) return;
-    const double s = (double)slots / n_reads, i = (double)items / n_reads;
-    const double s0 = c->slots_a_read * 0.875, i0 = c->items_a_read * 0.875;
-    c->slots_a_read = s > s0 ? s : s0;
-    c->items_a_read = i > i0 ? i : i0;
+    c->ran = true;
+    const auto note = [n_reads](double &e, uint64_t v) {
+        const double a = (double)v / n_reads, e0 = e * 0.875;
+        e = a > e0 ? a : e0;
+    };
+    note(c->a_read.slots, slots);
+    note(c->a_read.items, items);
+    note(c->a_read.seeds, c->n_seeds);
+    note(c->a_read.pos, c->n_pos);
 }
 
 /* what the end of a batched pass leaves in the queue words: the diagnostics,
@@ -701,11 +708,15 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     /* a bit for every slot there is, also where a pass before had no memory
      * for the bits of the slots it got */
     RC(grow(c->recmask, c->cap_recmask, (c->cap_slots + 31) / 32 + 1, st));
-    /* a read has a handful of seeds, a seed a position or two */
-    const uint64_t want_s = 8ull * n_reads + n_slots / 32 + 256;
-    const uint64_t want_p = 16ull * n_reads + n_slots / 16 + 1024;
-    RC(grow_outputs(c, want_s, want_p));
-    if (fetch) RC(grow_fetch(c, nr1, want_s, want_p));
+    /* what is expected, for which a context that ran has its buffers, or a
+     * handful of seeds a read and a position or two a seed */
+    const double n = (double)n_reads;
+    const uint64_t want_s = (uint64_t)(n * (c->ran ? c->a_read.seeds : 4.));
+    const uint64_t want_p = (uint64_t)(n * (c->ran ? c->a_read.pos : 8.));
+    RC(grow_outputs(c, want_s < c->cap_seeds ? want_s : want_s + 512u, want_p < c->cap_pos ? want_p : want_p + 8192u));
+    if (fetch)
+        RC(grow_fetch(c, nr1, want_s < c->cap_h_seeds ? want_s : want_s + 512u,
+                      want_p < c->cap_h_pos ? want_p : want_p + 8192u));
     memset(c->work, 0, sizeof(c->work));
     memset(c->walk_counts, 0, sizeof(c->walk_counts));
     GsBatch B;
@@ -1063,20 +1074,25 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
  * note_sizes kept, and a quarter more; where its buffers hold that, the batch
  * runs without waiting for its sizes, and again with them if it needed more.
  * Few reads may differ much and many lie near their average, so that a batch
- * is also expected to be a small one of any kind.  For up to GS_ONCE_READS
- * reads: two waits of about 10 us each are what it saves (60,007 short reads
- * 527 -> 457 us), and a batch that has to run again pays for little. */
+ * is also expected to be a small one of any kind.  Two waits of about 10 us
+ * each are what it saves.  Reads of 100 to 250 bases on 100 Mbp, so and sized:
+ * 3,000 277 and 298 us, 30,000 514 and 537, 130,000 1168 and 1189; beyond
+ * GS_ONCE_READS a batch that has to run again would pay for more.  Results
+ * that go to the host are written there by a kernel, sized by copies that
+ * overlap the locating: 10,000 417 and 450 us, 30,000 577 and 594, 60,000 805
+ * and 810, 100,000 1125 and 1110. */
 #define GS_ONCE_READS (1u << 17)
+#define GS_ONCE_FETCH_READS (1u << 16)
 #define GS_ONCE_SLOTS (1ull << 26)   /* the record mask is cleared for all of them */
 
 static int run_device(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
                       const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p, int fetch)
 {
-    if (p->kernel == GS_KERNEL_BATCHED && !p->count_work && n_reads && n_reads <= GS_ONCE_READS &&
-        c->slots_a_read > 0.) {
+    if (p->kernel == GS_KERNEL_BATCHED && !p->count_work && c->ran && n_reads &&
+        n_reads <= (fetch ? GS_ONCE_FETCH_READS : GS_ONCE_READS)) {
         const uint64_t least_s = 64ull * n_reads + 16384u, least_i = (uint64_t)n_reads + 256u;
-        uint64_t slots = (uint64_t)(1.25 * c->slots_a_read * (double)n_reads) + 1;
-        uint64_t items = (uint64_t)(1.25 * c->items_a_read * (double)n_reads) + 1;
+        uint64_t slots = (uint64_t)(1.25 * c->a_read.slots * (double)n_reads) + 1;
+        uint64_t items = (uint64_t)(1.25 * c->a_read.items * (double)n_reads) + 1;
         if ((slots < c->cap_slots || slots <= least_s) && (items < c->cap_item_read || items <= least_i) &&
             slots <= GS_ONCE_SLOTS) {
             slots = slots > least_s ? slots : least_s;
@@ -1195,11 +1211,14 @@ static int seed_chunked(gs_ctx *c, const char *seqs, const uint64_t *offsets, ui
     return GS_OK;
 }
 
-/* gs_seed batches that the host sizes: at a few nanoseconds a read and a
- * copy of the input into pinned memory, against the launches and the wait
- * that size it on the device (about 40 us) */
-#define GS_HOST_READS 8192u
-#define GS_STAGE_BYTES ((uint64_t)4 << 20)
+/* gs_seed batches that the host sizes and copies into pinned memory of the
+ * context's, a few nanoseconds a read and a byte, instead of the launches and
+ * waits that size them on the device.  Reads of 100 to 250 bases on 100 Mbp,
+ * so and not: one 87 and 106 us, 300 167 and 187, 1,000 209 and 219, 2,000 265
+ * and 262, 4,000 350 and 328, 8,000 470 and 398; a context's first call, with
+ * that pinned memory to be had, 1,000 405 and 458, 2,000 670 and 553. */
+#define GS_HOST_READS 4096u
+#define GS_STAGE_BYTES ((uint64_t)256 << 10)
 
 extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
                        const uint32_t *lengths, uint32_t n_reads, const gs_params *p)

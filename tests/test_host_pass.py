@@ -143,3 +143,21 @@ def test_timing_after_a_failed_pass(host, ask, graph):
         if rc and ask:
             assert (search, total) == want
         s.close()
+
+
+@pytest.mark.parametrize("reads", [300, 3000, 60_000])
+def test_results_take_pinned_memory_once(host, reads):
+    """A context that seeds batches of one kind from host buffers takes the
+    memory it pins in its first pass, and no more than a first guess or a
+    quarter above its results and its input."""
+    s = Seeder(host)
+    before = host.fake_pinned_bytes()
+    taken = []
+    for _ in range(4):
+        assert s.run([100] * reads, device=False) == 0
+        taken.append(host.fake_pinned_bytes() - before)
+    assert taken[0] == taken[3]
+    result = reads * (16 + 2 * 32 + 3 * 4)
+    if reads > 4096:
+        assert taken[0] < 1.3 * result
+    s.close()
