@@ -1220,13 +1220,10 @@ static int seed_chunked(gs_ctx *c, const char *seqs, const uint64_t *offsets, ui
 #define GS_HOST_READS 4096u
 #define GS_STAGE_BYTES ((uint64_t)256 << 10)
 
-extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
-                       const uint32_t *lengths, uint32_t n_reads, const gs_params *p)
+/* Seeds a batch from host memory; stage: where it lies as a stage, or NULL */
+static int seed_host(gs_ctx *c, const char *seqs, const uint64_t *offsets, const uint32_t *lengths,
+                     uint32_t n_reads, const gs_params *p, const char *stage)
 {
-    if (!c || (n_reads && (!seqs || !offsets || !lengths))) {
-        gs_set_error("gs_seed: null argument");
-        return GS_EINVAL;
-    }
     RC(check_params(p));
     GS_ON_DEVICE(gs_index_device(c->idx));
     if (n_reads && n_reads <= GS_HOST_READS && p->kernel == GS_KERNEL_BATCHED && !p->count_work) {
@@ -1244,13 +1241,16 @@ extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
             end = e > end ? e : end;
         }
         if (end <= GS_STAGE_BYTES && items <= 0xffffffffull) {
-            const size_t at_len = (size_t)n_reads * 8, at_seq = (at_len + (size_t)n_reads * 4 + 15) & ~(size_t)15;
-            RC(grow_host(c->h_stage, c->cap_stage, at_seq + end));
+            const size_t at_len = (size_t)n_reads * 8, at_seq = gs_stage_bases(n_reads);
             RC(grow(c->d_stage, c->cap_d_stage, at_seq + end + 16, c->st));
-            memcpy(c->h_stage, offsets, at_len);
-            memcpy(c->h_stage + at_len, lengths, (size_t)n_reads * 4);
-            memcpy(c->h_stage + at_seq, seqs, end);
-            GS_CUDA(cudaMemcpyAsync(c->d_stage, c->h_stage, at_seq + end, cudaMemcpyHostToDevice, c->st));
+            if (!stage) {
+                RC(grow_host(c->h_stage, c->cap_stage, at_seq + end));
+                memcpy(c->h_stage, offsets, at_len);
+                memcpy(c->h_stage + at_len, lengths, (size_t)n_reads * 4);
+                memcpy(c->h_stage + at_seq, seqs, end);
+                stage = c->h_stage;
+            }
+            GS_CUDA(cudaMemcpyAsync(c->d_stage, stage, at_seq + end, cudaMemcpyHostToDevice, c->st));
             return run_once(c, c->d_stage + at_seq, (const uint64_t *)c->d_stage,
                             (const uint32_t *)(c->d_stage + at_len), n_reads, p, 1, slots,
                             (uint32_t)items, true);
@@ -1281,6 +1281,22 @@ extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
     RC(grow(c->d_seqs, c->cap_seqs, bytes + 1, c->st));
     if (bytes) GS_CUDA(cudaMemcpyAsync(c->d_seqs, seqs, bytes, cudaMemcpyHostToDevice, c->st));
     return run_device(c, c->d_seqs, c->d_offsets, c->d_lengths, n_reads, p, 1);
+}
+
+extern "C" int gs_seed(gs_ctx *c, const char *seqs, const uint64_t *offsets,
+                       const uint32_t *lengths, uint32_t n_reads, const gs_params *p)
+{
+    if (!c || (n_reads && (!seqs || !offsets || !lengths))) {
+        gs_set_error("gs_seed: null argument");
+        return GS_EINVAL;
+    }
+    return seed_host(c, seqs, offsets, lengths, n_reads, p, NULL);
+}
+
+int gs_seed_stage(gs_ctx *c, const char *stage, uint32_t n_reads, const gs_params *p)
+{
+    return seed_host(c, stage + gs_stage_bases(n_reads), (const uint64_t *)stage,
+                     (const uint32_t *)(stage + (size_t)n_reads * 8u), n_reads, p, stage);
 }
 
 extern "C" int gs_result_host(gs_ctx *c, gs_result_view *out)

@@ -334,6 +334,12 @@ int gs_index_from_device(uint32_t primary, const uint32_t L2_1to4[4], const uint
                          uint32_t sa_intv, const uint32_t *d_samples, uint64_t n_samples, int device,
                          gs_index **out);
 
+/* A batch in one stretch of pinned memory: its offsets, its lengths and, at
+ * gs_stage_bases, its bases.  gs_seed_stage is gs_seed of such a batch, which a
+ * small one's is copied to the device from as it is. */
+static inline size_t gs_stage_bases(uint32_t n_reads) { return ((size_t)n_reads * 12u + 15u) & ~(size_t)15; }
+int gs_seed_stage(gs_ctx *c, const char *stage, uint32_t n_reads, const gs_params *p);
+
 /* kernel launchers (defined next to their kernels) */
 int gs_build_kmer_table(const GsDevIndex &idx, uint2 *table, cudaStream_t st);
 int gs_launch_text_lengths(const GsTextArgs &a, cudaStream_t st);

@@ -105,11 +105,9 @@ static void worker_main(gs_server *s, int slot)
         s->cv_done.notify_all();
         return;
     }
-    /* merged batch in pinned host memory: the H2D copy runs at link speed */
-    char *seqs = NULL;
-    uint64_t *offs = NULL;
-    uint32_t *lens = NULL;
-    size_t cap_b = 0, cap_r = 0;
+    /* merged batch in pinned host memory, as the pass copies it in */
+    char *stage = NULL;
+    size_t cap = 0;
     std::vector<Req *> batch;
     for (;;) {
         uint64_t est = 0;
@@ -156,20 +154,15 @@ static void worker_main(gs_server *s, int slot)
             nr += r->lens.size();
         }
         rc = GS_OK;
-        if (nb + 1 > cap_b) {
-            cudaFreeHost(seqs);
-            cap_b = nb + nb / 2 + 4096;
-            if (cudaMallocHost(&seqs, cap_b) != cudaSuccess) { seqs = NULL; cap_b = 0; rc = GS_ENOMEM; }
+        const size_t at_seq = gs_stage_bases((uint32_t)nr);
+        if (at_seq + nb + 1 > cap) {
+            cudaFreeHost(stage);
+            cap = at_seq + nb + (at_seq + nb) / 2 + 4096;
+            if (cudaMallocHost(&stage, cap) != cudaSuccess) { stage = NULL; cap = 0; rc = GS_ENOMEM; }
         }
-        if (nr + 1 > cap_r) {
-            cudaFreeHost(offs);
-            cudaFreeHost(lens);
-            cap_r = nr + nr / 2 + 256;
-            if (cudaMallocHost(&offs, cap_r * 8) != cudaSuccess ||
-                cudaMallocHost(&lens, cap_r * 4) != cudaSuccess) {
-                offs = NULL; lens = NULL; cap_r = 0; rc = GS_ENOMEM;
-            }
-        }
+        char *const seqs = stage + at_seq;
+        uint64_t *const offs = (uint64_t *)stage;
+        uint32_t *const lens = (uint32_t *)(stage + nr * 8);
         double t0 = now_ms();
         uint64_t wb = 0, wr = 0;
         double t_merged = 0, t_seeded = 0, t_split = 0;
@@ -185,7 +178,7 @@ static void worker_main(gs_server *s, int slot)
                 wb += r->bases;
             }
         t_merged = now_ms();
-        if (rc == GS_OK) rc = gs_seed(ctx, seqs, offs, lens, (uint32_t)nr, &s->opts.params);
+        if (rc == GS_OK) rc = gs_seed_stage(ctx, stage, (uint32_t)nr, &s->opts.params);
         t_seeded = now_ms();
         gs_result_view v;
         if (rc == GS_OK) rc = gs_result_host(ctx, &v);
@@ -231,9 +224,7 @@ static void worker_main(gs_server *s, int slot)
         s->cv_done.notify_all();
         s->cv_work.notify_all();
     }
-    cudaFreeHost(seqs);
-    cudaFreeHost(offs);
-    cudaFreeHost(lens);
+    cudaFreeHost(stage);
     gs_ctx_free(ctx);
 }
 

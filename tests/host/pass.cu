@@ -1,10 +1,12 @@
 /*
- * pass.cu -- the seeding context's host code (gs_api.cu) on the fake runtime.
+ * pass.cu -- the host code of the seeding context (gs_api.cu) and the serving
+ * loop (gs_server.cu) on the fake runtime.
  * The launchers here stand for the kernels: they count slots and work items
  * as those do, raise the overflow flag where a batch does not fit, and
  * give each read the seeds and positions that the test asks for.
  */
 #include "../../gpuseed_gb300/csrc/gs_api.cu"
+#include "../../gpuseed_gb300/csrc/gs_server.cu"
 
 #include "fake_cuda.h"
 

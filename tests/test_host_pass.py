@@ -161,3 +161,27 @@ def test_results_take_pinned_memory_once(host, reads):
     if reads > 4096:
         assert taken[0] < 1.3 * result
     s.close()
+
+
+def test_served_requests_are_pinned_once(host):
+    """A server's worker pins a merged batch's reads once, not once more for
+    the pass to take them from."""
+    import gpuseed_gb300 as gs
+    p = host.fake_pass().contents
+    p.seeds_a_read = p.pos_a_read = 0
+    opts = gs.ServerOpts(1, 0, 0, gs.Context.params(k=19, smem=True))
+    srv, rid = C.c_void_p(), C.c_uint64()
+    before = host.fake_pinned_bytes()
+    assert host.gs_server_start(C.c_void_p(host.fake_index()), C.byref(opts), C.byref(srv)) == 0
+    n, length = 1000, 200
+    lens = np.full(n, length, np.uint32)
+    offs = np.arange(n, dtype=np.uint64) * length
+    seqs = np.zeros(n * length, np.uint8)
+    a = [C.c_void_p(v.ctypes.data) for v in (seqs, offs, lens)]
+    assert host.gs_server_submit(srv, *a, n, C.byref(rid)) == 0
+    assert host.gs_server_wait(srv, rid, -1) == 0
+    host.gs_server_stop(srv)
+    # with the offsets and lengths, and half as much again for the next; the
+    # results' room: two offsets a read, and a guess at seeds and positions
+    results = 1.25 * (n * 16 + (4 * n + 512) * 32 + (8 * n + 8192) * 4)
+    assert host.fake_pinned_bytes() - before < 1.5 * n * (length + 12) + results + 16384
