@@ -60,12 +60,19 @@ struct GsDevIndex {
     int32_t text_min;
 };
 
-/* whether a walker's jl is text mode's state: an index without text mode has
- * rows up to 2^32 - 2, the marks among them (with it, gs_index_set_text keeps
- * the rows below) */
-__host__ __device__ static inline bool gs_text_mode(int32_t text_min, uint32_t jl)
+/* A kernel's part in text mode: none, where the index has none and rows go up
+ * to 2^32 - 2, the marks among them (with it, gs_index_set_text keeps the rows
+ * below); walkers that enter it are given to the text pass; or it runs here.
+ * By instance: asked of the index at every step it was 1.6 % of a pass over
+ * long reads. */
+#define GS_TEXT_NONE 0
+#define GS_TEXT_GIVEN 1
+#define GS_TEXT_RUN 2
+
+/* whether a walker's jl is text mode's state, not a row */
+__host__ __device__ static inline bool gs_text_mode(int part, uint32_t jl)
 {
-    return text_min != 0 && jl >= GS_TEXT_MARK;
+    return part != GS_TEXT_NONE && jl >= GS_TEXT_MARK;
 }
 
 /* Candidate slot written by the search kernels; y == 0 marks "no record". */

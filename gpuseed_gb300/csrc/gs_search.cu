@@ -1305,7 +1305,7 @@ struct GsAhead {
     bool alone;
 };
 
-template <int NSTOP, int COUNT, bool TEXT, bool PRE = false>
+template <int NSTOP, int COUNT, int TEXT, bool PRE = false>
 __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned char *seq, int iL,
                                              bool fwd, int dir, uint32_t &l, uint32_t &u,
                                              uint32_t &jl, uint32_t &ju, int &pos, bool &jpend,
@@ -1313,9 +1313,7 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
                                              GsWalkCounts *wc = nullptr,
                                              GsAhead *pre = nullptr)
 {
-    /* TEXT: text-mode states run here; otherwise the caller hands a walker
-     * that enters text mode to the text pass */
-    const bool text = TEXT && gs_text_mode(I.text_min, jl);
+    const bool text = TEXT == GS_TEXT_RUN && gs_text_mode(TEXT, jl);
     bool settle = false, two = false, fused = false;
     int np = pos;
     uint32_t c;
@@ -1414,7 +1412,7 @@ __device__ __forceinline__ bool gs_walk_step(const GsDevIndex &I, const unsigned
     /* one row and no J: count the steps taken so (J's words are free);
      * after text_min of them the occurrence is no chance hit, and with 16
      * bases or more left the walker enters text mode */
-    if (I.text_min && l == u && jl > ju) {
+    if (TEXT != GS_TEXT_NONE && I.text_min && l == u && jl > ju) {
         if (jl < GS_REGIME_MARK) {
             jl = GS_REGIME_MARK;
             ju = 0u;
@@ -1797,7 +1795,7 @@ __device__ __forceinline__ uint32_t gs_list_room(GsListPart &part, uint32_t *cou
     return (uint32_t)min(j, (uint64_t)cap);
 }
 
-template <int NSTOP, int COUNT>
+template <int NSTOP, int COUNT, int TEXT>
 __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_walk(GsDevIndex I, GsBatch B)
 {
     gs_after_previous();
@@ -1873,14 +1871,16 @@ __global__ void __launch_bounds__(GS_WALK_WARPS * 32, GS_WALK_CTAS) gs_search_wa
             if (exhausted) break;
             continue;
         }
-        if (have && !gs_walk_step<NSTOP, COUNT, false, true>(I, seq, iL, fwd, dir, l, u, jl, ju, pos,
+        if (have && !gs_walk_step<NSTOP, COUNT, TEXT, true>(I, seq, iL, fwd, dir, l, u, jl, ju, pos,
                                                              jpend, killed, wb, &wc, &pre)) {
             gs_write_record(B, r, n, fwd, anchor, pos, l, u, true, killed);
             have = false;
         }
         /* walkers that entered text mode go to the text pass, so that no
-         * lane of this pass runs the compare; without room they walk on */
-        const bool tx = have && gs_text_mode(I.text_min, jl);
+         * lane of this pass runs the compare; without room they walk on
+         * (gs_text_mode written out: compiled through it, a pass over long
+         * reads took 1 % more) */
+        const bool tx = TEXT != GS_TEXT_NONE && have && jl >= GS_TEXT_MARK;
         const uint32_t tm = __ballot_sync(0xffffffffu, tx);
         if (tm) {
             const uint32_t cap = (uint32_t)B.text_cap;
@@ -1942,7 +1942,7 @@ __global__ void __launch_bounds__(256) gs_search_text(GsDevIndex I, GsBatch B)
         int pos = (int)t.pos;
         uint32_t l = t.l, u = t.l, jl = GS_TEXT_MARK, ju = 0u;
         bool jpend = false, killed = false;
-        while (gs_walk_step<NSTOP, COUNT, true>(I, seq, iL, fwd, dir, l, u, jl, ju, pos, jpend,
+        while (gs_walk_step<NSTOP, COUNT, GS_TEXT_RUN>(I, seq, iL, fwd, dir, l, u, jl, ju, pos, jpend,
                                                 killed, wb)) {
         }
         gs_write_record(B, r, Lr - (uint32_t)B.k + 1u, fwd, anchor, pos, l, u, true, killed);
@@ -1958,7 +1958,7 @@ __global__ void __launch_bounds__(256) gs_search_text(GsDevIndex I, GsBatch B)
  * again with its J as the start pass would have made it; the slot gets the
  * walk's record, or loses its record bit.  Returns at once when the start
  * pass left none. */
-template <int NSTOP, int COUNT>
+template <int NSTOP, int COUNT, int TEXT>
 __global__ void __launch_bounds__(256) gs_search_leftover(GsDevIndex I, GsBatch B)
 {
     gs_after_previous();
@@ -2003,7 +2003,7 @@ __global__ void __launch_bounds__(256) gs_search_leftover(GsDevIndex I, GsBatch 
                     jpend = true;
                 }
             }
-            while (alive && gs_walk_step<NSTOP, COUNT, true>(I, seq, iL, fwd, dir, l, u, jl, ju, pos,
+            while (alive && gs_walk_step<NSTOP, COUNT, TEXT>(I, seq, iL, fwd, dir, l, u, jl, ju, pos,
                                                              jpend, killed, wb)) {
             }
             /* no record: drop the slot's bit (gs_write_record leaves it) */
@@ -2115,8 +2115,10 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
                  : (nstop ? (cnt ? gs_search_start<1, 1, false> : gs_search_start<1, 0, false>)
                           : (cnt ? gs_search_start<0, 1, false> : gs_search_start<0, 0, false>));
     void (*walk)(GsDevIndex, GsBatch) =
-        nstop ? (cnt ? gs_search_walk<1, 1> : gs_search_walk<1, 0>)
-              : (cnt ? gs_search_walk<0, 1> : gs_search_walk<0, 0>);
+        I.text_min ? (nstop ? (cnt ? gs_search_walk<1, 1, GS_TEXT_GIVEN> : gs_search_walk<1, 0, GS_TEXT_GIVEN>)
+                            : (cnt ? gs_search_walk<0, 1, GS_TEXT_GIVEN> : gs_search_walk<0, 0, GS_TEXT_GIVEN>))
+                   : (nstop ? (cnt ? gs_search_walk<1, 1, GS_TEXT_NONE> : gs_search_walk<1, 0, GS_TEXT_NONE>)
+                            : (cnt ? gs_search_walk<0, 1, GS_TEXT_NONE> : gs_search_walk<0, 0, GS_TEXT_NONE>));
     if (ctas_per_sm <= 0) ctas_per_sm = GS_START_CTAS;
     uint32_t grid = (uint32_t)sms * (uint32_t)ctas_per_sm;
     /* a captured pass knows its items only on the device: as many as the
@@ -2154,8 +2156,11 @@ static int gs_launch_batched(const GsDevIndex &I, GsBatch &B, int queue_chunk, i
         }
     }
     void (*leftover)(GsDevIndex, GsBatch) =
-        nstop ? (cnt ? gs_search_leftover<1, 1> : gs_search_leftover<1, 0>)
-              : (cnt ? gs_search_leftover<0, 1> : gs_search_leftover<0, 0>);
+        I.text_min
+            ? (nstop ? (cnt ? gs_search_leftover<1, 1, GS_TEXT_RUN> : gs_search_leftover<1, 0, GS_TEXT_RUN>)
+                     : (cnt ? gs_search_leftover<0, 1, GS_TEXT_RUN> : gs_search_leftover<0, 0, GS_TEXT_RUN>))
+            : (nstop ? (cnt ? gs_search_leftover<1, 1, GS_TEXT_NONE> : gs_search_leftover<1, 0, GS_TEXT_NONE>)
+                     : (cnt ? gs_search_leftover<0, 1, GS_TEXT_NONE> : gs_search_leftover<0, 0, GS_TEXT_NONE>));
     uint32_t lgrid = (uint32_t)sms * 8u;
     if (B.n_reads < lgrid * 8u) lgrid = B.n_reads / 8u + 1u;
     GS_CUDA(gs_launch_after(leftover, lgrid, 256, st, I, B));
