@@ -1211,13 +1211,17 @@ static int seed_chunked(gs_ctx *c, const char *seqs, const uint64_t *offsets, ui
     return GS_OK;
 }
 
-/* gs_seed batches that the host sizes and copies into pinned memory of the
- * context's, a few nanoseconds a read and a byte, instead of the launches and
- * waits that size them on the device.  Reads of 100 to 250 bases on 100 Mbp,
- * so and not: one 87 and 106 us, 300 167 and 187, 1,000 209 and 219, 2,000 265
- * and 262, 4,000 350 and 328, 8,000 470 and 398; a context's first call, with
- * that pinned memory to be had, 1,000 405 and 458, 2,000 670 and 553. */
-#define GS_HOST_READS 4096u
+/* gs_seed batches that the host sizes, a few nanoseconds a read, instead of the
+ * launches and waits that size them on the device; up to GS_STAGE_BYTES of them
+ * are copied into pinned memory of the context's, a part of a nanosecond a
+ * byte.  Reads of 100 to 250 bases on 100 Mbp, so and not: one 87 and 106 us,
+ * 300 167 and 187, 1,000 209 and 219, 2,000 265 and 262, 4,000 350 and 328,
+ * 8,000 470 and 398; a context's first call, with that pinned memory to be had,
+ * 1,000 405 and 458, 2,000 670 and 553.  Where they lie in such memory already
+ * (gs_seed_stage) any number of bytes: requests on a server of one slot, 300
+ * 173 and 220, 1,000 248 and 303, 4,000 390 and 402, 8,000 544 and 549, 12,000
+ * 660 and 645. */
+#define GS_HOST_READS 8192u
 #define GS_STAGE_BYTES ((uint64_t)256 << 10)
 
 /* Seeds a batch from host memory; stage: where it lies as a stage, or NULL */
@@ -1240,7 +1244,7 @@ static int seed_host(gs_ctx *c, const char *seqs, const uint64_t *offsets, const
             const uint64_t e = offsets[i] + lengths[i];
             end = e > end ? e : end;
         }
-        if (end <= GS_STAGE_BYTES && items <= 0xffffffffull) {
+        if ((stage || end <= GS_STAGE_BYTES) && items <= 0xffffffffull) {
             const size_t at_len = (size_t)n_reads * 8, at_seq = gs_stage_bases(n_reads);
             RC(grow(c->d_stage, c->cap_d_stage, at_seq + end + 16, c->st));
             if (!stage) {
