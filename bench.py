@@ -691,6 +691,9 @@ def main():
     achieved = canon_bytes / mean_search_s / 1e9 if canon_bytes else own_achieved
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
+                "frac_note": "of bytes that the start table, its rows' contexts and text mode "
+                             "answer without reading: no bound; traffic_frac is what moved",
+                "traffic_frac": traffic / mean_search_s / 1e9 / peak if traffic else None,
                 "peak_source": f"{peak_src} copy bandwidth (MEASURED_PEAKS.json hbm_gbs)",
                 "kernel": "gs_search_start + gs_search_walk + gs_search_text + gs_search_leftover (one search pass)",
                 "algorithmic_bytes_per_launch": canon_bytes if canon_bytes else own_bytes,

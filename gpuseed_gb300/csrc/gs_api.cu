@@ -616,11 +616,11 @@ static int size_walkers(gs_ctx *c, const GsDevIndex &I, const gs_params *p, uint
 /* What a batch has a read -- slots, work items, seeds, positions -- is expected
  * to be what the last one had, or those of batches before it that had more, an
  * eighth less for each since: two kinds of batches taking turns are both
- * expected. */
-static void note_sizes(gs_ctx *c, uint32_t n_reads, uint64_t slots, uint32_t items)
+ * expected.  (Other kernels' work items are others.) */
+static void note_sizes(gs_ctx *c, int kernel, uint32_t n_reads, uint64_t slots, uint32_t items)
 {
     c->last_items = items;
-    if (!n_reads) return;
+    if (!n_reads || kernel != GS_KERNEL_BATCHED) return;
     c->ran = true;
     const auto note = [n_reads](double &e, uint64_t v) {
         const double a = (double)v / n_reads, e0 = e * 0.875;
@@ -764,7 +764,7 @@ static int run_once(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets, co
     }
     timed(c, GS_TIMING_PASS);
     if (read_queue(c, p) & GS_FLAG_WALK) return walk_limit_error();
-    note_sizes(c, n_reads, c->h_small[GS_H_TOTALS], (uint32_t)c->h_small[GS_H_TOTALS + 1]);
+    note_sizes(c, p->kernel, n_reads, c->h_small[GS_H_TOTALS], (uint32_t)c->h_small[GS_H_TOTALS + 1]);
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;
@@ -915,7 +915,7 @@ static int run_pipeline(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets
     if (B.work) memcpy(c->walk_counts, &c->h_small[16], sizeof(c->walk_counts));
     timed(c, GS_TIMING_PASS);
     if (flags & GS_FLAG_WALK) return walk_limit_error();
-    note_sizes(c, n_reads, n_slots, n_items);
+    note_sizes(c, p->kernel, n_reads, n_slots, n_items);
     c->have_dev = 1;
     c->have_host = fetch;
     return GS_OK;
@@ -1071,8 +1071,9 @@ static int run_graph(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
 
 /* A pass over device-resident reads whose sizes the host does not know.  A
  * context that has run before expects as many slots and work items a read as
- * note_sizes kept, and a quarter more; where its buffers hold that, the batch
- * runs without waiting for its sizes, and again with them if it needed more.
+ * note_sizes kept, and a quarter more; unless that is more than twice the room
+ * it has, the batch runs without waiting for its sizes, and again with them if
+ * it needed more.
  * Few reads may differ much and many lie near their average, so that a batch
  * is also expected to be a small one of any kind.  Two waits of about 10 us
  * each are what it saves.  Reads of 100 to 250 bases on 100 Mbp, so and sized:
@@ -1093,8 +1094,8 @@ static int run_device(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
         const uint64_t least_s = 64ull * n_reads + 16384u, least_i = (uint64_t)n_reads + 256u;
         uint64_t slots = (uint64_t)(1.25 * c->a_read.slots * (double)n_reads) + 1;
         uint64_t items = (uint64_t)(1.25 * c->a_read.items * (double)n_reads) + 1;
-        if ((slots < c->cap_slots || slots <= least_s) && (items < c->cap_item_read || items <= least_i) &&
-            slots <= GS_ONCE_SLOTS) {
+        if ((slots <= 2 * c->cap_slots || slots <= least_s) &&
+            (items <= 2 * c->cap_item_read || items <= least_i) && slots <= GS_ONCE_SLOTS) {
             slots = slots > least_s ? slots : least_s;
             items = items > least_i ? items : least_i;
             const int rc = run_once(c, d_seqs, d_offsets, d_lengths, n_reads, p, fetch, slots,

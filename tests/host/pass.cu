@@ -124,7 +124,10 @@ int fake_replayed_when_larger(gs_ctx *c, int which)
 FakePass *fake_pass(void) { return &pass; }
 gs_index *fake_index(void)
 {
+    static const uint4 start_table = {0, 0, 0, 0};   /* there is one; nothing reads it */
     the_index.dev.seq_len = 1000000;
+    the_index.dev.kmerx = &start_table;
+    the_index.dev.kx = 13;
     return &the_index;
 }
 }

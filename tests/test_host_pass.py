@@ -119,6 +119,22 @@ def test_alike_batches_run_once(seeder):
             assert i < 2 or seeder.last.clear_words, "in one go"
 
 
+@pytest.mark.parametrize("device", [True, False])
+@pytest.mark.parametrize("before", [[(10_000, 2)], [(10_000, 1)], [(9000, 0)], [(9000, 0), (10_000, 2), (10_000, 0)]])
+def test_other_batches_do_not_keep_one_from_running_once(host, device, before):
+    """After passes (reads, kernel) of a smaller batch, whose room holds this
+    one, and of the other kernels, which count work items otherwise."""
+    s = Seeder(host)
+    for n, kernel in before:
+        assert s.run([100] * n, kernel=kernel) == 0
+    for i in range(3):
+        passes = s.last.passes
+        assert s.run([100] * 10_000, device=device) == 0
+        assert s.last.passes == passes + 1
+        assert i < 1 or s.last.clear_words, "in one go"
+    s.close()
+
+
 def _timing(s):
     t = C.c_float(), C.c_float()
     assert s.L.gs_ctx_last_timing(s.h, C.byref(t[0]), C.byref(t[1])) == 0
