@@ -7,12 +7,16 @@
  * calls instead of ~15 cudaMalloc/cudaFree per batch (:3029-3102,
  * :3750-3770):
  *
- *   prepare  -> slot / work-item counts per read, exclusive scans
+ *   prepare  -> slot / work-item counts and offsets per read, and the read
+ *               of each work item
  *   search   -> one record slot per candidate (gs_search.cu)
  *   count    -> per-read compaction + filter counts (gs_post.cu)
- *   scan     -> seed / position offsets
- *   emit     -> output seeds in output order
+ *   emit     -> seed / position offsets, output seeds in output order
  *   locate   -> positions by the sampled-SA walk
+ *
+ * A pass is sized on the way (run_pipeline: two waits for totals), by what is
+ * known or expected beforehand (run_once: none but the last), or is replayed
+ * as it was captured (run_graph).
  */
 #include "gs_internal.h"
 
@@ -503,8 +507,7 @@ static int check_params(const gs_params *p)
         if (_rc) return _rc;     \
     } while (0)
 
-/* the arguments of a pass that its sizes do not change; zero: the prepare
- * kernels clear the queue and the first `mask_words` words of the record mask */
+/* the arguments of a pass that its sizes do not change */
 static void batch_of(gs_ctx *c, const char *d_seqs, const uint64_t *d_offsets,
                      const uint32_t *d_lengths, uint32_t n_reads, const gs_params *p, GsBatch &B)
 {
@@ -592,7 +595,9 @@ static int size_walkers(gs_ctx *c, const GsDevIndex &I, const gs_params *p, uint
     if (!p->walker_slots && c->walker_per16 > per16) per16 = c->walker_per16;
     const uint64_t units = (uint64_t)n_items * (B.paired ? 2u : 1u);
     uint64_t want = (units * per16 + 15u) / 16u + 32u;
-    /* a start-pass warp reserves 64 entries or more at a time */
+    /* a start-pass warp's last reservation, of 32 entries or all of an item's
+     * up to 60 walkers where the buffer is small (gs_walker_chunk), may stay
+     * unused but for one */
     if (!p->walker_slots) want += 64ull * (n_items < 8192u ? n_items : 8192u);
     if (want > (1ull << 31)) want = 1ull << 31;   /* 32-bit buffer counter */
     RC(grow(c->walkers, c->cap_walkers, (size_t)want, c->st));

@@ -13,15 +13,14 @@
  * Results are the reference's integers (seed_gen.cu:195-216 occ, :329-368
  * occ pair, :455-484 LF).
  *
- * Before, a block of 32 bytes held 64 rows of the $-removed string as four
- * counts and bit-sliced bases.  A query took two loads and about 30
- * instructions, and the walk pass, which executes them without end, issued
- * on two thirds of its slots.  The wider block costs HBM (3.1 GB at 3.1 Gbp
- * instead of 1.55) and L2 reach, not loads: either form is one 64-byte fill
- * a bound, and bounds 64 to 127 rows apart no longer share one.
- * Measured (whole pass, the walk in brackets): 2 M reads on 3.1 Gbp 16.3 ->
- * 15.5 ms (9.5 -> 8.7, its DRAM reads 16.0 -> 18.3 GB), 1 M reads on 100
- * Mbp 7.7 -> 7.3 ms (4.1 -> 3.6), 40,000 long reads 7.1 -> 6.9 ms.
+ * The walk pass executes such queries without end and is bound by fills and by
+ * instructions, so a bound is one load of one 64-byte fill.  Against 32 bytes
+ * for 64 rows, four counts and bit-sliced bases, also one fill but two loads
+ * and about 30 instructions, this form takes twice the HBM (3.1 GB at 3.1 Gbp)
+ * and reaches half as far in L2, and a whole pass (the walk in brackets) takes,
+ * with steps of one base, 15.5 ms instead of 16.3 for 2 M reads on 3.1 Gbp (8.7
+ * of 9.5), 7.3 instead of 7.7 for 1 M on 100 Mbp (3.6 of 4.1), 6.9 instead of
+ * 7.1 for 40,000 long reads.
  */
 #ifndef GS_FM_CUH
 #define GS_FM_CUH

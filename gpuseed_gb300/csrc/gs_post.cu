@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(128) gs_mem_next_kernel(GsBatch B)
  * next, so that a warp does not wait for the longest chain of each 32 (1 M
  * reads on 100 Mbp, 2.3 M positions 246 -> 208 us; 150,001 reads 166 -> 131).
  * A tile of one round has nothing to hand out: each lane runs its own chain
- * (10,000 reads on 5 Mbp 38 us, 47 through shared memory). */
+ * (10,000 reads on 1 Mbp 35 us, 47 through shared memory). */
 #define GS_LOCATE_MOST 256u
 
 /* the row of position p (in the round from pb), and its seed */

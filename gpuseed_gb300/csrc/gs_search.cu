@@ -213,16 +213,14 @@ __global__ void __launch_bounds__(256, 8) gs_kmerx_code_kernel(GsDevIndex I, con
  * A candidate whose extension by the bases its read has next does not occur
  * can reach no minimum length past it, and one whose extension is a single
  * row that its neighbour's string shares is contained there: both end at
- * their start, without a walk.  The walk pass was bound by the walks'
- * dependent block loads, most of them of strings that a chance hit kept
- * alive for a base or two: with the extensions, and with the item's bases
- * loaded by the warp and its read found in a map instead of a search, a
- * 2 M-read SMEM pass on 3.1 Gbp takes 16.6 ms instead of 24.2, a 40,000-read
- * (2 kbp) MEM pass 7.2 instead of 10.4, a 1 M-read pass on 100 Mbp 7.9
- * instead of 10.5.  With the few rows' contexts a start plays its walk out
- * over up to six bases, its neighbour's with it, and a quarter (3.1 Gbp) to
- * half (100 Mbp) of the walkers that were left end there: walk passes of the
- * same three 8.45 -> 7.28, 3.33 -> 2.89 and 3.45 -> 2.70 ms.
+ * their start, without a walk.  A walk is a chain of dependent loads, and most
+ * are of strings that a chance hit keeps alive for a base or two.  What the
+ * forms are worth: the extensions (with the item's bases loaded by the warp,
+ * and its read from a map) 7.6 of 24.2 ms of a 2 M-read SMEM pass on 3.1 Gbp,
+ * 3.2 of 10.4 of a 40,000-read (2 kbp) MEM pass, 2.6 of 10.5 of a 1 M-read pass
+ * on 100 Mbp; the few rows' contexts, by which a start plays its walk out over
+ * up to six bases, its neighbour's with it, a quarter (3.1 Gbp) to half (100
+ * Mbp) of the walkers that are left, 1.17, 0.44 and 0.75 ms of the same three.
  * 255 rows is what the size's byte holds. */
 #define GS_EXT_ROWS 255u
 #define GS_ENTRY_EXT 8u
